@@ -110,7 +110,37 @@ struct BlockList {
   // kernels leave the blocks of a finished problem alone.  Null otherwise.
   const int *comp = nullptr;
   const FState *stc = nullptr;
+  // a list reduced to its active blocks (MacGpu::build_active): the entries
+  // are [*pa, *pb) of the arrays above (n stays the full list's length), and
+  // orig[entry] is the entry's place in the full list, by which sa and ia
+  // are laid out.  Null: the list is blocks[0 .. n).
+  const int *pa = nullptr, *pb = nullptr;
+  const int *orig = nullptr;
 };
+
+// one list and the arrays of its reduced form (mac_active.cu)
+struct ActiveList {
+  const int *blocks;
+  const uint16_t *ftypes;
+  const int *hx, *links;
+  int nlinks, n;
+  int *ablocks;
+  uint16_t *aftypes;
+  int *ahx, *alinks;
+  int *pre, *orig;
+};
+
+// entries [first, second) of a list
+struct ListRange {
+  int a, b;
+};
+__device__ __forceinline__ ListRange list_range(const BlockList &L) {
+  return L.pa ? ListRange{*L.pa, *L.pb} : ListRange{0, L.n};
+}
+// number of entries of a list that starts at its arrays' first entry
+__device__ __forceinline__ int list_count(const BlockList &L) { return L.pb ? *L.pb : L.n; }
+// place of entry p in the factor arrays sa and ia
+__device__ __forceinline__ long factor_entry(const BlockList &L, int p) { return L.orig ? L.orig[p] : p; }
 
 // chunks of a block list listed problem by problem (one BiCGSTAB state per
 // problem): the BiCGSTAB kernels run one CTA per chunk of at most kChunkCells

@@ -369,7 +369,7 @@ template <typename T, bool MULTI>
 __global__ void k_pupdate(BlockList L, int ncell, Chunks ch, FState *stb, const double *r, double *p, const double *v,
                           const double *vf, T *resid) {
   pdl_enter();
-  const Work wk = work_of<MULTI>(ch, stb, L.n * ncell, nullptr);
+  const Work wk = work_of<MULTI>(ch, stb, list_count(L) * ncell, nullptr);
   const FState *st = wk.st;
   if (st->done) return;
   const bool first = st->iter == 1 || st->restart;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kTPB) k_supdate(BlockList L, int ncell, Chunks
                                                 const double *v, double *s, double *x, const TP *phat,
                                                 const double *vf, T *resid, double *partials, unsigned *counter) {
   pdl_enter();
-  const Work wk = work_of<MULTI>(ch, stb, L.n * ncell, counter);
+  const Work wk = work_of<MULTI>(ch, stb, list_count(L) * ncell, counter);
   FState *st = wk.st;
   if (st->done) return;
   const double a = st->alpha;
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kTPB) k_rupdate(BlockList L, int ncell, Chunks
                                                 const T *shat, double *r, const double *s, const double *t,
                                                 const double *rhat, double *partials, unsigned *counter) {
   pdl_enter();
-  const Work wk = work_of<MULTI>(ch, stb, L.n * ncell, counter);
+  const Work wk = work_of<MULTI>(ch, stb, list_count(L) * ncell, counter);
   FState *st = wk.st;
   if (st->done) return;
   const double om = st->omega;
@@ -440,7 +440,7 @@ template <bool MULTI>
 __global__ void k_finish(BlockList L, int ncell, Chunks ch, const FState *stb, double *x0, const double *x,
                          double *sol) {
   pdl_enter();
-  const Work wk = work_of<MULTI>(ch, const_cast<FState *>(stb), L.n * ncell, nullptr);
+  const Work wk = work_of<MULTI>(ch, const_cast<FState *>(stb), list_count(L) * ncell, nullptr);
   if (!wk.st->conv) return;
   for (int it = wk.it0; it < wk.it1; it += wk.step) {
     const long q = cell_of(L, ncell, it);
@@ -455,7 +455,7 @@ template <typename T>
 __global__ void k_vc_out(BlockList L, int ncell, const FState *st, const T *corr, double *out) {
   pdl_enter();
   if (st->done) return;
-  const int total = L.n * ncell;
+  const int total = list_count(L) * ncell;
   for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < total; it += gridDim.x * blockDim.x) {
     const int p = it / ncell;
     if (block_off(L, L.blocks[p])) continue;
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(kTPB) k_op_red(Topo t, Coef<double> c, BlockLi
   pdl_enter();
   // DFOP: modes 0 and 1 of an FP32 input in double-float
   constexpr bool DF = DFOP && sizeof(TX) == 4 && MODE < 2;
-  const Work wk = work_of<MULTI>(ch, stb, L.n * t.ncell, counter);
+  const Work wk = work_of<MULTI>(ch, stb, list_count(L) * t.ncell, counter);
   FState *st = wk.st;
   if (MODE == 3 && !st->verify) return;
   if (MODE < 2 && st->done) return;
@@ -774,7 +774,7 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kTPB) k_verify_fold(BlockList L, int ncell, Chunks ch, const FState *stb,
                                                     double *x0, double *x) {
   pdl_enter();
-  const Work wk = work_of<MULTI>(ch, const_cast<FState *>(stb), L.n * ncell, nullptr);
+  const Work wk = work_of<MULTI>(ch, const_cast<FState *>(stb), list_count(L) * ncell, nullptr);
   if (!wk.st->verify) return;
   for (int it = wk.it0; it < wk.it1; it += wk.step) {
     const long q = cell_of(L, ncell, it);
@@ -987,7 +987,9 @@ void MacGpu::tune_smoother(int precision) {
     return;
   }
   if (rbgs_variant_[pi] >= 0 && rbgs_us_[pi][0] > 0) return;
+  solve_lists_ = true;  // the list the solve will walk
   const BlockList sl = sublevel_list(finest_, finest_);
+  solve_lists_ = false;
   if (sl.n == 0) {
     rbgs_variant_[pi] = 2;
     return;
@@ -1750,6 +1752,7 @@ void MacGpu::capture_loop(int precision) {
   graph_pform_ = prm_.prolong_form;
   graph_vout_ = prm_.vcycle_out;
   graph_omega_ = prm_.relax_omega;
+  graph_act_ = (int)act_on_;
 }
 
 // the captured graph was recorded with other parameters than the current ones
@@ -1760,7 +1763,7 @@ bool MacGpu::graph_stale() const {
          graph_order_ != prm_.sublevel_order || graph_smoother_ != prm_.smoother ||
          graph_inner_ != prm_.inner_sweeps || graph_multi_ != (int)multi() || graph_uniform_ != prm_.uniform ||
          graph_pform_ != prm_.prolong_form || graph_vout_ != prm_.vcycle_out ||
-         graph_omega_ != prm_.relax_omega;
+         graph_omega_ != prm_.relax_omega || graph_act_ != (int)act_on_;
 }
 
 int MacGpu::cg_solve_device(SolveInfo *info) {
@@ -1809,6 +1812,7 @@ int MacGpu::enqueue_solve() {
     for (int c = 0; c < ncomp_; c++) h_stc_[c] = init;
     CKR_(cudaMemcpyAsync(d_stc_, h_stc_, ncomp_ * sizeof(FState), cudaMemcpyHostToDevice, stream_), -1);
   }
+  if (act_on_) zero_solid();
   // prologue: x0 = sol, x = 0, r = rhs - A x0, rhat = r, |r0|, rho
   k_pro_copy<<<ew_grid(w), kTPB, 0, stream_>>>(TL, ncell_, vec_[kSOL], vec_[kX0], vec_[kX]);
   double *PART = mp ? d_cpart_ : d_part_;
@@ -1900,6 +1904,7 @@ int MacGpu::prepare_device() {
     if (!err_.empty()) return -1;
   }
   bind_uniform();
+  choose_active();
   // the FP64 smoother factors serve the FP64 V-cycle and the learned
   // correction only: an FP32 solve does not build them
   if (prm_.precision == 0 || learned_active()) ensure_smooth_factors();

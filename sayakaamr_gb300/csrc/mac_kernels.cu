@@ -26,6 +26,11 @@ namespace sayaka_gb300 {
 namespace {
 
 constexpr int kThreads = 256;
+// CTAs over a reduced list (BlockList::pb), whose length the host does not
+// know: about two rounds of resident CTAs, which walk it in strides, instead
+// of one CTA per entry of the full list, most of which would only read the
+// bounds and leave
+constexpr int kReducedGrid = 152 * 16;
 using namespace stencil;
 
 // ---------------------------------------------------------------------------
@@ -83,8 +88,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs(Topo t, Coef<T> c, Bloc
   if (h >= (t.ncell >> 1)) return;
   int ijk[3];
   color_cell_fast<ND>(h, t, color, ijk);
-  for (int p = blockIdx.y; p < L.n; p += gridDim.y) {
-    const long fo = (long)p * t.ncell;
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.y; p < lr.b; p += gridDim.y) {
+    const long fo = factor_entry(L, p) * t.ncell;
     if (L.stc && block_off(L, L.hx ? L.hx[(long)p * kHX + kHXBlock] : L.blocks[p])) continue;
     if (L.hx) {
       const int *e = L.hx + (long)p * kHX;
@@ -112,15 +118,16 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_ilp(Topo t, Coef<T> c, 
   int ijk[3];
   color_cell_fast<ND>(h, t, color, ijk);
   const int G = gridDim.y;
-  for (int p0 = blockIdx.y; p0 < L.n; p0 += CPT * G) {
+  const ListRange lr = list_range(L);
+  for (int p0 = lr.a + blockIdx.y; p0 < lr.b; p0 += CPT * G) {
     SmoothOps<T, ND> o[CPT];
     bool on[CPT];
 #pragma unroll
     for (int k = 0; k < CPT; k++) {
       const int p = p0 + k * G;
       on[k] = false;
-      if (p >= L.n) continue;
-      const long fo = (long)p * t.ncell;
+      if (p >= lr.b) continue;
+      const long fo = factor_entry(L, p) * t.ncell;
       const int *e = L.hx ? L.hx + (long)p * kHX : nullptr;
       const int b = e ? e[kHXBlock] : L.blocks[p];
       if (L.stc && block_off(L, b)) continue;
@@ -264,10 +271,12 @@ __global__ void __launch_bounds__(kThreads, MINB) k_prolong_red_warp16(Topo t, C
   pdl_enter();
   if (guard && *guard) return;
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  for (int p = blockIdx.x * warps + (threadIdx.x >> 5); p < L.n + X.n; p += gridDim.x * warps) {
-    const bool top = p < L.n;
+  const ListRange lr = list_range(L), xr = list_range(X);
+  const int nl = lr.b - lr.a, nx = xr.b - xr.a;
+  for (int p = blockIdx.x * warps + (threadIdx.x >> 5); p < nl + nx; p += gridDim.x * warps) {
+    const bool top = p < nl;
     const BlockList &Q = top ? L : X;
-    const int q = top ? p : p - L.n;
+    const int q = top ? lr.a + p : xr.a + p - nl;
     const int *e = Q.hx ? Q.hx + (long)q * kHX : nullptr;
     const int b = e ? e[kHXBlock] : Q.blocks[q];
     if (Q.stc && block_off(Q, b)) continue;  // uniform over the warp
@@ -301,7 +310,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_warp16(Topo t, Coef<flo
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh;
-  for (int p = blockIdx.x * warps + (threadIdx.x >> 5); p < L.n; p += gridDim.x * warps) {
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.x * warps + (threadIdx.x >> 5); p < lr.b; p += gridDim.x * warps) {
     const int *e = L.hx ? L.hx + (long)p * kHX : nullptr;
     const int b = e ? e[kHXBlock] : L.blocks[p];
     if (L.stc && block_off(L, b)) continue;  // uniform over the warp
@@ -436,7 +446,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_warp16_flat(Topo t, Coe
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh;
-  for (int p = blockIdx.x * warps + (threadIdx.x >> 5); p < L.n; p += gridDim.x * warps) {
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.x * warps + (threadIdx.x >> 5); p < lr.b; p += gridDim.x * warps) {
     const int *e = L.hx + (long)p * kHX;
     const int4 nb4 = *reinterpret_cast<const int4 *>(e);           // face neighbours 0..3
     const int2 ib = *reinterpret_cast<const int2 *>(e + kHXInfo);  // info, block
@@ -535,7 +546,7 @@ __global__ void __launch_bounds__(kThreads) k_restrict(Topo t, Coef<T> c, BlockL
   pdl_enter();
   if (guard && *guard) return;
   const int ncell = t.ncell;
-  const long total = (long)L.n * ncell;
+  const long total = (long)list_count(L) * ncell;
   for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
     const int p = (int)(it / ncell);
     if (block_off(L, L.blocks[p])) continue;
@@ -550,7 +561,7 @@ __global__ void __launch_bounds__(kThreads) k_prolong(Topo t, Coef<T> c, BlockLi
   pdl_enter();
   if (guard && *guard) return;
   const int ncell = t.ncell;
-  const long total = (long)L.n * ncell;
+  const long total = (long)list_count(L) * ncell;
   for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
     const int p = (int)(it / ncell);
     if (block_off(L, L.blocks[p])) continue;
@@ -763,7 +774,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_tile(Topo t, Coef<T> c,
   T *hc = tile + ncell;
   T *hk = hc + 2 * ND * nface;
   T *hv = hk + 2 * ND * nface;
-  for (int p = blockIdx.x; p < L.n; p += gridDim.x) {
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.x; p < lr.b; p += gridDim.x) {
     const int *hxe = L.hx ? L.hx + (long)p * kHX : nullptr;
     const int b = hxe ? hxe[kHXBlock] : L.blocks[p];
     if (block_off(L, b)) continue;  // uniform over the CTA
@@ -853,7 +865,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_tile(Topo t, Coef<T> c,
           o.sa = u[6];
           o.ia = u[7];
         } else {
-          const long fo = (long)p * ncell + o.ci;
+          const long fo = factor_entry(L, p) * ncell + o.ci;
           o.sa = L.sa[fo];
           o.ia = L.ia[fo];
         }
@@ -933,7 +945,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bhgs(Topo t, Coef<T> c, Bloc
   T *tile = reinterpret_cast<T *>(bhgs_smem);
   T *hc = tile + ncell;            // diagonal part of every boundary face of the block
   T *ho = hc + 2 * ND * nface;     // its off-diagonal part (frozen neighbour values)
-  for (int p = blockIdx.x; p < L.n; p += gridDim.x) {
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.x; p < lr.b; p += gridDim.x) {
     const int *hxe = L.hx ? L.hx + (long)p * kHX : nullptr;
     const int b = hxe ? hxe[kHXBlock] : L.blocks[p];
     if (block_off(L, b)) continue;  // uniform over the CTA
@@ -1019,7 +1032,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bhgs(Topo t, Coef<T> c, Bloc
             bool inner = true;
 #pragma unroll
             for (int q = 0; q < ND; q++) inner = inner && ijk[q] > 0 && ijk[q] < nb - 1;
-            const long fo = (long)p * ncell + ci;
+            const long fo = factor_entry(L, p) * ncell + ci;
             const bool ui = u && inner;
             const T iav = ui ? u[7] : (T)L.ia[fo];  // 0 in a solid cell
             unew = fma_t(rhs[cb + ci], ui ? u[6] : (T)L.sa[fo], off * iav);
@@ -1050,7 +1063,7 @@ __global__ void __launch_bounds__(kThreads) k_copy_blocks(BlockList L, int ncell
                                                           T *__restrict__ dst, const int *guard) {
   pdl_enter();
   if (guard && *guard) return;
-  const long total = (long)L.n * ncell;
+  const long total = (long)list_count(L) * ncell;
   for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
     const int p = (int)(it / ncell);
     if (block_off(L, L.blocks[p])) continue;
@@ -1457,12 +1470,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
   T *hc = tile + ncell;
   T *hk = hc + 2 * ND * nface;
   T *hv = hk + 2 * ND * nface;
-  for (int p = blockIdx.x; p < L.n + X.n; p += gridDim.x) {
-    if (p >= L.n) {
+  const ListRange lr = list_range(L), xr = list_range(X);
+  const int nl = lr.b - lr.a, nx = xr.b - xr.a;
+  for (int p = blockIdx.x; p < nl + nx; p += gridDim.x) {
+    if (p >= nl) {
       // the red sweep of a block of X: blocks two or more levels coarser,
       // which neither read nor are read by the level being prolonged
-      const int px = p - L.n;
-      const long fo = (long)px * ncell;
+      const int px = xr.a + p - nl;
+      const long fo = factor_entry(X, px) * ncell;
       const int *e = X.hx + (long)px * kHX;
       if (block_off(X, e[kHXBlock])) continue;
       for (int h = threadIdx.x; h < nhalf; h += blockDim.x) {
@@ -1473,10 +1488,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
       }
       continue;
     }
-    const int *hxe = L.hx ? L.hx + (long)p * kHX : nullptr;
-    const int b = hxe ? hxe[kHXBlock] : L.blocks[p];
+    const int pl = lr.a + p;
+    const int *hxe = L.hx ? L.hx + (long)pl * kHX : nullptr;
+    const int b = hxe ? hxe[kHXBlock] : L.blocks[pl];
     if (block_off(L, b)) continue;  // uniform over the CTA
-    const uint16_t ft = hxe ? (uint16_t)(hxe[kHXInfo] & 0xffff) : L.ftypes[p];
+    const uint16_t ft = hxe ? (uint16_t)(hxe[kHXInfo] & 0xffff) : L.ftypes[pl];
     const long cb = (long)b * ncell;
     const long fb = (long)b * t.nfb;
     const T *u = uniform_of(c, b);  // constant coefficients: no face or vf loads
@@ -1560,7 +1576,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
         bool inner = true;
 #pragma unroll
         for (int q = 0; q < ND; q++) inner = inner && ijk[q] > 0 && ijk[q] < nb - 1;
-        const long fo = (long)p * ncell + ci;
+        const long fo = factor_entry(L, pl) * ncell + ci;
         const bool ui = u && inner;
         const T iav = ui ? u[7] : (T)L.ia[fo];  // 0 in a solid cell
         unew = fma_t(rhs[cb + ci], ui ? u[6] : (T)L.sa[fo], off * iav);
@@ -1593,7 +1609,7 @@ void launch_prolong_red(const Topo &t, const Coef<T> &c, const BlockList &L, T *
   const size_t smem = sizeof(T) * ((size_t)t.ncell + 3 * 2 * t.ndim * (size_t)nface);
   ensure_max_smem(t.ndim == 2 ? (const void *)k_prolong_red<T, 2> : (const void *)k_prolong_red<T, 3>, 200 * 1024);
   const int threads = std::min(kThreads, ((t.ncell >> 1) + 31) / 32 * 32);
-  const int grid = std::min(L.n + X.n, 152 * 64);
+  const int grid = std::min(L.n + X.n, L.pb ? kReducedGrid : 152 * 64);
   if (t.ndim == 2)
     launch_k(pdl, k_prolong_red<T, 2>, grid, threads, smem, s, t, c, L, phi, rhs, guard, X);
   else
@@ -1612,7 +1628,7 @@ static void rbgs_tile_go(const Topo &t, const Coef<T> &c, const BlockList &L, in
   const size_t smem = rbgs_tile_smem<T, ND>(t);
   ensure_max_smem((const void *)k_rbgs_tile<T, ND, MINB>, 200 * 1024);
   const int threads = std::min(kThreads, ((t.ncell >> 1) + 31) / 32 * 32);
-  const int grid = std::min(L.n, 152 * 64);
+  const int grid = std::min(L.n, L.pb ? kReducedGrid : 152 * 64);
   launch_k(pdl, k_rbgs_tile<T, ND, MINB>, grid, threads, smem, s, t, c, L, color, phi, rhs, guard);
 }
 
@@ -1633,7 +1649,7 @@ static void rbgs_go(const Topo &t, const Coef<T> &c, const BlockList &L, int col
 template <typename T, int ND, int MINB, int CPT>
 static void rbgs_ilp_go(const Topo &t, const Coef<T> &c, const BlockList &L, int color, T *phi, const T *rhs,
                         const int *guard, cudaStream_t s, bool pdl, dim3 grid, int threads) {
-  grid.y = std::min((L.n + CPT - 1) / CPT, 65535);
+  grid.y = std::min((L.n + CPT - 1) / CPT, L.pb ? kReducedGrid : 65535);
   launch_k(pdl, k_rbgs_ilp<T, ND, MINB, CPT>, grid, threads, 0, s, t, c, L, color, phi, rhs, guard);
 }
 
@@ -1686,7 +1702,8 @@ void launch_rbgs(const Topo &t, const Coef<T> &c, const BlockList &L, int color,
   const size_t tile = t.ndim == 2 ? rbgs_tile_smem<T, 2>(t) : rbgs_tile_smem<T, 3>(t);
   if (variant >= 5 && variant <= 9 && tile > 200 * 1024) variant = 3;
   const bool aligned = (t.ncell * sizeof(T)) % 16 == 0 && (t.nfb * sizeof(T)) % 16 == 0;
-  if (L.stc && (variant == 8 || variant == 9)) variant = 7;  // the bulk-copy variants know no per-problem states
+  // the bulk-copy variants know no per-problem states and no reduced lists
+  if ((L.stc || L.pb) && (variant == 8 || variant == 9)) variant = 7;
   if (variant == 8) {
     const size_t bulk = t.ndim == 2 ? rbgs_bulk_smem<T, 2>(t) : rbgs_bulk_smem<T, 3>(t);
     if (bulk > 200 * 1024 || !aligned) variant = 7;
@@ -1696,7 +1713,7 @@ void launch_rbgs(const Topo &t, const Coef<T> &c, const BlockList &L, int color,
     if (st > 227 * 1024 || !aligned) variant = 7;
   }
   const int threads = std::min(kThreads, (nhalf + 31) / 32 * 32);
-  const dim3 grid((nhalf + threads - 1) / threads, std::min(L.n, 65535));
+  const dim3 grid((nhalf + threads - 1) / threads, std::min(L.n, L.pb ? kReducedGrid : 65535));
   if (t.ndim == 2)
     rbgs_nd<T, 2>(variant, t, c, L, color, phi, rhs, guard, s, pdl, grid, threads);
   else
@@ -1711,7 +1728,7 @@ void launch_bhgs(const Topo &t, const Coef<T> &c, const BlockList &L, int nsweep
   const int nface = t.ndim == 3 ? t.nb * t.nb : t.nb;
   const size_t smem = sizeof(T) * ((size_t)t.ncell + 2 * 2 * t.ndim * (size_t)nface);
   const int threads = std::min(kThreads, (nhalf + 31) / 32 * 32);
-  const int grid = std::min(L.n, 152 * 64);
+  const int grid = std::min(L.n, L.pb ? kReducedGrid : 152 * 64);
   if (t.ndim == 2) {
     ensure_max_smem((const void *)k_bhgs<T, 2, 2>, 200 * 1024);
     launch_k(pdl, k_bhgs<T, 2, 2>, grid, threads, smem, s, t, c, L, nsweep, src, dst, rhs, guard);

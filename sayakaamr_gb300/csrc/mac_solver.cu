@@ -572,6 +572,7 @@ MacGpu::~MacGpu() {
   fr(d_corr32_);
   fr(d_corr32b_);
   fr(d_corr64b_);
+  fr(d_active_mem_);
   fr(tlc_.blocks);
   fr(tlc_.ftypes);
   fr(tlc_.hx);
@@ -612,7 +613,7 @@ BlockList MacGpu::tower_list(int L) const {
   const DevTower &t = towers_[L];
   BlockList r{t.all.blocks, t.all.ftypes, t.all.n};
   r.hx = t.all.hx;
-  return attach(r);
+  return attach(active(r, t.all, 0, t.all.n));
 }
 // lists built while a solve is recorded carry the per-problem states
 BlockList MacGpu::attach(BlockList r) const {
@@ -629,10 +630,11 @@ BlockList MacGpu::sublevel_list(int L, int l) const {
   r.hx = t.all.hx + (long)b * kHX;
   if (L < (int)d_sfac_.size() && d_sfac_[L]) {
     const long w = (long)t.all.n * ncell_;
-    r.sa = d_sfac_[L] + (long)b * ncell_;
-    r.ia = d_sfac_[L] + w + (long)b * ncell_;
+    const long o = solve_lists_ && act_on_ ? 0 : (long)b * ncell_;  // reduced: by the entry's full place
+    r.sa = d_sfac_[L] + o;
+    r.ia = d_sfac_[L] + w + o;
   }
-  return attach(r);
+  return attach(active(r, t.all, b, e));
 }
 BlockList MacGpu::smooth_list(int L) const {
   BlockList r = tower_list(L);
@@ -650,20 +652,21 @@ BlockList MacGpu::parity_list(int L, int g, bool skip_top) const {
   r.hx = t.par.hx + (long)b * kHX;
   if (L < (int)d_pfac_.size() && d_pfac_[L]) {
     const long w = (long)t.par.n * ncell_;
-    r.sa = d_pfac_[L] + (long)b * ncell_;
-    r.ia = d_pfac_[L] + w + (long)b * ncell_;
+    const long o = solve_lists_ && act_on_ ? 0 : (long)b * ncell_;
+    r.sa = d_pfac_[L] + o;
+    r.ia = d_pfac_[L] + w + o;
   }
-  return attach(r);
+  return attach(active(r, t.par, b, e));
 }
 BlockList MacGpu::level_list(int l) const {
   BlockList r{levels_[l].blocks, nullptr, levels_[l].n};
   r.links = levels_[l].links;
-  return attach(r);
+  return attach(active(r, levels_[l], 0, levels_[l].n));
 }
 BlockList MacGpu::nonleaf_list(int l) const {
   BlockList r{nonleaf_[l].blocks, nullptr, nonleaf_[l].n};
   r.links = nonleaf_[l].links;
-  return attach(r);
+  return attach(active(r, nonleaf_[l], 0, nonleaf_[l].n));
 }
 
 // ---------------------------------------------------------------------------

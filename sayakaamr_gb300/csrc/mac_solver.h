@@ -202,6 +202,12 @@ class MacGpu {
     int *hx = nullptr;     // halo descriptors (tower lists)
     int *links = nullptr;  // parents (level lists) or children (non-leaf lists)
     int n = 0;
+    // the list without its solid blocks (see mac_active.cu)
+    struct {
+      int *blocks = nullptr;
+      uint16_t *ftypes = nullptr;
+      int *hx = nullptr, *links = nullptr, *pre = nullptr, *orig = nullptr;
+    } act;
   };
   struct DevTower {
     DevList all;
@@ -362,6 +368,17 @@ class MacGpu {
   bool solve_lists_ = false;  // block lists carry the states (set while a solve is recorded)
   bool multi() const { return ncomp_ > 1 && prm_.per_problem != 0 && d_stc_ != nullptr; }
   BlockList attach(BlockList r) const;
+  // blocks that hold fluid, and the lists reduced to them (mac_active.cu)
+  void build_active();
+  void choose_active();
+  void zero_solid();
+  BlockList active(BlockList r, const DevList &d, int a, int b) const;
+  char *d_active_mem_ = nullptr;       // the allocation behind these
+  int *d_active_ = nullptr;            // per block: holds fluid
+  ActiveList *d_act_lists_ = nullptr;  // every list and its reduced form
+  int n_act_lists_ = 0, n_act_ = 0;    // active blocks of the finest tower
+  long act_version_ = -1;              // coefficient version of the reduced lists
+  bool act_on_ = false;                // the solve walks the reduced lists
   Coef<float> c32_{};
   FState *d_st_ = nullptr, *h_st_ = nullptr;
   double *d_part_ = nullptr;
@@ -409,7 +426,7 @@ class MacGpu {
   int kernels_per_iter_ = 0;
   int graph_coop_ = -1, graph_pdl_ = -1, graph_cc_ = -1, graph_var_ = -1, graph_nn_ = -1, graph_order_ = -1;
   int graph_smoother_ = -1, graph_inner_ = -1, graph_multi_ = -1, graph_uniform_ = -1, graph_pform_ = -1,
-      graph_vout_ = -1;
+      graph_vout_ = -1, graph_act_ = -1;
   double graph_omega_ = -1.0;
   bool last_multi_ = false;  // the last device solve kept one state per problem
   Chunks chunks() const;
