@@ -154,386 +154,222 @@ __device__ __forceinline__ T prolonged_value(const Topo &t, const Coef<T> &c, in
   return (fluid || c.vf[q] > 0) ? phi[(long)P * t.ncell + encode(pc, nb)] : (T)0;
 }
 
-// One warp updates the cells of colour `color` of one 16x16 block of a 2D
-// FP32 sweep, any block: lane l holds row l/2, columns 8(l%2) .. +7 in
-// registers, v[] (PROLONG: the block's values prolonged from its parent,
-// masked by vf, as k_prolong_red's tile; else phi), neighbours inside the
-// block from registers and shuffles, every boundary face by its type as
-// smooth_cell_fast and k_prolong_red take it (same-level: the neighbour's
-// value, prolonged from its own parent when PROLONG; coarse/fine: the
-// coarse ghost or the fine-side sum; physical: the diagonal term), face
-// coefficients from the block record or the face arrays; the whole block is
-// written back.  Per cell the operations are those of smooth_cell_fast /
-// k_prolong_red in the same order: the same bits.
+// ---- 2D FP32 blocks of 16x16 cells, one warp per block --------------------
+// Lane l holds the cells of row l/2, columns 8(l%2) .. 8(l%2)+7, in registers.
+// What crosses the block's boundary is gathered first, one boundary face cell
+// per lane, into 64 slots of the warp's shared memory (slot 16 f + m: face f,
+// m-th cell along it): the face's part of the diagonal, its off-diagonal
+// factor and the value behind it, by face type as smooth_cell_fast takes them
+// (same-level: T, T and the neighbour's cell; physical: 0 or 2T, 0 and 0;
+// FINE_CRSE: T/1.5 twice and the coarse cell; CRSE_FINE: T/0.75, 1 and the
+// sum over the fine faces).  Blocks with a body's surface, a density front
+// or a coarse/fine face then take the same few instructions per cell as the
+// others; cell by cell (smooth_cell_fast) they took about five times as many,
+// and they are the greater part of a tree's finest level, which is refined
+// where they lie.  Bound by the latency of the loads (descriptor, then
+// record, rows, halo and coefficients at once) and by issue, not by bytes.
+constexpr int kW16Slots = 64;
+struct W16Halo {
+  float dp[kW16Slots], k[kW16Slots], v[kW16Slots];
+};
+
+// slot of face f, m-th face cell: its contribution to the cell of the block
+// behind it (PROLONG: a same-level neighbour's value prolonged from that
+// neighbour's parent).  The gathers of mac_stencil.cuh for 2D blocks of 16,
+// without their arrays: the direction differs from lane to lane, and arrays
+// indexed by it would live in local memory.
+struct W16Dir {  // the coefficient arrays of a lane's direction
+  const float *tff, *bc, *af;
+};
+__device__ __forceinline__ float w16_cf_coef(const Coef<float> &c, const W16Dir &a, int d, long fx, int b, float h) {
+  float v = c.beta * geom(c, b, 3 + d) / (geom(c, b, d) * h);
+  v = v * a.bc[fx];
+  v = v * a.af[fx];
+  return v;
+}
 template <bool PROLONG>
-__device__ __forceinline__ void warp_block16(const Topo &t, const Coef<float> &c, int b, uint16_t ft, const int *e,
-                                             int color, float *__restrict__ phi, const float *__restrict__ rhs,
-                                             int lane) {
+__device__ __forceinline__ void w16_halo_slot(const Topo &t, const Coef<float> &c, const int *e, int b, int info,
+                                              const float *u, int f, int m, const float *__restrict__ phi, float &dp,
+                                              float &k, float &v) {
   constexpr int NB = 16, NC = 256;
-  const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh;
+  const int d = f >> 1, s = f & 1;
+  const int ty = face_type_of((uint16_t)(info & 0xffff), f);
+  const W16Dir a = d ? W16Dir{c.tff[1], c.bcoef[1], c.afrac[1]} : W16Dir{c.tff[0], c.bcoef[0], c.afrac[0]};
+  const long fx = (long)b * t.nfb + (d ? m + NB * (s * NB) : s * NB + (NB + 1) * m);
+  const int across = s ? 0 : NB - 1;  // the neighbour's cell layer at the face
+  dp = k = v = 0.f;
+  if (ty == 0) {
+    const long n = e[f];
+    dp = k = u ? u[d] : a.tff[fx];
+    if constexpr (PROLONG) {
+      const int pw = e[kHXPar + f], wc = pw & 7;
+      const int i = d ? m : across, j = d ? across : m;
+      const bool fluid = c.vf[n * NC + i + NB * j] > 0;
+      const float pv = phi[(long)(pw >> 3) * NC + 8 * (wc & 1) + (i >> 1) + NB * (8 * ((wc >> 1) & 1) + (j >> 1))];
+      v = fluid ? pv : 0.f;
+    } else {
+      v = phi[n * NC + (d ? m + NB * across : across + NB * m)];
+    }
+  } else if (ty == 1) {
+    if (t.bc_type[b * 6 + f] != kBCNeumann) dp = (u ? u[d] : a.tff[fx]) * 2.0f;
+  } else if (ty == 2) {
+    const int tc = 8 * ((info >> (17 - d)) & 1) + (m >> 1);  // which_child >> (1 - d)
+    dp = k = w16_cf_coef(c, a, d, fx, b, 1.5f);
+    v = phi[(long)e[f] * NC + (d ? tc + NB * across : across + NB * tc)];
+  } else {
+    const int half = m >> 3, F = e[kHXKids + 4 * f + half], t0 = 2 * (m - 8 * half);
+    const int fl = across + 1 - s;  // the fine block's face layer toward b
+    dp = w16_cf_coef(c, a, d, fx, b, 0.75f);
+    k = 1.f;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const float tf =
+          w16_cf_coef(c, a, d, (long)F * t.nfb + (d ? t0 + q + NB * fl : fl + (NB + 1) * (t0 + q)), F, 1.5f);
+      v += tf * phi[(long)F * NC + (d ? t0 + q + NB * across : across + NB * (t0 + q))];
+    }
+  }
+}
+
+// the cells of colour `color` of list entry e (its halo descriptor): the
+// values and operations of smooth_cell_fast (PROLONG: of k_prolong_red) in
+// the same order, so the same bits.  A row's cells of the colour are the
+// columns 2q + par, q < 4; they stay in cc, the others in oc.
+template <bool PROLONG>
+__device__ __forceinline__ void w16_sweep(const Topo &t, const Coef<float> &c, const BlockList &L, const int *e,
+                                          int color, float *__restrict__ phi, const float *__restrict__ rhs, int lane,
+                                          W16Halo &sh) {
+  constexpr int NB = 16, NC = 256;
+  const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh, par = (color + j) & 1;
+  const int2 ib = *reinterpret_cast<const int2 *>(e + kHXInfo);
+  const int b = ib.y;
   const long cb = (long)b * NC, fb = (long)b * t.nfb;
   const float *u = uniform_of(c, b);
-  float v[8];
+  const float dv = geom(c, b, 6);
+  float cc[4], oc[4];
   if constexpr (PROLONG) {
-    const int pw = e ? e[kHXPar + 6] : t.parent[b] * 8 + t.which_child[b];
-    const int P = pw >> 3, wc = pw & 7;
+    // columns 2q and 2q+1 of the row have the same parent cell
+    const int pw = e[kHXPar + 6], P = pw >> 3, wc = pw & 7;
     const float4 q4 = *reinterpret_cast<const float4 *>(phi + (long)P * NC + (8 * ((wc >> 1) & 1) + (j >> 1)) * NB +
                                                          8 * (wc & 1) + 4 * hh);
-    const float pv[4] = {q4.x, q4.y, q4.z, q4.w};
-#pragma unroll
-    for (int k = 0; k < 8; k++) v[k] = (u || c.vf[cb + j * NB + c0 + k] > 0) ? pv[k >> 1] : 0.f;
+    cc[0] = oc[0] = q4.x, cc[1] = oc[1] = q4.y, cc[2] = oc[2] = q4.z, cc[3] = oc[3] = q4.w;
   } else {
     const float4 *src = reinterpret_cast<const float4 *>(phi + cb + j * NB + c0);
     const float4 p0 = src[0], p1 = src[1];
-    v[0] = p0.x, v[1] = p0.y, v[2] = p0.z, v[3] = p0.w, v[4] = p1.x, v[5] = p1.y, v[6] = p1.z, v[7] = p1.w;
+    cc[0] = par ? p0.y : p0.x, cc[1] = par ? p0.w : p0.z, cc[2] = par ? p1.y : p1.x, cc[3] = par ? p1.w : p1.z;
+    oc[0] = par ? p0.x : p0.y, oc[1] = par ? p0.z : p0.w, oc[2] = par ? p1.x : p1.y, oc[3] = par ? p1.z : p1.w;
   }
   const float4 *rsrc = reinterpret_cast<const float4 *>(rhs + cb + j * NB + c0);
   const float4 r0 = rsrc[0], r1 = rsrc[1];
-  const float r[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-  const float dv = geom(c, b, 6);
-  const float from_left = __shfl_up_sync(0xffffffffu, v[7], 1);
-  const float from_right = __shfl_down_sync(0xffffffffu, v[0], 1);
-  const int par = (color + j) & 1;
-  // value across boundary face f of cell ijk (same-level, coarse/fine)
-  auto across = [&](int f, const int ijk[3], int ty) -> float {
-    if (ty == 0) {
-      const int n = e ? e[f] : t.neighbor[b * 6 + f];
-      int ni[3] = {ijk[0], ijk[1], 0};
-      ni[f >> 1] = (f & 1) ? 0 : NB - 1;
-      if constexpr (PROLONG)
-        return prolonged_value<float, 2>(t, c, n, ni, phi, e ? e[kHXPar + f] : -1);
-      else
-        return phi[(long)n * NC + ni[0] + NB * ni[1]];
-    }
-    return fine_crse_ghost<float, 2, false>(t, b, f, ijk, phi, e);
-  };
+  const float r[4] = {par ? r0.y : r0.x, par ? r0.w : r0.z, par ? r1.y : r1.x, par ? r1.w : r1.z};
+  // the boundary face cells of the colour: eight per face, one per lane
+  const int hf = lane >> 3, hm = 2 * (lane & 7) + ((color + (hf & 1)) & 1);
+  float hdp, hk, hv;
+  w16_halo_slot<PROLONG>(t, c, e, b, ib.x, u, hf, hm, phi, hdp, hk, hv);
+  // face coefficients and volume fractions of the colour's cells
+  float tx[8], ty0[4], ty1[4], vf[4];
+  if (u) {
+    const float T0 = u[0], T1 = u[1];
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const float dnk = __shfl_up_sync(0xffffffffu, v[k], 2);
-    const float upk = __shfl_down_sync(0xffffffffu, v[k], 2);
-    if ((k & 1) != par) continue;
-    const int i = c0 + k;
-    const int ijk[3] = {i, j, 0};
-    float diag = c.alpha * dv;
-    float off = 0.f;
+    for (int q = 0; q < 4; q++) tx[2 * q] = tx[2 * q + 1] = T0, ty0[q] = ty1[q] = T1, vf[q] = 1.f;
+  } else {
+    const float *x = c.tff[0] + fb + (NB + 1) * j + c0 + par;
 #pragma unroll
-    for (int f = 0; f < 4; f++) {
-      const int d = f >> 1, sd = f & 1;
-      const bool bnd = d == 0 ? (sd ? i == NB - 1 : i == 0) : (sd ? j == NB - 1 : j == 0);
-      const int fx = d == 0 ? i + sd + (NB + 1) * j : i + NB * (j + sd);
-      if (!bnd) {
-        const float coef = u ? u[d] : c.tff[d][fb + fx];
-        float nbv;
-        if (f == 0)
-          nbv = k > 0 ? v[k - 1] : from_left;
-        else if (f == 1)
-          nbv = k < 7 ? v[k + 1] : from_right;
-        else if (f == 2)
-          nbv = dnk;
-        else
-          nbv = upk;
-        diag += coef;
-        off = fma_t(coef, nbv, off);
-        continue;
-      }
-      const int ty = face_type_of(ft, f);
-      if (ty == 0) {
-        const float coef = u ? u[d] : c.tff[d][fb + fx];
-        diag += coef;
-        off = fma_t(coef, across(f, ijk, 0), off);
-      } else if (ty == 1) {
-        if (t.bc_type[b * 6 + f] != kBCNeumann) diag += (u ? u[d] : c.tff[d][fb + fx]) * 2.0f;
-      } else if (ty == 2) {
-        const float coef = cf_coef(c, t, b, d, fx, 1.5f);
-        diag += coef;
-        off = fma_t(coef, across(f, ijk, 2), off);
-      } else {
-        diag += cf_coef(c, t, b, d, fx, 0.75f);
-        off = fma_t(1.0f, crse_fine_sum<float, 2, false>(t, c, b, f, ijk, phi, e), off);
+    for (int n = 0; n < 8; n++) tx[n] = x[n];
+    const float *y = c.tff[1] + fb + NB * j + c0 + par;
+    const float *w = c.vf + cb + NB * j + c0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) ty0[q] = y[2 * q], ty1[q] = y[2 * q + NB];
+    const float4 w0 = *reinterpret_cast<const float4 *>(w), w1 = *reinterpret_cast<const float4 *>(w + 4);
+    vf[0] = par ? w0.y : w0.x, vf[1] = par ? w0.w : w0.z, vf[2] = par ? w1.y : w1.x, vf[3] = par ? w1.w : w1.z;
+    if constexpr (PROLONG) {
+      const float ov[4] = {par ? w0.x : w0.y, par ? w0.z : w0.w, par ? w1.x : w1.y, par ? w1.z : w1.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (!(vf[q] > 0.f)) cc[q] = 0.f;
+        if (!(ov[q] > 0.f)) oc[q] = 0.f;
       }
     }
-    const float vfv = u ? 1.0f : c.vf[cb + j * NB + i];
-    v[k] = (vfv > 0.f && diag > 0.f) ? relax(c.omega, fast_div(fma_t(r[k] * dv, vfv, off), diag), v[k]) : 0.f;
   }
+  if (L.stc && block_off(L, b)) return;  // a finished problem; uniform over the warp
+  __syncwarp();                          // the slots of the warp's previous block have been read
+  sh.dp[16 * hf + hm] = hdp;
+  sh.k[16 * hf + hm] = hk;
+  sh.v[16 * hf + hm] = hv;
+  __syncwarp();
+  // the neighbours of a cell have the other colour: rows j-1 and j+1 hold
+  // them in oc of lanes l-2 and l+2, the row's own are oc[q-1], oc[q] (par 0)
+  // or oc[q], oc[q+1] (par 1), the outermost from the other half of the row
+  const float fl = __shfl_up_sync(0xffffffffu, oc[3], 1), fr = __shfl_down_sync(0xffffffffu, oc[0], 1);
+  float dn[4], up[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    dn[q] = __shfl_up_sync(0xffffffffu, oc[q], 2);
+    up[q] = __shfl_down_sync(0xffffffffu, oc[q], 2);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    float kl = tx[2 * q], kr = tx[2 * q + 1], kd = ty0[q], ku = ty1[q];
+    float dl = kl, dr = kr, dd = kd, du = ku;
+    float vl = par ? oc[q] : (q > 0 ? oc[q > 0 ? q - 1 : 0] : fl);
+    float vr = par ? (q < 3 ? oc[q < 3 ? q + 1 : 3] : fr) : oc[q];
+    float vd = dn[q], vu = up[q];
+    const int i = c0 + 2 * q + par;
+    if (q == 0 && i == 0) dl = sh.dp[j], kl = sh.k[j], vl = sh.v[j];
+    if (q == 3 && i == NB - 1) dr = sh.dp[16 + j], kr = sh.k[16 + j], vr = sh.v[16 + j];
+    if (j == 0) dd = sh.dp[32 + i], kd = sh.k[32 + i], vd = sh.v[32 + i];
+    if (j == NB - 1) du = sh.dp[48 + i], ku = sh.k[48 + i], vu = sh.v[48 + i];
+    float diag = c.alpha * dv, off = 0.f;
+    diag += dl;
+    off = fma_t(kl, vl, off);
+    diag += dr;
+    off = fma_t(kr, vr, off);
+    diag += dd;
+    off = fma_t(kd, vd, off);
+    diag += du;
+    off = fma_t(ku, vu, off);
+    cc[q] = (vf[q] > 0.f && diag > 0.f) ? relax(c.omega, fast_div(fma_t(r[q] * dv, vf[q], off), diag), cc[q]) : 0.f;
+  }
+  // the block is written back whole, the other colour's cells with the values
+  // that concurrent readers see in any case
   float4 *dst = reinterpret_cast<float4 *>(phi + cb + j * NB + c0);
-  dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-  dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+  dst[0] = par ? make_float4(oc[0], cc[0], oc[1], cc[1]) : make_float4(cc[0], oc[0], cc[1], oc[1]);
+  dst[1] = par ? make_float4(oc[2], cc[2], oc[3], cc[3]) : make_float4(cc[2], oc[2], cc[3], oc[3]);
 }
 
 // prolongation of a level fused with its first red sweep (k_prolong_red's
-// values), 2D FP32 16x16 blocks, one warp per block of L, then one warp per
-// block of X for the red sweep of the coarser same-parity sublevels
+// values), one warp per block of L, then one warp per block of X for the red
+// sweep of the coarser same-parity sublevels
 template <int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) k_prolong_red_warp16(Topo t, Coef<float> c, BlockList L,
                                                                        float *__restrict__ phi,
                                                                        const float *__restrict__ rhs,
                                                                        const int *guard, BlockList X) {
+  __shared__ W16Halo sh[kThreads / 32];
   pdl_enter();
   if (guard && *guard) return;
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const ListRange lr = list_range(L), xr = list_range(X);
   const int nl = lr.b - lr.a, nx = xr.b - xr.a;
   for (int p = blockIdx.x * warps + (threadIdx.x >> 5); p < nl + nx; p += gridDim.x * warps) {
-    const bool top = p < nl;
-    const BlockList &Q = top ? L : X;
-    const int q = top ? lr.a + p : xr.a + p - nl;
-    const int *e = Q.hx ? Q.hx + (long)q * kHX : nullptr;
-    const int b = e ? e[kHXBlock] : Q.blocks[q];
-    if (Q.stc && block_off(Q, b)) continue;  // uniform over the warp
-    const uint16_t ft = e ? (uint16_t)(e[kHXInfo] & 0xffff) : Q.ftypes[q];
-    if (top)
-      warp_block16<true>(t, c, b, ft, e, 0, phi, rhs, lane);
+    if (p < nl)
+      w16_sweep<true>(t, c, L, L.hx + (long)(lr.a + p) * kHX, 0, phi, rhs, lane, sh[threadIdx.x >> 5]);
     else
-      warp_block16<false>(t, c, b, ft, e, 0, phi, rhs, lane);
+      w16_sweep<false>(t, c, X, X.hx + (long)(xr.a + p - nl) * kHX, 0, phi, rhs, lane, sh[threadIdx.x >> 5]);
   }
 }
 
-// The 2D sweep of 16x16 blocks with one warp per block: lane l holds row
-// l/2, columns 8(l%2) .. 8(l%2)+7 of phi and rhs in registers (two 16-byte
-// loads each), neighbours inside the block come from the lane's own
-// registers and from lanes l-1, l+1 (columns) and l-2, l+2 (rows) by
-// shuffles, and the block is written back whole (the cells of the other
-// colour with their unchanged values) with two 16-byte stores per lane.  The
-// fast path takes constant-coefficient blocks (a block record) whose faces
-// are all same-level or physical; their halo cells are loaded from the
-// neighbour block (one value per lane for the side faces, two 16-byte loads
-// for the bottom and top rows).  Any other block is swept cell by cell with
-// smooth_cell_fast.  Per cell the arithmetic is smooth_cell_fast's, face by
-// face in the same order, so every path gives the same bits.
+// one colour of a red-black sweep, one warp per block
 template <int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_warp16(Topo t, Coef<float> c, BlockList L, int color,
                                                                 float *__restrict__ phi, const float *__restrict__ rhs,
                                                                 const int *guard) {
+  __shared__ W16Halo sh[kThreads / 32];
   pdl_enter();
   if (guard && *guard) return;
-  constexpr int NB = 16, NC = 256;
-  const int lane = threadIdx.x & 31;
-  const int warps = blockDim.x >> 5;
-  const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const ListRange lr = list_range(L);
-  for (int p = lr.a + blockIdx.x * warps + (threadIdx.x >> 5); p < lr.b; p += gridDim.x * warps) {
-    const int *e = L.hx ? L.hx + (long)p * kHX : nullptr;
-    const int b = e ? e[kHXBlock] : L.blocks[p];
-    if (L.stc && block_off(L, b)) continue;  // uniform over the warp
-    const uint16_t ft = e ? (uint16_t)(e[kHXInfo] & 0xffff) : L.ftypes[p];
-    const float *u = uniform_of(c, b);
-    bool fast = u != nullptr;
-#pragma unroll
-    for (int f = 0; f < 4; f++) fast = fast && face_type_of(ft, f) <= 1;
-    if (!fast) {
-      // four cells of the colour per lane, as k_rbgs does them (measured
-      // faster for these blocks than warp_block16's register form)
-      for (int k = 0; k < 4; k++) {
-        const int h = lane * 4 + k;  // half-cell index 0..127
-        int ijk[3];
-        color_cell_fast<2>(h, t, color, ijk);
-        smooth_cell_fast<float, 2>(t, c, b, ft, ijk, phi, rhs, nullptr, nullptr, e);
-      }
-      continue;
-    }
-    const long cb = (long)b * NC;
-    const float4 *src = reinterpret_cast<const float4 *>(phi + cb + j * NB + c0);
-    const float4 *rsrc = reinterpret_cast<const float4 *>(rhs + cb + j * NB + c0);
-    const float4 p0 = src[0], p1 = src[1], r0 = rsrc[0], r1 = rsrc[1];
-    float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-    const float r[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-    const int ty[4] = {face_type_of(ft, 0), face_type_of(ft, 1), face_type_of(ft, 2), face_type_of(ft, 3)};
-    // halo values (same-level faces only; physical faces have no off-diagonal term)
-    float hl = 0.f, hr = 0.f;
-    if (hh == 0 && ty[0] == 0) {
-      const int n = e ? e[0] : t.neighbor[b * 6 + 0];
-      hl = phi[(long)n * NC + j * NB + (NB - 1)];
-    }
-    if (hh == 1 && ty[1] == 0) {
-      const int n = e ? e[1] : t.neighbor[b * 6 + 1];
-      hr = phi[(long)n * NC + j * NB];
-    }
-    float hv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if ((j == 0 && ty[2] == 0) || (j == NB - 1 && ty[3] == 0)) {
-      const int f = j == 0 ? 2 : 3;
-      const int n = e ? e[f] : t.neighbor[b * 6 + f];
-      const int row = j == 0 ? NB - 1 : 0;
-      const float4 *hs = reinterpret_cast<const float4 *>(phi + (long)n * NC + row * NB + c0);
-      const float4 a0 = hs[0], a1 = hs[1];
-      hv[0] = a0.x, hv[1] = a0.y, hv[2] = a0.z, hv[3] = a0.w, hv[4] = a1.x, hv[5] = a1.y, hv[6] = a1.z, hv[7] = a1.w;
-    }
-    const float dv = geom(c, b, 6);
-    const float T0 = u[0], T1 = u[1];
-    const bool dir[4] = {t.bc_type[b * 6 + 0] != kBCNeumann, t.bc_type[b * 6 + 1] != kBCNeumann,
-                         t.bc_type[b * 6 + 2] != kBCNeumann, t.bc_type[b * 6 + 3] != kBCNeumann};
-    // neighbours across lanes: v[7] of the left half, v[0] of the right half
-    const float from_left = __shfl_up_sync(0xffffffffu, v[7], 1);
-    const float from_right = __shfl_down_sync(0xffffffffu, v[0], 1);
-    const int par = (color + j) & 1;  // column parity of this row's cells of the colour
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      // rows j-1 and j+1 from lanes l-2 and l+2; their column-k cell has the
-      // other colour (their row parity differs), so it is still the old value
-      // even after those lanes updated their own cells in place
-      const float dnk = __shfl_up_sync(0xffffffffu, v[k], 2);
-      const float upk = __shfl_down_sync(0xffffffffu, v[k], 2);
-      if ((k & 1) != par) continue;
-      const int i = c0 + k;
-      float diag = c.alpha * dv;
-      float off = 0.f;
-      // f = 0: left
-      if (i > 0 || ty[0] == 0) {
-        const float nbv = k > 0 ? v[k - 1] : (hh == 1 ? from_left : hl);
-        diag += T0;
-        off = fma_t(T0, nbv, off);
-      } else if (dir[0]) {
-        diag += T0 * 2.0f;
-      }
-      // f = 1: right
-      if (i < NB - 1 || ty[1] == 0) {
-        const float nbv = k < 7 ? v[k + 1] : (hh == 0 ? from_right : hr);
-        diag += T0;
-        off = fma_t(T0, nbv, off);
-      } else if (dir[1]) {
-        diag += T0 * 2.0f;
-      }
-      // f = 2: down
-      if (j > 0 || ty[2] == 0) {
-        const float nbv = j > 0 ? dnk : hv[k];
-        diag += T1;
-        off = fma_t(T1, nbv, off);
-      } else if (dir[2]) {
-        diag += T1 * 2.0f;
-      }
-      // f = 3: up
-      if (j < NB - 1 || ty[3] == 0) {
-        const float nbv = j < NB - 1 ? upk : hv[k];
-        diag += T1;
-        off = fma_t(T1, nbv, off);
-      } else if (dir[3]) {
-        diag += T1 * 2.0f;
-      }
-      v[k] = diag > 0.f ? relax(c.omega, fast_div(fma_t(r[k] * dv, 1.0f, off), diag), v[k]) : 0.f;
-    }
-    float4 *dst = reinterpret_cast<float4 *>(phi + cb + j * NB + c0);
-    dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-    dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-  }
-}
-
-// the cell-by-cell sweep of one block (four cells of the colour per lane)
-__device__ __forceinline__ void warp16_slow_block(const Topo &t, const Coef<float> &c, int b, uint16_t ft, int color,
-                                               float *__restrict__ phi, const float *__restrict__ rhs, const int *e,
-                                               int lane) {
-  for (int k = 0; k < 4; k++) {
-    const int h = lane * 4 + k;
-    int ijk[3];
-    color_cell_fast<2>(h, t, color, ijk);
-    smooth_cell_fast<float, 2>(t, c, b, ft, ijk, phi, rhs, nullptr, nullptr, e);
-  }
-}
-
-// k_rbgs_warp16 with every load of a block issued before its first branch:
-// the descriptor (two vector loads), then at once the block record, dv, the
-// face BC types, phi and rhs and the halo values (their ids and face types
-// come with the descriptor), and only then the problem's done flag, the
-// fast-path test and the sweep.  The latency of a block is then about three
-// dependent loads (descriptor, data, done flag) instead of six.  Same
-// arithmetic, same bits.  Needs the list's halo descriptors.
-template <int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_rbgs_warp16_flat(Topo t, Coef<float> c, BlockList L, int color,
-                                                                     float *__restrict__ phi,
-                                                                     const float *__restrict__ rhs,
-                                                                     const int *guard) {
-  pdl_enter();
-  if (guard && *guard) return;
-  constexpr int NB = 16, NC = 256;
-  const int lane = threadIdx.x & 31;
-  const int warps = blockDim.x >> 5;
-  const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh;
-  const ListRange lr = list_range(L);
-  for (int p = lr.a + blockIdx.x * warps + (threadIdx.x >> 5); p < lr.b; p += gridDim.x * warps) {
-    const int *e = L.hx + (long)p * kHX;
-    const int4 nb4 = *reinterpret_cast<const int4 *>(e);           // face neighbours 0..3
-    const int2 ib = *reinterpret_cast<const int2 *>(e + kHXInfo);  // info, block
-    const int b = ib.y;
-    const uint16_t ft = (uint16_t)(ib.x & 0xffff);
-    const int ty[4] = {face_type_of(ft, 0), face_type_of(ft, 1), face_type_of(ft, 2), face_type_of(ft, 3)};
-    const long cb = (long)b * NC;
-    // ---- every load of the block
-    const int comp = L.stc ? L.comp[b] : 0;
-    const float4 rec = c.ut ? *reinterpret_cast<const float4 *>(c.ut + (long)b * kUni) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float dv = geom(c, b, 6);
-    const int2 bc01 = *reinterpret_cast<const int2 *>(t.bc_type + b * 6);
-    const int2 bc23 = *reinterpret_cast<const int2 *>(t.bc_type + b * 6 + 2);
-    const int par = (color + j) & 1;  // column parity of this row's cells of the colour
-    const float4 *src = reinterpret_cast<const float4 *>(phi + cb + j * NB + c0);
-    const float4 *rsrc = reinterpret_cast<const float4 *>(rhs + cb + j * NB + c0);
-    const float4 p0 = src[0], p1 = src[1], r0 = rsrc[0], r1 = rsrc[1];
-    float hl = 0.f, hr = 0.f;
-    if (hh == 0 && ty[0] == 0) hl = phi[(long)nb4.x * NC + j * NB + (NB - 1)];
-    if (hh == 1 && ty[1] == 0) hr = phi[(long)nb4.y * NC + j * NB];
-    float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-    if ((j == 0 && ty[2] == 0) || (j == NB - 1 && ty[3] == 0)) {
-      const int n = j == 0 ? nb4.z : nb4.w;
-      const float4 *hs = reinterpret_cast<const float4 *>(phi + (long)n * NC + (j == 0 ? NB - 1 : 0) * NB + c0);
-      a0 = hs[0];
-      a1 = hs[1];
-    }
-    // ---- then the decisions
-    if (L.stc && L.stc[comp].done) continue;  // uniform over the warp
-    bool fast = c.ut != nullptr && __float_as_uint(rec.w) != 0u;
-#pragma unroll
-    for (int f = 0; f < 4; f++) fast = fast && ty[f] <= 1;
-    if (!fast) {
-      warp16_slow_block(t, c, b, ft, color, phi, rhs, e, lane);
-      continue;
-    }
-    float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-    // rhs and the halo row of the colour's four cells only (cell k = 2q + par)
-    const float rs[4] = {par ? r0.y : r0.x, par ? r0.w : r0.z, par ? r1.y : r1.x, par ? r1.w : r1.z};
-    const float hs4[4] = {par ? a0.y : a0.x, par ? a0.w : a0.z, par ? a1.y : a1.x, par ? a1.w : a1.z};
-    const float T0 = rec.x, T1 = rec.y;
-    const bool dir[4] = {bc01.x != kBCNeumann, bc01.y != kBCNeumann, bc23.x != kBCNeumann, bc23.y != kBCNeumann};
-    const float from_left = __shfl_up_sync(0xffffffffu, v[7], 1);
-    const float from_right = __shfl_down_sync(0xffffffffu, v[0], 1);
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const float dnk = __shfl_up_sync(0xffffffffu, v[k], 2);
-      const float upk = __shfl_down_sync(0xffffffffu, v[k], 2);
-      if ((k & 1) != par) continue;
-      const int i = c0 + k;
-      float diag = c.alpha * dv;
-      float off = 0.f;
-      if (i > 0 || ty[0] == 0) {
-        const float nbv = k > 0 ? v[k - 1] : (hh == 1 ? from_left : hl);
-        diag += T0;
-        off = fma_t(T0, nbv, off);
-      } else if (dir[0]) {
-        diag += T0 * 2.0f;
-      }
-      if (i < NB - 1 || ty[1] == 0) {
-        const float nbv = k < 7 ? v[k + 1] : (hh == 0 ? from_right : hr);
-        diag += T0;
-        off = fma_t(T0, nbv, off);
-      } else if (dir[1]) {
-        diag += T0 * 2.0f;
-      }
-      if (j > 0 || ty[2] == 0) {
-        const float nbv = j > 0 ? dnk : hs4[k >> 1];
-        diag += T1;
-        off = fma_t(T1, nbv, off);
-      } else if (dir[2]) {
-        diag += T1 * 2.0f;
-      }
-      if (j < NB - 1 || ty[3] == 0) {
-        const float nbv = j < NB - 1 ? upk : hs4[k >> 1];
-        diag += T1;
-        off = fma_t(T1, nbv, off);
-      } else if (dir[3]) {
-        diag += T1 * 2.0f;
-      }
-      v[k] = diag > 0.f ? relax(c.omega, fast_div(fma_t(rs[k >> 1] * dv, 1.0f, off), diag), v[k]) : 0.f;
-    }
-    float4 *dst = reinterpret_cast<float4 *>(phi + cb + j * NB + c0);
-    dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-    dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-  }
+  for (int p = lr.a + blockIdx.x * warps + (threadIdx.x >> 5); p < lr.b; p += gridDim.x * warps)
+    w16_sweep<false>(t, c, L, L.hx + (long)p * kHX, color, phi, rhs, lane, sh[threadIdx.x >> 5]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1599,7 +1435,7 @@ void launch_prolong_red(const Topo &t, const Coef<T> &c, const BlockList &L, T *
   if (L.n == 0) return;
   if (X.n > 0 && !X.hx) return;  // the extra sweep reads its blocks through halo descriptors
   if constexpr (sizeof(T) == 4) {
-    if (form == 1 && t.ndim == 2 && t.nb == 16) {
+    if (form == 1 && t.ndim == 2 && t.nb == 16 && L.hx) {
       const int g = std::min((L.n + X.n + 7) / 8, 152 * 64);
       launch_k(pdl, k_prolong_red_warp16<5>, g, kThreads, 0, s, t, c, L, phi, rhs, guard, X);
       return;
@@ -1662,14 +1498,14 @@ static void rbgs_nd(int variant, const Topo &t, const Coef<T> &c, const BlockLis
     case 12:
     case 13:
       if constexpr (ND == 2 && sizeof(T) == 4) {
-        if (t.nb == 16) {
+        if (t.nb == 16 && L.hx) {
           const int g = std::min((L.n + 7) / 8, 152 * 64);
           if (variant == 11)
             launch_k(pdl, k_rbgs_warp16<4>, g, kThreads, 0, s, t, c, L, color, phi, rhs, guard);
-          else if (variant == 12 || !L.hx)
+          else if (variant == 12)
             launch_k(pdl, k_rbgs_warp16<5>, g, kThreads, 0, s, t, c, L, color, phi, rhs, guard);
           else
-            launch_k(pdl, k_rbgs_warp16_flat<4>, g, kThreads, 0, s, t, c, L, color, phi, rhs, guard);
+            launch_k(pdl, k_rbgs_warp16<3>, g, kThreads, 0, s, t, c, L, color, phi, rhs, guard);
           return;
         }
       }
