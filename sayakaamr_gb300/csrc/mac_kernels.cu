@@ -372,6 +372,151 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_warp16(Topo t, Coef<flo
     w16_sweep<false>(t, c, L, L.hx + (long)p * kHX, color, phi, rhs, lane, sh[threadIdx.x >> 5]);
 }
 
+// The block-hybrid pass (k_bhgs) over 2D FP32 blocks of 16x16 cells, one warp
+// per block: nsweep red-black sweeps of the block in registers with the values
+// outside it frozen, from src into dst.  Everything the sweeps read is loaded
+// once, at the start; a sweep is then shuffles and arithmetic, without the
+// shared-memory tile, the reloads of coefficients and right-hand side and the
+// two CTA barriers per sweep that the CTA form has.  The values and operations
+// of k_bhgs in the same order: a frozen neighbour's part enters as 1 * (T
+// value), its rounded product.  Bound by the latency of one round of loads.
+__device__ __forceinline__ void h16_pass(const Topo &t, const Coef<float> &c, const BlockList &L, const int *e,
+                                         int nsweep, const float *__restrict__ src, float *__restrict__ dst,
+                                         const float *__restrict__ rhs, int lane, W16Halo &sh) {
+  constexpr int NB = 16, NC = 256;
+  const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh, par = j & 1;  // red cells: columns 2q + par
+  const int2 ib = *reinterpret_cast<const int2 *>(e + kHXInfo);
+  const int b = ib.y;
+  const long cb = (long)b * NC, fb = (long)b * t.nfb;
+  const float *u = uniform_of(c, b);
+  const float dv = geom(c, b, 6);
+  const float4 *s4 = reinterpret_cast<const float4 *>(src + cb + j * NB + c0);
+  const float4 p0 = s4[0], p1 = s4[1];
+  const float4 *rsrc = reinterpret_cast<const float4 *>(rhs + cb + j * NB + c0);
+  const float4 r0 = rsrc[0], r1 = rsrc[1];
+  float hdp[2], hk[2], hv[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+    w16_halo_slot<false>(t, c, e, b, ib.x, u, (lane >> 4) + 2 * h, lane & 15, src, hdp[h], hk[h], hv[h]);
+  // v[color][q]; the face coefficients, diagonal, rhs * dv and vf of the cell
+  float v[2][4], kl[2][4], kr[2][4], kd[2][4], ku[2][4], diag[2][4], rd[2][4], vf[2][4];
+  const float pv[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+  const float rv[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    v[0][q] = par ? pv[2 * q + 1] : pv[2 * q];
+    v[1][q] = par ? pv[2 * q] : pv[2 * q + 1];
+    rd[0][q] = (par ? rv[2 * q + 1] : rv[2 * q]) * dv;
+    rd[1][q] = (par ? rv[2 * q] : rv[2 * q + 1]) * dv;
+  }
+  if (u) {
+    const float T0 = u[0], T1 = u[1];
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) kl[k][q] = kr[k][q] = T0, kd[k][q] = ku[k][q] = T1, vf[k][q] = 1.f;
+  } else {
+    const float *x = c.tff[0] + fb + (NB + 1) * j + c0;
+    float tx[9];
+#pragma unroll
+    for (int n = 0; n < 9; n++) tx[n] = x[n];
+    const float4 *y = reinterpret_cast<const float4 *>(c.vf + cb + NB * j + c0);
+    const float4 w0 = y[0], w1 = y[1];
+    const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+    const float *yd = c.tff[1] + fb + NB * j + c0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      kl[0][q] = par ? tx[2 * q + 1] : tx[2 * q];
+      kr[0][q] = par ? tx[2 * q + 2] : tx[2 * q + 1];
+      kl[1][q] = par ? tx[2 * q] : tx[2 * q + 1];
+      kr[1][q] = par ? tx[2 * q + 1] : tx[2 * q + 2];
+      kd[0][q] = yd[2 * q + par];
+      kd[1][q] = yd[2 * q + 1 - par];
+      ku[0][q] = yd[2 * q + par + NB];
+      ku[1][q] = yd[2 * q + 1 - par + NB];
+      vf[0][q] = par ? wv[2 * q + 1] : wv[2 * q];
+      vf[1][q] = par ? wv[2 * q] : wv[2 * q + 1];
+    }
+  }
+  if (L.stc && block_off(L, b)) return;  // a finished problem; uniform over the warp
+  __syncwarp();                          // the slots of the warp's previous block have been read
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    // the frozen part: T * value (CRSE_FINE: the sum itself), rounded
+    sh.dp[lane + 32 * h] = hdp[h];
+    sh.v[lane + 32 * h] = hk[h] * hv[h];
+  }
+  __syncwarp();
+  // boundary cells: the slot's diagonal part, factor 1, the frozen part as
+  // the neighbour's value (hx: left or right, hy: below or above)
+  float hx = 0.f, hy[2][4];
+  const bool edge_y = j == 0 || j == NB - 1;
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int pk = k ? 1 - par : par, i = c0 + 2 * q + pk;
+      float dl = kl[k][q], dr = kr[k][q], dd = kd[k][q], du = ku[k][q];
+      if (q == 0 && i == 0) dl = sh.dp[j], kl[k][q] = 1.f, hx = sh.v[j];
+      if (q == 3 && i == NB - 1) dr = sh.dp[16 + j], kr[k][q] = 1.f, hx = sh.v[16 + j];
+      hy[k][q] = 0.f;
+      if (j == 0) dd = sh.dp[32 + i], kd[k][q] = 1.f, hy[k][q] = sh.v[32 + i];
+      if (j == NB - 1) du = sh.dp[48 + i], ku[k][q] = 1.f, hy[k][q] = sh.v[48 + i];
+      float g = c.alpha * dv;
+      g += dl;
+      g += dr;
+      g += dd;
+      g += du;
+      diag[k][q] = vf[k][q] > 0.f ? g : 0.f;  // 0: the cell stays at 0
+    }
+  for (int sw = 0; sw < nsweep; sw++) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const int pk = k ? 1 - par : par;
+      float(&o)[4] = v[1 - k];
+      const float fl = __shfl_up_sync(0xffffffffu, o[3], 1), fr = __shfl_down_sync(0xffffffffu, o[0], 1);
+      float nd[4], nu[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        nd[q] = __shfl_up_sync(0xffffffffu, o[q], 2);
+        nu[q] = __shfl_down_sync(0xffffffffu, o[q], 2);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        float vl = pk ? o[q] : (q > 0 ? o[q > 0 ? q - 1 : 0] : (hh ? fl : hx));
+        float vr = pk ? (q < 3 ? o[q < 3 ? q + 1 : 3] : (hh ? hx : fr)) : o[q];
+        const float vd = edge_y && j == 0 ? hy[k][q] : nd[q], vu = edge_y && j != 0 ? hy[k][q] : nu[q];
+        float off = 0.f;
+        off = fma_t(kl[k][q], vl, off);
+        off = fma_t(kr[k][q], vr, off);
+        off = fma_t(kd[k][q], vd, off);
+        off = fma_t(ku[k][q], vu, off);
+        v[k][q] = diag[k][q] > 0.f
+                      ? relax(c.omega, fast_div(fma_t(rd[k][q], vf[k][q], off), diag[k][q]), v[k][q])
+                      : 0.f;
+      }
+    }
+  }
+  float4 *d4 = reinterpret_cast<float4 *>(dst + cb + j * NB + c0);
+  d4[0] = par ? make_float4(v[1][0], v[0][0], v[1][1], v[0][1]) : make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
+  d4[1] = par ? make_float4(v[1][2], v[0][2], v[1][3], v[0][3]) : make_float4(v[0][2], v[1][2], v[0][3], v[1][3]);
+}
+
+constexpr int kH16Threads = 128;
+template <int MINB>
+__global__ void __launch_bounds__(kH16Threads, MINB) k_bhgs_warp16(Topo t, Coef<float> c, BlockList L, int nsweep,
+                                                                   const float *__restrict__ src,
+                                                                   float *__restrict__ dst,
+                                                                   const float *__restrict__ rhs, const int *guard) {
+  __shared__ W16Halo sh[kH16Threads / 32];
+  pdl_enter();
+  if (guard && *guard) return;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.x * warps + (threadIdx.x >> 5); p < lr.b; p += gridDim.x * warps)
+    h16_pass(t, c, L, L.hx + (long)p * kHX, nsweep, src, dst, rhs, lane, sh[threadIdx.x >> 5]);
+}
+
 // ---------------------------------------------------------------------------
 // volume-weighted restriction onto the non-leaf blocks of a level:
 // coarse = avg(fine*vf_fine)/vf_coarse (src/SayakaMacIB.cpp:157-232 with
@@ -890,6 +1035,195 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bhgs(Topo t, Coef<T> c, Bloc
       for (int i = threadIdx.x; i < ncell; i += blockDim.x) dst[cb + i] = tile[i];
     }
     __syncthreads();
+  }
+}
+
+// ---- The block-hybrid pass over 3D FP32 blocks of 16^3 or 8^3 cells --------
+// One CTA per block, one thread per row of cells along x, which keeps the
+// row's values, diagonal and right-hand side in registers, split by colour.
+// The tile in shared memory is split by colour too (tile[colour][quarter]
+// [row], a float4 of four cells of one colour): the cells of a row that a
+// half sweep updates have their y and z neighbours at the same places of the
+// adjoining rows' other-colour part, so a thread reads them 16 bytes at a
+// time without bank conflicts, and its x neighbours are in its registers.
+// Rows outside the block hold the frozen neighbours' parts (T value, rounded)
+// and enter with factor 1, so no cell takes a branch.  The values and
+// operations of k_bhgs in the same order: the same bits.
+//
+// k_bhgs spends about 80 instructions on an update (index arithmetic, six
+// boundary tests, reloads from global memory) and this form about 16; its
+// bound moves from issue towards the three streams of a pass (src, rhs, dst).
+template <int NB>
+struct H3 {
+  static constexpr int kRows = (NB + 2) * (NB + 2), kQ = NB / 2, kH = NB / 8, kFace = NB * NB;
+  float4 tile[2][kH][kRows];
+  float hc[6][kFace];   // diagonal part of every boundary face cell
+  float hox[2][kFace];  // frozen parts across the x faces
+  static __device__ __forceinline__ int row(int j, int k) { return j + 1 + (NB + 2) * (k + 1); }
+};
+
+// the sweeps of one block: row (j, k) of thread (U: a constant-coefficient
+// block, coefficients T[]; else from the face arrays)
+template <int NB, bool U>
+__device__ __forceinline__ void h3_sweeps(const Topo &t, const Coef<float> &c, int b, const float *u, float dv,
+                                          int nsweep, const float *__restrict__ rhs, H3<NB> &sh) {
+  constexpr int Q = NB / 2, H = NB / 8;
+  const int j = threadIdx.x % NB, k = threadIdx.x / NB, pr = (j + k) & 1, m = threadIdx.x;
+  const long cb = (long)b * NB * NB * NB, fb = (long)b * t.nfb;
+  const int r = H3<NB>::row(j, k);
+  const float T0 = U ? u[0] : 0.f, T1 = U ? u[1] : 0.f, T2 = U ? u[2] : 0.f;
+  // x faces i .. i+1 of cell i; y and z faces below, the ones above NB and
+  // NB^2 further
+  const float *fx = c.tff[0] + fb + (NB + 1) * (j + NB * k);
+  const float *fy = c.tff[1] + fb + NB * (j + (NB + 1) * k);
+  const float *fz = c.tff[2] + fb + NB * (j + NB * k);
+  const float *vf = c.vf + cb + NB * m, *rp = rhs + cb + NB * m;
+  float v[2][Q], rd[2][Q], dg[2][Q];
+  const float kd = j == 0 ? 1.f : T1, ku = j == NB - 1 ? 1.f : T1;
+  const float kb = k == 0 ? 1.f : T2, kf = k == NB - 1 ? 1.f : T2;
+  const float hl = sh.hox[0][m], hr = sh.hox[1][m];
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    const float2 r2 = *reinterpret_cast<const float2 *>(rp + 2 * q);
+    rd[0][q] = (pr ? r2.y : r2.x) * dv;
+    rd[1][q] = (pr ? r2.x : r2.y) * dv;
+  }
+#pragma unroll
+  for (int col = 0; col < 2; col++) {
+    const int pk = col ? 1 - pr : pr;
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+      const float4 w = sh.tile[col][h][r];
+      v[col][4 * h] = w.x, v[col][4 * h + 1] = w.y, v[col][4 * h + 2] = w.z, v[col][4 * h + 3] = w.w;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const int i = 2 * q + pk;
+      float g = c.alpha * dv;
+      g += q == 0 && i == 0 ? sh.hc[0][m] : (U ? T0 : fx[i]);
+      g += q == Q - 1 && i == NB - 1 ? sh.hc[1][m] : (U ? T0 : fx[i + 1]);
+      g += j == 0 ? sh.hc[2][i + NB * k] : (U ? T1 : fy[i]);
+      g += j == NB - 1 ? sh.hc[3][i + NB * k] : (U ? T1 : fy[i + NB]);
+      g += k == 0 ? sh.hc[4][i + NB * j] : (U ? T2 : fz[i]);
+      g += k == NB - 1 ? sh.hc[5][i + NB * j] : (U ? T2 : fz[i + NB * NB]);
+      if (!U && !(vf[i] > 0.f)) g = 0.f;  // 0: the cell stays at 0
+      dg[col][q] = g;
+    }
+  }
+  for (int sw = 0; sw < nsweep; sw++) {
+#pragma unroll
+    for (int col = 0; col < 2; col++) {
+      const int pk = col ? 1 - pr : pr;
+      const float(&o)[Q] = v[1 - col];
+#pragma unroll
+      for (int h = 0; h < H; h++) {
+        const float4 d4 = sh.tile[1 - col][h][r - 1], u4 = sh.tile[1 - col][h][r + 1];
+        const float4 b4 = sh.tile[1 - col][h][r - (NB + 2)], f4 = sh.tile[1 - col][h][r + (NB + 2)];
+        const float vd[4] = {d4.x, d4.y, d4.z, d4.w}, vu[4] = {u4.x, u4.y, u4.z, u4.w};
+        const float vb[4] = {b4.x, b4.y, b4.z, b4.w}, vz[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+          const int q = 4 * h + n, i = 2 * q + pk;
+          float vl = pk ? o[q] : (q > 0 ? o[q > 0 ? q - 1 : 0] : hl);
+          float vr = pk ? (q < Q - 1 ? o[q < Q - 1 ? q + 1 : q] : hr) : o[q];
+          const float kl = q == 0 && i == 0 ? 1.f : (U ? T0 : fx[i]);
+          const float kr = q == Q - 1 && i == NB - 1 ? 1.f : (U ? T0 : fx[i + 1]);
+          float off = 0.f;
+          off = fma_t(kl, vl, off);
+          off = fma_t(kr, vr, off);
+          off = fma_t(U || j == 0 ? kd : fy[i], vd[n], off);
+          off = fma_t(U || j == NB - 1 ? ku : fy[i + NB], vu[n], off);
+          off = fma_t(U || k == 0 ? kb : fz[i], vb[n], off);
+          off = fma_t(U || k == NB - 1 ? kf : fz[i + NB * NB], vz[n], off);
+          const float g = dg[col][q];
+          v[col][q] = g > 0.f ? relax(c.omega, fast_div(fma_t(rd[col][q], U ? 1.f : vf[i], off), g), v[col][q]) : 0.f;
+        }
+        sh.tile[col][h][r] = make_float4(v[col][4 * h], v[col][4 * h + 1], v[col][4 * h + 2], v[col][4 * h + 3]);
+      }
+      __syncthreads();
+    }
+  }
+}
+
+template <int NB, int MINB>
+__global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> c, BlockList L, int nsweep,
+                                                            const float *__restrict__ src, float *__restrict__ dst,
+                                                            const float *__restrict__ rhs, const int *guard) {
+  __shared__ H3<NB> sh;
+  pdl_enter();
+  if (guard && *guard) return;
+  constexpr int NT = NB * NB, NC = NB * NB * NB;
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.x; p < lr.b; p += gridDim.x) {
+    const int *e = L.hx + (long)p * kHX;
+    const int2 ib = *reinterpret_cast<const int2 *>(e + kHXInfo);
+    const int b = ib.y;
+    if (L.stc && block_off(L, b)) continue;  // uniform over the CTA
+    const uint16_t ft = (uint16_t)(ib.x & 0xffff);
+    const long cb = (long)b * NC, fb = (long)b * t.nfb;
+    const float *u = uniform_of(c, b);
+    // the tile, four cells of a row per step: two of each colour
+    const float4 *s4 = reinterpret_cast<const float4 *>(src + cb);
+#pragma unroll
+    for (int n = threadIdx.x; n < NC / 4; n += NT) {
+      const float4 w = s4[n];
+      const int row = n / (NB / 4), q = 2 * (n % (NB / 4)), j = row % NB, k = row / NB, pr = (j + k) & 1;
+      const int at = H3<NB>::row(j, k);
+      float2 *r2 = reinterpret_cast<float2 *>(&sh.tile[0][q >> 2][at]) + ((q >> 1) & 1);
+      float2 *b2 = reinterpret_cast<float2 *>(&sh.tile[1][q >> 2][at]) + ((q >> 1) & 1);
+      *r2 = pr ? make_float2(w.y, w.w) : make_float2(w.x, w.z);
+      *b2 = pr ? make_float2(w.x, w.z) : make_float2(w.y, w.w);
+    }
+    // the boundary face cells: diagonal and frozen parts
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+      const int d = f >> 1, s = f & 1, m = threadIdx.x, a0 = m % NB, a1 = m / NB;
+      const int ijk[3] = {d == 0 ? (s ? NB - 1 : 0) : a0, d == 0 ? a0 : (d == 1 ? (s ? NB - 1 : 0) : a1),
+                          d == 2 ? (s ? NB - 1 : 0) : a1};
+      const int fx = d == 0   ? ijk[0] + s + (NB + 1) * (ijk[1] + NB * ijk[2])
+                     : d == 1 ? ijk[0] + NB * (ijk[1] + s + (NB + 1) * ijk[2])
+                              : ijk[0] + NB * (ijk[1] + NB * (ijk[2] + s));
+      const int ty = face_type_of(ft, f);
+      float vc = 0.f, vo = 0.f;
+      if (ty == 0) {
+        vc = u ? u[d] : c.tff[d][fb + fx];
+        vo = vc * same_level_ghost<float, false>(t, b, f, ijk, src, e);
+      } else if (ty == 1) {
+        if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * 2.0f;
+      } else if (ty == 2) {
+        vc = cf_coef(c, t, b, d, fx, 1.5f);
+        vo = vc * fine_crse_ghost<float, 3, false>(t, b, f, ijk, src, e);
+      } else {
+        vc = cf_coef(c, t, b, d, fx, 0.75f);
+        vo = crse_fine_sum<float, 3, false>(t, c, b, f, ijk, src, e);
+      }
+      sh.hc[f][m] = vc;
+      if (d == 0) {
+        sh.hox[s][m] = vo;
+      } else {
+        // seen by the cell as its neighbour: the other colour, the same place
+        const int col = (ijk[0] + ijk[1] + ijk[2]) & 1, q = ijk[0] >> 1;
+        const int at = d == 1 ? H3<NB>::row(s ? NB : -1, ijk[2]) : H3<NB>::row(ijk[1], s ? NB : -1);
+        reinterpret_cast<float *>(&sh.tile[1 - col][q >> 2][at])[q & 3] = vo;
+      }
+    }
+    __syncthreads();
+    const float dv = geom(c, b, 6);
+    if (u)
+      h3_sweeps<NB, true>(t, c, b, u, dv, nsweep, rhs, sh);
+    else
+      h3_sweeps<NB, false>(t, c, b, u, dv, nsweep, rhs, sh);
+    if (nsweep == 0) __syncthreads();
+    float4 *d4 = reinterpret_cast<float4 *>(dst + cb);
+#pragma unroll
+    for (int n = threadIdx.x; n < NC / 4; n += NT) {
+      const int row = n / (NB / 4), q = 2 * (n % (NB / 4)), j = row % NB, k = row / NB, pr = (j + k) & 1;
+      const int at = H3<NB>::row(j, k);
+      const float2 r2 = *(reinterpret_cast<const float2 *>(&sh.tile[0][q >> 2][at]) + ((q >> 1) & 1));
+      const float2 b2 = *(reinterpret_cast<const float2 *>(&sh.tile[1][q >> 2][at]) + ((q >> 1) & 1));
+      d4[n] = pr ? make_float4(b2.x, r2.x, b2.y, r2.y) : make_float4(r2.x, b2.x, r2.y, b2.y);
+    }
+    __syncthreads();  // the tile is free for the next block
   }
 }
 
@@ -1561,6 +1895,21 @@ void launch_bhgs(const Topo &t, const Coef<T> &c, const BlockList &L, int nsweep
                  const T *rhs, const int *guard, cudaStream_t s, bool pdl) {
   const int nhalf = t.ncell / 2;
   if (L.n == 0 || nhalf == 0) return;
+  if constexpr (sizeof(T) == 4) {
+    if (t.ndim == 2 && t.nb == 16 && L.hx) {
+      const int warps = kH16Threads / 32, g = std::min((L.n + warps - 1) / warps, 152 * 64);
+      launch_k(pdl, k_bhgs_warp16<4>, g, kH16Threads, 0, s, t, c, L, nsweep, src, dst, rhs, guard);
+      return;
+    }
+    if (t.ndim == 3 && (t.nb == 16 || t.nb == 8) && L.hx) {
+      const int g = std::min(L.n, L.pb ? kReducedGrid : 152 * 64);
+      if (t.nb == 16)
+        launch_k(pdl, k_bhgs_rows<16, 2>, g, 256, 0, s, t, c, L, nsweep, src, dst, rhs, guard);
+      else
+        launch_k(pdl, k_bhgs_rows<8, 8>, g, 64, 0, s, t, c, L, nsweep, src, dst, rhs, guard);
+      return;
+    }
+  }
   const int nface = t.ndim == 3 ? t.nb * t.nb : t.nb;
   const size_t smem = sizeof(T) * ((size_t)t.ncell + 2 * 2 * t.ndim * (size_t)nface);
   const int threads = std::min(kThreads, (nhalf + 31) / 32 * 32);
