@@ -91,6 +91,21 @@ __global__ void __launch_bounds__(256) k_active_copy(const ActiveList *__restric
       l.alinks[i] = l.links[(long)l.orig[i / l.nlinks] * l.nlinks + i % l.nlinks];
 }
 
+// of the active blocks of the finest tower: all (head[0]) and those with one
+// face coefficient (head[1], see k_iso)
+__global__ void __launch_bounds__(kScanThreads) k_active_head(ActiveList top, const double *__restrict__ iso, int *head) {
+  const int n = top.pre[top.n];
+  int k = 0;
+  for (int i0 = 0; i0 < n; i0 += kScanThreads) {
+    const int i = i0 + threadIdx.x;
+    k += __syncthreads_count(i < n && iso[top.ablocks[i]] != 0.0);
+  }
+  if (threadIdx.x == 0) {
+    head[0] = n;
+    head[1] = k;
+  }
+}
+
 // zeros on the solid blocks of up to four vectors
 template <typename T>
 __global__ void __launch_bounds__(256) k_zero_solid(int nblocks, int ncell, const int *__restrict__ flag, T *a, T *b,
@@ -116,6 +131,7 @@ void MacGpu::build_active() {
   const int nbk = tt_.num_blocks;
   const DevList &top = towers_[finest_].all;
   n_act_ = top.n;
+  n_iso_ = 0;
   if (top.n == 0) return;
   if (!d_active_) {
     std::vector<ActiveList> h;
@@ -125,12 +141,13 @@ void MacGpu::build_active() {
       p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base ? base + used : nullptr);
       used += (n * sizeof(*p) + 15) / 16 * 16;
     };
-    int *flags = nullptr;
+    int *flags = nullptr, *head = nullptr;
     ActiveList *lists = nullptr;
     auto lay = [&] {  // sizes first, then places
       used = 0;
       h.clear();
       take(flags, nbk);
+      take(head, 2);
       auto reduce = [&](DevList &d, int nlinks) {
         if (d.n == 0) return;
         take(d.act.blocks, d.n);
@@ -162,13 +179,21 @@ void MacGpu::build_active() {
     CK_(cudaStreamSynchronize(stream_));
     d_act_lists_ = lists;
     d_active_ = flags;
+    d_act_head_ = head;
   }
   k_block_active<<<std::min((nbk + 7) / 8, 152 * 8), 256, 0, stream_>>>(nbk, ncell_, d_vf_, d_active_);
   k_active_scan<<<n_act_lists_, kScanThreads, 0, stream_>>>(d_act_lists_, d_active_);
   k_active_copy<<<dim3(152, n_act_lists_), 256, 0, stream_>>>(d_act_lists_);
   CK_(cudaGetLastError());
-  CK_(cudaMemcpyAsync(&n_act_, top.act.pre + top.n, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+  const ActiveList t{top.blocks, nullptr, nullptr, nullptr, 0, top.n, top.act.blocks, nullptr, nullptr, nullptr,
+                     top.act.pre, top.act.orig};
+  k_active_head<<<1, kScanThreads, 0, stream_>>>(t, d_iso_, d_act_head_);
+  CK_(cudaGetLastError());
+  int head[2] = {0, 0};
+  CK_(cudaMemcpyAsync(head, d_act_head_, sizeof(head), cudaMemcpyDeviceToHost, stream_));
   CK_(cudaStreamSynchronize(stream_));
+  n_act_ = head[0];
+  n_iso_ = head[1];
 }
 
 // whether the next solve walks the reduced lists: one shared BiCGSTAB state,

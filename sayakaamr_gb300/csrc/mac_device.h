@@ -51,6 +51,11 @@ struct Coef {
   // [6] sa and [7] ia of the FP64 smoother.  Kernels read these instead of
   // the face arrays and vf, with the same arithmetic in the same order.
   const T *ut = nullptr;
+  // coefficients of the coarse/fine faces (device solve only; null
+  // elsewhere): [block][face][cell of the face], stencil::cf_coef of a face
+  // at a coarser neighbour (spacing 1.5) or at a refined one (0.75), which
+  // costs two divisions' worth of FP64 where a kernel evaluates it
+  const T *cf = nullptr;
 };
 constexpr int kUni = 8;
 

@@ -49,6 +49,45 @@ __device__ __forceinline__ df two_prod(float a, float b) {
   return {p, __fmaf_rn(a, b, -p)};
 }
 
+// n x - (sum of the 2 ND values v) for floats x, v and a small whole number n
+// as FP64: every product and sum splits into its rounded value and its exact
+// error, the errors are summed the same way, and what is left of them after
+// the second float (bits below 2^-48 of the largest term, which appear only
+// where neighbouring values differ by more than 2^20) is added too.  The
+// result is off by one FP64 rounding of itself, about 2^-53, where the FP64
+// sum of products rounds at the size of its terms.
+template <int ND>
+__device__ __forceinline__ double exact_delta(float n, float x, const float (&v)[2 * ND]) {
+  df s = two_sum(v[0], v[1]), err = {0.f, 0.f};
+  float rest = 0.f;
+  auto more = [&](float e, bool first) {  // e joins the errors
+    if (first) {
+      err.hi = e;
+    } else {
+      const df a = two_sum(err.hi, e);
+      err.hi = a.hi;
+      rest = __fadd_rn(rest, a.lo);
+    }
+  };
+  more(s.lo, true);
+#pragma unroll
+  for (int d = 1; d < ND; d++) {
+    const df p = two_sum(v[2 * d], v[2 * d + 1]);
+    const df q = two_sum(s.hi, p.hi);
+    s.hi = q.hi;
+    more(p.lo, false);
+    more(q.lo, false);
+  }
+  const df p = two_prod(n, x);
+  const df h = two_sum(p.hi, -s.hi);
+  more(-p.lo, false);
+  const df l = two_sum(h.lo, -err.hi);
+  const float m = __fsub_rn(l.lo, rest);
+  if (fpint::rare(h.hi) || fpint::rare(l.hi) || m != 0.f)
+    return (fpint::widen(h.hi) + fpint::widen(l.hi)) + fpint::widen(m);
+  return fpint::widen_common(h.hi) + fpint::widen_common(l.hi);
+}
+
 __device__ __forceinline__ df add(df x, df y) {
   df s = two_sum(x.hi, y.hi);
   const df t = two_sum(x.lo, y.lo);

@@ -628,6 +628,34 @@ __global__ void __launch_bounds__(kTPB) k_uniform(Topo t, Coef<double> c, Coef<f
   }
 }
 
+// the coefficients of the faces at coarser and at refined neighbours
+// (Coef::cf), in the arithmetic of cf_coef
+template <typename T, int ND>
+__global__ void __launch_bounds__(kTPB) k_cf_faces(Topo t, Coef<T> c, T *__restrict__ cf) {
+  using namespace stencil;
+  const int nface = ND == 3 ? t.nb * t.nb : t.nb;
+  const long total = (long)t.nblocks * 2 * ND * nface;
+  for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
+    const int m = (int)(it % nface), f = (int)(it / nface % (2 * ND)), b = (int)(it / nface / (2 * ND));
+    const int n = t.neighbor[b * 6 + f];
+    const bool coarser = n == -1, refined = n >= 0 && t.child[n * 8] >= 0;
+    if (!coarser && !refined) continue;
+    const int d = f >> 1, s = f & 1, m0 = ND == 3 ? m % t.nb : m, m1 = ND == 3 ? m / t.nb : 0;
+    const int ijk[3] = {d == 0 ? (s ? t.nb - 1 : 0) : m0, d == 0 ? m0 : (d == 1 ? (s ? t.nb - 1 : 0) : m1),
+                        ND == 3 ? (d == 2 ? (s ? t.nb - 1 : 0) : m1) : 0};
+    cf[it] = cf_coef(c, t, b, d, face_index(d, ijk, s, t.nb), coarser ? (T)1.5 : (T)0.75);
+  }
+}
+
+// T S of the blocks whose faces all carry one coefficient (see k_op_rows), else 0
+__global__ void k_iso(int nblocks, int nd, double alpha, const double *__restrict__ u64, double *__restrict__ iso) {
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nblocks; b += gridDim.x * blockDim.x) {
+    const double *u = u64 + (long)b * kUni;
+    const bool on = u[3] != 0.0 && alpha == 0.0 && u[0] == u[1] && (nd == 2 || u[0] == u[2]);
+    iso[b] = on ? u[0] * u[5] : 0.0;
+  }
+}
+
 // sum T * phi_nb over the faces of cell ijk that are not physical boundaries
 template <int ND, typename TX>
 __device__ __forceinline__ double op_offdiag(const Topo &t, const Coef<double> &c, int b, uint16_t ft,
@@ -652,7 +680,7 @@ __device__ __forceinline__ double op_offdiag(const Topo &t, const Coef<double> &
         off = __fma_rn(u ? u[d] : c.tff[d][(long)b * t.nfb + fx],
                        widen_from<TX>(same_level_ghost<TX, false>(t, b, f, ijk, x, hx)), off);
       else if (ty == 2)
-        off = __fma_rn(cf_coef(c, t, b, d, fx, 1.5), widen_from<TX>(fine_crse_ghost<TX, ND, false>(t, b, f, ijk, x, hx)),
+        off = __fma_rn(cf_face<double, ND>(c, t, b, f, ijk, fx, 1.5), widen_from<TX>(fine_crse_ghost<TX, ND, false>(t, b, f, ijk, x, hx)),
                        off);
       else if (ty == 3)
         off += crse_fine_sum<double, ND, false>(t, c, b, f, ijk, x, hx);
@@ -705,7 +733,7 @@ __device__ __forceinline__ dfl::df op_offdiag_df(const Topo &t, const Coef<doubl
 }
 
 template <int ND, int MODE, typename TX, bool MULTI, bool DFOP = false>
-__global__ void __launch_bounds__(kTPB) k_op_red(Topo t, Coef<double> c, BlockList L, Chunks ch,
+__global__ void __launch_bounds__(kTPB, 4) k_op_red(Topo t, Coef<double> c, BlockList L, Chunks ch,
                                                const TX *__restrict__ x, double *__restrict__ y,
                                                const double *__restrict__ w, const double *__restrict__ P,
                                                const double *__restrict__ S, FState *stb, double *partials,
@@ -767,6 +795,166 @@ __global__ void __launch_bounds__(kTPB) k_op_red(Topo t, Coef<double> c, BlockLi
   if (MODE == 1) seg_reduce<2>(acc, 0u, partials, wk.counter, wk.first, wk.count, wk.slot, EpiOmega{st});
   if (MODE == 2) seg_reduce<2>(acc, 1u, partials, wk.counter, wk.first, wk.count, wk.slot, EpiInit{st});
   if (MODE == 3) seg_reduce<2>(acc, 1u, partials, wk.counter, wk.first, wk.count, wk.slot, EpiVerify{st});
+}
+
+// The operator with its dot products (modes 0 and 1 of k_op_red) on an FP32
+// input, blocks whose edge is a multiple of 4 cells: a thread takes four cells
+// of a row, whose neighbours along y and z are four cells of another row (of
+// the block, or of the neighbour behind a same-level face) and lie in the
+// thread's own 16 bytes along x, so the loads are 16 bytes wide and no cell
+// inside a warp takes another path than the next one.
+//
+// In a block whose faces all carry one coefficient T and whose cells are
+// fluid (iso: T S, alpha 0), y = T S (n x_c - sum x_nb), n counting same-level
+// faces once, Dirichlet faces twice (their ghost is -x_c), Neumann faces not
+// at all.  The difference is formed exactly on the FP32 pipe
+// (dfl::exact_delta): a cell then takes an addition and a product of FP64
+// instead of 2 ND + 2 multiply-adds, which is what bounds this kernel (GB300:
+// two FP64 lanes per SM and clock).  Other blocks take the general form of
+// k_op_red on the same loads, the coarse/fine faces among them from their
+// table (Coef::cf: without it each costs a division on the FP64 pipe).
+template <int ND, int MODE, bool MULTI>
+__global__ void __launch_bounds__(kTPB, 4) k_op_rows(Topo t, Coef<double> c, BlockList L, Chunks ch,
+                                                   const float *__restrict__ x, double *__restrict__ y,
+                                                   const double *__restrict__ w, const double *__restrict__ P,
+                                                   const double *__restrict__ S, FState *stb, double *partials,
+                                                   unsigned *counter, const double *__restrict__ iso) {
+  using namespace stencil;
+  pdl_enter();
+  Work wk = work_of<MULTI>(ch, stb, list_count(L) * t.ncell, counter);
+  FState *st = wk.st;
+  if (st->done) return;
+  if (MULTI) wk.it0 -= threadIdx.x;  // cells of the chunk; its threads take four each
+  const int nb = t.nb, nc = t.ncell;
+  double acc[2] = {0.0, 0.0};
+  const int first = MULTI ? wk.it0 + 4 * (int)threadIdx.x : 4 * wk.it0;
+  for (int it = first; it < wk.it1; it += 4 * wk.step) {
+    int p, ci, ijk[3];
+    split_cell<ND>(it, t, p, ci);
+    decode_fast<ND>(ci, t, ijk);
+    const int *e = L.hx + (long)p * kHX;
+    const int2 ib = *reinterpret_cast<const int2 *>(e + kHXInfo);
+    const int b = ib.y;
+    const uint16_t ft = (uint16_t)(ib.x & 0xffff);
+    const long cb = (long)b * nc;
+    const float *xb = x + cb + ci;
+    const double K = iso[b];
+    // the six (four) neighbour rows: v[0], v[1] the cells left and right of
+    // the four, r[] the four cells below and above them per direction
+    float4 r[2 * (ND - 1)];
+    float vx[2] = {0.f, 0.f};
+    float nrow = 2.f * ND, nl = 0.f, nr = 0.f;  // multiplicity of x_c, and of the first and last cell
+    bool cf = false;
+    const float4 xc = *reinterpret_cast<const float4 *>(xb);
+#pragma unroll
+    for (int f = 0; f < 2 * ND; f++) {
+      const int d = f >> 1, s = f & 1, stride = d == 0 ? 1 : (d == 1 ? nb : nb * nb);
+      const bool bnd = d == 0 ? (s ? ijk[0] + 4 == nb : ijk[0] == 0) : (s ? ijk[d] == nb - 1 : ijk[d] == 0);
+      const float *q = xb + (d == 0 ? (s ? 4 : -1) : (s ? stride : -stride));
+      bool there = true;
+      if (bnd) {
+        const int ty = face_type_of(ft, f);
+        there = ty == 0;
+        cf = cf || ty > 1;
+        if (ty == 0) {
+          q = x + (long)e[f] * nc + ci + (d == 0 ? (s ? 4 - nb : nb - 1) : (s ? (1 - nb) * stride : (nb - 1) * stride));
+        } else if (ty == 1) {
+          const float n = t.bc_type[b * 6 + f] == kBCNeumann ? -1.f : 1.f;
+          if (d > 0)
+            nrow += n;
+          else if (s)
+            nr = n;
+          else
+            nl = n;
+        }
+      }
+      if (d == 0)
+        vx[s] = there ? *q : 0.f;
+      else
+        r[f >= 2 ? f - 2 : 0] = there ? *reinterpret_cast<const float4 *>(q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const double2 wa = *reinterpret_cast<const double2 *>(w + cb + ci);
+    const double2 wb = *reinterpret_cast<const double2 *>(w + cb + ci + 2);
+    const float xv[6] = {vx[0], xc.x, xc.y, xc.z, xc.w, vx[1]};
+    double yv[4];
+    bool done = false;
+    if (__double_as_longlong(K) != 0 && !cf) {  // uniform over a block but for its coarse/fine faces
+      done = true;
+#pragma unroll
+      for (int n = 0; n < 4; n++) {
+        float v[2 * ND];
+        v[0] = xv[n];
+        v[1] = xv[n + 2];
+#pragma unroll
+        for (int q = 0; q < 2 * (ND - 1); q++) v[2 + q] = n == 0 ? r[q].x : n == 1 ? r[q].y : n == 2 ? r[q].z : r[q].w;
+        const double dl = dfl::exact_delta<ND>(nrow + (n == 0 ? nl : 0.f) + (n == 3 ? nr : 0.f), xv[n + 1], v);
+        // an overflow of the FP32 sums: the general form
+        done = done && (__double2hiint(dl) & 0x7ff00000) != 0x7ff00000;
+        yv[n] = K * dl;
+      }
+    }
+    if (!done) {
+      const long fb = (long)b * t.nfb;
+      const double *u = uniform_of(c, b);
+      // factor and value of a face at a coarser or refined neighbour
+      auto cross = [&](int f, int n, double &k, double &v) {
+        const int at[3] = {ijk[0] + n, ijk[1], ijk[2]};
+        if (face_type_of(ft, f) == 2) {
+          k = cf_face<double, ND>(c, t, b, f, at, 0, 1.5);
+          v = fpint::widen(fine_crse_ghost<float, ND, false>(t, b, f, at, x, e));
+        } else {
+          k = 1.0;
+          v = crse_fine_sum<double, ND, false>(t, c, b, f, at, x, e);
+        }
+      };
+      const int row = ijk[1] + nb * ijk[2];
+      const double *tx = c.tff[0] + fb + (nb + 1) * row + ijk[0];
+      double off[4], xw[6];
+#pragma unroll
+      for (int n = 0; n < 6; n++) xw[n] = fpint::widen(xv[n]);
+      double tl = u ? u[0] : tx[0];
+      if (cf && ijk[0] == 0 && face_type_of(ft, 0) > 1) cross(0, 0, tl, xw[0]);
+#pragma unroll
+      for (int n = 0; n < 4; n++) {
+        const double ti = u ? u[0] : tx[n + 1];
+        double tr = ti;
+        if (n == 3 && cf && ijk[0] + 4 == nb && face_type_of(ft, 1) > 1) cross(1, 3, tr, xw[5]);
+        off[n] = __fma_rn(tr, xw[n + 2], __fma_rn(tl, xw[n], 0.0));
+        tl = ti;
+      }
+#pragma unroll
+      for (int f = 2; f < 2 * ND; f++) {
+        const int d = f >> 1, s = f & 1;
+        const long fx = d == 1 ? ijk[0] + nb * (ijk[1] + s + (nb + 1) * ijk[2]) : ci + s * nb * nb;
+        const double *tf = c.tff[d] + fb + fx;
+        const float4 q = r[f - 2];
+        const float qv[4] = {q.x, q.y, q.z, q.w};
+        const bool over = cf && (s ? ijk[d] == nb - 1 : ijk[d] == 0) && face_type_of(ft, f) > 1;
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+          double k = u ? u[d] : tf[n], v = fpint::widen(qv[n]);
+          if (over) cross(f, n, k, v);
+          off[n] = __fma_rn(k, v, off[n]);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 4; n++) yv[n] = __fma_rn(xw[n + 1], P[cb + ci + n], -off[n] * S[cb + ci + n]);
+    }
+    *reinterpret_cast<double2 *>(y + cb + ci) = make_double2(yv[0], yv[1]);
+    *reinterpret_cast<double2 *>(y + cb + ci + 2) = make_double2(yv[2], yv[3]);
+    const double wv[4] = {wa.x, wa.y, wb.x, wb.y};
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+      acc[0] = __fma_rn(wv[n], yv[n], acc[0]);
+      if (MODE == 1) acc[1] = __fma_rn(yv[n], yv[n], acc[1]);
+    }
+  }
+  if (MODE == 0) {
+    double a[1] = {acc[0]};
+    seg_reduce<1>(a, 0u, partials, wk.counter, wk.first, wk.count, wk.slot, EpiAlpha{st});
+  } else {
+    seg_reduce<2>(acc, 0u, partials, wk.counter, wk.first, wk.count, wk.slot, EpiOmega{st});
+  }
 }
 
 // while verifying: x0 += x, x = 0 (the pass's solution folded into x0)
@@ -907,10 +1095,12 @@ void MacGpu::ensure_fast_buffers() {
   else
     cudaMemsetAsync(d_uni2_, 0, (size_t)std::max(nbk, 1) * kUni * sizeof(float2), stream_);
   if (dev_malloc(&d_uni64_, (size_t)std::max(nbk, 1) * kUni * sizeof(double)) != cudaSuccess ||
-      dev_malloc(&d_uni32_, (size_t)std::max(nbk, 1) * kUni * sizeof(float)) != cudaSuccess)
+      dev_malloc(&d_uni32_, (size_t)std::max(nbk, 1) * kUni * sizeof(float)) != cudaSuccess ||
+      dev_malloc(&d_iso_, (size_t)std::max(nbk, 1) * sizeof(double)) != cudaSuccess)
     fail("out of device memory (block records)");
   else {
     cudaMemsetAsync(d_uni64_, 0, (size_t)std::max(nbk, 1) * kUni * sizeof(double), stream_);
+    cudaMemsetAsync(d_iso_, 0, (size_t)std::max(nbk, 1) * sizeof(double), stream_);
     cudaMemsetAsync(d_uni32_, 0, (size_t)std::max(nbk, 1) * kUni * sizeof(float), stream_);
   }
   if (dev_malloc(&d_st_, sizeof(FState)) != cudaSuccess) fail("alloc state");
@@ -918,6 +1108,16 @@ void MacGpu::ensure_fast_buffers() {
   if (dev_malloc(&d_part_, sizeof(double) * kMaxRedBlocks * 4) != cudaSuccess) fail("alloc partials");
   if (dev_malloc(&d_cnt_, sizeof(unsigned) * 4) != cudaSuccess) fail("alloc counter");
   cudaMemsetAsync(d_cnt_, 0, sizeof(unsigned) * 4, stream_);
+  {
+    const size_t ncf = (size_t)std::max(nbk, 1) * 2 * nd * (nd == 3 ? tt_.nb * tt_.nb : tt_.nb);
+    if (dev_malloc(&d_cf64_, ncf * sizeof(double)) != cudaSuccess ||
+        dev_malloc(&d_cf32_, ncf * sizeof(float)) != cudaSuccess) {
+      fail("out of device memory (coarse/fine faces)");
+    } else {
+      cudaMemsetAsync(d_cf64_, 0, ncf * sizeof(double), stream_);
+      cudaMemsetAsync(d_cf32_, 0, ncf * sizeof(float), stream_);
+    }
+  }
   c32_.geom = d_geom32_;
   for (int d = 0; d < 3; d++) {
     const int dd = d < nd ? d : 0;
@@ -1058,6 +1258,21 @@ void MacGpu::build_op_factors() {
   CK(cudaGetLastError());
 }
 
+// the coarse/fine face tables from the current coefficients
+void MacGpu::build_cf() {
+  const long n = (long)tt_.num_blocks * 2 * tt_.ndim * (tt_.ndim == 3 ? tt_.nb * tt_.nb : tt_.nb);
+  if (n == 0) return;
+  auto go = [&](auto k64, auto k32) {
+    k64<<<ew_grid(n), kTPB, 0, stream_>>>(topo_, c64_, d_cf64_);
+    k32<<<ew_grid(n), kTPB, 0, stream_>>>(topo_, c32_, d_cf32_);
+  };
+  if (tt_.ndim == 2)
+    go(k_cf_faces<double, 2>, k_cf_faces<float, 2>);
+  else
+    go(k_cf_faces<double, 3>, k_cf_faces<float, 3>);
+  CK(cudaGetLastError());
+}
+
 // constant-coefficient block records from the current coefficients (after
 // refresh_fp32: the FP32 record takes the FP32 face coefficients)
 void MacGpu::build_uniform() {
@@ -1070,6 +1285,7 @@ void MacGpu::build_uniform() {
     k_uniform<3><<<grid, kTPB, 0, stream_>>>(topo_, c64_, c32_, d_uni64_, d_uni32_);
   const long nu = (long)nbk * kUni;
   k_split_df<<<ew_grid(nu), kTPB, 0, stream_>>>(nu, d_uni64_, d_uni2_);
+  k_iso<<<std::min((nbk + kTPB - 1) / kTPB, 152 * 8), kTPB, 0, stream_>>>(nbk, tt_.ndim, alpha_, d_uni64_, d_iso_);
   CK(cudaGetLastError());
 }
 
@@ -1079,6 +1295,8 @@ void MacGpu::bind_uniform() {
   cd64_ = c64_;
   cd64_.ut = prm_.uniform ? d_uni64_ : nullptr;
   c32_.ut = prm_.uniform ? d_uni32_ : nullptr;
+  cd64_.cf = d_cf64_;
+  c32_.cf = d_cf32_;
   // the smoothers' relaxation weight (1: plain Gauss-Seidel, the reference's)
   cd64_.omega = prm_.relax_omega;
   c32_.omega = (float)prm_.relax_omega;
@@ -1570,19 +1788,24 @@ void MacGpu::precondition(int L, T *resid, T *corr, const Coef<T> &c, double *ou
 // on the integer pipe where they read it, or widened once into FP64 phat /
 // shat.  params.vcycle_out 0 (auto): in place in 2D and on 3D towers of at
 // most 2M cells, where it saves two launches per iteration (batch workload,
-// 2D, 29M cells: 58.8 in place vs 60.4 ms widened); larger 3D towers widen,
-// since the 3D operator reads seven cells and their integer widenings cost
-// more than the launches (config3, 15.9M cells: 31.6 in place vs 27.3 ms).
-// 1 = in place with the operator in double-float, 2 = always widened, 3 =
-// always in place.
+// 2D, 29M cells: 58.8 in place vs 60.4 ms widened), and on larger 3D towers
+// of which at least half the blocks have one face coefficient, whose operator
+// is formed on the FP32 pipe from the FP32 values (k_op_rows).  Other large 3D
+// towers widen, since the general 3D operator reads seven cells and their
+// integer widenings cost more than the launches (15.9M cells: 31.6 in place
+// vs 27.3 ms).  1 = in place with the operator in double-float, 2 = always
+// widened, 3 = always in place.
 constexpr long kDirectF32Cells = 1l << 21;
+bool MacGpu::vcycle_in_place() const {
+  if (learned_active() || prm_.precision != 1) return false;
+  if (prm_.vcycle_out != 0) return prm_.vcycle_out != 2;
+  const DevList &top = towers_[finest_].all;
+  return tt_.ndim == 2 || (long)top.n * ncell_ <= kDirectF32Cells || (!multi() && 2l * n_iso_ >= n_act_);
+}
 template <typename T>
 void MacGpu::iteration_device(T *resid, T *corr, const Coef<T> &c) {
   if constexpr (sizeof(T) == 4) {
-    const long w = (long)tower_list(finest_).n * ncell_;
-    const bool direct = prm_.vcycle_out == 1 || prm_.vcycle_out == 3 ||
-                        (prm_.vcycle_out == 0 && (tt_.ndim == 2 || w <= kDirectF32Cells));
-    if (!learned_active() && direct) {
+    if (vcycle_in_place()) {
       iteration_body<T, float>(resid, corr, c, corr, corr, nullptr, nullptr);
       return;
     }
@@ -1615,6 +1838,7 @@ void MacGpu::iteration_body(T *resid, T *corr, const Coef<T> &c, const TO *PH, c
   const bool pdl = prm_.pdl != 0;
   const double *OP = d_opP_, *OS = d_opS_;
   const float2 *OP2 = d_opP2_, *OS2 = d_opS2_, *U2 = d_uni2_;
+  const double *ISO = d_iso_;
   // params.vcycle_out 1: the operator of the FP32 V-cycle's output in double-float
   const bool dfop = prm_.vcycle_out == 1;
   auto op = [&](auto mode, const auto *x, double *y, const double *wv, double *y2) {
@@ -1639,6 +1863,17 @@ void MacGpu::iteration_body(T *resid, T *corr, const Coef<T> &c, const TO *PH, c
       }
     };
     if constexpr (sizeof(TX) == 4 && M < 2) {
+      if (!dfop && tt_.nb % 4 == 0) {
+        const int g = mp ? nchunks_ : std::min(red_grid(w), (int)std::max<long>(1, (w / 4 + kTPB - 1) / kTPB));
+        auto rows = [&](auto kern) {
+          launch_k(pdl, kern, g, kTPB, 0, stream_, topo_, cd64_, TL, ch, x, y, wv, OP, OS, ST, PART, CNT, ISO);
+        };
+        if (tt_.ndim == 2)
+          mp ? rows(k_op_rows<2, M, true>) : rows(k_op_rows<2, M, false>);
+        else
+          mp ? rows(k_op_rows<3, M, true>) : rows(k_op_rows<3, M, false>);
+        return;
+      }
       if (dfop) {
         go(std::true_type{});
         return;
@@ -1753,6 +1988,7 @@ void MacGpu::capture_loop(int precision) {
   graph_vout_ = prm_.vcycle_out;
   graph_omega_ = prm_.relax_omega;
   graph_act_ = (int)act_on_;
+  graph_direct_ = (int)vcycle_in_place();
 }
 
 // the captured graph was recorded with other parameters than the current ones
@@ -1763,7 +1999,8 @@ bool MacGpu::graph_stale() const {
          graph_order_ != prm_.sublevel_order || graph_smoother_ != prm_.smoother ||
          graph_inner_ != prm_.inner_sweeps || graph_multi_ != (int)multi() || graph_uniform_ != prm_.uniform ||
          graph_pform_ != prm_.prolong_form || graph_vout_ != prm_.vcycle_out ||
-         graph_omega_ != prm_.relax_omega || graph_act_ != (int)act_on_;
+         graph_omega_ != prm_.relax_omega || graph_act_ != (int)act_on_ ||
+         graph_direct_ != (int)vcycle_in_place();
 }
 
 int MacGpu::cg_solve_device(SolveInfo *info) {
@@ -1887,6 +2124,7 @@ int MacGpu::prepare_device() {
     // bottom solve's arrays had to be allocated afresh.
     const BottomDev before = bot_;
     refresh_fp32();
+    build_cf();
     build_uniform();
     build_op_factors();
     if (prm_.bottom_refresh || !bottom_ready_ || bot_param_ != prm_.bottom_level || bot_half_ != prm_.bottom_half)

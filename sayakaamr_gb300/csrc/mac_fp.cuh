@@ -52,6 +52,18 @@ __device__ __forceinline__ double widen(float f) {
   return from_bits(sign | ((unsigned long long)(897 - s) << 52) | ((unsigned long long)((m << s) & 0x7fffffu) << 29));
 }
 
+// the same without branches for zeros and normal floats; `rare` tells the
+// others (denormals, inf, NaN), which take widen
+__device__ __forceinline__ bool rare(float f) {
+  const unsigned a = __float_as_uint(f) << 1;
+  return a != 0u && a - 0x01000000u >= 0xfe000000u;
+}
+__device__ __forceinline__ double widen_common(float f) {
+  const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+  const unsigned hi = (a ? (a >> 3) + 0x38000000u : 0u) | (u & 0x80000000u);
+  return from_bits(((unsigned long long)hi << 32) | (u << 29));
+}
+
 // 0.0 + (double)f: as widen, with -0 turned into +0
 __device__ __forceinline__ double widen_plus0(float f) {
   return (__float_as_uint(f) & 0x7fffffffu) == 0u ? 0.0 : widen(f);

@@ -178,15 +178,6 @@ struct W16Halo {
 // neighbour's parent).  The gathers of mac_stencil.cuh for 2D blocks of 16,
 // without their arrays: the direction differs from lane to lane, and arrays
 // indexed by it would live in local memory.
-struct W16Dir {  // the coefficient arrays of a lane's direction
-  const float *tff, *bc, *af;
-};
-__device__ __forceinline__ float w16_cf_coef(const Coef<float> &c, const W16Dir &a, int d, long fx, int b, float h) {
-  float v = c.beta * geom(c, b, 3 + d) / (geom(c, b, d) * h);
-  v = v * a.bc[fx];
-  v = v * a.af[fx];
-  return v;
-}
 template <bool PROLONG>
 __device__ __forceinline__ void w16_halo_slot(const Topo &t, const Coef<float> &c, const int *e, int b, int info,
                                               const float *u, int f, int m, const float *__restrict__ phi, float &dp,
@@ -194,13 +185,13 @@ __device__ __forceinline__ void w16_halo_slot(const Topo &t, const Coef<float> &
   constexpr int NB = 16, NC = 256;
   const int d = f >> 1, s = f & 1;
   const int ty = face_type_of((uint16_t)(info & 0xffff), f);
-  const W16Dir a = d ? W16Dir{c.tff[1], c.bcoef[1], c.afrac[1]} : W16Dir{c.tff[0], c.bcoef[0], c.afrac[0]};
+  const float *tff = d ? c.tff[1] : c.tff[0];
   const long fx = (long)b * t.nfb + (d ? m + NB * (s * NB) : s * NB + (NB + 1) * m);
   const int across = s ? 0 : NB - 1;  // the neighbour's cell layer at the face
   dp = k = v = 0.f;
   if (ty == 0) {
     const long n = e[f];
-    dp = k = u ? u[d] : a.tff[fx];
+    dp = k = u ? u[d] : tff[fx];
     if constexpr (PROLONG) {
       const int pw = e[kHXPar + f], wc = pw & 7;
       const int i = d ? m : across, j = d ? across : m;
@@ -211,20 +202,18 @@ __device__ __forceinline__ void w16_halo_slot(const Topo &t, const Coef<float> &
       v = phi[n * NC + (d ? m + NB * across : across + NB * m)];
     }
   } else if (ty == 1) {
-    if (t.bc_type[b * 6 + f] != kBCNeumann) dp = (u ? u[d] : a.tff[fx]) * 2.0f;
+    if (t.bc_type[b * 6 + f] != kBCNeumann) dp = (u ? u[d] : tff[fx]) * 2.0f;
   } else if (ty == 2) {
     const int tc = 8 * ((info >> (17 - d)) & 1) + (m >> 1);  // which_child >> (1 - d)
-    dp = k = w16_cf_coef(c, a, d, fx, b, 1.5f);
+    dp = k = c.cf[((long)b * 4 + f) * NB + m];
     v = phi[(long)e[f] * NC + (d ? tc + NB * across : across + NB * tc)];
   } else {
     const int half = m >> 3, F = e[kHXKids + 4 * f + half], t0 = 2 * (m - 8 * half);
-    const int fl = across + 1 - s;  // the fine block's face layer toward b
-    dp = w16_cf_coef(c, a, d, fx, b, 0.75f);
+    dp = c.cf[((long)b * 4 + f) * NB + m];
     k = 1.f;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
-      const float tf =
-          w16_cf_coef(c, a, d, (long)F * t.nfb + (d ? t0 + q + NB * fl : fl + (NB + 1) * (t0 + q)), F, 1.5f);
+      const float tf = c.cf[((long)F * 4 + (f ^ 1)) * NB + t0 + q];
       v += tf * phi[(long)F * NC + (d ? t0 + q + NB * across : across + NB * (t0 + q))];
     }
   }
@@ -798,10 +787,10 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_tile(Topo t, Coef<T> c,
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        vc = vk = cf_coef(c, t, b, d, fx, (T)1.5);
+        vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
         vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
       } else {
-        vc = cf_coef(c, t, b, d, fx, (T)0.75);
+        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
         vk = (T)1;
         vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
       }
@@ -965,10 +954,10 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bhgs(Topo t, Coef<T> c, Bloc
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        vc = cf_coef(c, t, b, d, fx, (T)1.5);
+        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
         vo = vc * fine_crse_ghost<T, ND, false>(t, b, f, ijk, src, hxe);
       } else {
-        vc = cf_coef(c, t, b, d, fx, (T)0.75);
+        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
         vo = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, src, hxe);
       }
       hc[e] = vc;
@@ -1191,10 +1180,10 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * 2.0f;
       } else if (ty == 2) {
-        vc = cf_coef(c, t, b, d, fx, 1.5f);
+        vc = cf_face<float, 3>(c, t, b, f, ijk, fx, 1.5f);
         vo = vc * fine_crse_ghost<float, 3, false>(t, b, f, ijk, src, e);
       } else {
-        vc = cf_coef(c, t, b, d, fx, 0.75f);
+        vc = cf_face<float, 3>(c, t, b, f, ijk, fx, 0.75f);
         vo = crse_fine_sum<float, 3, false>(t, c, b, f, ijk, src, e);
       }
       sh.hc[f][m] = vc;
@@ -1337,10 +1326,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_rbgs_bulk(Topo t, Coef<T> c, Bl
     } else if (ty == 1) {
       if (t.bc_type[b * 6 + f] != kBCNeumann) vc = c.tff[d][fb + fx] * (T)2.0;
     } else if (ty == 2) {
-      vc = vk = cf_coef(c, t, b, d, fx, (T)1.5);
+      vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
       vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
     } else {
-      vc = cf_coef(c, t, b, d, fx, (T)0.75);
+      vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
       vk = (T)1;
       vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
     }
@@ -1490,10 +1479,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_rbgs_stream(Topo t, Coef<
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = c.tff[d][fb + fx] * (T)2.0;
       } else if (ty == 2) {
-        vc = vk = cf_coef(c, t, b, d, fx, (T)1.5);
+        vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
         vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
       } else {
-        vc = cf_coef(c, t, b, d, fx, (T)0.75);
+        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
         vk = (T)1;
         vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
       }
@@ -1698,10 +1687,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        vc = vk = cf_coef(c, t, b, d, fx, (T)1.5);
+        vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
         vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
       } else {  // not at the finest level of a tower
-        vc = cf_coef(c, t, b, d, fx, (T)0.75);
+        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
         vk = (T)1;
         vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
       }
@@ -1769,7 +1758,7 @@ void launch_prolong_red(const Topo &t, const Coef<T> &c, const BlockList &L, T *
   if (L.n == 0) return;
   if (X.n > 0 && !X.hx) return;  // the extra sweep reads its blocks through halo descriptors
   if constexpr (sizeof(T) == 4) {
-    if (form == 1 && t.ndim == 2 && t.nb == 16 && L.hx) {
+    if (form == 1 && t.ndim == 2 && t.nb == 16 && L.hx && c.cf) {
       const int g = std::min((L.n + X.n + 7) / 8, 152 * 64);
       launch_k(pdl, k_prolong_red_warp16<5>, g, kThreads, 0, s, t, c, L, phi, rhs, guard, X);
       return;
@@ -1832,7 +1821,7 @@ static void rbgs_nd(int variant, const Topo &t, const Coef<T> &c, const BlockLis
     case 12:
     case 13:
       if constexpr (ND == 2 && sizeof(T) == 4) {
-        if (t.nb == 16 && L.hx) {
+        if (t.nb == 16 && L.hx && c.cf) {
           const int g = std::min((L.n + 7) / 8, 152 * 64);
           if (variant == 11)
             launch_k(pdl, k_rbgs_warp16<4>, g, kThreads, 0, s, t, c, L, color, phi, rhs, guard);
@@ -1896,12 +1885,12 @@ void launch_bhgs(const Topo &t, const Coef<T> &c, const BlockList &L, int nsweep
   const int nhalf = t.ncell / 2;
   if (L.n == 0 || nhalf == 0) return;
   if constexpr (sizeof(T) == 4) {
-    if (t.ndim == 2 && t.nb == 16 && L.hx) {
+    if (t.ndim == 2 && t.nb == 16 && L.hx && c.cf) {
       const int warps = kH16Threads / 32, g = std::min((L.n + warps - 1) / warps, 152 * 64);
       launch_k(pdl, k_bhgs_warp16<4>, g, kH16Threads, 0, s, t, c, L, nsweep, src, dst, rhs, guard);
       return;
     }
-    if (t.ndim == 3 && (t.nb == 16 || t.nb == 8) && L.hx) {
+    if (t.ndim == 3 && (t.nb == 16 || t.nb == 8) && L.hx && c.cf) {
       const int g = std::min(L.n, L.pb ? kReducedGrid : 152 * 64);
       if (t.nb == 16)
         launch_k(pdl, k_bhgs_rows<16, 2>, g, 256, 0, s, t, c, L, nsweep, src, dst, rhs, guard);

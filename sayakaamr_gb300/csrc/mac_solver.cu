@@ -596,6 +596,9 @@ MacGpu::~MacGpu() {
   free_coef_lists();
   fr(d_uni64_);
   fr(d_uni32_);
+  fr(d_iso_);
+  fr(d_cf64_);
+  fr(d_cf32_);
   fr(d_cnt_);
   bottom_free();
   fr(d_phases_);

@@ -376,7 +376,11 @@ class MacGpu {
   char *d_active_mem_ = nullptr;       // the allocation behind these
   int *d_active_ = nullptr;            // per block: holds fluid
   ActiveList *d_act_lists_ = nullptr;  // every list and its reduced form
-  int n_act_lists_ = 0, n_act_ = 0;    // active blocks of the finest tower
+  int n_act_lists_ = 0;
+  int n_act_ = 0, n_iso_ = 0;  // active blocks of the finest tower, and those with one face coefficient
+  int *d_act_head_ = nullptr;
+  // the BiCGSTAB kernels read the FP32 V-cycle's output in place
+  bool vcycle_in_place() const;
   long act_version_ = -1;              // coefficient version of the reduced lists
   bool act_on_ = false;                // the solve walks the reduced lists
   Coef<float> c32_{};
@@ -389,6 +393,10 @@ class MacGpu {
   // the device solve's kernels read (c64_ with the records when enabled)
   double *d_uni64_ = nullptr;
   float *d_uni32_ = nullptr;
+  void build_cf();
+  double *d_cf64_ = nullptr;  // coarse/fine face coefficients (Coef::cf)
+  float *d_cf32_ = nullptr;
+  double *d_iso_ = nullptr;  // per block: T S where one coefficient holds on every face, else 0
   Coef<double> cd64_{};
   void build_uniform();
   void bind_uniform();
@@ -426,7 +434,7 @@ class MacGpu {
   int kernels_per_iter_ = 0;
   int graph_coop_ = -1, graph_pdl_ = -1, graph_cc_ = -1, graph_var_ = -1, graph_nn_ = -1, graph_order_ = -1;
   int graph_smoother_ = -1, graph_inner_ = -1, graph_multi_ = -1, graph_uniform_ = -1, graph_pform_ = -1,
-      graph_vout_ = -1, graph_act_ = -1;
+      graph_vout_ = -1, graph_act_ = -1, graph_direct_ = -1;
   double graph_omega_ = -1.0;
   bool last_multi_ = false;  // the last device solve kept one state per problem
   Chunks chunks() const;

@@ -95,6 +95,16 @@ __device__ __forceinline__ T cf_coef(const Coef<T> &c, const Topo &t, int b, int
   return v;
 }
 
+// the same from the table when there is one: face f of cell ijk
+template <typename T, int ND>
+__device__ __forceinline__ T cf_face(const Coef<T> &c, const Topo &t, int b, int f, const int ijk[3], int fidx, T h) {
+  if (!c.cf) return cf_coef(c, t, b, f >> 1, fidx, h);
+  const int d = f >> 1;
+  const int m0 = d == 0 ? ijk[1] : ijk[0], m1 = d == 2 ? ijk[1] : ijk[2];
+  const int m = ND == 3 ? m0 + t.nb * m1 : m0;
+  return c.cf[((long)b * (2 * ND) + f) * (ND == 3 ? t.nb * t.nb : t.nb) + m];
+}
+
 // CRSE_FINE face: sum of the fine-side contributions T_f * phi_f over the
 // fine faces covering coarse face (d, s) of cell ijk of block b, in the
 // reference's RESTRICT_SUM order (lower transverse dimension fastest)
@@ -127,7 +137,7 @@ __device__ __forceinline__ T crse_fine_sum(const Topo &t, const Coef<T> &c, int 
       if (ND == 3) fi[tq[1]] = base[tq[1]] + a1;
       if (ND == 2) fi[2] = 0;
       const int fx = face_index(d, fi, fside, nb);
-      const T tf = cf_coef(c, t, F, d, fx, h15);
+      const T tf = cf_face<T, ND>(c, t, F, f ^ 1, fi, fx, h15);
       val += tf * fpint::cvt<T>(ld<CG>(&x[(long)F * t.ncell + encode(fi, nb)]));
     }
   }
@@ -327,11 +337,11 @@ __device__ __forceinline__ void smooth_cell_fast(const Topo &t, const Coef<T> &c
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) diag += (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        const T coef = cf_coef(c, t, b, d, fx, (T)1.5);
+        const T coef = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
         diag += coef;
         off = fma_t(coef, fine_crse_ghost<T, ND, CG>(t, b, f, ijk, phi, hx), off);
       } else {
-        diag += cf_coef(c, t, b, d, fx, (T)0.75);
+        diag += cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
         off += crse_fine_sum<T, ND, CG>(t, c, b, f, ijk, phi, hx);
       }
     }
@@ -410,10 +420,10 @@ __device__ __forceinline__ void smooth_gather(const Topo &t, const Coef<T> &c, i
       o.kc[f] = (T)0;
       o.v[f] = (T)0;
     } else if (ty == 2) {
-      o.dp[f] = o.kc[f] = cf_coef(c, t, b, d, fx, (T)1.5);
+      o.dp[f] = o.kc[f] = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
       o.v[f] = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hx);
     } else {
-      o.dp[f] = cf_coef(c, t, b, d, fx, (T)0.75);
+      o.dp[f] = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
       o.kc[f] = (T)1;
       o.v[f] = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hx);
     }
