@@ -179,27 +179,30 @@ __global__ void k_restrict_cells(int nd, int nb, int ncell, const int *__restric
 // ls > 0, a face open when the cells on both sides are
 __global__ void k_ls_frac(int nd, int nb, int ncell, int nfb, const int *__restrict__ blocks, int n,
                           const double *__restrict__ ls, int ng, double *vf, Faces F) {
-  const int G = nb + 2 * ng;
+  // one CTA per block, one thread per point (i, j, k) of 0 .. nb: it owns the
+  // cell and the lower face of each direction there, so the index arithmetic
+  // and the point's own level-set test serve up to four values (a thread per
+  // value: 378 us for 13.75 M cells).  The sign test is on the bits (ls <= 0
+  // or a NaN's comparison false), off the FP64 pipe.
+  const int G = nb + 2 * ng, m = nb + 1, m2 = nd == 3 ? m : 1;
   const long gsz = nd == 3 ? (long)G * G * G : (long)G * G;
-  const int per = ncell + nd * nfb;
-  const long total = (long)n * per;
-  for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
-    const int k = (int)(it / per), r = (int)(it - (long)k * per);
+  auto solid = [](double v) {  // v <= 0
+    const long long u = __double_as_longlong(v);
+    return (u << 1) == 0 || (u < 0 && (unsigned long long)(u << 1) <= 0xffe0000000000000ull);
+  };
+  for (int k = blockIdx.x; k < n; k += gridDim.x) {
     const int b = blocks[k];
-    auto L = [&](int i, int j, int kz) {
-      return ls[(long)b * gsz + (i + ng) + (long)G * ((j + ng) + (long)G * (nd == 3 ? kz + ng : 0))];
-    };
-    if (r < ncell) {
-      const int i = r % nb, j = (r / nb) % nb, kz = nd == 3 ? r / (nb * nb) : 0;
-      vf[(long)b * ncell + r] = L(i, j, kz) <= 0 ? 0.0 : 1.0;
-      continue;
+    const double *lb = ls + (long)b * gsz + ng + (long)G * (ng + (nd == 3 ? (long)G * ng : 0));
+    for (int r = threadIdx.x; r < m * m * m2; r += blockDim.x) {
+      const int row = r / m, i = r - row * m, kz = row / m, j = row - kz * m;
+      const double *q = lb + i + (long)G * (j + (long)G * kz);
+      const bool ij = i < nb && j < nb, in2 = nd == 2 || kz < nb;
+      const bool s0 = solid(*q);
+      if (ij && in2) vf[(long)b * ncell + i + nb * (j + nb * kz)] = s0 ? 0.0 : 1.0;
+      if (j < nb && in2) F.f[0][(long)b * nfb + i + m * (j + nb * kz)] = s0 || solid(q[-1]) ? 0.0 : 1.0;
+      if (i < nb && in2) F.f[1][(long)b * nfb + i + nb * (j + m * kz)] = s0 || solid(q[-G]) ? 0.0 : 1.0;
+      if (nd == 3 && ij) F.f[2][(long)b * nfb + i + nb * (j + nb * kz)] = s0 || solid(q[-(long)G * G]) ? 0.0 : 1.0;
     }
-    const int q = r - ncell, d = q / nfb, fx = q - d * nfb;
-    const int e0 = nb + (d == 0), e1 = nb + (d == 1);
-    const int i = fx % e0, j = (fx / e0) % e1, kz = nd == 3 ? fx / (e0 * e1) : 0;
-    const int ii = d == 0, jj = d == 1, kk = d == 2;
-    const bool solid = L(i - ii, j - jj, kz - kk) <= 0 || L(i, j, kz) <= 0;
-    F.f[d][(long)b * nfb + fx] = solid ? 0.0 : 1.0;
   }
 }
 
@@ -354,9 +357,8 @@ void MacGpu::set_ib_frac_by_ls(const double *ls, int ng, bool dev) {
   }
   const DevTower &tw = towers_[finest_];
   Faces fa{{d_afrac_[0], d_afrac_[1], d_afrac_[2]}};
-  const long work = (long)tw.all.n * (ncell_ + nd * nfb_);
-  if (work)
-    k_ls_frac<<<cgrid(work), kCT, 0, stream_>>>(nd, tt_.nb, ncell_, nfb_, tw.all.blocks, tw.all.n, src, ng, d_vf_,
+  if (tw.all.n)
+    k_ls_frac<<<std::min(tw.all.n, 152 * 64), kCT, 0, stream_>>>(nd, tt_.nb, ncell_, nfb_, tw.all.blocks, tw.all.n, src, ng, d_vf_,
                                                 fa);
   coef_average((1 << nd) - 1, d_afrac_, d_vf_);
   coef_changed();

@@ -71,11 +71,13 @@ constexpr int kUni = 8;
 //   [kHXPar+f]     FINE_FINE face f of a block below level 1: the
 //                  neighbour's parent * 8 + its which_child, else -1
 //   [kHXPar+6]     the block's own parent * 8 + which_child, or -1
+//   [kHXLevel]     the block's level
 constexpr int kHX = 40;
 constexpr int kHXInfo = 6;
 constexpr int kHXBlock = 7;
 constexpr int kHXKids = 8;
 constexpr int kHXPar = 32;
+constexpr int kHXLevel = 39;
 
 // BiCGSTAB state kept on the device (FP64 scalars and control flags) by the
 // graph-captured solve of mac_fast.cu
@@ -242,13 +244,14 @@ void launch_prolong_red(const Topo &t, const Coef<T> &c, const BlockList &L, T *
 // block-hybrid Gauss-Seidel pass (Gauss-Seidel inside a block, Jacobi
 // between blocks): nsweep red-black sweeps of every block of L from src's
 // values into dst (src unchanged); L may hold several sublevels
+// top > 0 (where bhgs_prolongs): the blocks of level top start from their
+// parents' values (launch_prolong's), in src or next to it as neighbours
 template <typename T>
 void launch_bhgs(const Topo &t, const Coef<T> &c, const BlockList &L, int nsweep, const T *src, T *dst,
-                 const T *rhs, const int *guard, cudaStream_t s, bool pdl = false);
+                 const T *rhs, const int *guard, cudaStream_t s, bool pdl = false, int top = 0);
+// the pass over these blocks can prolong
 template <typename T>
-void launch_copy_blocks(const BlockList &L, int ncell, const T *src, T *dst, const int *guard, cudaStream_t s,
-                        bool pdl = false);
-
+bool bhgs_prolongs(const Topo &t, const Coef<T> &c, const BlockList &L);
 void launch_flux(const Topo &t, const Coef<double> &c, const BlockList &L, int dir,
                  const double *phi, double *flux, cudaStream_t s);
 

@@ -495,40 +495,43 @@ __global__ void k_set_cond_multi(cudaGraphConditionalHandle h, const FState *stc
 // faces that are not physical boundaries, with FMA: 7 FMA + 1 multiply per
 // cell instead of about 40 FP64 operations.  The result differs from the
 // reference's operator by rounding only (about 1e-16 relative).
+// (one CTA per block, so that a thread divides once for its full cells)
 template <int ND>
 __global__ void __launch_bounds__(kTPB) k_op_prep(Topo t, Coef<double> c, BlockList L, double *P, double *S) {
   using namespace stencil;
-  const int nb = t.nb, total = L.n * t.ncell;
-  for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < total; it += gridDim.x * blockDim.x) {
-    int p, ci, ijk[3];
-    split_cell<ND>(it, t, p, ci);
-    decode_fast<ND>(ci, t, ijk);
+  const int nb = t.nb;
+  for (int p = blockIdx.x; p < L.n; p += gridDim.x) {
     const int b = L.blocks[p];
     const uint16_t ft = L.ftypes[p];
-    const double dv = geom(c, b, 6);
-    double diag = c.alpha * dv;
-    for (int f = 0; f < 2 * ND; f++) {
-      const int d = f >> 1, s = f & 1;
-      const bool bnd = s ? ijk[d] == nb - 1 : ijk[d] == 0;
-      const int fx = face_index(d, ijk, s, nb);
-      const double tf = c.tff[d][(long)b * t.nfb + fx];
-      if (!bnd) {
-        diag += tf;
-        continue;
+    const double dv = geom(c, b, 6), full = 1.0 / (dv * 1.0);
+    for (int ci = threadIdx.x; ci < t.ncell; ci += blockDim.x) {
+      int ijk[3];
+      decode_fast<ND>(ci, t, ijk);
+      double diag = c.alpha * dv;
+      for (int f = 0; f < 2 * ND; f++) {
+        const int d = f >> 1, s = f & 1;
+        const bool bnd = s ? ijk[d] == nb - 1 : ijk[d] == 0;
+        const int fx = face_index(d, ijk, s, nb);
+        const double tf = c.tff[d][(long)b * t.nfb + fx];
+        if (!bnd) {
+          diag += tf;
+          continue;
+        }
+        const int ty = face_type_of(ft, f);
+        if (ty == 0)
+          diag += tf;
+        else if (ty == 1)
+          diag += t.bc_type[b * 6 + f] == kBCNeumann ? 0.0 : 2.0 * tf;
+        else
+          diag += cf_face<double, ND>(c, t, b, f, ijk, fx, ty == 2 ? 1.5 : 0.75);
       }
-      const int ty = face_type_of(ft, f);
-      if (ty == 0)
-        diag += tf;
-      else if (ty == 1)
-        diag += t.bc_type[b * 6 + f] == kBCNeumann ? 0.0 : 2.0 * tf;
-      else
-        diag += cf_coef(c, t, b, d, fx, ty == 2 ? 1.5 : 0.75);
+      const long q = (long)b * t.ncell + ci;
+      const double vfv = c.vf[q];
+      const bool one = __double_as_longlong(vfv) == __double_as_longlong(1.0);
+      const double sc = one ? full : (vfv > 0 ? 1.0 / (dv * vfv) : 0.0);
+      S[q] = sc;
+      P[q] = diag * sc;
     }
-    const long q = (long)b * t.ncell + ci;
-    const double vfv = c.vf[q];
-    const double sc = vfv > 0 ? 1.0 / (dv * vfv) : 0.0;
-    S[q] = sc;
-    P[q] = diag * sc;
   }
 }
 
@@ -578,7 +581,8 @@ __global__ void __launch_bounds__(kTPB) k_smooth_factors(Topo t, Coef<double> c,
 
 // Constant-coefficient block records (Coef::ut), one CTA per block: a block
 // qualifies when every face of direction d carries the same coefficient T_d
-// (boundary faces included) and every cell has vf = 1.  Its interior cells'
+// (boundary faces included) and every cell has vf = 1, compared as bits (off
+// the FP64 pipe).  Its interior cells'
 // factors are those k_op_prep and k_smooth_factors compute, in the same
 // order: diag = alpha*dv + T_0 + T_0 + T_1 + T_1 (+ T_2 + T_2).  The FP32
 // record holds the FP32 coefficients, equal throughout the block too.
@@ -593,9 +597,11 @@ __global__ void __launch_bounds__(kTPB) k_uniform(Topo t, Coef<double> c, Coef<f
     bool good = true;
     for (int d = 0; d < ND; d++) {
       const double t0 = c.tff[d][fb];
-      for (int i = threadIdx.x; i < t.nfb; i += blockDim.x) good = good && c.tff[d][fb + i] == t0;
+      for (int i = threadIdx.x; i < t.nfb; i += blockDim.x)
+        good = good && __double_as_longlong(c.tff[d][fb + i]) == __double_as_longlong(t0);
     }
-    for (int i = threadIdx.x; i < t.ncell; i += blockDim.x) good = good && c.vf[cb + i] == 1.0;
+    for (int i = threadIdx.x; i < t.ncell; i += blockDim.x)
+      good = good && __double_as_longlong(c.vf[cb + i]) == __double_as_longlong(1.0);
     if (!good) ok = 0;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -630,8 +636,9 @@ __global__ void __launch_bounds__(kTPB) k_uniform(Topo t, Coef<double> c, Coef<f
 
 // the coefficients of the faces at coarser and at refined neighbours
 // (Coef::cf), in the arithmetic of cf_coef
+// (the FP32 table from the FP64 arrays, each value rounded to T first)
 template <typename T, int ND>
-__global__ void __launch_bounds__(kTPB) k_cf_faces(Topo t, Coef<T> c, T *__restrict__ cf) {
+__global__ void __launch_bounds__(kTPB) k_cf_faces(Topo t, Coef<double> c, T *__restrict__ cf) {
   using namespace stencil;
   const int nface = ND == 3 ? t.nb * t.nb : t.nb;
   const long total = (long)t.nblocks * 2 * ND * nface;
@@ -643,7 +650,10 @@ __global__ void __launch_bounds__(kTPB) k_cf_faces(Topo t, Coef<T> c, T *__restr
     const int d = f >> 1, s = f & 1, m0 = ND == 3 ? m % t.nb : m, m1 = ND == 3 ? m / t.nb : 0;
     const int ijk[3] = {d == 0 ? (s ? t.nb - 1 : 0) : m0, d == 0 ? m0 : (d == 1 ? (s ? t.nb - 1 : 0) : m1),
                         ND == 3 ? (d == 2 ? (s ? t.nb - 1 : 0) : m1) : 0};
-    cf[it] = cf_coef(c, t, b, d, face_index(d, ijk, s, t.nb), coarser ? (T)1.5 : (T)0.75);
+    const long fx = (long)b * t.nfb + face_index(d, ijk, s, t.nb);
+    T v = (T)c.beta * (T)geom(c, b, 3 + d) / ((T)geom(c, b, d) * (coarser ? (T)1.5 : (T)0.75));
+    v = v * (T)c.bcoef[d][fx];
+    cf[it] = v * (T)c.afrac[d][fx];
   }
 }
 
@@ -691,7 +701,7 @@ __device__ __forceinline__ double op_offdiag(const Topo &t, const Coef<double> &
 
 // operator fused with its dot products:
 // MODE 0: y = A x, rhat.y (EpiAlpha) ; MODE 1: y = A x, y.w, y.y (EpiOmega) ;
-// MODE 2: y = w - A x (0 where vf = 0), |y|, y.y (EpiInit) ;
+// MODE 2: y = y2 = w - A x (0 where vf = 0), |y|, y.y (EpiInit) ;
 // MODE 3: only while verifying: y = y2 = w - A x, |y|, y.y (EpiVerify)
 // The operator in double-float (mac_df.cuh) for an FP32 input x: the sum of
 // T * x over the faces, then P * x - S * sum, with T, P and S as double-float
@@ -779,7 +789,7 @@ __global__ void __launch_bounds__(kTPB, 4) k_op_red(Topo t, Coef<double> c, Bloc
     }
     if constexpr (MODE >= 2) yv = fpint::positive(u ? u[5] : S[q]) ? w[q] - yv : 0.0;
     y[q] = yv;
-    if (MODE == 3) y2[q] = yv;
+    if (MODE >= 2) y2[q] = yv;
     if (MODE == 0) acc[0] = __fma_rn(w[q], yv, acc[0]);
     if (MODE == 1) {
       acc[0] = __fma_rn(yv, w[q], acc[0]);
@@ -896,46 +906,52 @@ __global__ void __launch_bounds__(kTPB, 4) k_op_rows(Topo t, Coef<double> c, Blo
     if (!done) {
       const long fb = (long)b * t.nfb;
       const double *u = uniform_of(c, b);
-      // factor and value of a face at a coarser or refined neighbour
-      auto cross = [&](int f, int n, double &k, double &v) {
-        const int at[3] = {ijk[0] + n, ijk[1], ijk[2]};
-        if (face_type_of(ft, f) == 2) {
-          k = cf_face<double, ND>(c, t, b, f, at, 0, 1.5);
-          v = fpint::widen(fine_crse_ghost<float, ND, false>(t, b, f, at, x, e));
-        } else {
-          k = 1.0;
-          v = crse_fine_sum<double, ND, false>(t, c, b, f, at, x, e);
+      // factors and values of cells n0 .. n1-1 at face f toward a coarser or
+      // refined neighbour; the cells' loads are independent of each other
+      auto cross = [&](int f, auto n0, auto n1, double *k, double *v) {
+        const bool coarser = face_type_of(ft, f) == 2;
+#pragma unroll
+        for (int n = decltype(n0)::value; n < decltype(n1)::value; n++) {
+          const int at[3] = {ijk[0] + n, ijk[1], ijk[2]};
+          const double own = cf_face<double, ND>(c, t, b, f, at, 0, 1.5);
+          v[n - decltype(n0)::value] = coarser ? fpint::widen(fine_crse_ghost<float, ND, false>(t, b, f, at, x, e))
+                                               : crse_fine_sum<double, ND, false>(t, c, b, f, at, x, e);
+          k[n - decltype(n0)::value] = coarser ? own : 1.0;
         }
       };
+      constexpr std::integral_constant<int, 0> c0{};
+      constexpr std::integral_constant<int, 1> c1{};
+      constexpr std::integral_constant<int, 3> c3{};
+      constexpr std::integral_constant<int, 4> c4{};
       const int row = ijk[1] + nb * ijk[2];
       const double *tx = c.tff[0] + fb + (nb + 1) * row + ijk[0];
-      double off[4], xw[6];
+      double off[4], xw[6], tk[5];
 #pragma unroll
       for (int n = 0; n < 6; n++) xw[n] = fpint::widen(xv[n]);
-      double tl = u ? u[0] : tx[0];
-      if (cf && ijk[0] == 0 && face_type_of(ft, 0) > 1) cross(0, 0, tl, xw[0]);
 #pragma unroll
-      for (int n = 0; n < 4; n++) {
-        const double ti = u ? u[0] : tx[n + 1];
-        double tr = ti;
-        if (n == 3 && cf && ijk[0] + 4 == nb && face_type_of(ft, 1) > 1) cross(1, 3, tr, xw[5]);
-        off[n] = __fma_rn(tr, xw[n + 2], __fma_rn(tl, xw[n], 0.0));
-        tl = ti;
-      }
+      for (int n = 0; n < 5; n++) tk[n] = u ? u[0] : tx[n];
+      double tr = tk[4];
+      if (cf && ijk[0] == 0 && face_type_of(ft, 0) > 1) cross(0, c0, c1, &tk[0], &xw[0]);
+      if (cf && ijk[0] + 4 == nb && face_type_of(ft, 1) > 1) cross(1, c3, c4, &tr, &xw[5]);
+#pragma unroll
+      for (int n = 0; n < 4; n++)
+        off[n] = __fma_rn(n == 3 ? tr : tk[n + 1], xw[n + 2], __fma_rn(tk[n], xw[n], 0.0));
 #pragma unroll
       for (int f = 2; f < 2 * ND; f++) {
         const int d = f >> 1, s = f & 1;
         const long fx = d == 1 ? ijk[0] + nb * (ijk[1] + s + (nb + 1) * ijk[2]) : ci + s * nb * nb;
         const double *tf = c.tff[d] + fb + fx;
         const float4 q = r[f - 2];
-        const float qv[4] = {q.x, q.y, q.z, q.w};
-        const bool over = cf && (s ? ijk[d] == nb - 1 : ijk[d] == 0) && face_type_of(ft, f) > 1;
+        double k[4], v[4];
+        if (cf && (s ? ijk[d] == nb - 1 : ijk[d] == 0) && face_type_of(ft, f) > 1) {
+          cross(f, c0, c4, k, v);
+        } else {
+          v[0] = fpint::widen(q.x), v[1] = fpint::widen(q.y), v[2] = fpint::widen(q.z), v[3] = fpint::widen(q.w);
 #pragma unroll
-        for (int n = 0; n < 4; n++) {
-          double k = u ? u[d] : tf[n], v = fpint::widen(qv[n]);
-          if (over) cross(f, n, k, v);
-          off[n] = __fma_rn(k, v, off[n]);
+          for (int n = 0; n < 4; n++) k[n] = u ? u[d] : tf[n];
         }
+#pragma unroll
+        for (int n = 0; n < 4; n++) off[n] = __fma_rn(k[n], v[n], off[n]);
       }
 #pragma unroll
       for (int n = 0; n < 4; n++) yv[n] = __fma_rn(xw[n + 1], P[cb + ci + n], -off[n] * S[cb + ci + n]);
@@ -1058,7 +1074,7 @@ __global__ void k_split_df(long n, const double *src, float2 *dst) {
 
 __global__ void k_to_f32(long n, const double *src, float *dst) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    dst[i] = (float)src[i];
+    dst[i] = fpint::narrow(src[i]);  // a hardware conversion is an FP64-pipe operation
 }
 
 }  // namespace
@@ -1248,14 +1264,25 @@ void MacGpu::build_op_factors() {
   const BlockList TL = tower_list(finest_);
   const long w = (long)TL.n * ncell_;
   if (w == 0) return;
+  Coef<double> cc = c64_;
+  cc.cf = d_cf64_;
   if (tt_.ndim == 2)
-    k_op_prep<2><<<ew_grid(w), kTPB, 0, stream_>>>(topo_, c64_, TL, d_opP_, d_opS_);
+    k_op_prep<2><<<std::min(TL.n, 152 * 64), kTPB, 0, stream_>>>(topo_, cc, TL, d_opP_, d_opS_);
   else
-    k_op_prep<3><<<ew_grid(w), kTPB, 0, stream_>>>(topo_, c64_, TL, d_opP_, d_opS_);
-  const long nc = (long)tt_.num_blocks * ncell_;
+    k_op_prep<3><<<std::min(TL.n, 152 * 64), kTPB, 0, stream_>>>(topo_, cc, TL, d_opP_, d_opS_);
+  CK(cudaGetLastError());
+}
+
+// double-float pairs of the operator factors and block records, for the
+// double-float operator only (params.vcycle_out 1)
+void MacGpu::ensure_df_factors() {
+  if (df_version_ == coef_version_) return;
+  const long nc = (long)tt_.num_blocks * ncell_, nu = (long)tt_.num_blocks * kUni;
   k_split_df<<<ew_grid(nc), kTPB, 0, stream_>>>(nc, d_opP_, d_opP2_);
   k_split_df<<<ew_grid(nc), kTPB, 0, stream_>>>(nc, d_opS_, d_opS2_);
+  k_split_df<<<ew_grid(nu), kTPB, 0, stream_>>>(nu, d_uni64_, d_uni2_);
   CK(cudaGetLastError());
+  df_version_ = coef_version_;
 }
 
 // the coarse/fine face tables from the current coefficients
@@ -1264,7 +1291,7 @@ void MacGpu::build_cf() {
   if (n == 0) return;
   auto go = [&](auto k64, auto k32) {
     k64<<<ew_grid(n), kTPB, 0, stream_>>>(topo_, c64_, d_cf64_);
-    k32<<<ew_grid(n), kTPB, 0, stream_>>>(topo_, c32_, d_cf32_);
+    k32<<<ew_grid(n), kTPB, 0, stream_>>>(topo_, c64_, d_cf32_);
   };
   if (tt_.ndim == 2)
     go(k_cf_faces<double, 2>, k_cf_faces<float, 2>);
@@ -1283,8 +1310,6 @@ void MacGpu::build_uniform() {
     k_uniform<2><<<grid, kTPB, 0, stream_>>>(topo_, c64_, c32_, d_uni64_, d_uni32_);
   else
     k_uniform<3><<<grid, kTPB, 0, stream_>>>(topo_, c64_, c32_, d_uni64_, d_uni32_);
-  const long nu = (long)nbk * kUni;
-  k_split_df<<<ew_grid(nu), kTPB, 0, stream_>>>(nu, d_uni64_, d_uni2_);
   k_iso<<<std::min((nbk + kTPB - 1) / kTPB, 152 * 8), kTPB, 0, stream_>>>(nbk, tt_.ndim, alpha_, d_uni64_, d_iso_);
   CK(cudaGetLastError());
 }
@@ -1308,13 +1333,24 @@ void MacGpu::refresh_fp32() {
   const long nc = (long)nbk * ncell_, nf = (long)nbk * nfb_;
   for (int d = 0; d < nd; d++) {
     k_to_f32<<<ew_grid(nf), kTPB, 0, stream_>>>(nf, d_tff_[d], d_tff32_[d]);
-    k_to_f32<<<ew_grid(nf), kTPB, 0, stream_>>>(nf, d_bcoef_[d], d_bcoef32_[d]);
-    k_to_f32<<<ew_grid(nf), kTPB, 0, stream_>>>(nf, d_afrac_[d], d_afrac32_[d]);
   }
   k_to_f32<<<ew_grid(nc), kTPB, 0, stream_>>>(nc, d_vf_, d_vf32_);
   k_to_f32<<<ew_grid((long)nbk * 8), kTPB, 0, stream_>>>((long)nbk * 8, d_geom_, d_geom32_);
   c32_.alpha = (float)alpha_;
   c32_.beta = (float)beta_;
+}
+
+// FP32 copies of B and the area fractions, which only the learned correction
+// reads (the V-cycle takes its coarse/fine coefficients from Coef::cf)
+void MacGpu::ensure_fp32_faces() {
+  if (faces32_version_ == coef_version_) return;
+  const long nf = (long)tt_.num_blocks * nfb_;
+  for (int d = 0; d < tt_.ndim; d++) {
+    k_to_f32<<<ew_grid(nf), kTPB, 0, stream_>>>(nf, d_bcoef_[d], d_bcoef32_[d]);
+    k_to_f32<<<ew_grid(nf), kTPB, 0, stream_>>>(nf, d_afrac_[d], d_afrac32_[d]);
+  }
+  CK(cudaGetLastError());
+  faces32_version_ = coef_version_;
 }
 
 // Level of the dense bottom solve.  Level 1 always works (it is uniform and
@@ -1685,20 +1721,30 @@ void MacGpu::vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *o
     if (l - 1 >= tt_.max_level || levels_[l - 1].n == 0 || levels_[l].n == 0) continue;
     launch_restrict<T>(topo_, c, nonleaf_list(l - 1), resid, guard, stream_, prm_.pdl != 0);
   }
-  bottom_launch<T>(resid, corr);
+  // Block-hybrid passes read one correction vector and write the other.  A
+  // tower holds every block that the next one reads (its leaves and the
+  // parents of the next level), so the vectors simply change places from
+  // tower to tower, and the bottom starts in the one from which the last pass
+  // of the finest tower ends in corr.
+  T *main = corr, *other = prm_.smoother == 1 ? corr_alt<T>() : corr;
+  if (prm_.smoother == 1) {
+    int passes = 0;
+    for (int l = LB + 1; l <= L; l++) passes += levels_[l].n > 0 ? prm_.n_post : 0;
+    if (passes & 1) std::swap(main, other);
+  }
+  bottom_launch<T>(resid, main);
   for (int l = LB + 1; l <= L; l++) {
     if (levels_[l].n == 0) continue;
     if (prm_.smoother == 1) {
-      // block-hybrid passes over every sublevel of tower l at once, reading
-      // one correction vector and writing the other
-      launch_prolong<T>(topo_, c, level_list(l), corr, guard, stream_, prm_.pdl != 0);
+      // over every sublevel of tower l at once; the first pass prolongs
       const BlockList TL = smooth_list(l);
-      T *a = corr, *b = corr_alt<T>();
+      const bool fused = prm_.n_post > 0 && bhgs_prolongs<T>(topo_, c, TL) && sublevel_list(l, l).n == levels_[l].n;
+      if (!fused) launch_prolong<T>(topo_, c, level_list(l), main, guard, stream_, prm_.pdl != 0);
       for (int s = 0; s < prm_.n_post; s++) {
-        launch_bhgs<T>(topo_, c, TL, prm_.inner_sweeps, a, b, resid, guard, stream_, prm_.pdl != 0);
-        std::swap(a, b);
+        launch_bhgs<T>(topo_, c, TL, prm_.inner_sweeps, main, other, resid, guard, stream_, prm_.pdl != 0,
+                       fused && s == 0 ? l : 0);
+        std::swap(main, other);
       }
-      if (a != corr) launch_copy_blocks<T>(TL, ncell_, a, corr, guard, stream_, prm_.pdl != 0);
       continue;
     }
     // the level's own sublevel of tower l holds every block of the level, so
@@ -2054,22 +2100,17 @@ int MacGpu::enqueue_solve() {
   k_pro_copy<<<ew_grid(w), kTPB, 0, stream_>>>(TL, ncell_, vec_[kSOL], vec_[kX0], vec_[kX]);
   double *PART = mp ? d_cpart_ : d_part_;
   unsigned *CNT = mp ? d_ccnt_ : d_cnt_;
-  if (tt_.ndim == 2) {
-    if (mp)
-      k_op_red<2, 2, double, true><<<gr, kTPB, 0, stream_>>>(topo_, cd64_, TL, ch, vec_[kX0], vec_[kR], vec_[kRHS],
-                                                             d_opP_, d_opS_, ST, PART, CNT);
-    else
-      k_op_red<2, 2, double, false><<<gr, kTPB, 0, stream_>>>(topo_, cd64_, TL, ch, vec_[kX0], vec_[kR], vec_[kRHS],
-                                                              d_opP_, d_opS_, ST, PART, CNT);
-  } else {
-    if (mp)
-      k_op_red<3, 2, double, true><<<gr, kTPB, 0, stream_>>>(topo_, cd64_, TL, ch, vec_[kX0], vec_[kR], vec_[kRHS],
-                                                             d_opP_, d_opS_, ST, PART, CNT);
-    else
-      k_op_red<3, 2, double, false><<<gr, kTPB, 0, stream_>>>(topo_, cd64_, TL, ch, vec_[kX0], vec_[kR], vec_[kRHS],
-                                                              d_opP_, d_opS_, ST, PART, CNT);
-  }
-  vcopy(TL, vec_[kRHAT], vec_[kR]);
+  solve_lists_ = true;  // r and rhat are read on the blocks the solve walks
+  const BlockList RL = mp ? TL : tower_list(L);
+  solve_lists_ = false;
+  auto resid = [&](auto kern) {
+    kern<<<gr, kTPB, 0, stream_>>>(topo_, cd64_, RL, ch, vec_[kX0], vec_[kR], vec_[kRHS], d_opP_, d_opS_, ST, PART,
+                                   CNT, vec_[kRHAT], nullptr, nullptr, nullptr);
+  };
+  if (tt_.ndim == 2)
+    mp ? resid(k_op_red<2, 2, double, true>) : resid(k_op_red<2, 2, double, false>);
+  else
+    mp ? resid(k_op_red<3, 2, double, true>) : resid(k_op_red<3, 2, double, false>);
   if (mp) k_set_cond_multi<<<1, 256, 0, stream_>>>(0, d_stc_, ncomp_, d_st_);
   if (prm_.max_iter > 0) {
     if (prm_.graph) {
@@ -2147,7 +2188,11 @@ int MacGpu::prepare_device() {
   // correction only: an FP32 solve does not build them
   if (prm_.precision == 0 || learned_active()) ensure_smooth_factors();
   tune_smoother(prm_.precision);
-  if (learned_active()) learned_prepare();
+  if (prm_.vcycle_out == 1) ensure_df_factors();
+  if (learned_active()) {
+    ensure_fp32_faces();
+    learned_prepare();
+  }
   if (!err_.empty()) return -1;
   if (prm_.vcycle_kernel && (program_npost_ != prm_.n_post || program_order_ != prm_.sublevel_order ||
                              program_bot_ != bot_level_))
@@ -2309,6 +2354,7 @@ int MacGpu::device_kernel_compact(int which, int L, int variant, const double *i
     CKR_(cudaGetLastError(), 2);
     CKR_(cudaMemcpyAsync(out, vec_[kV], n * sizeof(double), cudaMemcpyDeviceToHost, stream_), 2);
   } else if (which == 3) {
+    ensure_df_factors();
     // the operator of the BiCGSTAB iteration on an FP32 input (double-float
     // path): in rounded to FP32, then y = A x on the finest tower
     const BlockList TL = tower_list(finest_);

@@ -178,7 +178,9 @@ struct W16Halo {
 // neighbour's parent).  The gathers of mac_stencil.cuh for 2D blocks of 16,
 // without their arrays: the direction differs from lane to lane, and arrays
 // indexed by it would live in local memory.
-template <bool PROLONG>
+// (FINE: the finer blocks behind a refined face hold prolonged values too,
+// those of this block's neighbour there, their parent)
+template <bool PROLONG, bool FINE = false>
 __device__ __forceinline__ void w16_halo_slot(const Topo &t, const Coef<float> &c, const int *e, int b, int info,
                                               const float *u, int f, int m, const float *__restrict__ phi, float &dp,
                                               float &k, float &v) {
@@ -214,7 +216,11 @@ __device__ __forceinline__ void w16_halo_slot(const Topo &t, const Coef<float> &
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const float tf = c.cf[((long)F * 4 + (f ^ 1)) * NB + t0 + q];
-      v += tf * phi[(long)F * NC + (d ? t0 + q + NB * across : across + NB * (t0 + q))];
+      const long fc = (long)F * NC + (d ? t0 + q + NB * across : across + NB * (t0 + q));
+      if constexpr (FINE)
+        v += tf * (c.vf[fc] > 0 ? phi[(long)t.neighbor[b * 6 + f] * NC + (d ? m + NB * across : across + NB * m)] : 0.f);
+      else
+        v += tf * phi[fc];
     }
   }
 }
@@ -369,8 +375,11 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_warp16(Topo t, Coef<flo
 // two CTA barriers per sweep that the CTA form has.  The values and operations
 // of k_bhgs in the same order: a frozen neighbour's part enters as 1 * (T
 // value), its rounded product.  Bound by the latency of one round of loads.
+// TOP: src holds no values yet for the blocks of level `top`, which start from
+// their parents' (k_prolong's values).
+template <bool TOP>
 __device__ __forceinline__ void h16_pass(const Topo &t, const Coef<float> &c, const BlockList &L, const int *e,
-                                         int nsweep, const float *__restrict__ src, float *__restrict__ dst,
+                                         int top, int nsweep, const float *__restrict__ src, float *__restrict__ dst,
                                          const float *__restrict__ rhs, int lane, W16Halo &sh) {
   constexpr int NB = 16, NC = 256;
   const int j = lane >> 1, hh = lane & 1, c0 = 8 * hh, par = j & 1;  // red cells: columns 2q + par
@@ -379,14 +388,31 @@ __device__ __forceinline__ void h16_pass(const Topo &t, const Coef<float> &c, co
   const long cb = (long)b * NC, fb = (long)b * t.nfb;
   const float *u = uniform_of(c, b);
   const float dv = geom(c, b, 6);
-  const float4 *s4 = reinterpret_cast<const float4 *>(src + cb + j * NB + c0);
-  const float4 p0 = s4[0], p1 = s4[1];
+  const int below = TOP ? top - e[kHXLevel] : -1;  // 0: the block itself is prolonged, 1: the finer ones at its faces
+  float4 p0, p1;
+  if (TOP && below == 0) {
+    const int pw = e[kHXPar + 6], wc = pw & 7;
+    const float4 q4 = *reinterpret_cast<const float4 *>(src + (long)(pw >> 3) * NC +
+                                                         (8 * ((wc >> 1) & 1) + (j >> 1)) * NB + 8 * (wc & 1) + 4 * hh);
+    p0 = make_float4(q4.x, q4.x, q4.y, q4.y);
+    p1 = make_float4(q4.z, q4.z, q4.w, q4.w);
+  } else {
+    const float4 *s4 = reinterpret_cast<const float4 *>(src + cb + j * NB + c0);
+    p0 = s4[0], p1 = s4[1];
+  }
   const float4 *rsrc = reinterpret_cast<const float4 *>(rhs + cb + j * NB + c0);
   const float4 r0 = rsrc[0], r1 = rsrc[1];
   float hdp[2], hk[2], hv[2];
 #pragma unroll
-  for (int h = 0; h < 2; h++)
-    w16_halo_slot<false>(t, c, e, b, ib.x, u, (lane >> 4) + 2 * h, lane & 15, src, hdp[h], hk[h], hv[h]);
+  for (int h = 0; h < 2; h++) {
+    const int f = (lane >> 4) + 2 * h, m = lane & 15;
+    if (TOP && below == 0)
+      w16_halo_slot<true>(t, c, e, b, ib.x, u, f, m, src, hdp[h], hk[h], hv[h]);
+    else if (TOP && below == 1)
+      w16_halo_slot<false, true>(t, c, e, b, ib.x, u, f, m, src, hdp[h], hk[h], hv[h]);
+    else
+      w16_halo_slot<false>(t, c, e, b, ib.x, u, f, m, src, hdp[h], hk[h], hv[h]);
+  }
   // v[color][q]; the face coefficients, diagonal, rhs * dv and vf of the cell
   float v[2][4], kl[2][4], kr[2][4], kd[2][4], ku[2][4], diag[2][4], rd[2][4], vf[2][4];
   const float pv[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
@@ -425,6 +451,10 @@ __device__ __forceinline__ void h16_pass(const Topo &t, const Coef<float> &c, co
       ku[1][q] = yd[2 * q + 1 - par + NB];
       vf[0][q] = par ? wv[2 * q + 1] : wv[2 * q];
       vf[1][q] = par ? wv[2 * q] : wv[2 * q + 1];
+      if (TOP && below == 0) {
+        if (!(vf[0][q] > 0.f)) v[0][q] = 0.f;
+        if (!(vf[1][q] > 0.f)) v[1][q] = 0.f;
+      }
     }
   }
   if (L.stc && block_off(L, b)) return;  // a finished problem; uniform over the warp
@@ -492,18 +522,19 @@ __device__ __forceinline__ void h16_pass(const Topo &t, const Coef<float> &c, co
 }
 
 constexpr int kH16Threads = 128;
-template <int MINB>
+template <int MINB, bool TOP>
 __global__ void __launch_bounds__(kH16Threads, MINB) k_bhgs_warp16(Topo t, Coef<float> c, BlockList L, int nsweep,
                                                                    const float *__restrict__ src,
                                                                    float *__restrict__ dst,
-                                                                   const float *__restrict__ rhs, const int *guard) {
+                                                                   const float *__restrict__ rhs, const int *guard,
+                                                                   int top) {
   __shared__ W16Halo sh[kH16Threads / 32];
   pdl_enter();
   if (guard && *guard) return;
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const ListRange lr = list_range(L);
   for (int p = lr.a + blockIdx.x * warps + (threadIdx.x >> 5); p < lr.b; p += gridDim.x * warps)
-    h16_pass(t, c, L, L.hx + (long)p * kHX, nsweep, src, dst, rhs, lane, sh[threadIdx.x >> 5]);
+    h16_pass<TOP>(t, c, L, L.hx + (long)p * kHX, top, nsweep, src, dst, rhs, lane, sh[threadIdx.x >> 5]);
 }
 
 // ---------------------------------------------------------------------------
@@ -543,20 +574,22 @@ __global__ void __launch_bounds__(kThreads) k_prolong(Topo t, Coef<T> c, BlockLi
 template <typename T>
 __global__ void k_face_coef(Topo t, const double *geom64, const T *b0, const T *b1, const T *b2, const T *a0,
                             const T *a1, const T *a2, double beta, T *t0, T *t1, T *t2) {
-  const long per = (long)t.nfb;
-  const long total = (long)t.nblocks * per * t.ndim;
-  for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
-    const int d = (int)(it / ((long)t.nblocks * per));
-    const long r = it - (long)d * t.nblocks * per;
-    const int b = (int)(r / per);
+  // one CTA per block and direction: a thread divides once for all its faces
+  // (a division per face is about 15 operations of the FP64 pipe: 13.75 M
+  // cells took 1050 us)
+  for (long it = blockIdx.x; it < (long)t.nblocks * t.ndim; it += gridDim.x) {
+    const int b = (int)(it / t.ndim), d = (int)(it - (long)b * t.ndim);
     const T *B = d == 0 ? b0 : (d == 1 ? b1 : b2);
     const T *A = d == 0 ? a0 : (d == 1 ? a1 : a2);
     T *O = d == 0 ? t0 : (d == 1 ? t1 : t2);
     const T ds = (T)geom64[b * 8 + 3 + d], dx = (T)geom64[b * 8 + d];
-    T v = (T)beta * ds / dx;
-    v = v * B[r];
-    v = v * A[r];
-    O[r] = v;
+    const T q = (T)beta * ds / dx;
+    const long fb = (long)b * t.nfb;
+    for (int i = threadIdx.x; i < t.nfb; i += blockDim.x) {
+      T v = q * B[fb + i];
+      v = v * A[fb + i];
+      O[fb + i] = v;
+    }
   }
 }
 
@@ -707,7 +740,7 @@ void launch_face_coef(const Topo &t, const double *geom64, const T *bcoef[3], co
                       T *tff[3], cudaStream_t s) {
   const long work = (long)t.nblocks * t.nfb * t.ndim;
   if (work == 0) return;
-  k_face_coef<T><<<grid_for(work), kThreads, 0, s>>>(t, geom64, bcoef[0], bcoef[1], bcoef[2], afrac[0], afrac[1],
+  k_face_coef<T><<<(int)std::min<long>((long)t.nblocks * t.ndim, 152 * 64), std::min(kThreads, (t.nfb + 31) / 32 * 32), 0, s>>>(t, geom64, bcoef[0], bcoef[1], bcoef[2], afrac[0], afrac[1],
                                                      afrac[2], beta, tff[0], tff[1], tff[2]);
 }
 
@@ -1134,10 +1167,11 @@ __device__ __forceinline__ void h3_sweeps(const Topo &t, const Coef<float> &c, i
   }
 }
 
-template <int NB, int MINB>
+// TOP: as in h16_pass
+template <int NB, int MINB, bool TOP>
 __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> c, BlockList L, int nsweep,
                                                             const float *__restrict__ src, float *__restrict__ dst,
-                                                            const float *__restrict__ rhs, const int *guard) {
+                                                            const float *__restrict__ rhs, const int *guard, int top) {
   __shared__ H3<NB> sh;
   pdl_enter();
   if (guard && *guard) return;
@@ -1151,12 +1185,30 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
     const uint16_t ft = (uint16_t)(ib.x & 0xffff);
     const long cb = (long)b * NC, fb = (long)b * t.nfb;
     const float *u = uniform_of(c, b);
+    const int below = TOP ? top - e[kHXLevel] : -1;  // 0: the block itself is prolonged, 1: the finer ones at its faces
     // the tile, four cells of a row per step: two of each colour
     const float4 *s4 = reinterpret_cast<const float4 *>(src + cb);
 #pragma unroll
     for (int n = threadIdx.x; n < NC / 4; n += NT) {
-      const float4 w = s4[n];
       const int row = n / (NB / 4), q = 2 * (n % (NB / 4)), j = row % NB, k = row / NB, pr = (j + k) & 1;
+      float4 w;
+      if (TOP && below == 0) {
+        const int pw = e[kHXPar + 6], wc = pw & 7;
+        constexpr int hb = NB / 2;
+        const float2 v2 = *reinterpret_cast<const float2 *>(src + (long)(pw >> 3) * NC + hb * (wc & 1) + q +
+                                                             NB * (hb * ((wc >> 1) & 1) + (j >> 1) +
+                                                                   NB * (hb * ((wc >> 2) & 1) + (k >> 1))));
+        w = make_float4(v2.x, v2.x, v2.y, v2.y);
+        if (!u) {
+          const float4 m4 = *reinterpret_cast<const float4 *>(c.vf + cb + 4 * n);
+          if (!(m4.x > 0.f)) w.x = 0.f;
+          if (!(m4.y > 0.f)) w.y = 0.f;
+          if (!(m4.z > 0.f)) w.z = 0.f;
+          if (!(m4.w > 0.f)) w.w = 0.f;
+        }
+      } else {
+        w = s4[n];
+      }
       const int at = H3<NB>::row(j, k);
       float2 *r2 = reinterpret_cast<float2 *>(&sh.tile[0][q >> 2][at]) + ((q >> 1) & 1);
       float2 *b2 = reinterpret_cast<float2 *>(&sh.tile[1][q >> 2][at]) + ((q >> 1) & 1);
@@ -1176,7 +1228,13 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
       float vc = 0.f, vo = 0.f;
       if (ty == 0) {
         vc = u ? u[d] : c.tff[d][fb + fx];
-        vo = vc * same_level_ghost<float, false>(t, b, f, ijk, src, e);
+        if (TOP && below == 0) {
+          const int ni[3] = {d == 0 ? NB - 1 - ijk[0] : ijk[0], d == 1 ? NB - 1 - ijk[1] : ijk[1],
+                             d == 2 ? NB - 1 - ijk[2] : ijk[2]};
+          vo = vc * prolonged_value<float, 3>(t, c, e[f], ni, src, e[kHXPar + f]);
+        } else {
+          vo = vc * same_level_ghost<float, false>(t, b, f, ijk, src, e);
+        }
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * 2.0f;
       } else if (ty == 2) {
@@ -1184,7 +1242,7 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
         vo = vc * fine_crse_ghost<float, 3, false>(t, b, f, ijk, src, e);
       } else {
         vc = cf_face<float, 3>(c, t, b, f, ijk, fx, 0.75f);
-        vo = crse_fine_sum<float, 3, false>(t, c, b, f, ijk, src, e);
+        vo = crse_fine_sum<float, 3, false>(t, c, b, f, ijk, src, e, TOP && below == 1);
       }
       sh.hc[f][m] = vc;
       if (d == 0) {
@@ -1213,21 +1271,6 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
       d4[n] = pr ? make_float4(b2.x, r2.x, b2.y, r2.y) : make_float4(r2.x, b2.x, r2.y, b2.y);
     }
     __syncthreads();  // the tile is free for the next block
-  }
-}
-
-// dst = src over the blocks of a list
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_copy_blocks(BlockList L, int ncell, const T *__restrict__ src,
-                                                          T *__restrict__ dst, const int *guard) {
-  pdl_enter();
-  if (guard && *guard) return;
-  const long total = (long)list_count(L) * ncell;
-  for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
-    const int p = (int)(it / ncell);
-    if (block_off(L, L.blocks[p])) continue;
-    const long q = (long)L.blocks[p] * ncell + (it - (long)p * ncell);
-    dst[q] = src[q];
   }
 }
 
@@ -1880,22 +1923,30 @@ void launch_rbgs(const Topo &t, const Coef<T> &c, const BlockList &L, int color,
 }
 
 template <typename T>
+bool bhgs_prolongs(const Topo &t, const Coef<T> &c, const BlockList &L) {
+  return sizeof(T) == 4 && L.hx && c.cf && (t.ndim == 2 ? t.nb == 16 : t.nb == 16 || t.nb == 8);
+}
+
+template <typename T>
 void launch_bhgs(const Topo &t, const Coef<T> &c, const BlockList &L, int nsweep, const T *src, T *dst,
-                 const T *rhs, const int *guard, cudaStream_t s, bool pdl) {
+                 const T *rhs, const int *guard, cudaStream_t s, bool pdl, int top) {
   const int nhalf = t.ncell / 2;
   if (L.n == 0 || nhalf == 0) return;
   if constexpr (sizeof(T) == 4) {
     if (t.ndim == 2 && t.nb == 16 && L.hx && c.cf) {
       const int warps = kH16Threads / 32, g = std::min((L.n + warps - 1) / warps, 152 * 64);
-      launch_k(pdl, k_bhgs_warp16<4>, g, kH16Threads, 0, s, t, c, L, nsweep, src, dst, rhs, guard);
+      launch_k(pdl, top ? k_bhgs_warp16<4, true> : k_bhgs_warp16<4, false>, g, kH16Threads, 0, s, t, c, L, nsweep, src,
+               dst, rhs, guard, top);
       return;
     }
     if (t.ndim == 3 && (t.nb == 16 || t.nb == 8) && L.hx && c.cf) {
       const int g = std::min(L.n, L.pb ? kReducedGrid : 152 * 64);
       if (t.nb == 16)
-        launch_k(pdl, k_bhgs_rows<16, 2>, g, 256, 0, s, t, c, L, nsweep, src, dst, rhs, guard);
+        launch_k(pdl, top ? k_bhgs_rows<16, 2, true> : k_bhgs_rows<16, 2, false>, g, 256, 0, s, t, c, L, nsweep, src,
+                 dst, rhs, guard, top);
       else
-        launch_k(pdl, k_bhgs_rows<8, 8>, g, 64, 0, s, t, c, L, nsweep, src, dst, rhs, guard);
+        launch_k(pdl, top ? k_bhgs_rows<8, 8, true> : k_bhgs_rows<8, 8, false>, g, 64, 0, s, t, c, L, nsweep, src, dst,
+                 rhs, guard, top);
       return;
     }
   }
@@ -1910,14 +1961,6 @@ void launch_bhgs(const Topo &t, const Coef<T> &c, const BlockList &L, int nsweep
     ensure_max_smem((const void *)k_bhgs<T, 3, 2>, 200 * 1024);
     launch_k(pdl, k_bhgs<T, 3, 2>, grid, threads, smem, s, t, c, L, nsweep, src, dst, rhs, guard);
   }
-}
-
-template <typename T>
-void launch_copy_blocks(const BlockList &L, int ncell, const T *src, T *dst, const int *guard, cudaStream_t s,
-                        bool pdl) {
-  const long work = (long)L.n * ncell;
-  if (work == 0) return;
-  launch_k(pdl, k_copy_blocks<T>, grid_for(work), kThreads, 0, s, L, ncell, src, dst, guard);
 }
 
 template <typename T>
@@ -1989,8 +2032,8 @@ void launch_fix_bc(const Topo &t, const Coef<double> &c, const BlockList &L, con
   template void launch_prolong_red<T>(const Topo &, const Coef<T> &, const BlockList &, T *, const T *,        \
                                       const int *, cudaStream_t, bool, const BlockList &, int);                 \
   template void launch_bhgs<T>(const Topo &, const Coef<T> &, const BlockList &, int, const T *, T *,          \
-                               const T *, const int *, cudaStream_t, bool);                                     \
-  template void launch_copy_blocks<T>(const BlockList &, int, const T *, T *, const int *, cudaStream_t, bool);
+                               const T *, const int *, cudaStream_t, bool, int);                                \
+  template bool bhgs_prolongs<T>(const Topo &, const Coef<T> &, const BlockList &);
 SAYAKA_INST(double)
 SAYAKA_INST(float)
 #undef SAYAKA_INST

@@ -845,6 +845,7 @@ int MacGpu::learned_collect(int max_iters, int max_samples) {
     return -1;
   }
   CKR_(cudaStreamSynchronize(stream_), -1);
+  ensure_fp32_faces();
   const int L = finest_;
   const BlockList TL = tower_list(L);
   const long w = (long)TL.n * ncell_;

@@ -169,7 +169,7 @@ T *dalloc(size_t n) {
 __global__ void k_make_hx(int n, int nd, const int *__restrict__ blocks, const uint16_t *__restrict__ fts,
                           const int *__restrict__ neighbor, const int *__restrict__ parent,
                           const int *__restrict__ which_child, const int *__restrict__ child,
-                          const int *__restrict__ fc_neigh, int *__restrict__ hx) {
+                          const int *__restrict__ fc_neigh, const int *__restrict__ level, int *__restrict__ hx) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     const int b = blocks[p];
     const unsigned ft = fts[p];
@@ -177,6 +177,7 @@ __global__ void k_make_hx(int n, int nd, const int *__restrict__ blocks, const u
     for (int k = 0; k < kHX; k++) e[k] = -1;
     e[kHXInfo] = (int)(ft | ((unsigned)which_child[b] << 16));
     e[kHXBlock] = b;
+    e[kHXLevel] = level[b];
     if (parent[b] >= 0) e[kHXPar + 6] = parent[b] * 8 + which_child[b];
     for (int f = 0; f < 2 * nd; f++) {
       const int ty = (ft >> (2 * f)) & 3, d = f >> 1, s = f & 1;
@@ -315,11 +316,13 @@ MacGpu::MacGpu(const TreeTables &tt) : tt_(tt) {
   CK(cudaMemcpy(d_wc_, tt.which_child.data(), (size_t)nbk * sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(d_fc_neigh_, fc_neigh_.data(), (size_t)nbk * 6 * sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(d_geom_, geom_.data(), (size_t)nbk * 8 * sizeof(double), cudaMemcpyHostToDevice));
+  d_level_ = dalloc<int>(nbk);
+  CK(cudaMemcpy(d_level_, tt.level.data(), (size_t)nbk * sizeof(int), cudaMemcpyHostToDevice));
   // halo descriptors of a tower list (see kHX), built on the device
   auto make_hx = [&](const int *blk, const uint16_t *fts, int n, int *hx) {
     if (n <= 0) return;
     k_make_hx<<<std::min((n + 255) / 256, 152 * 8), 256, 0, stream_>>>(n, nd, blk, fts, d_neighbor_, d_parent_, d_wc_,
-                                                                      d_child_, d_fc_neigh_, hx);
+                                                                      d_child_, d_fc_neigh_, d_level_, hx);
   };
   for (int L = 1; L <= tt.max_level; L++) {
     const Tower &src = tw[L];
@@ -549,6 +552,7 @@ MacGpu::~MacGpu() {
   fr(d_parent_);
   fr(d_wc_);
   fr(d_fc_neigh_);
+  fr(d_level_);
   fr(d_bc_type_);
   fr(d_err_);
   fr(d_geom_);

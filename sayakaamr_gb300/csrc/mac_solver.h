@@ -318,7 +318,7 @@ class MacGpu {
 
   // device tables
   int *d_neighbor_ = nullptr, *d_child_ = nullptr, *d_parent_ = nullptr, *d_wc_ = nullptr;
-  int *d_fc_neigh_ = nullptr, *d_bc_type_ = nullptr;
+  int *d_fc_neigh_ = nullptr, *d_bc_type_ = nullptr, *d_level_ = nullptr;
   int *d_err_ = nullptr;  // error word of the bounded waits (Topo::err)
   double *d_geom_ = nullptr;
   double *d_bcoef_[3] = {nullptr, nullptr, nullptr}, *d_afrac_[3] = {nullptr, nullptr, nullptr};
@@ -394,6 +394,9 @@ class MacGpu {
   double *d_uni64_ = nullptr;
   float *d_uni32_ = nullptr;
   void build_cf();
+  void ensure_df_factors();
+  void ensure_fp32_faces();
+  long df_version_ = -1, faces32_version_ = -1;  // coefficient versions of those copies
   double *d_cf64_ = nullptr;  // coarse/fine face coefficients (Coef::cf)
   float *d_cf32_ = nullptr;
   double *d_iso_ = nullptr;  // per block: T S where one coefficient holds on every face, else 0
@@ -453,7 +456,7 @@ class MacGpu {
   // kernel launches of one captured BiCGSTAB iteration; a device solve
   // launches kPrologueKernels + iterations * this + kEpilogueKernels
   int kernels_per_iteration() const { return kernels_per_iter_; }
-  static constexpr int kPrologueKernels = 3, kEpilogueKernels = 1;
+  static constexpr int kPrologueKernels = 2, kEpilogueKernels = 1;
 };
 
 // integer-pipe precision conversions of the vector kernels against the

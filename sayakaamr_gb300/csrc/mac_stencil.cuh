@@ -110,7 +110,11 @@ __device__ __forceinline__ T cf_face(const Coef<T> &c, const Topo &t, int b, int
 // reference's RESTRICT_SUM order (lower transverse dimension fastest)
 template <typename T, int ND, bool CG = false, typename TX = T>
 __device__ __forceinline__ T crse_fine_sum(const Topo &t, const Coef<T> &c, int b, int f, const int ijk[3],
-                                           const TX *__restrict__ x, const int *__restrict__ hx = nullptr) {
+                                           const TX *__restrict__ x, const int *__restrict__ hx = nullptr,
+                                           bool prolonged = false) {
+  // prolonged: the fine blocks take their parent's values, masked by their
+  // volume fractions: those of this block's neighbour behind the face, whose
+  // cell next to it covers the fine cells
   const int nb = t.nb, half = nb >> 1;
   const int d = f >> 1, s = f & 1;
   int cidx = (1 - s) << d, k = 0;
@@ -138,6 +142,13 @@ __device__ __forceinline__ T crse_fine_sum(const Topo &t, const Coef<T> &c, int 
       if (ND == 2) fi[2] = 0;
       const int fx = face_index(d, fi, fside, nb);
       const T tf = cf_face<T, ND>(c, t, F, f ^ 1, fi, fx, h15);
+      if (prolonged) {
+        int pc[3] = {ijk[0], ijk[1], ijk[2]};
+        pc[d] = fi[d];
+        const T pv = fpint::cvt<T>(ld<CG>(&x[(long)t.neighbor[b * 6 + f] * t.ncell + encode(pc, nb)]));
+        val += tf * (c.vf[(long)F * t.ncell + encode(fi, nb)] > 0 ? pv : (T)0);
+        continue;
+      }
       val += tf * fpint::cvt<T>(ld<CG>(&x[(long)F * t.ncell + encode(fi, nb)]));
     }
   }
