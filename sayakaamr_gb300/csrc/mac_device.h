@@ -150,11 +150,13 @@ __device__ __forceinline__ int list_count(const BlockList &L) { return L.pb ? *L
 __device__ __forceinline__ long factor_entry(const BlockList &L, int p) { return L.orig ? L.orig[p] : p; }
 
 // chunks of a block list listed problem by problem (one BiCGSTAB state per
-// problem): the BiCGSTAB kernels run one CTA per chunk of at most kChunkCells
-// cells of one problem
-// 16 cells per thread: the batch workload solves in 58.8 ms with 4096-cell
-// chunks, 59.5 with 2048 or 8192
-constexpr int kChunkCells = 4096;
+// problem): the BiCGSTAB kernels run one CTA per chunk of at most
+// chunk_cells(total) cells of one problem.  4096 cells, 16 per thread, spread
+// the FP64 epilogue of a chunk's reduction thin (29M cells: 58.8 ms a solve,
+// 59.5 with 2048 or 8192); a smaller forest takes smaller chunks, so that its
+// launches still fill the 608 resident CTAs about twice over and a thread
+// waits for one round of loads instead of four.
+inline long chunk_cells(long total) { return total >= (1l << 24) ? 4096 : total >= (1l << 22) ? 2048 : 1024; }
 struct Chunks {
   const int *comp;       // per chunk: its problem
   const int *beg, *end;  // per chunk: first and past-last cell of the list

@@ -147,7 +147,7 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NV], unsigned maxmask, d
 // A forest of independent problems (the connected components of the tree)
 // solved with one BiCGSTAB state per problem: the finest tower's blocks are
 // listed problem by problem, and the BiCGSTAB kernels run one CTA per chunk
-// of at most kChunkCells consecutive cells of one problem, so that every
+// of at most chunk_cells() consecutive cells of one problem, so that every
 // reduction is a segment of whole CTAs (seg_reduce) and every CTA reads one
 // state.
 // the cells a CTA walks, the state it reads and its reduction segment
@@ -495,18 +495,35 @@ __global__ void k_set_cond_multi(cudaGraphConditionalHandle h, const FState *stc
 // faces that are not physical boundaries, with FMA: 7 FMA + 1 multiply per
 // cell instead of about 40 FP64 operations.  The result differs from the
 // reference's operator by rounding only (about 1e-16 relative).
-// (one CTA per block, so that a thread divides once for its full cells)
+// One warp per block divides once for the block's full cells; a solid cell's
+// factors are 0, and those of a constant-coefficient block's interior cells
+// are its record's (the same values, see k_uniform), so the FP64 pipe sees the
+// other cells only.
 template <int ND>
 __global__ void __launch_bounds__(kTPB) k_op_prep(Topo t, Coef<double> c, BlockList L, double *P, double *S) {
   using namespace stencil;
-  const int nb = t.nb;
-  for (int p = blockIdx.x; p < L.n; p += gridDim.x) {
+  const int nb = t.nb, lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < L.n; p += warps) {
     const int b = L.blocks[p];
     const uint16_t ft = L.ftypes[p];
+    const double *u = uniform_of(c, b);
     const double dv = geom(c, b, 6), full = 1.0 / (dv * 1.0);
-    for (int ci = threadIdx.x; ci < t.ncell; ci += blockDim.x) {
+    for (int ci = lane; ci < t.ncell; ci += 32) {
+      const long q = (long)b * t.ncell + ci;
       int ijk[3];
       decode_fast<ND>(ci, t, ijk);
+      bool inner = true;
+      for (int d = 0; d < ND; d++) inner = inner && ijk[d] > 0 && ijk[d] < nb - 1;
+      if (u && inner) {
+        P[q] = u[4];
+        S[q] = u[5];
+        continue;
+      }
+      const double vfv = c.vf[q];
+      if (!fpint::positive(vfv)) {
+        P[q] = S[q] = 0.0;
+        continue;
+      }
       double diag = c.alpha * dv;
       for (int f = 0; f < 2 * ND; f++) {
         const int d = f >> 1, s = f & 1;
@@ -523,12 +540,10 @@ __global__ void __launch_bounds__(kTPB) k_op_prep(Topo t, Coef<double> c, BlockL
         else if (ty == 1)
           diag += t.bc_type[b * 6 + f] == kBCNeumann ? 0.0 : 2.0 * tf;
         else
-          diag += cf_face<double, ND>(c, t, b, f, ijk, fx, ty == 2 ? 1.5 : 0.75);
+          diag += cf_face<double, ND>(c, t, b, f, ijk);
       }
-      const long q = (long)b * t.ncell + ci;
-      const double vfv = c.vf[q];
       const bool one = __double_as_longlong(vfv) == __double_as_longlong(1.0);
-      const double sc = one ? full : (vfv > 0 ? 1.0 / (dv * vfv) : 0.0);
+      const double sc = one ? full : 1.0 / (dv * vfv);
       S[q] = sc;
       P[q] = diag * sc;
     }
@@ -690,10 +705,10 @@ __device__ __forceinline__ double op_offdiag(const Topo &t, const Coef<double> &
         off = __fma_rn(u ? u[d] : c.tff[d][(long)b * t.nfb + fx],
                        widen_from<TX>(same_level_ghost<TX, false>(t, b, f, ijk, x, hx)), off);
       else if (ty == 2)
-        off = __fma_rn(cf_face<double, ND>(c, t, b, f, ijk, fx, 1.5), widen_from<TX>(fine_crse_ghost<TX, ND, false>(t, b, f, ijk, x, hx)),
+        off = __fma_rn(cf_face<double, ND>(c, t, b, f, ijk), widen_from<TX>(fine_crse_ghost<TX, ND, false>(t, b, f, ijk, x, hx)),
                        off);
       else if (ty == 3)
-        off += crse_fine_sum<double, ND, false>(t, c, b, f, ijk, x, hx);
+        off += refined_sum<double, ND, false>(t, c, b, f, ijk, x, hx);
     }
   }
   return off;
@@ -732,10 +747,10 @@ __device__ __forceinline__ dfl::df op_offdiag_df(const Topo &t, const Coef<doubl
         const dfl::df T = u2 ? dfl::load(u2 + d) : dfl::from_double(c.tff[d][(long)b * t.nfb + fx]);
         off = dfl::add(off, dfl::mul_f(T, same_level_ghost<float, false>(t, b, f, ijk, x, hx)));
       } else if (ty == 2) {
-        off = dfl::add(off, dfl::mul_f(dfl::from_double(cf_coef(c, t, b, d, fx, 1.5)),
+        off = dfl::add(off, dfl::mul_f(dfl::from_double(cf_face<double, ND>(c, t, b, f, ijk)),
                                        fine_crse_ghost<float, ND, false>(t, b, f, ijk, x, hx)));
       } else if (ty == 3) {
-        off = dfl::add(off, dfl::from_double(crse_fine_sum<double, ND, false>(t, c, b, f, ijk, x, hx)));
+        off = dfl::add(off, dfl::from_double(refined_sum<double, ND, false>(t, c, b, f, ijk, x, hx)));
       }
     }
   }
@@ -828,17 +843,20 @@ __global__ void __launch_bounds__(kTPB, 4) k_op_rows(Topo t, Coef<double> c, Blo
                                                    const float *__restrict__ x, double *__restrict__ y,
                                                    const double *__restrict__ w, const double *__restrict__ P,
                                                    const double *__restrict__ S, FState *stb, double *partials,
-                                                   unsigned *counter, const double *__restrict__ iso) {
+                                                   unsigned *counter, const double *__restrict__ iso, int per) {
   using namespace stencil;
   pdl_enter();
   Work wk = work_of<MULTI>(ch, stb, list_count(L) * t.ncell, counter);
   FState *st = wk.st;
   if (st->done) return;
-  if (MULTI) wk.it0 -= threadIdx.x;  // cells of the chunk; its threads take four each
   const int nb = t.nb, nc = t.ncell;
   double acc[2] = {0.0, 0.0};
-  const int first = MULTI ? wk.it0 + 4 * (int)threadIdx.x : 4 * wk.it0;
-  for (int it = first; it < wk.it1; it += 4 * wk.step) {
+  // MULTI: the CTA's chunk; else `per` threads of every CTA work, so that a
+  // small problem reaches as many SMs, each with its own FP64 pipe, as it can
+  const int tid = threadIdx.x;
+  const int first = MULTI ? wk.it0 + 3 * tid : 4 * ((int)blockIdx.x * per + tid);
+  const int step = 4 * (MULTI ? (int)blockDim.x : (int)gridDim.x * per);
+  for (int it = MULTI || tid < per ? first : wk.it1; it < wk.it1; it += step) {
     int p, ci, ijk[3];
     split_cell<ND>(it, t, p, ci);
     decode_fast<ND>(ci, t, ijk);
@@ -913,9 +931,9 @@ __global__ void __launch_bounds__(kTPB, 4) k_op_rows(Topo t, Coef<double> c, Blo
 #pragma unroll
         for (int n = decltype(n0)::value; n < decltype(n1)::value; n++) {
           const int at[3] = {ijk[0] + n, ijk[1], ijk[2]};
-          const double own = cf_face<double, ND>(c, t, b, f, at, 0, 1.5);
+          const double own = cf_face<double, ND>(c, t, b, f, at);
           v[n - decltype(n0)::value] = coarser ? fpint::widen(fine_crse_ghost<float, ND, false>(t, b, f, at, x, e))
-                                               : crse_fine_sum<double, ND, false>(t, c, b, f, at, x, e);
+                                               : refined_sum<double, ND, false>(t, c, b, f, at, x, e);
           k[n - decltype(n0)::value] = coarser ? own : 1.0;
         }
       };
@@ -1266,10 +1284,11 @@ void MacGpu::build_op_factors() {
   if (w == 0) return;
   Coef<double> cc = c64_;
   cc.cf = d_cf64_;
+  cc.ut = d_uni64_;
   if (tt_.ndim == 2)
-    k_op_prep<2><<<std::min(TL.n, 152 * 64), kTPB, 0, stream_>>>(topo_, cc, TL, d_opP_, d_opS_);
+    k_op_prep<2><<<ew_grid(32l * TL.n), kTPB, 0, stream_>>>(topo_, cc, TL, d_opP_, d_opS_);
   else
-    k_op_prep<3><<<std::min(TL.n, 152 * 64), kTPB, 0, stream_>>>(topo_, cc, TL, d_opP_, d_opS_);
+    k_op_prep<3><<<ew_grid(32l * TL.n), kTPB, 0, stream_>>>(topo_, cc, TL, d_opP_, d_opS_);
   CK(cudaGetLastError());
 }
 
@@ -1910,9 +1929,12 @@ void MacGpu::iteration_body(T *resid, T *corr, const Coef<T> &c, const TO *PH, c
     };
     if constexpr (sizeof(TX) == 4 && M < 2) {
       if (!dfop && tt_.nb % 4 == 0) {
-        const int g = mp ? nchunks_ : std::min(red_grid(w), (int)std::max<long>(1, (w / 4 + kTPB - 1) / kTPB));
+        // threads at work per CTA: 32 .. 256, enough for about two CTAs per SM
+        const long groups = std::max<long>(1, w / 4), cap = red_grid(w);
+        const int per = (int)std::min<long>(kTPB, std::max<long>(32, (groups / (152 * 2) + 31) / 32 * 32));
+        const int g = mp ? nchunks_ : (int)std::min<long>(std::max<long>(cap, 152 * 2), (groups + per - 1) / per);
         auto rows = [&](auto kern) {
-          launch_k(pdl, kern, g, kTPB, 0, stream_, topo_, cd64_, TL, ch, x, y, wv, OP, OS, ST, PART, CNT, ISO);
+          launch_k(pdl, kern, g, kTPB, 0, stream_, topo_, cd64_, TL, ch, x, y, wv, OP, OS, ST, PART, CNT, ISO, per);
         };
         if (tt_.ndim == 2)
           mp ? rows(k_op_rows<2, M, true>) : rows(k_op_rows<2, M, false>);

@@ -571,13 +571,21 @@ __global__ void __launch_bounds__(kThreads) k_prolong(Topo t, Coef<T> c, BlockLi
 }
 
 // same-level face coefficient ((beta*ds)/dx)*B*a for every face of every block
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
+
 template <typename T>
-__global__ void k_face_coef(Topo t, const double *geom64, const T *b0, const T *b1, const T *b2, const T *a0,
+__global__ void __launch_bounds__(kThreads) k_face_coef(Topo t, const double *geom64, const T *b0, const T *b1, const T *b2, const T *a0,
                             const T *a1, const T *a2, double beta, T *t0, T *t1, T *t2) {
-  // one CTA per block and direction: a thread divides once for all its faces
-  // (a division per face is about 15 operations of the FP64 pipe: 13.75 M
-  // cells took 1050 us)
-  for (long it = blockIdx.x; it < (long)t.nblocks * t.ndim; it += gridDim.x) {
+  // One warp per block and direction divides once for all its faces (a
+  // division is about 20 operations of the FP64 pipe, whatever the number of
+  // lanes that need it), and a product with 1 or 0 is not formed: B and the
+  // area fraction are 1 or 0 on most faces.  13.75 M cells: 1050 us with a
+  // division per face, 587 with one per thread of a CTA, XXX now.
+  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  for (long it = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; it < (long)t.nblocks * t.ndim; it += warps) {
     const int b = (int)(it / t.ndim), d = (int)(it - (long)b * t.ndim);
     const T *B = d == 0 ? b0 : (d == 1 ? b1 : b2);
     const T *A = d == 0 ? a0 : (d == 1 ? a1 : a2);
@@ -585,9 +593,11 @@ __global__ void k_face_coef(Topo t, const double *geom64, const T *b0, const T *
     const T ds = (T)geom64[b * 8 + 3 + d], dx = (T)geom64[b * 8 + d];
     const T q = (T)beta * ds / dx;
     const long fb = (long)b * t.nfb;
-    for (int i = threadIdx.x; i < t.nfb; i += blockDim.x) {
-      T v = q * B[fb + i];
-      v = v * A[fb + i];
+    for (int i = lane; i < t.nfb; i += 32) {
+      const T bv = B[fb + i], av = A[fb + i];
+      T v = q;
+      if (!same_bits(bv, (T)1)) v = v * bv;
+      if (!same_bits(av, (T)1)) v = v * av;
       O[fb + i] = v;
     }
   }
@@ -738,10 +748,10 @@ inline int grid_for(long work) {
 template <typename T>
 void launch_face_coef(const Topo &t, const double *geom64, const T *bcoef[3], const T *afrac[3], double beta,
                       T *tff[3], cudaStream_t s) {
-  const long work = (long)t.nblocks * t.nfb * t.ndim;
-  if (work == 0) return;
-  k_face_coef<T><<<(int)std::min<long>((long)t.nblocks * t.ndim, 152 * 64), std::min(kThreads, (t.nfb + 31) / 32 * 32), 0, s>>>(t, geom64, bcoef[0], bcoef[1], bcoef[2], afrac[0], afrac[1],
-                                                     afrac[2], beta, tff[0], tff[1], tff[2]);
+  const long rows = (long)t.nblocks * t.ndim;
+  if (rows == 0 || t.nfb == 0) return;
+  k_face_coef<T><<<grid_for(rows * 32), kThreads, 0, s>>>(t, geom64, bcoef[0], bcoef[1], bcoef[2], afrac[0], afrac[1],
+                                                          afrac[2], beta, tff[0], tff[1], tff[2]);
 }
 
 template <typename T>
@@ -820,12 +830,12 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_tile(Topo t, Coef<T> c,
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
+        vc = vk = cf_face<T, ND>(c, t, b, f, ijk);
         vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
       } else {
-        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
+        vc = cf_face<T, ND>(c, t, b, f, ijk);
         vk = (T)1;
-        vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
+        vv = refined_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
       }
       hc[e] = vc;
       hk[e] = vk;
@@ -987,11 +997,11 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bhgs(Topo t, Coef<T> c, Bloc
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
+        vc = cf_face<T, ND>(c, t, b, f, ijk);
         vo = vc * fine_crse_ghost<T, ND, false>(t, b, f, ijk, src, hxe);
       } else {
-        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
-        vo = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, src, hxe);
+        vc = cf_face<T, ND>(c, t, b, f, ijk);
+        vo = refined_sum<T, ND, false>(t, c, b, f, ijk, src, hxe);
       }
       hc[e] = vc;
       ho[e] = vo;
@@ -1238,11 +1248,11 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * 2.0f;
       } else if (ty == 2) {
-        vc = cf_face<float, 3>(c, t, b, f, ijk, fx, 1.5f);
+        vc = cf_face<float, 3>(c, t, b, f, ijk);
         vo = vc * fine_crse_ghost<float, 3, false>(t, b, f, ijk, src, e);
       } else {
-        vc = cf_face<float, 3>(c, t, b, f, ijk, fx, 0.75f);
-        vo = crse_fine_sum<float, 3, false>(t, c, b, f, ijk, src, e, TOP && below == 1);
+        vc = cf_face<float, 3>(c, t, b, f, ijk);
+        vo = refined_sum<float, 3, false>(t, c, b, f, ijk, src, e, TOP && below == 1);
       }
       sh.hc[f][m] = vc;
       if (d == 0) {
@@ -1369,12 +1379,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_rbgs_bulk(Topo t, Coef<T> c, Bl
     } else if (ty == 1) {
       if (t.bc_type[b * 6 + f] != kBCNeumann) vc = c.tff[d][fb + fx] * (T)2.0;
     } else if (ty == 2) {
-      vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
+      vc = vk = cf_face<T, ND>(c, t, b, f, ijk);
       vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
     } else {
-      vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
+      vc = cf_face<T, ND>(c, t, b, f, ijk);
       vk = (T)1;
-      vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
+      vv = refined_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
     }
     hc[e] = vc;
     hk[e] = vk;
@@ -1522,12 +1532,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_rbgs_stream(Topo t, Coef<
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = c.tff[d][fb + fx] * (T)2.0;
       } else if (ty == 2) {
-        vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
+        vc = vk = cf_face<T, ND>(c, t, b, f, ijk);
         vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
       } else {
-        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
+        vc = cf_face<T, ND>(c, t, b, f, ijk);
         vk = (T)1;
-        vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
+        vv = refined_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
       }
       hc[e] = vc;
       hk[e] = vk;
@@ -1730,12 +1740,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        vc = vk = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
+        vc = vk = cf_face<T, ND>(c, t, b, f, ijk);
         vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
       } else {  // not at the finest level of a tower
-        vc = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
+        vc = cf_face<T, ND>(c, t, b, f, ijk);
         vk = (T)1;
-        vv = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
+        vv = refined_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
       }
       hc[e] = vc;
       hk[e] = vk;

@@ -425,16 +425,16 @@ MacGpu::MacGpu(const TreeTables &tt) : tt_(tt) {
     CK(cudaMemcpy(tlc_.ftypes, pf.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice));
     make_hx(tlc_.blocks, tlc_.ftypes, n, tlc_.hx);
     std::vector<int> ccomp, cbeg, cend, c0(ncomp_, 0), cn(ncomp_, 0);
-    const long nc = ncell_;
+    const long nc = ncell_, chunk = chunk_cells((long)n * nc);
     for (int p = 0; p < n;) {
       const int c = comp_of_block_[pb[p]];
       int q = p;
       while (q < n && comp_of_block_[pb[q]] == c) q++;
       c0[c] = (int)ccomp.size();
-      for (long a = (long)p * nc; a < (long)q * nc; a += kChunkCells) {
+      for (long a = (long)p * nc; a < (long)q * nc; a += chunk) {
         ccomp.push_back(c);
         cbeg.push_back((int)a);
-        cend.push_back((int)std::min<long>(a + kChunkCells, (long)q * nc));
+        cend.push_back((int)std::min<long>(a + chunk, (long)q * nc));
       }
       cn[c] = (int)ccomp.size() - c0[c];
       p = q;

@@ -95,14 +95,62 @@ __device__ __forceinline__ T cf_coef(const Coef<T> &c, const Topo &t, int b, int
   return v;
 }
 
-// the same from the table when there is one: face f of cell ijk
+// the same from the table (device solve): face f of cell ijk
 template <typename T, int ND>
-__device__ __forceinline__ T cf_face(const Coef<T> &c, const Topo &t, int b, int f, const int ijk[3], int fidx, T h) {
-  if (!c.cf) return cf_coef(c, t, b, f >> 1, fidx, h);
+__device__ __forceinline__ T cf_face(const Coef<T> &c, const Topo &t, int b, int f, const int ijk[3]) {
   const int d = f >> 1;
   const int m0 = d == 0 ? ijk[1] : ijk[0], m1 = d == 2 ? ijk[1] : ijk[2];
   const int m = ND == 3 ? m0 + t.nb * m1 : m0;
   return c.cf[((long)b * (2 * ND) + f) * (ND == 3 ? t.nb * t.nb : t.nb) + m];
+}
+
+// CRSE_FINE face in the device solve: sum over the fine cells (t0 + 0..1,
+// t1 + 0..1) of fine block F behind face f of the coarse block, in the
+// reference's order.  cf: the block's table row of its face toward the coarse
+// one; x: its cells; vf (or null): the fine cells take the parent's value pv
+// where they hold fluid.  A call: inlined for every face of every cell of a
+// thread it made kernels of 50 to 290 KB, and a launch of a few microseconds
+// then waits for the instruction cache.
+template <typename T, int ND, bool CG, typename TX>
+static __device__ __noinline__ T fine_sum(const T *__restrict__ cf, const TX *__restrict__ x, int nb, int f, int t0,
+                                          int t1, const T *__restrict__ vf, T pv) {
+  const int d = f >> 1, across = (f & 1) ? 0 : nb - 1;
+  const int su = d == 0 ? nb : 1, sv = d == 2 ? nb : nb * nb;
+  const int o = across * (d == 0 ? 1 : (d == 1 ? nb : nb * nb)) + t0 * su + t1 * sv;
+  T val = 0;
+#pragma unroll
+  for (int a1 = 0; a1 < (ND == 3 ? 2 : 1); a1++)
+#pragma unroll
+    for (int a0 = 0; a0 < 2; a0++) {
+      const int q = o + a0 * su + a1 * sv;
+      const T v = vf ? (vf[q] > 0 ? pv : (T)0) : fpint::cvt<T>(ld<CG>(&x[q]));
+      val += cf[t0 + a0 + nb * (t1 + a1)] * v;
+    }
+  return val;
+}
+
+// that sum for face f of cell ijk of block b (hx: its halo descriptor or
+// null); prolonged: see fine_sum, with the block's neighbour behind the face,
+// the parent of the fine blocks, whose cell next to the face covers the cells
+template <typename T, int ND, bool CG = false, typename TX = T>
+__device__ __forceinline__ T refined_sum(const Topo &t, const Coef<T> &c, int b, int f, const int ijk[3],
+                                         const TX *__restrict__ x, const int *__restrict__ hx,
+                                         bool prolonged = false) {
+  const int nb = t.nb, half = nb >> 1, d = f >> 1, s = f & 1;
+  const int i0 = d == 0 ? ijk[1] : ijk[0], i1 = ND == 3 ? (d == 2 ? ijk[1] : ijk[2]) : 0;
+  const int h0 = i0 >= half ? 1 : 0, h1 = ND == 3 && i1 >= half ? 1 : 0;
+  const int q0 = d == 0 ? 1 : 0, q1 = d == 2 ? 1 : 2;
+  const int F = hx ? hx[kHXKids + f * 4 + h0 + 2 * h1]
+                   : t.child[t.neighbor[b * 6 + f] * 8 + (((1 - s) << d) | (h0 << q0) | (ND == 3 ? h1 << q1 : 0))];
+  T pv = 0;
+  if (prolonged) {
+    const int pc[3] = {d == 0 ? (s ? 0 : nb - 1) : ijk[0], d == 1 ? (s ? 0 : nb - 1) : ijk[1],
+                       ND == 3 ? (d == 2 ? (s ? 0 : nb - 1) : ijk[2]) : 0};
+    pv = fpint::cvt<T>(ld<CG>(&x[(long)t.neighbor[b * 6 + f] * t.ncell + encode(pc, nb)]));
+  }
+  return fine_sum<T, ND, CG, TX>(c.cf + ((long)F * (2 * ND) + (f ^ 1)) * (ND == 3 ? nb * nb : nb),
+                                 x + (long)F * t.ncell, nb, f, 2 * (i0 - h0 * half), ND == 3 ? 2 * (i1 - h1 * half) : 0,
+                                 prolonged ? c.vf + (long)F * t.ncell : nullptr, pv);
 }
 
 // CRSE_FINE face: sum of the fine-side contributions T_f * phi_f over the
@@ -110,11 +158,7 @@ __device__ __forceinline__ T cf_face(const Coef<T> &c, const Topo &t, int b, int
 // reference's RESTRICT_SUM order (lower transverse dimension fastest)
 template <typename T, int ND, bool CG = false, typename TX = T>
 __device__ __forceinline__ T crse_fine_sum(const Topo &t, const Coef<T> &c, int b, int f, const int ijk[3],
-                                           const TX *__restrict__ x, const int *__restrict__ hx = nullptr,
-                                           bool prolonged = false) {
-  // prolonged: the fine blocks take their parent's values, masked by their
-  // volume fractions: those of this block's neighbour behind the face, whose
-  // cell next to it covers the fine cells
+                                           const TX *__restrict__ x, const int *__restrict__ hx = nullptr) {
   const int nb = t.nb, half = nb >> 1;
   const int d = f >> 1, s = f & 1;
   int cidx = (1 - s) << d, k = 0;
@@ -141,14 +185,7 @@ __device__ __forceinline__ T crse_fine_sum(const Topo &t, const Coef<T> &c, int 
       if (ND == 3) fi[tq[1]] = base[tq[1]] + a1;
       if (ND == 2) fi[2] = 0;
       const int fx = face_index(d, fi, fside, nb);
-      const T tf = cf_face<T, ND>(c, t, F, f ^ 1, fi, fx, h15);
-      if (prolonged) {
-        int pc[3] = {ijk[0], ijk[1], ijk[2]};
-        pc[d] = fi[d];
-        const T pv = fpint::cvt<T>(ld<CG>(&x[(long)t.neighbor[b * 6 + f] * t.ncell + encode(pc, nb)]));
-        val += tf * (c.vf[(long)F * t.ncell + encode(fi, nb)] > 0 ? pv : (T)0);
-        continue;
-      }
+      const T tf = cf_coef(c, t, F, d, fx, h15);
       val += tf * fpint::cvt<T>(ld<CG>(&x[(long)F * t.ncell + encode(fi, nb)]));
     }
   }
@@ -348,12 +385,12 @@ __device__ __forceinline__ void smooth_cell_fast(const Topo &t, const Coef<T> &c
       } else if (ty == 1) {
         if (t.bc_type[b * 6 + f] != kBCNeumann) diag += (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
-        const T coef = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
+        const T coef = cf_face<T, ND>(c, t, b, f, ijk);
         diag += coef;
         off = fma_t(coef, fine_crse_ghost<T, ND, CG>(t, b, f, ijk, phi, hx), off);
       } else {
-        diag += cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
-        off += crse_fine_sum<T, ND, CG>(t, c, b, f, ijk, phi, hx);
+        diag += cf_face<T, ND>(c, t, b, f, ijk);
+        off += refined_sum<T, ND, CG>(t, c, b, f, ijk, phi, hx);
       }
     }
   }
@@ -431,12 +468,12 @@ __device__ __forceinline__ void smooth_gather(const Topo &t, const Coef<T> &c, i
       o.kc[f] = (T)0;
       o.v[f] = (T)0;
     } else if (ty == 2) {
-      o.dp[f] = o.kc[f] = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)1.5);
+      o.dp[f] = o.kc[f] = cf_face<T, ND>(c, t, b, f, ijk);
       o.v[f] = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hx);
     } else {
-      o.dp[f] = cf_face<T, ND>(c, t, b, f, ijk, fx, (T)0.75);
+      o.dp[f] = cf_face<T, ND>(c, t, b, f, ijk);
       o.kc[f] = (T)1;
-      o.v[f] = crse_fine_sum<T, ND, false>(t, c, b, f, ijk, phi, hx);
+      o.v[f] = refined_sum<T, ND, false>(t, c, b, f, ijk, phi, hx);
     }
   }
   o.r = rhs[cb + ci];
