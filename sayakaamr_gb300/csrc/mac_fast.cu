@@ -24,6 +24,7 @@
 #include "cuda_check.h"
 #include "mac_stencil.cuh"
 #include "mac_df.cuh"
+#include "mac_flow.h"
 #include "launch.cuh"
 #include "mac_fp.cuh"
 #include "tree.h"
@@ -1770,6 +1771,14 @@ void MacGpu::vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *o
     // the prolongation and the red sweep that follows it can be one launch
     const BlockList top = sublevel_list(l, l);
     const bool fused = prm_.fuse_prolong && prm_.n_post > 0 && top.n == levels_[l].n;
+    if constexpr (sizeof(T) == 4) {
+      // the whole tower in one launch, where its blocks fit the device
+      if (fused && flow_fits(l)) {
+        CK(launch_flow(topo_, c, parity_list(l, 0, false), parity_list(l, 1, false), l, prm_.n_post, corr, resid,
+                       guard, d_flow_words_, d_flow_epoch_, act_on_ ? d_active_ : nullptr, stream_));
+        continue;
+      }
+    }
     // with the parity order, the red sweep of the rest of group 0 (leaf
     // sublevels l-2, l-4, ...) rides in the same launch
     const BlockList rest0 = prm_.sublevel_order == 1 ? parity_list(l, 0, true) : BlockList{nullptr, nullptr, 0};
@@ -1801,6 +1810,30 @@ void MacGpu::vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *o
     }
   }
   if (out) vc_out_launch<T>(tower_list(L), corr, out);
+}
+
+// tower l can be smoothed by launch_flow
+bool MacGpu::flow_fits(int l) const {
+  return d_flow_words_ && solve_lists_ && prm_.smooth_variant < 0 && prm_.sublevel_order == 1 &&
+         prm_.prolong_form == 1 && prm_.n_post < (int)kFlowTags - 1 &&
+         towers_[l].par.n > 0 && towers_[l].par.n <= flow_capacity_;
+}
+
+// the exchange buffers of launch_flow, if any tower fits it
+void MacGpu::ensure_flow() {
+  if (flow_capacity_ >= 0) return;
+  flow_capacity_ = flow_capacity(topo_);
+  bool any = false;
+  for (int l = 2; l <= finest_; l++) any = any || (towers_[l].par.n > 0 && towers_[l].par.n <= flow_capacity_);
+  if (!any) return;
+  const size_t n = flow_words(topo_);
+  if (dev_malloc(&d_flow_words_, n * sizeof(unsigned long long)) != cudaSuccess ||
+      dev_malloc(&d_flow_epoch_, 2 * sizeof(unsigned)) != cudaSuccess) {
+    fail("out of device memory (edge exchange)");
+    return;
+  }
+  CK(cudaMemsetAsync(d_flow_words_, 0, n * sizeof(unsigned long long), stream_));
+  CK(cudaMemsetAsync(d_flow_epoch_, 0, 2 * sizeof(unsigned), stream_));
 }
 
 // V-cycle result on the tower, widened to FP64: out = 0 + corr
@@ -2210,6 +2243,7 @@ int MacGpu::prepare_device() {
   // correction only: an FP32 solve does not build them
   if (prm_.precision == 0 || learned_active()) ensure_smooth_factors();
   tune_smoother(prm_.precision);
+  if (prm_.precision == 1) ensure_flow();
   if (prm_.vcycle_out == 1) ensure_df_factors();
   if (learned_active()) {
     ensure_fp32_faces();
@@ -2241,7 +2275,7 @@ int MacGpu::solve_state(SolveInfo *info) {
     }
   }
   if (rbgs_bulk_error(topo_.err, stream_, true) > 0) {
-    fail("bulk-copy smoother: an mbarrier wait timed out");
+    fail("device smoother: a bounded wait timed out");
     return -1;
   }
   if (learned_active() && nn_tc_error(true) > 0) {

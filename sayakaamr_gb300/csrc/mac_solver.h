@@ -343,6 +343,12 @@ class MacGpu {
   // second correction vector of the block-hybrid smoother's passes (they
   // read one and write the other)
   float *d_corr32b_ = nullptr;
+  // one-launch smoothing of a tower (mac_flow.cu)
+  unsigned long long *d_flow_words_ = nullptr;
+  unsigned *d_flow_epoch_ = nullptr;
+  int flow_capacity_ = -1;  // blocks a launch can hold; -1 before the first look
+  bool flow_fits(int l) const;
+  void ensure_flow();
   double *d_corr64b_ = nullptr;
   template <typename T>
   T *corr_alt() {
