@@ -823,6 +823,59 @@ __global__ void __launch_bounds__(kTPB, 4) k_op_red(Topo t, Coef<double> c, Bloc
   if (MODE == 3) seg_reduce<2>(acc, 1u, partials, wk.counter, wk.first, wk.count, wk.slot, EpiVerify{st});
 }
 
+// N cells of k_op_rows at face f toward a coarser or refined neighbour, with
+// transverse indices (i0 .. i0+N-1, i1): off += factor * value per cell (e: the
+// block's halo descriptor).  A call keeps the kernel small; its N cells' loads
+// are in flight together (cell by cell, a small problem's launch waited four
+// times over: 15 us for 27 thousand cells).
+template <int ND, int N>
+static __device__ __noinline__ double4 op_cross(const double *__restrict__ cf, const float *__restrict__ x,
+                                                const int *__restrict__ e, int nb, int nc, int f, int i0, int i1,
+                                                double4 off) {
+  const int d = f >> 1, half = nb >> 1, nface = ND == 3 ? nb * nb : nb, across = (f & 1) ? 0 : nb - 1;
+  const int su = d == 0 ? nb : 1, sv = d == 2 ? nb : nb * nb, sd = d == 0 ? 1 : (d == 1 ? nb : nb * nb);
+  const int info = e[kHXInfo];
+  double k[N], v[N];
+  if (((info >> (2 * f)) & 3) == 2) {
+    const int wc = info >> 16, q0 = d == 0 ? 1 : 0, q1 = d == 2 ? 1 : 2;
+    const int t0 = ((wc >> q0) & 1) * half, t1 = ND == 3 ? ((wc >> q1) & 1) * half + (i1 >> 1) : 0;
+    const double *row = cf + ((long)e[kHXBlock] * (2 * ND) + f) * nface + i0 + nb * i1;
+    const float *xc = x + (long)e[f] * nc + across * sd + t1 * sv;
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      k[n] = row[n];
+      v[n] = fpint::widen(xc[(t0 + ((i0 + n) >> 1)) * su]);
+    }
+  } else {
+    // (four cells never straddle the halves of a face: nb / 2 is even, and
+    // where it is not a multiple of 4 each cell finds its own fine block)
+    const int h1 = ND == 3 && i1 >= half ? 1 : 0;
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      const int h0 = i0 + n >= half ? 1 : 0;
+      const long F = e[kHXKids + f * 4 + h0 + 2 * h1];
+      const int t0 = 2 * (i0 + n - h0 * half), t1 = 2 * (i1 - h1 * half);
+      const double *row = cf + (F * (2 * ND) + (f ^ 1)) * nface;
+      const float *xf = x + F * nc + across * sd;
+      double val = 0.0;
+#pragma unroll
+      for (int a1 = 0; a1 < (ND == 3 ? 2 : 1); a1++)
+#pragma unroll
+        for (int a0 = 0; a0 < 2; a0++)
+          val += row[t0 + a0 + nb * (t1 + a1)] * fpint::widen(xf[(t0 + a0) * su + (t1 + a1) * sv]);
+      k[n] = 1.0;
+      v[n] = val;
+    }
+  }
+  off.x = __fma_rn(k[0], v[0], off.x);
+  if (N > 1) {
+    off.y = __fma_rn(k[N > 1 ? 1 : 0], v[N > 1 ? 1 : 0], off.y);
+    off.z = __fma_rn(k[N > 2 ? 2 : 0], v[N > 2 ? 2 : 0], off.z);
+    off.w = __fma_rn(k[N > 3 ? 3 : 0], v[N > 3 ? 3 : 0], off.w);
+  }
+  return off;
+}
+
 // The operator with its dot products (modes 0 and 1 of k_op_red) on an FP32
 // input, blocks whose edge is a multiple of 4 cells: a thread takes four cells
 // of a row, whose neighbours along y and z are four cells of another row (of
@@ -924,56 +977,45 @@ __global__ void __launch_bounds__(kTPB, 4) k_op_rows(Topo t, Coef<double> c, Blo
     }
     if (!done) {
       const long fb = (long)b * t.nfb;
-      const double *u = uniform_of(c, b);
-      // factors and values of cells n0 .. n1-1 at face f toward a coarser or
-      // refined neighbour; the cells' loads are independent of each other
-      auto cross = [&](int f, auto n0, auto n1, double *k, double *v) {
-        const bool coarser = face_type_of(ft, f) == 2;
-#pragma unroll
-        for (int n = decltype(n0)::value; n < decltype(n1)::value; n++) {
-          const int at[3] = {ijk[0] + n, ijk[1], ijk[2]};
-          const double own = cf_face<double, ND>(c, t, b, f, at);
-          v[n - decltype(n0)::value] = coarser ? fpint::widen(fine_crse_ghost<float, ND, false>(t, b, f, at, x, e))
-                                               : refined_sum<double, ND, false>(t, c, b, f, at, x, e);
-          k[n - decltype(n0)::value] = coarser ? own : 1.0;
-        }
-      };
-      constexpr std::integral_constant<int, 0> c0{};
-      constexpr std::integral_constant<int, 1> c1{};
-      constexpr std::integral_constant<int, 3> c3{};
-      constexpr std::integral_constant<int, 4> c4{};
       const int row = ijk[1] + nb * ijk[2];
       const double *tx = c.tff[0] + fb + (nb + 1) * row + ijk[0];
-      double off[4], xw[6], tk[5];
+      const double2 *p2 = reinterpret_cast<const double2 *>(P + cb + ci), *s2 = reinterpret_cast<const double2 *>(S + cb + ci);
+      const double2 pa = p2[0], pb = p2[1], sa = s2[0], sb = s2[1];
+      double xw[6], tk[5];
 #pragma unroll
       for (int n = 0; n < 6; n++) xw[n] = fpint::widen(xv[n]);
 #pragma unroll
-      for (int n = 0; n < 5; n++) tk[n] = u ? u[0] : tx[n];
-      double tr = tk[4];
-      if (cf && ijk[0] == 0 && face_type_of(ft, 0) > 1) cross(0, c0, c1, &tk[0], &xw[0]);
-      if (cf && ijk[0] + 4 == nb && face_type_of(ft, 1) > 1) cross(1, c3, c4, &tr, &xw[5]);
-#pragma unroll
-      for (int n = 0; n < 4; n++)
-        off[n] = __fma_rn(n == 3 ? tr : tk[n + 1], xw[n + 2], __fma_rn(tk[n], xw[n], 0.0));
+      for (int n = 0; n < 5; n++) tk[n] = tx[n];
+      // left and right, the first and last cell's across the block's edge
+      const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
+      double l0 = __fma_rn(tk[0], xw[0], 0.0);
+      if (cf && ijk[0] == 0 && face_type_of(ft, 0) > 1) l0 = op_cross<ND, 1>(c.cf, x, e, nb, nc, 0, ijk[1], ijk[2], zero).x;
+      double4 off = make_double4(__fma_rn(tk[1], xw[2], l0), __fma_rn(tk[2], xw[3], __fma_rn(tk[1], xw[1], 0.0)),
+                                 __fma_rn(tk[3], xw[4], __fma_rn(tk[2], xw[2], 0.0)), __fma_rn(tk[3], xw[3], 0.0));
+      if (cf && ijk[0] + 4 == nb && face_type_of(ft, 1) > 1)
+        off.w = op_cross<ND, 1>(c.cf, x, e, nb, nc, 1, ijk[1], ijk[2], make_double4(off.w, 0.0, 0.0, 0.0)).x;
+      else
+        off.w = __fma_rn(tk[4], xw[5], off.w);
 #pragma unroll
       for (int f = 2; f < 2 * ND; f++) {
         const int d = f >> 1, s = f & 1;
-        const long fx = d == 1 ? ijk[0] + nb * (ijk[1] + s + (nb + 1) * ijk[2]) : ci + s * nb * nb;
-        const double *tf = c.tff[d] + fb + fx;
-        const float4 q = r[f - 2];
-        double k[4], v[4];
         if (cf && (s ? ijk[d] == nb - 1 : ijk[d] == 0) && face_type_of(ft, f) > 1) {
-          cross(f, c0, c4, k, v);
+          off = op_cross<ND, 4>(c.cf, x, e, nb, nc, f, ijk[0], d == 1 ? ijk[2] : ijk[1], off);
         } else {
-          v[0] = fpint::widen(q.x), v[1] = fpint::widen(q.y), v[2] = fpint::widen(q.z), v[3] = fpint::widen(q.w);
-#pragma unroll
-          for (int n = 0; n < 4; n++) k[n] = u ? u[d] : tf[n];
+          const long fx = d == 1 ? ijk[0] + nb * (ijk[1] + s + (nb + 1) * ijk[2]) : ci + s * nb * nb;
+          const double2 *tf = reinterpret_cast<const double2 *>(c.tff[d] + fb + fx);
+          const double2 ka = tf[0], kb = tf[1];
+          const float4 q = r[f - 2];
+          off.x = __fma_rn(ka.x, fpint::widen(q.x), off.x);
+          off.y = __fma_rn(ka.y, fpint::widen(q.y), off.y);
+          off.z = __fma_rn(kb.x, fpint::widen(q.z), off.z);
+          off.w = __fma_rn(kb.y, fpint::widen(q.w), off.w);
         }
-#pragma unroll
-        for (int n = 0; n < 4; n++) off[n] = __fma_rn(k[n], v[n], off[n]);
       }
-#pragma unroll
-      for (int n = 0; n < 4; n++) yv[n] = __fma_rn(xw[n + 1], P[cb + ci + n], -off[n] * S[cb + ci + n]);
+      yv[0] = __fma_rn(xw[1], pa.x, -off.x * sa.x);
+      yv[1] = __fma_rn(xw[2], pa.y, -off.y * sa.y);
+      yv[2] = __fma_rn(xw[3], pb.x, -off.z * sb.x);
+      yv[3] = __fma_rn(xw[4], pb.y, -off.w * sb.y);
     }
     *reinterpret_cast<double2 *>(y + cb + ci) = make_double2(yv[0], yv[1]);
     *reinterpret_cast<double2 *>(y + cb + ci + 2) = make_double2(yv[2], yv[3]);
