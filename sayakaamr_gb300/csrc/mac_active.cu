@@ -91,9 +91,11 @@ __global__ void __launch_bounds__(256) k_active_copy(const ActiveList *__restric
       l.alinks[i] = l.links[(long)l.orig[i / l.nlinks] * l.nlinks + i % l.nlinks];
 }
 
-// of the active blocks of the finest tower: all (head[0]) and those with one
-// face coefficient (head[1], see k_iso)
-__global__ void __launch_bounds__(kScanThreads) k_active_head(ActiveList top, const double *__restrict__ iso, int *head) {
+// head[0], head[1]: the active blocks of the finest tower, and those of them
+// with one face coefficient (see k_iso); head[2 + i]: active entries of list i
+__global__ void __launch_bounds__(kScanThreads) k_active_head(ActiveList top, const double *__restrict__ iso, int *head,
+                                                             const ActiveList *__restrict__ lists, int nlists) {
+  for (int i = threadIdx.x; i < nlists; i += blockDim.x) head[2 + i] = lists[i].pre[lists[i].n];
   const int n = top.pre[top.n];
   int k = 0;
   for (int i0 = 0; i0 < n; i0 += kScanThreads) {
@@ -147,7 +149,7 @@ void MacGpu::build_active() {
       used = 0;
       h.clear();
       take(flags, nbk);
-      take(head, 2);
+      take(head, 2 + 2 * towers_.size() + levels_.size() + nonleaf_.size());
       auto reduce = [&](DevList &d, int nlinks) {
         if (d.n == 0) return;
         take(d.act.blocks, d.n);
@@ -187,11 +189,17 @@ void MacGpu::build_active() {
   CK_(cudaGetLastError());
   const ActiveList t{top.blocks, nullptr, nullptr, nullptr, 0, top.n, top.act.blocks, nullptr, nullptr, nullptr,
                      top.act.pre, top.act.orig};
-  k_active_head<<<1, kScanThreads, 0, stream_>>>(t, d_iso_, d_act_head_);
+  k_active_head<<<1, kScanThreads, 0, stream_>>>(t, d_iso_, d_act_head_, d_act_lists_, n_act_lists_);
   CK_(cudaGetLastError());
-  int head[2] = {0, 0};
-  CK_(cudaMemcpyAsync(head, d_act_head_, sizeof(head), cudaMemcpyDeviceToHost, stream_));
+  std::vector<int> head(2 + n_act_lists_, 0);
+  CK_(cudaMemcpyAsync(head.data(), d_act_head_, head.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_));
   CK_(cudaStreamSynchronize(stream_));
+  // active entries of every tower's parity-grouped list
+  n_act_par_.assign(towers_.size(), 0);
+  for (size_t i = 0, q = 2; i < towers_.size(); i++) {
+    if (towers_[i].all.n) q++;
+    if (towers_[i].par.n) n_act_par_[i] = head[q++];
+  }
   n_act_ = head[0];
   n_iso_ = head[1];
 }

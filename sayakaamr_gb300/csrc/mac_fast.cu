@@ -1815,8 +1815,11 @@ void MacGpu::vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *o
     const bool fused = prm_.fuse_prolong && prm_.n_post > 0 && top.n == levels_[l].n;
     if constexpr (sizeof(T) == 4) {
       // the whole tower in one launch, where its blocks fit the device
-      if (fused && flow_fits(l)) {
-        CK(launch_flow(topo_, c, parity_list(l, 0, false), parity_list(l, 1, false), l, prm_.n_post, corr, resid,
+      if (fused && solve_lists_ && flow_fits(l)) {
+        // (a moving body may change the number of active blocks up to the
+        // capacity without another capture)
+        const int grid = std::min(towers_[l].par.n, flow_capacity_);
+        CK(launch_flow(topo_, c, parity_list(l, 0, false), parity_list(l, 1, false), l, prm_.n_post, grid, corr, resid,
                        guard, d_flow_words_, d_flow_epoch_, act_on_ ? d_active_ : nullptr, stream_));
         continue;
       }
@@ -1855,18 +1858,26 @@ void MacGpu::vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *o
 }
 
 // tower l can be smoothed by launch_flow
+int MacGpu::flow_entries(int l) const {
+  return act_on_ && l < (int)n_act_par_.size() ? n_act_par_[l] : towers_[l].par.n;
+}
 bool MacGpu::flow_fits(int l) const {
-  return d_flow_words_ && solve_lists_ && prm_.smooth_variant < 0 && prm_.sublevel_order == 1 &&
-         prm_.prolong_form == 1 && prm_.n_post < (int)kFlowTags - 1 &&
-         towers_[l].par.n > 0 && towers_[l].par.n <= flow_capacity_;
+  return d_flow_words_ && prm_.sublevel_order == 1 && prm_.prolong_form == 1 &&
+         prm_.n_post < (int)kFlowTags - 1 && flow_entries(l) > 0 && flow_entries(l) <= flow_capacity_;
+}
+unsigned MacGpu::flow_mask() const {
+  unsigned m = 0;
+  if (prm_.precision == 1 && prm_.smoother == 0 && prm_.vcycle_kernel == 0)
+    for (int l = 2; l <= finest_ && l < 32; l++) m |= flow_fits(l) ? 1u << l : 0u;
+  return m;
 }
 
 // the exchange buffers of launch_flow, if any tower fits it
 void MacGpu::ensure_flow() {
-  if (flow_capacity_ >= 0) return;
-  flow_capacity_ = flow_capacity(topo_);
+  if (d_flow_words_) return;
+  if (flow_capacity_ < 0) flow_capacity_ = flow_capacity(topo_);
   bool any = false;
-  for (int l = 2; l <= finest_; l++) any = any || (towers_[l].par.n > 0 && towers_[l].par.n <= flow_capacity_);
+  for (int l = 2; l <= finest_; l++) any = any || (flow_entries(l) > 0 && flow_entries(l) <= flow_capacity_);
   if (!any) return;
   const size_t n = flow_words(topo_);
   if (dev_malloc(&d_flow_words_, n * sizeof(unsigned long long)) != cudaSuccess ||
@@ -2132,6 +2143,7 @@ void MacGpu::capture_loop(int precision) {
   graph_omega_ = prm_.relax_omega;
   graph_act_ = (int)act_on_;
   graph_direct_ = (int)vcycle_in_place();
+  graph_flow_ = flow_mask();
 }
 
 // the captured graph was recorded with other parameters than the current ones
@@ -2143,7 +2155,7 @@ bool MacGpu::graph_stale() const {
          graph_inner_ != prm_.inner_sweeps || graph_multi_ != (int)multi() || graph_uniform_ != prm_.uniform ||
          graph_pform_ != prm_.prolong_form || graph_vout_ != prm_.vcycle_out ||
          graph_omega_ != prm_.relax_omega || graph_act_ != (int)act_on_ ||
-         graph_direct_ != (int)vcycle_in_place();
+         graph_direct_ != (int)vcycle_in_place() || graph_flow_ != flow_mask();
 }
 
 int MacGpu::cg_solve_device(SolveInfo *info) {

@@ -14,11 +14,11 @@ int flow_capacity(const Topo &t);
 size_t flow_words(const Topo &t);
 // Tower of parity groups A and B (with halo descriptors): the prolongation of
 // level `level` and nsweep red-black sweeps, launch_prolong_red's and
-// launch_rbgs's values in their order.  A.n + B.n <= flow_capacity(t), nsweep
-// < kFlowTags - 1.  alive: with reduced lists, the blocks they hold (else
-// null).
+// launch_rbgs's values in their order.  grid: at least the groups' entries (of
+// reduced lists: their active ones) and at most flow_capacity(t); nsweep <
+// kFlowTags - 1.  alive: with reduced lists, the blocks they hold (else null).
 cudaError_t launch_flow(const Topo &t, const Coef<float> &c, const BlockList &A, const BlockList &B, int level,
-                        int nsweep, float *phi, const float *rhs, const int *guard, unsigned long long *words,
-                        unsigned *epoch, const int *alive, cudaStream_t s);
+                        int nsweep, int grid, float *phi, const float *rhs, const int *guard,
+                        unsigned long long *words, unsigned *epoch, const int *alive, cudaStream_t s);
 
 }  // namespace sayaka_gb300

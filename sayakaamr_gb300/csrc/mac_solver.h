@@ -348,6 +348,8 @@ class MacGpu {
   unsigned *d_flow_epoch_ = nullptr;
   int flow_capacity_ = -1;  // blocks a launch can hold; -1 before the first look
   bool flow_fits(int l) const;
+  int flow_entries(int l) const;  // blocks that a launch for tower l holds
+  unsigned flow_mask() const;     // the towers that fit, as the captured graph has them
   void ensure_flow();
   double *d_corr64b_ = nullptr;
   template <typename T>
@@ -385,6 +387,7 @@ class MacGpu {
   int n_act_lists_ = 0;
   int n_act_ = 0, n_iso_ = 0;  // active blocks of the finest tower, and those with one face coefficient
   int *d_act_head_ = nullptr;
+  std::vector<int> n_act_par_;  // active entries of every tower's parity-grouped list
   // the BiCGSTAB kernels read the FP32 V-cycle's output in place
   bool vcycle_in_place() const;
   long act_version_ = -1;              // coefficient version of the reduced lists
@@ -444,6 +447,7 @@ class MacGpu {
   int graph_coop_ = -1, graph_pdl_ = -1, graph_cc_ = -1, graph_var_ = -1, graph_nn_ = -1, graph_order_ = -1;
   int graph_smoother_ = -1, graph_inner_ = -1, graph_multi_ = -1, graph_uniform_ = -1, graph_pform_ = -1,
       graph_vout_ = -1, graph_act_ = -1, graph_direct_ = -1;
+  unsigned graph_flow_ = 0;
   double graph_omega_ = -1.0;
   bool last_multi_ = false;  // the last device solve kept one state per problem
   Chunks chunks() const;

@@ -1,5 +1,5 @@
-"""The smoothing of a tower in one cooperative launch (2D FP32 blocks of 8 or
-16 cells, prolong_form 1 with the tuned smoother) against the separate
+"""The smoothing of a tower in one cooperative launch (FP32; 2D blocks of 8 or
+16 cells, 3D blocks of 8; prolong_form 1) against the separate
 launches (prolong_form 0): the same bits, on trees of one block per problem up
 to more blocks than a launch can hold, with coarse/fine and physical faces,
 cut cells, solid blocks (reduced lists), over-relaxation, one to five sweeps,
@@ -60,3 +60,37 @@ def test_mostly_solid(nb):
     p = W._finish("disk", t, tb, vol, area, [np.ones_like(a) for a in area], f, False, {}, dirichlet_faces=(3,))
     assert 4 * (p.vol.reshape(p.num_blocks, -1).max(axis=1) == 0).sum() > p.num_blocks
     _both(p)
+
+
+@pytest.mark.parametrize("levels", [2, 4, 5])
+@pytest.mark.parametrize("kw", [dict(), dict(relax_omega=1.1, n_post_smooth=4), dict(n_post_smooth=1, uniform=0)],
+                         ids=["2", "4-relaxed", "1-arrays"])
+def test_3d(levels, kw):
+    # at 5 levels the finest tower holds more blocks than a launch
+    _both(W.config3(nb=8, max_level=levels, band=1.0), **kw)
+
+
+@pytest.mark.parametrize("kw", [dict(n_post_smooth=4, relax_omega=1.1), dict(n_post_smooth=3)], ids=["4", "3"])
+def test_3d_moving_body(kw):
+    """mostly solid (reduced lists); the fractions change under a captured
+    graph, by a little and by so much that other towers fit a launch"""
+    seq = list(W.config5_sequence(steps=3, regrid_every=100, max_level=5))
+    out = []
+    for form in (1, 0):
+        S = W.make_solver(seq[0][2], **dict(PARAMS, prolong_form=form, bottom_level=1, **kw))
+        got = []
+        for _, _, p in seq + seq[:1]:
+            S.set_ib_frac_compact(p.vol, p.area)
+            S.set_rhs_compact(p.rhs)
+            S.set_zero_sol()
+            info = S.cg_solve()
+            got.append((info["status"], info["iterations"], S.get_sol_compact()))
+        full = np.ones_like(p.vol)
+        S.set_ib_frac_compact(full, [np.ones_like(a) for a in p.area])
+        S.set_zero_sol()
+        info = S.cg_solve()
+        got.append((info["status"], info["iterations"], S.get_sol_compact()))
+        out.append(got)
+    for a, b in zip(*out):
+        assert a[:2] == b[:2]
+        assert np.array_equal(a[2], b[2])
