@@ -1094,54 +1094,82 @@ struct H3 {
   static __device__ __forceinline__ int row(int j, int k) { return j + 1 + (NB + 2) * (k + 1); }
 };
 
+// Coefficients and volume fractions of a block without a record, staged once:
+// read from global memory row by row, every load of a warp touches 32 lines,
+// and a pass of one such block took 19 us.  y and z faces and volume fractions
+// are split by the parity of their indices like the tile: the lower face of a
+// cell of colour c is in part c of its own row, its upper face in part 1 - c
+// of the next row, at the same place.
+template <int NB>
+struct H3Var {
+  static constexpr int kH = NB / 8;
+  float fx[NB * NB][NB + 1];
+  float4 fy[2][kH][NB * (NB + 1)], fz[2][kH][NB * (NB + 1)], vf[2][kH][NB * NB];
+};
+// rows x NB values of src, row m split by the parity of i + par(m)
+template <int NB, int ROWS, class Par>
+__device__ __forceinline__ void h3_stage(const float *__restrict__ src, float4 (&dst)[2][NB / 8][ROWS], Par par) {
+  const float4 *s4 = reinterpret_cast<const float4 *>(src);
+#pragma unroll
+  for (int n = threadIdx.x; n < ROWS * (NB / 4); n += NB * NB) {
+    const float4 w = s4[n];
+    const int row = n / (NB / 4), q = 2 * (n % (NB / 4)), pr = par(row) & 1;
+    float2 *e2 = reinterpret_cast<float2 *>(&dst[0][q >> 2][row]) + ((q >> 1) & 1);
+    float2 *o2 = reinterpret_cast<float2 *>(&dst[1][q >> 2][row]) + ((q >> 1) & 1);
+    *e2 = pr ? make_float2(w.y, w.w) : make_float2(w.x, w.z);
+    *o2 = pr ? make_float2(w.x, w.z) : make_float2(w.y, w.w);
+  }
+}
+
 // the sweeps of one block: row (j, k) of thread (U: a constant-coefficient
-// block, coefficients T[]; else from the face arrays)
+// block, coefficients T[]; else from the face arrays).  The diagonal is not
+// kept per cell: in a constant-coefficient block every cell of a row but its
+// two ends has the same (a boundary face's part is one value per face there,
+// coarse/fine faces included), elsewhere it is summed along with the
+// off-diagonal from the same loads.  With 16 registers less, three CTAs of a
+// 16^3 block fit an SM instead of two.
 template <int NB, bool U>
 __device__ __forceinline__ void h3_sweeps(const Topo &t, const Coef<float> &c, int b, const float *u, float dv,
-                                          int nsweep, const float *__restrict__ rhs, H3<NB> &sh) {
+                                          int nsweep, const float4 (&r4)[NB / 4], H3<NB> &sh,
+                                          const H3Var<NB> &sv) {
   constexpr int Q = NB / 2, H = NB / 8;
   const int j = threadIdx.x % NB, k = threadIdx.x / NB, pr = (j + k) & 1, m = threadIdx.x;
-  const long cb = (long)b * NB * NB * NB, fb = (long)b * t.nfb;
   const int r = H3<NB>::row(j, k);
   const float T0 = U ? u[0] : 0.f, T1 = U ? u[1] : 0.f, T2 = U ? u[2] : 0.f;
-  // x faces i .. i+1 of cell i; y and z faces below, the ones above NB and
-  // NB^2 further
-  const float *fx = c.tff[0] + fb + (NB + 1) * (j + NB * k);
-  const float *fy = c.tff[1] + fb + NB * (j + (NB + 1) * k);
-  const float *fz = c.tff[2] + fb + NB * (j + NB * k);
-  const float *vf = c.vf + cb + NB * m, *rp = rhs + cb + NB * m;
-  float v[2][Q], rd[2][Q], dg[2][Q];
+  const float *fx = sv.fx[m];
+  const int ry = j + (NB + 1) * k;  // row of the y faces below; above: the next
+  float v[2][Q], rd[2][Q];
   const float kd = j == 0 ? 1.f : T1, ku = j == NB - 1 ? 1.f : T1;
   const float kb = k == 0 ? 1.f : T2, kf = k == NB - 1 ? 1.f : T2;
-  const float hl = sh.hox[0][m], hr = sh.hox[1][m];
-#pragma unroll
-  for (int q = 0; q < Q; q++) {
-    const float2 r2 = *reinterpret_cast<const float2 *>(rp + 2 * q);
-    rd[0][q] = (pr ? r2.y : r2.x) * dv;
-    rd[1][q] = (pr ? r2.x : r2.y) * dv;
+  const float hl = sh.hox[0][m], hr = sh.hox[1][m], cl = sh.hc[0][m], cr = sh.hc[1][m];
+  // diagonal of the row's first, inner and last cells (U)
+  float g0 = 0.f, gm = 0.f, g1 = 0.f;
+  if (U) {
+    const float ad = c.alpha * dv;
+    const float yd = j == 0 ? sh.hc[2][NB * k] : T1, yu = j == NB - 1 ? sh.hc[3][NB * k] : T1;
+    const float zb = k == 0 ? sh.hc[4][NB * j] : T2, zf = k == NB - 1 ? sh.hc[5][NB * j] : T2;
+    g0 = ad + cl, gm = ad + T0, g1 = ad + T0;
+    g0 += T0, gm += T0, g1 += cr;
+    g0 += yd, gm += yd, g1 += yd;
+    g0 += yu, gm += yu, g1 += yu;
+    g0 += zb, gm += zb, g1 += zb;
+    g0 += zf, gm += zf, g1 += zf;
   }
 #pragma unroll
-  for (int col = 0; col < 2; col++) {
-    const int pk = col ? 1 - pr : pr;
+  for (int q = 0; q < Q; q += 2) {
+    const float4 w = r4[q / 2];
+    rd[0][q] = (pr ? w.y : w.x) * dv;
+    rd[1][q] = (pr ? w.x : w.y) * dv;
+    rd[0][q + 1] = (pr ? w.w : w.z) * dv;
+    rd[1][q + 1] = (pr ? w.z : w.w) * dv;
+  }
+#pragma unroll
+  for (int col = 0; col < 2; col++)
 #pragma unroll
     for (int h = 0; h < H; h++) {
       const float4 w = sh.tile[col][h][r];
       v[col][4 * h] = w.x, v[col][4 * h + 1] = w.y, v[col][4 * h + 2] = w.z, v[col][4 * h + 3] = w.w;
     }
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const int i = 2 * q + pk;
-      float g = c.alpha * dv;
-      g += q == 0 && i == 0 ? sh.hc[0][m] : (U ? T0 : fx[i]);
-      g += q == Q - 1 && i == NB - 1 ? sh.hc[1][m] : (U ? T0 : fx[i + 1]);
-      g += j == 0 ? sh.hc[2][i + NB * k] : (U ? T1 : fy[i]);
-      g += j == NB - 1 ? sh.hc[3][i + NB * k] : (U ? T1 : fy[i + NB]);
-      g += k == 0 ? sh.hc[4][i + NB * j] : (U ? T2 : fz[i]);
-      g += k == NB - 1 ? sh.hc[5][i + NB * j] : (U ? T2 : fz[i + NB * NB]);
-      if (!U && !(vf[i] > 0.f)) g = 0.f;  // 0: the cell stays at 0
-      dg[col][q] = g;
-    }
-  }
   for (int sw = 0; sw < nsweep; sw++) {
 #pragma unroll
     for (int col = 0; col < 2; col++) {
@@ -1153,22 +1181,49 @@ __device__ __forceinline__ void h3_sweeps(const Topo &t, const Coef<float> &c, i
         const float4 b4 = sh.tile[1 - col][h][r - (NB + 2)], f4 = sh.tile[1 - col][h][r + (NB + 2)];
         const float vd[4] = {d4.x, d4.y, d4.z, d4.w}, vu[4] = {u4.x, u4.y, u4.z, u4.w};
         const float vb[4] = {b4.x, b4.y, b4.z, b4.w}, vz[4] = {f4.x, f4.y, f4.z, f4.w};
+        float4 tdv, tuv, tbv, tfv, vfv;
+        if (!U) {
+          tdv = sv.fy[col][h][ry], tuv = sv.fy[1 - col][h][ry + 1];
+          tbv = sv.fz[col][h][m], tfv = sv.fz[1 - col][h][m + NB];
+          vfv = sv.vf[col][h][m];
+        }
 #pragma unroll
         for (int n = 0; n < 4; n++) {
           const int q = 4 * h + n, i = 2 * q + pk;
+          const bool first = q == 0 && i == 0, last = q == Q - 1 && i == NB - 1;
           float vl = pk ? o[q] : (q > 0 ? o[q > 0 ? q - 1 : 0] : hl);
           float vr = pk ? (q < Q - 1 ? o[q < Q - 1 ? q + 1 : q] : hr) : o[q];
-          const float kl = q == 0 && i == 0 ? 1.f : (U ? T0 : fx[i]);
-          const float kr = q == Q - 1 && i == NB - 1 ? 1.f : (U ? T0 : fx[i + 1]);
-          float off = 0.f;
-          off = fma_t(kl, vl, off);
-          off = fma_t(kr, vr, off);
-          off = fma_t(U || j == 0 ? kd : fy[i], vd[n], off);
-          off = fma_t(U || j == NB - 1 ? ku : fy[i + NB], vu[n], off);
-          off = fma_t(U || k == 0 ? kb : fz[i], vb[n], off);
-          off = fma_t(U || k == NB - 1 ? kf : fz[i + NB * NB], vz[n], off);
-          const float g = dg[col][q];
-          v[col][q] = g > 0.f ? relax(c.omega, fast_div(fma_t(rd[col][q], U ? 1.f : vf[i], off), g), v[col][q]) : 0.f;
+          float off = 0.f, g, w = 1.f;
+          if (U) {
+            g = first ? g0 : last ? g1 : gm;
+            off = fma_t(first ? 1.f : T0, vl, off);
+            off = fma_t(last ? 1.f : T0, vr, off);
+            off = fma_t(kd, vd[n], off);
+            off = fma_t(ku, vu[n], off);
+            off = fma_t(kb, vb[n], off);
+            off = fma_t(kf, vz[n], off);
+          } else {
+            const float tl = fx[i], tr = fx[i + 1];
+            const float td = n == 0 ? tdv.x : n == 1 ? tdv.y : n == 2 ? tdv.z : tdv.w;
+            const float tu = n == 0 ? tuv.x : n == 1 ? tuv.y : n == 2 ? tuv.z : tuv.w;
+            const float tb = n == 0 ? tbv.x : n == 1 ? tbv.y : n == 2 ? tbv.z : tbv.w;
+            const float tf = n == 0 ? tfv.x : n == 1 ? tfv.y : n == 2 ? tfv.z : tfv.w;
+            g = c.alpha * dv;
+            g += first ? cl : tl;
+            g += last ? cr : tr;
+            g += j == 0 ? sh.hc[2][i + NB * k] : td;
+            g += j == NB - 1 ? sh.hc[3][i + NB * k] : tu;
+            g += k == 0 ? sh.hc[4][i + NB * j] : tb;
+            g += k == NB - 1 ? sh.hc[5][i + NB * j] : tf;
+            off = fma_t(first ? 1.f : tl, vl, off);
+            off = fma_t(last ? 1.f : tr, vr, off);
+            off = fma_t(j == 0 ? 1.f : td, vd[n], off);
+            off = fma_t(j == NB - 1 ? 1.f : tu, vu[n], off);
+            off = fma_t(k == 0 ? 1.f : tb, vb[n], off);
+            off = fma_t(k == NB - 1 ? 1.f : tf, vz[n], off);
+            w = n == 0 ? vfv.x : n == 1 ? vfv.y : n == 2 ? vfv.z : vfv.w;
+          }
+          v[col][q] = (w > 0.f && g > 0.f) ? relax(c.omega, fast_div(fma_t(rd[col][q], w, off), g), v[col][q]) : 0.f;
         }
         sh.tile[col][h][r] = make_float4(v[col][4 * h], v[col][4 * h + 1], v[col][4 * h + 2], v[col][4 * h + 3]);
       }
@@ -1183,6 +1238,8 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
                                                             const float *__restrict__ src, float *__restrict__ dst,
                                                             const float *__restrict__ rhs, const int *guard, int top) {
   __shared__ H3<NB> sh;
+  extern __shared__ __align__(16) unsigned char h3_smem[];
+  H3Var<NB> &sv = *reinterpret_cast<H3Var<NB> *>(h3_smem);
   pdl_enter();
   if (guard && *guard) return;
   constexpr int NT = NB * NB, NC = NB * NB * NB;
@@ -1196,6 +1253,10 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
     const long cb = (long)b * NC, fb = (long)b * t.nfb;
     const float *u = uniform_of(c, b);
     const int below = TOP ? top - e[kHXLevel] : -1;  // 0: the block itself is prolonged, 1: the finer ones at its faces
+    float4 r4[NB / 4];  // the thread's row of the right-hand side, in flight with the tile
+#pragma unroll
+    for (int n = 0; n < NB / 4; n++) r4[n] = reinterpret_cast<const float4 *>(rhs + cb + NB * (int)threadIdx.x)[n];
+    const float dv = geom(c, b, 6);
     // the tile, four cells of a row per step: two of each colour
     const float4 *s4 = reinterpret_cast<const float4 *>(src + cb);
 #pragma unroll
@@ -1264,12 +1325,17 @@ __global__ void __launch_bounds__(NB *NB, MINB) k_bhgs_rows(Topo t, Coef<float> 
         reinterpret_cast<float *>(&sh.tile[1 - col][q >> 2][at])[q & 3] = vo;
       }
     }
+    if (!u) {
+      h3_stage<NB, NB *(NB + 1)>(c.tff[1] + fb, sv.fy, [](int row) { return row % (NB + 1) + row / (NB + 1); });
+      h3_stage<NB, NB *(NB + 1)>(c.tff[2] + fb, sv.fz, [](int row) { return row % NB + row / NB; });
+      h3_stage<NB, NB * NB>(c.vf + cb, sv.vf, [](int row) { return row % NB + row / NB; });
+      for (int n = threadIdx.x; n < NT * (NB + 1); n += NT) (&sv.fx[0][0])[n] = c.tff[0][fb + n];
+    }
     __syncthreads();
-    const float dv = geom(c, b, 6);
     if (u)
-      h3_sweeps<NB, true>(t, c, b, u, dv, nsweep, rhs, sh);
+      h3_sweeps<NB, true>(t, c, b, u, dv, nsweep, r4, sh, sv);
     else
-      h3_sweeps<NB, false>(t, c, b, u, dv, nsweep, rhs, sh);
+      h3_sweeps<NB, false>(t, c, b, u, dv, nsweep, r4, sh, sv);
     if (nsweep == 0) __syncthreads();
     float4 *d4 = reinterpret_cast<float4 *>(dst + cb);
 #pragma unroll
@@ -1932,6 +1998,15 @@ void launch_rbgs(const Topo &t, const Coef<T> &c, const BlockList &L, int color,
     rbgs_nd<T, 3>(variant, t, c, L, color, phi, rhs, guard, s, pdl, grid, threads);
 }
 
+template <int NB, int MINB>
+static void bhgs_rows_go(const Topo &t, const Coef<float> &c, const BlockList &L, int nsweep, const float *src,
+                         float *dst, const float *rhs, const int *guard, cudaStream_t s, bool pdl, int top, int grid) {
+  const auto kern = top ? k_bhgs_rows<NB, MINB, true> : k_bhgs_rows<NB, MINB, false>;
+  const int smem = (int)sizeof(H3Var<NB>);
+  ensure_max_smem((const void *)kern, smem);
+  launch_k(pdl, kern, grid, NB * NB, smem, s, t, c, L, nsweep, src, dst, rhs, guard, top);
+}
+
 template <typename T>
 bool bhgs_prolongs(const Topo &t, const Coef<T> &c, const BlockList &L) {
   return sizeof(T) == 4 && L.hx && c.cf && (t.ndim == 2 ? t.nb == 16 : t.nb == 16 || t.nb == 8);
@@ -1952,11 +2027,9 @@ void launch_bhgs(const Topo &t, const Coef<T> &c, const BlockList &L, int nsweep
     if (t.ndim == 3 && (t.nb == 16 || t.nb == 8) && L.hx && c.cf) {
       const int g = std::min(L.n, L.pb ? kReducedGrid : 152 * 64);
       if (t.nb == 16)
-        launch_k(pdl, top ? k_bhgs_rows<16, 2, true> : k_bhgs_rows<16, 2, false>, g, 256, 0, s, t, c, L, nsweep, src,
-                 dst, rhs, guard, top);
+        bhgs_rows_go<16, 2>(t, c, L, nsweep, src, dst, rhs, guard, s, pdl, top, g);
       else
-        launch_k(pdl, top ? k_bhgs_rows<8, 8, true> : k_bhgs_rows<8, 8, false>, g, 64, 0, s, t, c, L, nsweep, src, dst,
-                 rhs, guard, top);
+        bhgs_rows_go<8, 8>(t, c, L, nsweep, src, dst, rhs, guard, s, pdl, top, g);
       return;
     }
   }
