@@ -1059,35 +1059,37 @@ __global__ void __launch_bounds__(kTPB) k_bottom_gemv(BottomDev bd, const T *__r
   stencil::bottom_tile<T>(bd, blockIdx.x, resid, corr, rv);
 }
 
-// in-place Gauss-Jordan inversion step k of nmat matrices of order m at
-// offsets offs (no pivoting: the pinned, row-scaled level-1 operator has
-// positive pivots)
-__global__ void k_gj_save(int m, int k, int nmat, const long long *offs, const double *a, double *row, double *col,
-                          double *ipiv) {
-  const long total = (long)nmat * m;
-  for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
-    const int mat = (int)(it / m), i = (int)(it - (long)mat * m);
-    const double *am = a + offs[mat];
-    row[it] = am[(long)k * m + i];
-    col[it] = am[(long)i * m + k];
-    if (i == k) ipiv[mat] = 1.0 / am[(long)k * m + k];
-  }
+// Gauss-Jordan inversion step k of nmat matrices of order m at offsets offs
+// (no pivoting: the pinned, row-scaled bottom operator has positive pivots),
+// from a into b, so that one launch per step is enough: the pivot row and
+// column are read where they are while every other entry is written.  One
+// CTA per matrix row; the row of the next pivot also writes its reciprocal,
+// ipiv[mat][k + 1], so that no CTA waits for a division.  (With the row and
+// column saved by a launch of their own and the step in place, an inversion
+// of order 512 took 2.6 ms, half of it the saving launches.)
+__global__ void k_gj_first(int m, int nmat, const long long *__restrict__ offs, const double *__restrict__ a,
+                           double *__restrict__ ipiv) {
+  const int mat = blockIdx.x * blockDim.x + threadIdx.x;
+  if (mat < nmat) ipiv[(long)mat * m] = 1.0 / a[offs[mat]];
 }
-// one CTA per matrix row: every element uses the step's saved pivot row,
-// pivot column and pivot reciprocal (no division per element)
-__global__ void __launch_bounds__(kTPB) k_gj_step(int m, int k, int nmat, const long long *offs, double *a,
-                                                const double *row, const double *col, const double *ipiv) {
+__global__ void __launch_bounds__(kTPB) k_gj_step(int m, int k, int nmat, const long long *__restrict__ offs,
+                                                const double *__restrict__ a, double *__restrict__ b,
+                                                double *__restrict__ ipiv) {
   const long rows = (long)nmat * m;
   for (long r = blockIdx.x; r < rows; r += gridDim.x) {
     const int mat = (int)(r / m), i = (int)(r - (long)mat * m);
-    const double *rw = row + (long)mat * m;
-    const double ip = ipiv[mat], ci = col[r];
-    double *ar = a + offs[mat] + (long)i * m;
+    const double *am = a + offs[mat], *rw = am + (long)k * m, *ar = am + (long)i * m;
+    double *br = b + offs[mat] + (long)i * m;
+    const double ip = ipiv[(long)mat * m + k];
     if (i == k) {
-      for (int j = threadIdx.x; j < m; j += blockDim.x) ar[j] = j == k ? ip : rw[j] * ip;
+      for (int j = threadIdx.x; j < m; j += blockDim.x) br[j] = j == k ? ip : rw[j] * ip;
     } else {
-      const double f = ci * ip;
-      for (int j = threadIdx.x; j < m; j += blockDim.x) ar[j] = j == k ? -f : __fma_rn(-f, rw[j], ar[j]);
+      const double f = ar[k] * ip;
+      for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const double v = j == k ? -f : __fma_rn(-f, rw[j], ar[j]);
+        br[j] = v;
+        if (i == k + 1 && j == i) ipiv[(long)mat * m + i] = 1.0 / v;
+      }
     }
   }
 }
@@ -1682,22 +1684,31 @@ void MacGpu::build_bottom() {
       if (comp_n[c] == m) offs.push_back(comp_off[c]);
     const int nmat = (int)offs.size();
     long long *d_offs = nullptr;
-    double *row = nullptr, *col = nullptr;
+    double *other = nullptr;  // the matrices after every other step, at the same offsets
     CK_(dev_malloc(&d_offs, nmat * sizeof(long long)));
-    CK_(dev_malloc(&row, (size_t)nmat * m * sizeof(double)));
-    CK_(dev_malloc(&col, (size_t)nmat * m * sizeof(double)));
     double *ipiv = nullptr;
-    CK_(dev_malloc(&ipiv, nmat * sizeof(double)));
+    CK_(dev_malloc(&other, (size_t)tot * sizeof(double)));
+    CK_(dev_malloc(&ipiv, (size_t)nmat * m * sizeof(double)));
     CK_(cudaMemcpyAsync(d_offs, offs.data(), nmat * sizeof(long long), cudaMemcpyHostToDevice, stream_));
     const int step_grid = (int)std::min<long>((long)nmat * m, 152 * 16);
+    // an odd order starts from a copy, so that the last step ends in d_binv_
+    const double *from = d_binv_;
+    double *to = other;
+    if (m & 1) {
+      CK_(cudaMemcpyAsync(other, d_binv_, (size_t)tot * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
+      from = other;
+      to = d_binv_;
+    }
+    k_gj_first<<<(nmat + kTPB - 1) / kTPB, kTPB, 0, stream_>>>(m, nmat, d_offs, from, ipiv);
     for (int k = 0; k < m; k++) {
-      k_gj_save<<<ew_grid((long)nmat * m), kTPB, 0, stream_>>>(m, k, nmat, d_offs, d_binv_, row, col, ipiv);
-      k_gj_step<<<step_grid, kTPB, 0, stream_>>>(m, k, nmat, d_offs, d_binv_, row, col, ipiv);
+      k_gj_step<<<step_grid, kTPB, 0, stream_>>>(m, k, nmat, d_offs, from, to, ipiv);
+      double *t = const_cast<double *>(from);
+      from = to;
+      to = t;
     }
     CK_(cudaStreamSynchronize(stream_));
     dev_free(d_offs);
-    dev_free(row);
-    dev_free(col);
+    dev_free(other);
     dev_free(ipiv);
   }
   for (int r0 : pins) {
