@@ -1691,14 +1691,9 @@ void MacGpu::build_bottom() {
     CK_(dev_malloc(&ipiv, (size_t)nmat * m * sizeof(double)));
     CK_(cudaMemcpyAsync(d_offs, offs.data(), nmat * sizeof(long long), cudaMemcpyHostToDevice, stream_));
     const int step_grid = (int)std::min<long>((long)nmat * m, 152 * 16);
-    // an odd order starts from a copy, so that the last step ends in d_binv_
+    // (the order is even, as the blocks' sides are: the last step ends in d_binv_)
     const double *from = d_binv_;
     double *to = other;
-    if (m & 1) {
-      CK_(cudaMemcpyAsync(other, d_binv_, (size_t)tot * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
-      from = other;
-      to = d_binv_;
-    }
     k_gj_first<<<(nmat + kTPB - 1) / kTPB, kTPB, 0, stream_>>>(m, nmat, d_offs, from, ipiv);
     for (int k = 0; k < m; k++) {
       k_gj_step<<<step_grid, kTPB, 0, stream_>>>(m, k, nmat, d_offs, from, to, ipiv);

@@ -537,6 +537,222 @@ __global__ void __launch_bounds__(kH16Threads, MINB) k_bhgs_warp16(Topo t, Coef<
     h16_pass<TOP>(t, c, L, L.hx + (long)p * kHX, top, nsweep, src, dst, rhs, lane, sh[threadIdx.x >> 5]);
 }
 
+// ---- 3D FP32 blocks of 8^3 cells, one thread per row of cells along x ------
+// A thread updates the four cells of the colour in its row.  Their neighbours
+// are in the row itself and, at the same places, in the four adjoining rows,
+// which it loads 32 bytes at a time from the block or from the block behind a
+// same-level face, so a sweep needs no shared memory and no barrier and only
+// coarse/fine faces take another path.  One thread per cell spends most of its
+// instructions on indices and boundary tests.  PROLONG: the values are those of
+// the parents (k_prolong_red's).  Bound by the latency of the loads.  13.75 M
+// cells, 5,366 of 30,697 blocks without a cut: a sweep 16.5 -> 11.0 us, the
+// fused prolongation 93 -> 29 us.  CTAs per SM of a sweep of the finest level:
+// 23.1 us at 8, 19.0 at 12, 18.8 at 16 (one thread per cell: 33.2).
+struct Row4 {  // diagonal and off-diagonal sums of the four cells
+  float g[4], o[4];
+};
+// a coarser or refined neighbour behind y or z face f, cells a0, a0 + 2, ..
+// along x, other transverse index a1 (with d = 0: one cell, a0 = j, a1 = k)
+template <int N>
+static __device__ __noinline__ Row4 rows8_cross(const float *__restrict__ cf, const float *__restrict__ phi,
+                                                const int *__restrict__ e, int f, int a0, int a1, Row4 s) {
+  constexpr int NB = 8, NC = 512, NF = 64;
+  const int d = f >> 1, across = (f & 1) ? 0 : NB - 1, info = e[kHXInfo], b = e[kHXBlock];
+  const int su = d == 0 ? NB : 1, sv = d == 2 ? NB : NB * NB, sd = d == 0 ? 1 : (d == 1 ? NB : NB * NB);
+  const float *own = cf + ((long)b * 6 + f) * NF + NB * a1;
+  if (((info >> (2 * f)) & 3) == 2) {
+    const int wc = info >> 16, q0 = d == 0 ? 1 : 0, q1 = d == 2 ? 1 : 2;
+    const float *x = phi + (long)e[f] * NC + across * sd + (4 * ((wc >> q1) & 1) + (a1 >> 1)) * sv;
+    const int t0 = 4 * ((wc >> q0) & 1);
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      const float k = own[a0 + 2 * n];
+      s.g[n] += k;
+      s.o[n] = fma_t(k, x[(t0 + ((a0 + 2 * n) >> 1)) * su], s.o[n]);
+    }
+    return s;
+  }
+  const int h1 = a1 >> 2;
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    const int i = a0 + 2 * n, h0 = i >> 2;
+    const long F = e[kHXKids + 4 * f + h0 + 2 * h1];
+    const int t0 = 2 * (i - 4 * h0), t1 = 2 * (a1 - 4 * h1);
+    const float *w = cf + (F * 6 + (f ^ 1)) * NF + t0 + NB * t1;
+    const float *x = phi + F * NC + across * sd + t0 * su + t1 * sv;
+    float v = 0.f;
+    v += w[0] * x[0];
+    v += w[1] * x[su];
+    v += w[NB] * x[sv];
+    v += w[NB + 1] * x[su + sv];
+    s.g[n] += own[i];
+    s.o[n] += v;
+  }
+  return s;
+}
+
+template <bool PROLONG>
+__device__ __forceinline__ void rows8_sweep(const Topo &t, const Coef<float> &c, const BlockList &L, const int *e,
+                                            int color, float *__restrict__ phi, const float *__restrict__ rhs) {
+  constexpr int NB = 8, NC = 512;
+  const int tid = threadIdx.x, j = tid & 7, k = tid >> 3, pk = (color + j + k) & 1;  // cells 2q + pk
+  const int4 n03 = *reinterpret_cast<const int4 *>(e), n47 = *reinterpret_cast<const int4 *>(e + 4);
+  const int info = n47.z, b = n47.w;
+  const long cb = (long)b * NC, fb = (long)b * t.nfb;
+  if (L.stc && block_off(L, b)) return;
+  const float *u = uniform_of(c, b);
+  const bool U = u != nullptr;
+  const float dv = geom(c, b, 6);
+  const float T0 = U ? u[0] : 0.f, T1 = U ? u[1] : 0.f, T2 = U ? u[2] : 0.f;
+  struct Row {
+    float4 a, b;
+    __device__ __forceinline__ float at(int q, int odd) const {  // cell 2q + odd
+      return q == 0 ? (odd ? a.y : a.x) : q == 1 ? (odd ? a.w : a.z) : q == 2 ? (odd ? b.y : b.x) : (odd ? b.w : b.z);
+    }
+  };
+  auto load = [](const float *p) { return Row{reinterpret_cast<const float4 *>(p)[0], reinterpret_cast<const float4 *>(p)[1]}; };
+  // row (jj, kk) of block n, prolonged from its parent pw (parent * 8 + child);
+  // fluid: every cell of n is
+  auto row_of = [&](long n, int pw, bool fluid, int jj, int kk) {
+    if constexpr (PROLONG) {
+      const int wc = pw & 7;
+      const float4 q = *reinterpret_cast<const float4 *>(phi + (long)(pw >> 3) * NC + 4 * (wc & 1) +
+                                                          NB * (4 * ((wc >> 1) & 1) + (jj >> 1) +
+                                                                NB * (4 * ((wc >> 2) & 1) + (kk >> 1))));
+      Row r{make_float4(q.x, q.x, q.y, q.y), make_float4(q.z, q.z, q.w, q.w)};
+      if (!fluid) {
+        const Row m = load(c.vf + n * NC + NB * (jj + NB * kk));
+        if (!(m.a.x > 0.f)) r.a.x = 0.f;
+        if (!(m.a.y > 0.f)) r.a.y = 0.f;
+        if (!(m.a.z > 0.f)) r.a.z = 0.f;
+        if (!(m.a.w > 0.f)) r.a.w = 0.f;
+        if (!(m.b.x > 0.f)) r.b.x = 0.f;
+        if (!(m.b.y > 0.f)) r.b.y = 0.f;
+        if (!(m.b.z > 0.f)) r.b.z = 0.f;
+        if (!(m.b.w > 0.f)) r.b.w = 0.f;
+      }
+      return r;
+    } else {
+      return load(phi + n * NC + NB * (jj + NB * kk));
+    }
+  };
+  const int pw = PROLONG ? e[kHXPar + 6] : 0;
+  const Row own = row_of(b, pw, U, j, k), rr = load(rhs + cb + NB * tid);
+  Row vf{make_float4(1.f, 1.f, 1.f, 1.f), make_float4(1.f, 1.f, 1.f, 1.f)};
+  if (!U) vf = load(c.vf + cb + NB * tid);
+  const int nbr[6] = {n03.x, n03.y, n03.z, n03.w, n47.x, n47.y};
+  Row4 s;
+#pragma unroll
+  for (int q = 0; q < 4; q++) s.g[q] = c.alpha * dv, s.o[q] = 0.f;
+  // x faces
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+    const float *fx = c.tff[0] + fb + (NB + 1) * tid + f;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const bool edge = f == 0 ? q == 0 && pk == 0 : q == 3 && pk == 1;
+      const float T = U ? T0 : fx[2 * q + pk];
+      if (!edge) {
+        // left: cell 2q + pk - 1, right: 2q + pk + 1, both of the other colour
+        const float v = f == 0 ? (pk ? own.at(q, 0) : own.at(q > 0 ? q - 1 : 0, 1)) : (pk ? own.at(q < 3 ? q + 1 : 3, 0) : own.at(q, 1));
+        s.g[q] += T;
+        s.o[q] = fma_t(T, v, s.o[q]);
+        continue;
+      }
+      const int ty = (info >> (2 * f)) & 3, across = f ? 0 : NB - 1;
+      if (ty == 0) {
+        float v;
+        if constexpr (PROLONG) {
+          const int ijk[3] = {across, j, k};
+          v = prolonged_value<float, 3>(t, c, nbr[f], ijk, phi, e[kHXPar + f]);
+        } else {
+          v = phi[(long)nbr[f] * NC + NB * tid + across];
+        }
+        s.g[q] += T;
+        s.o[q] = fma_t(T, v, s.o[q]);
+      } else if (ty == 1) {
+        if (t.bc_type[b * 6 + f] != kBCNeumann) s.g[q] += T * 2.0f;
+      } else {
+        Row4 one;
+        one.g[0] = s.g[q], one.o[0] = s.o[q];
+        one = rows8_cross<1>(c.cf, phi, e, f, j, k, one);
+        s.g[q] = one.g[0], s.o[q] = one.o[0];
+      }
+    }
+  }
+  // y and z faces: the row across, cells at the same places
+#pragma unroll
+  for (int f = 2; f < 6; f++) {
+    const int d = f >> 1, side = f & 1, at = d == 1 ? j : k;
+    const bool edge = side ? at == NB - 1 : at == 0;
+    const int ty = edge ? (info >> (2 * f)) & 3 : 0;
+    if (ty >= 2) {
+      s = rows8_cross<4>(c.cf, phi, e, f, pk, d == 1 ? k : j, s);
+      continue;
+    }
+    float T[4];
+    if (U) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) T[q] = d == 1 ? T1 : T2;
+    } else {
+      const Row w = load(c.tff[d] + fb + (d == 1 ? NB * (j + side + (NB + 1) * k) : NB * (j + NB * (k + side))));
+#pragma unroll
+      for (int q = 0; q < 4; q++) T[q] = pk ? w.at(q, 1) : w.at(q, 0);
+    }
+    if (ty == 1) {
+      if (t.bc_type[b * 6 + f] != kBCNeumann) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) s.g[q] += T[q] * 2.0f;
+      }
+      continue;
+    }
+    const int to = edge ? (side ? 0 : NB - 1) : (side ? at + 1 : at - 1);
+    const Row v = row_of(edge ? nbr[f] : b, PROLONG ? (edge ? e[kHXPar + f] : pw) : 0, U && !edge, d == 1 ? to : j,
+                         d == 1 ? k : to);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      s.g[q] += T[q];
+      s.o[q] = fma_t(T[q], pk ? v.at(q, 1) : v.at(q, 0), s.o[q]);
+    }
+  }
+  float n[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const float r = pk ? rr.at(q, 1) : rr.at(q, 0), w = pk ? vf.at(q, 1) : vf.at(q, 0);
+    const float old = pk ? own.at(q, 1) : own.at(q, 0);
+    n[q] = (w > 0.f && s.g[q] > 0.f) ? relax(c.omega, fast_div(fma_t(r * dv, w, s.o[q]), s.g[q]), old) : 0.f;
+  }
+  // the other colour's cells with the values that concurrent readers see anyway
+  float4 *dst = reinterpret_cast<float4 *>(phi + cb + NB * tid);
+  dst[0] = pk ? make_float4(own.a.x, n[0], own.a.z, n[1]) : make_float4(n[0], own.a.y, n[1], own.a.w);
+  dst[1] = pk ? make_float4(own.b.x, n[2], own.b.z, n[3]) : make_float4(n[2], own.b.y, n[3], own.b.w);
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(64, MINB) k_rbgs_rows8(Topo t, Coef<float> c, BlockList L, int color,
+                                                         float *__restrict__ phi, const float *__restrict__ rhs,
+                                                         const int *guard) {
+  pdl_enter();
+  if (guard && *guard) return;
+  const ListRange lr = list_range(L);
+  for (int p = lr.a + blockIdx.x; p < lr.b; p += gridDim.x)
+    rows8_sweep<false>(t, c, L, L.hx + (long)p * kHX, color, phi, rhs);
+}
+__global__ void __launch_bounds__(64, 12) k_prolong_red_rows8(Topo t, Coef<float> c, BlockList L,
+                                                              float *__restrict__ phi, const float *__restrict__ rhs,
+                                                              const int *guard, BlockList X) {
+  pdl_enter();
+  if (guard && *guard) return;
+  const ListRange lr = list_range(L), xr = list_range(X);
+  const int nl = lr.b - lr.a, nx = xr.b - xr.a;
+  for (int p = blockIdx.x; p < nl + nx; p += gridDim.x) {
+    if (p < nl)
+      rows8_sweep<true>(t, c, L, L.hx + (long)(lr.a + p) * kHX, 0, phi, rhs);
+    else
+      rows8_sweep<false>(t, c, X, X.hx + (long)(xr.a + p - nl) * kHX, 0, phi, rhs);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // volume-weighted restriction onto the non-leaf blocks of a level:
 // coarse = avg(fine*vf_fine)/vf_coarse (src/SayakaMacIB.cpp:157-232 with
@@ -1883,6 +2099,13 @@ void launch_prolong_red(const Topo &t, const Coef<T> &c, const BlockList &L, T *
       return;
     }
   }
+  if constexpr (sizeof(T) == 4) {
+    if (form == 1 && t.ndim == 3 && t.nb == 8 && L.hx && c.cf) {
+      const int g = std::min(L.n + X.n, 152 * 32);
+      launch_k(pdl, k_prolong_red_rows8, g, 64, 0, s, t, c, L, phi, rhs, guard, X);
+      return;
+    }
+  }
   const int nface = t.ndim == 3 ? t.nb * t.nb : t.nb;
   const size_t smem = sizeof(T) * ((size_t)t.ncell + 3 * 2 * t.ndim * (size_t)nface);
   ensure_max_smem(t.ndim == 2 ? (const void *)k_prolong_red<T, 2> : (const void *)k_prolong_red<T, 3>, 200 * 1024);
@@ -1918,12 +2141,10 @@ static void rbgs_go(const Topo &t, const Coef<T> &c, const BlockList &L, int col
   launch_k(pdl, k_rbgs<T, ND, MINB>, grid, threads, 0, s, t, c, L, color, phi, rhs, guard);
 }
 
-// variant 10: CPT = 2 cells per thread (k_rbgs_ilp), cap 64; variants 11, 12:
-// one warp per 16x16 block in 2D FP32 (k_rbgs_warp16, caps 64 and 48);
-// variant 13: the same with every load issued before the first branch
-// (k_rbgs_warp16_flat, cap 64: at 48 registers it spills and loses,
-// 20.8 vs 16.9 us on the batch workload's first 64 problems); elsewhere
-// variant 3
+// variant 10: CPT = 2 cells per thread (k_rbgs_ilp), cap 64; variants 11 .. 13
+// of an FP32 sweep: one warp per 16x16 block in 2D (k_rbgs_warp16, register
+// caps 64, 48, 80), one thread per row of an 8^3 block in 3D (k_rbgs_rows8,
+// 8, 12, 16 CTAs of 64 threads per SM); elsewhere variant 3
 template <typename T, int ND, int MINB, int CPT>
 static void rbgs_ilp_go(const Topo &t, const Coef<T> &c, const BlockList &L, int color, T *phi, const T *rhs,
                         const int *guard, cudaStream_t s, bool pdl, dim3 grid, int threads) {
@@ -1948,6 +2169,14 @@ static void rbgs_nd(int variant, const Topo &t, const Coef<T> &c, const BlockLis
             launch_k(pdl, k_rbgs_warp16<5>, g, kThreads, 0, s, t, c, L, color, phi, rhs, guard);
           else
             launch_k(pdl, k_rbgs_warp16<3>, g, kThreads, 0, s, t, c, L, color, phi, rhs, guard);
+          return;
+        }
+      }
+      if constexpr (ND == 3 && sizeof(T) == 4) {
+        if (t.nb == 8 && L.hx && c.cf) {
+          const int g = std::min(L.n, 152 * 32);
+          const auto k = variant == 11 ? k_rbgs_rows8<8> : variant == 12 ? k_rbgs_rows8<12> : k_rbgs_rows8<16>;
+          launch_k(pdl, k, g, 64, 0, s, t, c, L, color, phi, rhs, guard);
           return;
         }
       }

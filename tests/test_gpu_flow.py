@@ -94,3 +94,19 @@ def test_3d_moving_body(kw):
     for a, b in zip(*out):
         assert a[:2] == b[:2]
         assert np.array_equal(a[2], b[2])
+
+
+@pytest.mark.parametrize("variant", [11, 12, 13])
+@pytest.mark.parametrize("kw", [dict(), dict(relax_omega=1.1, n_post_smooth=3), dict(uniform=0)],
+                         ids=["2", "3-relaxed", "arrays"])
+def test_row_sweeps_of_3d_blocks(variant, kw):
+    """3D blocks of 8^3 cells, one thread per row, in towers too large for one
+    launch: the same bits as one thread per cell (variant 3)"""
+    p = W.config3(nb=8)
+    out = []
+    for v, form in ((variant, 1), (3, 0)):
+        S = W.make_solver(p, **dict(PARAMS, smooth_variant=v, prolong_form=form, **kw))
+        info = S.cg_solve()
+        out.append((info["status"], info["iterations"], info["rnorm"], S.get_sol_compact()))
+    assert out[0][:3] == out[1][:3]
+    assert np.array_equal(out[0][3], out[1][3])
