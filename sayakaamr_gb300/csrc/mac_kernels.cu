@@ -753,6 +753,11 @@ __global__ void __launch_bounds__(64, 12) k_prolong_red_rows8(Topo t, Coef<float
   }
 }
 
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
+
 // ---------------------------------------------------------------------------
 // volume-weighted restriction onto the non-leaf blocks of a level:
 // coarse = avg(fine*vf_fine)/vf_coarse (src/SayakaMacIB.cpp:157-232 with
@@ -768,6 +773,87 @@ __global__ void __launch_bounds__(kThreads) k_restrict(Topo t, Coef<T> c, BlockL
     const int p = (int)(it / ncell);
     if (block_off(L, L.blocks[p])) continue;
     restrict_cell<T, ND>(t, c, L.blocks[p], (int)(it - (long)p * ncell), phi, L.links ? L.links + (long)p * 8 : nullptr);
+  }
+}
+
+// the same with two coarse cells next to each other along x per thread, whose
+// fine rows of four cells it loads at once (blocks' sides a multiple of four).
+// A factor vf = 1 is not multiplied or divided by (the same bits; in FP64 the
+// division alone is half of the kernel's FP64 work), and where a block's record
+// says that all its cells have vf = 1 it isn't read.
+template <typename T>
+struct alignas(16) Quad {
+  T v[4];
+};
+template <typename T, int ND>
+__global__ void __launch_bounds__(kThreads) k_restrict_pairs(Topo t, Coef<T> c, BlockList L, T *__restrict__ phi,
+                                                             const int *guard) {
+  pdl_enter();
+  if (guard && *guard) return;
+  const int nb = t.nb, half = nb >> 1, pairs = t.ncell >> 1, sh = t.lnb >= 0 ? ND * t.lnb - 1 : -1;
+  const long total = (long)list_count(L) * pairs;
+  const T wgt = (T)1.0 / (T)(1 << ND);
+  for (long it = blockIdx.x * (long)blockDim.x + threadIdx.x; it < total; it += (long)gridDim.x * blockDim.x) {
+    const int p = sh >= 0 ? (int)(it >> sh) : (int)(it / pairs);
+    const int ci = 2 * (int)(it - (long)p * pairs), b = L.blocks[p];
+    int ijk[3];
+    if (t.lnb >= 0) {
+      ijk[0] = ci & (nb - 1);
+      ijk[1] = (ci >> t.lnb) & (nb - 1);
+      ijk[2] = ND == 3 ? ci >> (2 * t.lnb) : 0;
+    } else {
+      decode<ND>(ci, nb, ijk);
+    }
+    int cidx = 0, f0 = 0, stride = 1;
+#pragma unroll
+    for (int q = 0; q < ND; q++) {
+      const int sq = ijk[q] >= half ? 1 : 0;
+      cidx |= sq << q;
+      f0 += 2 * (ijk[q] - sq * half) * stride;
+      stride *= nb;
+    }
+    const int F = L.links ? L.links[(long)p * 8 + cidx] : t.child[b * 8 + cidx];
+    if (block_off(L, b)) continue;
+    const long fine = (long)F * t.ncell + f0, coarse = (long)b * t.ncell + ci;
+    constexpr int R = ND == 3 ? 4 : 2;
+    Quad<T> x[R];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      x[r] = *reinterpret_cast<const Quad<T> *>(phi + fine + (r & 1) * nb + (r >> 1) * nb * nb);
+    const T one = (T)1;
+    if (!uniform_of(c, F)) {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const Quad<T> w = *reinterpret_cast<const Quad<T> *>(c.vf + fine + (r & 1) * nb + (r >> 1) * nb * nb);
+        bool fluid = true;
+#pragma unroll
+        for (int q = 0; q < 4; q++) fluid = fluid && same_bits(w.v[q], one);
+        if (!fluid) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) x[r].v[q] = x[r].v[q] * w.v[q];
+        }
+      }
+    }
+    T vc[2] = {one, one};
+    if (!uniform_of(c, b)) vc[0] = c.vf[coarse], vc[1] = c.vf[coarse + 1];
+    const bool fluid = same_bits(vc[0], one) && same_bits(vc[1], one);
+    T out[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      T sum = 0;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        sum += x[r].v[2 * k];
+        sum += x[r].v[2 * k + 1];
+      }
+      out[k] = sum * wgt;
+    }
+    if (!fluid) {
+#pragma unroll
+      for (int k = 0; k < 2; k++) out[k] = vc[k] > 0 ? out[k] / vc[k] : (T)0;
+    }
+    phi[coarse] = out[0];
+    phi[coarse + 1] = out[1];
   }
 }
 
@@ -787,11 +873,6 @@ __global__ void __launch_bounds__(kThreads) k_prolong(Topo t, Coef<T> c, BlockLi
 }
 
 // same-level face coefficient ((beta*ds)/dx)*B*a for every face of every block
-__device__ __forceinline__ bool same_bits(double a, double b) {
-  return __double_as_longlong(a) == __double_as_longlong(b);
-}
-__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
-
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_face_coef(Topo t, const double *geom64, const T *b0, const T *b1, const T *b2, const T *a0,
                             const T *a1, const T *a2, double beta, T *t0, T *t1, T *t2) {
@@ -2291,6 +2372,11 @@ void launch_restrict(const Topo &t, const Coef<T> &c, const BlockList &L, T *phi
                      cudaStream_t s, bool pdl) {
   const long work = (long)L.n * t.ncell;
   if (work == 0) return;
+  if (t.nb % 4 == 0) {
+    const auto k = t.ndim == 2 ? k_restrict_pairs<T, 2> : k_restrict_pairs<T, 3>;
+    launch_k(pdl, k, grid_for(work / 2), kThreads, 0, s, t, c, L, phi, guard);
+    return;
+  }
   if (t.ndim == 2)
     launch_k(pdl, k_restrict<T, 2>, grid_for(work), kThreads, 0, s, t, c, L, phi, guard);
   else
