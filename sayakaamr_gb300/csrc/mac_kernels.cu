@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs(Topo t, Coef<T> c, Bloc
 // (entries p, p + G, ..., G = gridDim.y): every cell's operands are gathered
 // before any is updated, so that a thread keeps CPT cells' loads in flight
 // (smooth_gather / smooth_update: the values of smooth_cell_fast)
-template <typename T, int ND, int MINB, int CPT>
+template <typename T, int ND, int MINB, int CPT, bool FAC>
 __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_ilp(Topo t, Coef<T> c, BlockList L, int color,
                                                              T *__restrict__ phi, const T *__restrict__ rhs,
                                                              const int *guard) {
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_ilp(Topo t, Coef<T> c, 
   const int G = gridDim.y;
   const ListRange lr = list_range(L);
   for (int p0 = lr.a + blockIdx.y; p0 < lr.b; p0 += CPT * G) {
-    SmoothOps<T, ND> o[CPT];
+    SmoothOps<T, ND, FAC> o[CPT];
     bool on[CPT];
 #pragma unroll
     for (int k = 0; k < CPT; k++) {
@@ -132,13 +132,13 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_ilp(Topo t, Coef<T> c, 
       const int b = e ? e[kHXBlock] : L.blocks[p];
       if (L.stc && block_off(L, b)) continue;
       const uint16_t ft = e ? (uint16_t)(e[kHXInfo] & 0xffff) : L.ftypes[p];
-      smooth_gather<T, ND>(t, c, b, ft, ijk, phi, rhs, L.sa ? L.sa + fo : nullptr, L.ia ? L.ia + fo : nullptr, e,
-                           o[k]);
+      smooth_gather<T, ND, FAC>(t, c, b, ft, ijk, phi, rhs, FAC ? L.sa + fo : nullptr, FAC ? L.ia + fo : nullptr, e,
+                                o[k]);
       on[k] = true;
     }
 #pragma unroll
     for (int k = 0; k < CPT; k++)
-      if (on[k]) smooth_update<T, ND>(c, o[k], phi);
+      if (on[k]) smooth_update<T, ND, FAC>(c, o[k], phi);
   }
 }
 
@@ -151,7 +151,7 @@ __device__ __forceinline__ T prolonged_value(const Topo &t, const Coef<T> &c, in
   int pc[3] = {0, 0, 0};
   for (int q = 0; q < ND; q++) pc[q] = ((wc >> q) & 1) * half + (ijk[q] >> 1);
   const long q = (long)b * t.ncell + encode(ijk, nb);
-  return (fluid || c.vf[q] > 0) ? phi[(long)P * t.ncell + encode(pc, nb)] : (T)0;
+  return (fluid || positive(c.vf[q])) ? phi[(long)P * t.ncell + encode(pc, nb)] : (T)0;
 }
 
 // ---- 2D FP32 blocks of 16x16 cells, one warp per block --------------------
@@ -2032,7 +2032,8 @@ int rbgs_bulk_error(int *err, cudaStream_t s, bool clear) {
 // are; the red cells are then updated with the tiled sweep's arithmetic and
 // the whole tile is written.  Same values as k_prolong + k_rbgs_tile.
 
-template <typename T, int ND>
+// FAC: L has the FP64 smoother's factors, which need no diagonal.
+template <typename T, int ND, bool FAC>
 __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, BlockList L, T *__restrict__ phi,
                                                             const T *__restrict__ rhs, const int *guard,
                                                             BlockList X) {
@@ -2101,16 +2102,16 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
         vc = vk = u ? u[d] : c.tff[d][fb + fx];
         vv = prolonged_value<T, ND>(t, c, n, ni, phi, hxe ? hxe[kHXPar + f] : -1);
       } else if (ty == 1) {
-        if (t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
+        if (!FAC && t.bc_type[b * 6 + f] != kBCNeumann) vc = (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0;
       } else if (ty == 2) {
         vc = vk = cf_face<T, ND>(c, t, b, f, ijk);
         vv = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hxe);
       } else {  // not at the finest level of a tower
-        vc = cf_face<T, ND>(c, t, b, f, ijk);
+        if constexpr (!FAC) vc = cf_face<T, ND>(c, t, b, f, ijk);
         vk = (T)1;
         vv = refined_sum<T, ND, false>(t, c, b, f, ijk, phi, hxe);
       }
-      hc[e] = vc;
+      if constexpr (!FAC) hc[e] = vc;
       hk[e] = vk;
       hv[e] = vv;
     }
@@ -2120,7 +2121,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
       int ijk[3];
       color_cell_fast<ND>(h, t, 0, ijk);
       const int ci = t.lnb >= 0 ? ijk[0] + ((ijk[1] + (ijk[2] << t.lnb)) << t.lnb) : encode(ijk, nb);
-      T diag = c.alpha * dv;
+      T diag = FAC ? (T)0 : c.alpha * dv;
       T off = 0;
 #pragma unroll
       for (int f = 0; f < 2 * ND; f++) {
@@ -2136,18 +2137,18 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
             fx = ci + s * nb * nb;
           const T coef = u ? u[d] : c.tff[d][fb + fx];
           const int stride = d == 0 ? 1 : (d == 1 ? nb : nb * nb);
-          diag += coef;
+          if constexpr (!FAC) diag += coef;
           off = fma_t(coef, tile[ci + (s ? stride : -stride)], off);
         } else {
           const int q0 = d == 0 ? 1 : 0, q1 = d == 2 ? 1 : 2;
           const int m = ijk[q0] + (ND == 3 ? nb * ijk[q1] : 0);
           const int e = f * nface + m;
-          diag += hc[e];
+          if constexpr (!FAC) diag += hc[e];
           off = fma_t(hk[e], hv[e], off);
         }
       }
       T unew = 0;
-      if (sizeof(T) == 8 && L.sa) {
+      if constexpr (FAC) {
         bool inner = true;
 #pragma unroll
         for (int q = 0; q < ND; q++) inner = inner && ijk[q] > 0 && ijk[q] < nb - 1;
@@ -2155,7 +2156,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, 
         const bool ui = u && inner;
         const T iav = ui ? u[7] : (T)L.ia[fo];  // 0 in a solid cell
         unew = fma_t(rhs[cb + ci], ui ? u[6] : (T)L.sa[fo], off * iav);
-        if (iav != (T)0) unew = relax(c.omega, unew, tile[ci]);
+        if (nonzero(iav)) unew = relax(c.omega, unew, tile[ci]);
       } else {
         const T vfv = u ? (T)1 : c.vf[cb + ci];
         if (vfv > 0 && diag > 0) unew = relax(c.omega, fast_div(fma_t(rhs[cb + ci] * dv, vfv, off), diag), tile[ci]);
@@ -2189,13 +2190,19 @@ void launch_prolong_red(const Topo &t, const Coef<T> &c, const BlockList &L, T *
   }
   const int nface = t.ndim == 3 ? t.nb * t.nb : t.nb;
   const size_t smem = sizeof(T) * ((size_t)t.ncell + 3 * 2 * t.ndim * (size_t)nface);
-  ensure_max_smem(t.ndim == 2 ? (const void *)k_prolong_red<T, 2> : (const void *)k_prolong_red<T, 3>, 200 * 1024);
   const int threads = std::min(kThreads, ((t.ncell >> 1) + 31) / 32 * 32);
   const int grid = std::min(L.n + X.n, L.pb ? kReducedGrid : 152 * 64);
-  if (t.ndim == 2)
-    launch_k(pdl, k_prolong_red<T, 2>, grid, threads, smem, s, t, c, L, phi, rhs, guard, X);
-  else
-    launch_k(pdl, k_prolong_red<T, 3>, grid, threads, smem, s, t, c, L, phi, rhs, guard, X);
+  auto go = [&](auto k) {
+    ensure_max_smem((const void *)k, 200 * 1024);
+    launch_k(pdl, k, grid, threads, smem, s, t, c, L, phi, rhs, guard, X);
+  };
+  if constexpr (sizeof(T) == 8) {
+    if (L.sa) {
+      t.ndim == 2 ? go(k_prolong_red<T, 2, true>) : go(k_prolong_red<T, 3, true>);
+      return;
+    }
+  }
+  t.ndim == 2 ? go(k_prolong_red<T, 2, false>) : go(k_prolong_red<T, 3, false>);
 }
 
 template <typename T, int ND>
@@ -2230,7 +2237,13 @@ template <typename T, int ND, int MINB, int CPT>
 static void rbgs_ilp_go(const Topo &t, const Coef<T> &c, const BlockList &L, int color, T *phi, const T *rhs,
                         const int *guard, cudaStream_t s, bool pdl, dim3 grid, int threads) {
   grid.y = std::min((L.n + CPT - 1) / CPT, L.pb ? kReducedGrid : 65535);
-  launch_k(pdl, k_rbgs_ilp<T, ND, MINB, CPT>, grid, threads, 0, s, t, c, L, color, phi, rhs, guard);
+  if constexpr (sizeof(T) == 8) {
+    if (L.sa) {
+      launch_k(pdl, k_rbgs_ilp<T, ND, MINB, CPT, true>, grid, threads, 0, s, t, c, L, color, phi, rhs, guard);
+      return;
+    }
+  }
+  launch_k(pdl, k_rbgs_ilp<T, ND, MINB, CPT, false>, grid, threads, 0, s, t, c, L, color, phi, rhs, guard);
 }
 
 template <typename T, int ND>

@@ -329,6 +329,13 @@ __device__ __forceinline__ double fast_div(double a, double b) { return a / b; }
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// v > 0 and v != 0 without the FP64 pipe (2 lanes per clock): +0 < bits <= +inf
+__device__ __forceinline__ bool positive(float v) { return v > 0.f; }
+__device__ __forceinline__ bool positive(double v) {
+  return (unsigned long long)__double_as_longlong(v) - 1ull < 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ bool nonzero(double v) { return (__double_as_longlong(v) << 1) != 0; }
+
 // the relaxed red-black update of a fluid cell, u_old + omega (u_gs - u_old)
 // (successive over-relaxation for omega > 1); omega 1 returns u_gs itself,
 // the plain Gauss-Seidel update with the same bits.  omega is a launch
@@ -337,6 +344,16 @@ template <typename T>
 __device__ __forceinline__ T relax(T omega, T unew, T old) {
   return omega == (T)1 ? unew : fma_t(omega, unew - old, old);
 }
+
+template <typename T, int ND, bool FAC>
+struct SmoothOps;
+template <typename T, int ND, bool FAC>
+__device__ __forceinline__ void smooth_gather(const Topo &t, const Coef<T> &c, int b, uint16_t ft, const int ijk[3],
+                                              const T *__restrict__ phi, const T *__restrict__ rhs,
+                                              const double *sa, const double *ia, const int *__restrict__ hx,
+                                              SmoothOps<T, ND, FAC> &o);
+template <typename T, int ND, bool FAC>
+__device__ __forceinline__ void smooth_update(const Coef<T> &c, const SmoothOps<T, ND, FAC> &o, T *__restrict__ phi);
 
 // red-black update of the device solve's V-cycle: the smoother of
 // smooth_cell with 32-bit shift indexing, FMA accumulation and a fast
@@ -349,6 +366,14 @@ __device__ __forceinline__ void smooth_cell_fast(const Topo &t, const Coef<T> &c
                                                  const int ijk[3], T *__restrict__ phi, const T *__restrict__ rhs,
                                                  const double *sa = nullptr, const double *ia = nullptr,
                                                  const int *__restrict__ hx = nullptr) {
+  if constexpr (sizeof(T) == 8 && !CG) {
+    if (sa) {  // (in code of its own: the sum of the diagonal is half of a sweep's FP64 work)
+      SmoothOps<T, ND, true> o;
+      smooth_gather<T, ND, true>(t, c, b, ft, ijk, phi, rhs, sa, ia, hx, o);
+      smooth_update<T, ND, true>(c, o, phi);
+      return;
+    }
+  }
   const int nb = t.nb;
   const int ci = t.lnb >= 0 ? ijk[0] + ((ijk[1] + (ijk[2] << t.lnb)) << t.lnb) : encode(ijk, nb);
   const long cb = (long)b * t.ncell;
@@ -394,7 +419,7 @@ __device__ __forceinline__ void smooth_cell_fast(const Topo &t, const Coef<T> &c
       }
     }
   }
-  if (sizeof(T) == 8 && sa) {
+  if (CG && sizeof(T) == 8 && sa) {
     const bool ui = u && inner;  // interior cell of a constant-coefficient block
     const T iav = ui ? u[7] : (T)ia[ci];  // 0 in a solid cell
     T unew = fma_t(ld<CG>(&rhs[cb + ci]), ui ? u[6] : (T)sa[ci], off * iav);
@@ -420,26 +445,32 @@ __device__ __forceinline__ void smooth_cell_fast(const Topo &t, const Coef<T> &c
 // same as smooth_cell_fast's.  A thread gathers all its cells before
 // updating any, so that their global loads are in flight together (none of
 // them reads a cell that the launch writes).
-template <typename T, int ND>
+// FAC: a list with the FP64 smoother's factors (sa, ia), which need no
+// diagonal: neither its parts nor their sum is formed, and a physical face
+// costs nothing.  An FP64 sweep is bound by the FP64 pipe (2 lanes per clock
+// and SM), and the diagonal was 5 of a 2D cell's 12 operations: 32 problems,
+// 5.4 M cells, 21.5 -> 13.3 us a launch (one cell per thread, k_rbgs, which
+// gains most from the registers; k_rbgs_ilp's two cells: 16.4).
+template <typename T, int ND, bool FAC>
 struct SmoothOps {
   long q;
-  T dv, r, vf;
-  T dp[2 * ND], kc[2 * ND], v[2 * ND];
-  double sa, ia;
-  bool fac;
+  T dv, r, vf;  // FAC: vf is sa, dv is ia
+  T dp[FAC ? 1 : 2 * ND], kc[2 * ND], v[2 * ND];
 };
-template <typename T, int ND>
+template <typename T, int ND, bool FAC>
 __device__ __forceinline__ void smooth_gather(const Topo &t, const Coef<T> &c, int b, uint16_t ft, const int ijk[3],
                                               const T *__restrict__ phi, const T *__restrict__ rhs,
                                               const double *sa, const double *ia, const int *__restrict__ hx,
-                                              SmoothOps<T, ND> &o) {
+                                              SmoothOps<T, ND, FAC> &o) {
   const int nb = t.nb;
   const int ci = t.lnb >= 0 ? ijk[0] + ((ijk[1] + (ijk[2] << t.lnb)) << t.lnb) : encode(ijk, nb);
   const long cb = (long)b * t.ncell;
   const long fb = (long)b * t.nfb;
   const T *u = uniform_of(c, b);
   o.q = cb + ci;
-  o.dv = geom(c, b, 6);
+  auto part = [&](int f, T v) {
+    if constexpr (!FAC) o.dp[f] = v;
+  };
   bool inner = true;
 #pragma unroll
   for (int f = 0; f < 2 * ND; f++) {
@@ -455,53 +486,53 @@ __device__ __forceinline__ void smooth_gather(const Topo &t, const Coef<T> &c, i
       fx = ci + s * nb * nb;
     if (!bnd) {
       const int stride = d == 0 ? 1 : (d == 1 ? nb : nb * nb);
-      o.dp[f] = o.kc[f] = u ? u[d] : c.tff[d][fb + fx];
+      part(f, o.kc[f] = u ? u[d] : c.tff[d][fb + fx]);
       o.v[f] = phi[cb + ci + (s ? stride : -stride)];
       continue;
     }
     const int ty = face_type_of(ft, f);
     if (ty == 0) {
-      o.dp[f] = o.kc[f] = u ? u[d] : c.tff[d][fb + fx];
+      part(f, o.kc[f] = u ? u[d] : c.tff[d][fb + fx]);
       o.v[f] = same_level_ghost<T, false>(t, b, f, ijk, phi, hx);
     } else if (ty == 1) {
-      o.dp[f] = t.bc_type[b * 6 + f] != kBCNeumann ? (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0 : (T)0;
+      if constexpr (!FAC) part(f, t.bc_type[b * 6 + f] != kBCNeumann ? (u ? u[d] : c.tff[d][fb + fx]) * (T)2.0 : (T)0);
       o.kc[f] = (T)0;
       o.v[f] = (T)0;
     } else if (ty == 2) {
-      o.dp[f] = o.kc[f] = cf_face<T, ND>(c, t, b, f, ijk);
+      part(f, o.kc[f] = cf_face<T, ND>(c, t, b, f, ijk));
       o.v[f] = fine_crse_ghost<T, ND, false>(t, b, f, ijk, phi, hx);
     } else {
-      o.dp[f] = cf_face<T, ND>(c, t, b, f, ijk);
+      if constexpr (!FAC) part(f, cf_face<T, ND>(c, t, b, f, ijk));
       o.kc[f] = (T)1;
       o.v[f] = refined_sum<T, ND, false>(t, c, b, f, ijk, phi, hx);
     }
   }
   o.r = rhs[cb + ci];
-  o.fac = sizeof(T) == 8 && sa;
-  if (o.fac) {
+  if constexpr (FAC) {
     const bool ui = u && inner;
-    o.sa = ui ? (double)u[6] : sa[ci];
-    o.ia = ui ? (double)u[7] : ia[ci];
-    o.vf = (T)0;
+    o.vf = ui ? u[6] : (T)sa[ci];
+    o.dv = ui ? u[7] : (T)ia[ci];
   } else {
     o.vf = u ? (T)1 : c.vf[cb + ci];
-    o.sa = o.ia = 0.0;
+    o.dv = geom(c, b, 6);
   }
 }
-template <typename T, int ND>
-__device__ __forceinline__ void smooth_update(const Coef<T> &c, const SmoothOps<T, ND> &o, T *__restrict__ phi) {
-  T diag = c.alpha * o.dv;
+template <typename T, int ND, bool FAC>
+__device__ __forceinline__ void smooth_update(const Coef<T> &c, const SmoothOps<T, ND, FAC> &o, T *__restrict__ phi) {
   T off = 0;
+  if constexpr (FAC) {
 #pragma unroll
-  for (int f = 0; f < 2 * ND; f++) {
-    diag += o.dp[f];
-    off = fma_t(o.kc[f], o.v[f], off);
-  }
-  if (o.fac) {
-    T unew = fma_t(o.r, (T)o.sa, off * (T)o.ia);
-    if (c.omega != (T)1 && o.ia != 0.0) unew = relax(c.omega, unew, phi[o.q]);
+    for (int f = 0; f < 2 * ND; f++) off = fma_t(o.kc[f], o.v[f], off);
+    T unew = fma_t(o.r, o.vf, off * o.dv);
+    if (c.omega != (T)1 && nonzero(o.dv)) unew = relax(c.omega, unew, phi[o.q]);
     phi[o.q] = unew;
     return;
+  }
+  T diag = c.alpha * o.dv;
+#pragma unroll
+  for (int f = 0; f < 2 * ND; f++) {
+    if constexpr (!FAC) diag += o.dp[f];
+    off = fma_t(o.kc[f], o.v[f], off);
   }
   T unew = 0;
   if (o.vf > 0 && diag > 0) {
