@@ -170,7 +170,7 @@ __host__ __device__ __forceinline__ bool block_off(const BlockList &L, int b) {
 
 // The dense FP64 bottom solve: one inverse per connected component of the
 // level-1 blocks (a forest of independent problems has one per problem),
-// rows grouped by component, one CTA tile per 8 rows.
+// rows grouped by component, one CTA per tile of tile_rows rows.
 struct BottomDev {
   const double *binv;          // the components' row-major inverses, back to back
   const int *blocks;           // bottom-level block of every ncell rows, in row order
@@ -184,8 +184,9 @@ struct BottomDev {
   // or, instead, an FP16 copy with one FP32 scale per row (entry = h * scale)
   const unsigned short *binv16 = nullptr;
   const float *rscale = nullptr;
+  int tile_rows = 8;
 };
-constexpr int kBottomTileRows = 8;
+constexpr int kBottomWarps = 8;  // of a CTA; a tile has one row per warp, or four
 
 // one phase of the cooperative V-cycle program (mac_vcycle.cu)
 enum PhaseOp { kPhaseRestrict = 0, kPhaseBottom = 1, kPhaseProlong = 2, kPhaseSmooth = 3, kPhaseOut = 4 };

@@ -880,7 +880,7 @@ __global__ void __launch_bounds__(kThreads) k_face_coef(Topo t, const double *ge
   // division is about 20 operations of the FP64 pipe, whatever the number of
   // lanes that need it), and a product with 1 or 0 is not formed: B and the
   // area fraction are 1 or 0 on most faces.  13.75 M cells: 1050 us with a
-  // division per face, 587 with one per thread of a CTA, XXX now.
+  // division per face, 587 with one per thread of a CTA, 262 now.
   const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
   for (long it = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; it < (long)t.nblocks * t.ndim; it += warps) {
     const int b = (int)(it / t.ndim), d = (int)(it - (long)b * t.ndim);
@@ -2032,9 +2032,11 @@ int rbgs_bulk_error(int *err, cudaStream_t s, bool clear) {
 // are; the red cells are then updated with the tiled sweep's arithmetic and
 // the whole tile is written.  Same values as k_prolong + k_rbgs_tile.
 
-// FAC: L has the FP64 smoother's factors, which need no diagonal.
+// FAC: L has the FP64 smoother's factors, which need no diagonal (and leave
+// registers for six CTAs per SM: 30.3 us at four, 26.5 at six; 33.5 with the
+// diagonal; 32 problems, 5.4 M cells).
 template <typename T, int ND, bool FAC>
-__global__ void __launch_bounds__(kThreads, 4) k_prolong_red(Topo t, Coef<T> c, BlockList L, T *__restrict__ phi,
+__global__ void __launch_bounds__(kThreads, FAC ? 6 : 4) k_prolong_red(Topo t, Coef<T> c, BlockList L, T *__restrict__ phi,
                                                             const T *__restrict__ rhs, const int *guard,
                                                             BlockList X) {
   extern __shared__ __align__(16) unsigned char pr_smem[];

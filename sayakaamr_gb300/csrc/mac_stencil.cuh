@@ -617,7 +617,7 @@ __device__ __forceinline__ void prolong_cell(const Topo &t, const Coef<T> &c, in
   phi[q] = c.vf[q] > 0 ? v : (T)0;
 }
 
-// rows [row0, row0 + 8) of one component of the bottom solve:
+// rows [row0, row0 + tile_rows) of one component of the bottom solve:
 // corr = Binv_c * resid_c, one warp per row; rv: shared memory for the
 // component's residual (max_n doubles); every thread of the CTA calls it
 // a component's residual (rows r0 .. r0+m, whole blocks of ncell rows) into
@@ -651,8 +651,8 @@ __device__ __forceinline__ void bottom_tile(const BottomDev &bd, int tile, const
     float *rf = reinterpret_cast<float *>(rv);
     bottom_gather<T, CG>(bd, r0, m, resid, rf);
     __syncthreads();
-    const int lane = threadIdx.x & 31, row = bd.tile_row0[tile] + (threadIdx.x >> 5);
-    if ((threadIdx.x >> 5) < kBottomTileRows && row < m) {
+    const int lane = threadIdx.x & 31, row0 = bd.tile_row0[tile], end = min(m, row0 + bd.tile_rows);
+    for (int row = row0 + (threadIdx.x >> 5); row < end && threadIdx.x < 32 * kBottomWarps; row += kBottomWarps) {
       // rows start on 16-byte boundaries: m and the component offsets are
       // multiples of the block size (at least 64 cells)
       const uint4 *a8 = reinterpret_cast<const uint4 *>(bd.binv16 + bd.comp_off[c] + (long long)row * m);
@@ -695,8 +695,8 @@ __device__ __forceinline__ void bottom_tile(const BottomDev &bd, int tile, const
     float *rf = reinterpret_cast<float *>(rv);
     bottom_gather<T, CG>(bd, r0, m, resid, rf);
     __syncthreads();
-    const int lane = threadIdx.x & 31, row = bd.tile_row0[tile] + (threadIdx.x >> 5);
-    if ((threadIdx.x >> 5) < kBottomTileRows && row < m) {
+    const int lane = threadIdx.x & 31, row0 = bd.tile_row0[tile], end = min(m, row0 + bd.tile_rows);
+    for (int row = row0 + (threadIdx.x >> 5); row < end && threadIdx.x < 32 * kBottomWarps; row += kBottomWarps) {
       const float4 *a4 = reinterpret_cast<const float4 *>(bd.binv32 + bd.comp_off[c] + (long long)row * m);
       const float4 *r4 = reinterpret_cast<const float4 *>(rf);
       float s = 0.f;
@@ -731,8 +731,8 @@ __device__ __forceinline__ void bottom_tile(const BottomDev &bd, int tile, const
   }
   bottom_gather<T, CG>(bd, r0, m, resid, rv);
   __syncthreads();
-  const int lane = threadIdx.x & 31, row = bd.tile_row0[tile] + (threadIdx.x >> 5);
-  if ((threadIdx.x >> 5) < kBottomTileRows && row < m) {
+  const int lane = threadIdx.x & 31, row0 = bd.tile_row0[tile], end = min(m, row0 + bd.tile_rows);
+  for (int row = row0 + (threadIdx.x >> 5); row < end && threadIdx.x < 32 * kBottomWarps; row += kBottomWarps) {
     const double *a = bd.binv + bd.comp_off[c] + (long long)row * m;
     // four independent loads in flight per lane, four partial sums
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;

@@ -73,3 +73,21 @@ def test_per_problem_states_take_fewer_iteration_blocks():
     cells = np.array([p.leaf_cells for p in parts])
     assert own["iterations"] <= shared["iterations"] + 1
     assert np.sum(its * cells) < shared["iterations"] * np.sum(cells), (its, shared["iterations"])
+
+
+@pytest.mark.parametrize("half", [1, 0])
+def test_many_small_components_share_a_bottom_cta(half):
+    """40 problems with one 16^2 block each at the bottom level: 10,240 rows of
+    256, four per warp; every copy of a problem has the solution of the forest
+    of five (one row per warp)"""
+    rng = np.random.default_rng(44)
+    parts = [workloads.batch_problem(rng, "b%d" % k) for k in range(5)]
+    out = []
+    for group in (parts, parts * 8):
+        S = workloads.make_solver(workloads.forest(group, "f"))
+        S.set_params(tol_rel=1e-8, tol_abs=0.0, use_mg_precond=1, max_iter=500, precision=1, bottom=1,
+                     bottom_half=half, bottom_level=1)
+        info = S.cg_solve()
+        assert info["status"] == 0, info
+        out.append(S.get_sol_compact().reshape(len(group) // 5, -1))
+    assert np.max(np.abs(out[1] - out[0])) < SOL_RTOL * np.max(np.abs(out[0]))
