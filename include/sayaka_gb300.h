@@ -116,7 +116,9 @@ typedef struct sayaka_params {
   int32_t cluster_cells;  /* vcycle_kernel 2: runs of consecutive phases that each touch at most this many
                              cells share one cluster launch; larger phases get their own launch (16384) */
   int32_t smooth_variant; /* device smoother launch bounds (register cap): -1 = autotuned at prepare by
-                             timing every variant on the finest level (default), 0..9 = fixed */
+                             timing every variant on the finest level (default), 0..13 = fixed: 10 two
+                             cells per thread; 11..13, FP32, one warp per 16x16 block (register caps 64, 48,
+                             80) or one thread per row of an 8^3 block, elsewhere as 3.  The same values */
   int32_t learned;        /* device path with the FP32 V-cycle: 1 = add the trained learned block
                              correction after every V-cycle (default 0); see sayaka_mac_learned_* */
   int32_t bottom_level;   /* device path: level of the dense bottom solve; 0 = auto (the finest level below the
@@ -150,13 +152,17 @@ typedef struct sayaka_params {
                              on tcgen05 with the accumulator in tensor memory (default); 0 = on mma.sync warp
                              MMAs (the same network, products summed in another order) */
   int32_t vcycle_out;     /* how the BiCGSTAB kernels read the FP32 V-cycle's output: 0 = in place (widened
-                             exactly on the integer pipe where they read it) in 2D and on 3D towers of at most
-                             2,097,152 cells, widened once into FP64 vectors on larger 3D towers (default); 1 =
+                             exactly on the integer pipe where they read it) in 2D, on 3D towers of at most
+                             2,097,152 cells and on larger ones at least half of whose blocks have equal
+                             spacings and constant coefficients, widened once into FP64 vectors on the others
+                             (default); 1 =
                              in place, the operator evaluated in double-float on the FP32 pipe; 2 = always
                              widened; 3 = always in place */
   int32_t prolong_form;   /* device V-cycle, the prolongation fused with the first red sweep of its level:
-                             1 = one warp per block with the block in registers (2D FP32 16x16 blocks,
-                             default; elsewhere form 0), 0 = one CTA per block with a shared-memory tile; the
+                             1 = one warp per 16x16 block with the block in registers, one thread per row of
+                             an 8^3 block (FP32; elsewhere form 0), and a tower's prolongation and sweeps in
+                             one cooperative launch where its blocks of 8 or 16 cells (2D) or 8 (3D) fit the
+                             device at once (default); 0 = one CTA per block with a shared-memory tile; the
                              same values */
   int32_t learned_loss;   /* training loss of the learned correction u: 0 = the residual u leaves under the
                              block-local operator (default); 1 = the distance of u to the block-local part of the
