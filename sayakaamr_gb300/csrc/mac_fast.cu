@@ -1349,6 +1349,18 @@ void MacGpu::ensure_df_factors() {
   df_version_ = coef_version_;
 }
 
+// The arrays that only some parameters read, from the current coefficients: the
+// FP64 smoother factors (the FP64 V-cycle and the learned correction), the
+// double-float factors (vcycle_out 1) and the FP32 copies of B and the area
+// fractions (the learned correction).  A solve without a captured graph may run
+// with other parameters than its preparation saw, so every solve asks for what
+// it reads; all three return at once where nothing changed.
+void MacGpu::ensure_derived() {
+  if (prm_.precision == 0 || learned_active()) ensure_smooth_factors();
+  if (prm_.vcycle_out == 1) ensure_df_factors();
+  if (learned_active()) ensure_fp32_faces();
+}
+
 // the coarse/fine face tables from the current coefficients
 void MacGpu::build_cf() {
   const long n = (long)tt_.num_blocks * 2 * tt_.ndim * (tt_.ndim == 3 ? tt_.nb * tt_.nb : tt_.nb);
@@ -2198,6 +2210,8 @@ int MacGpu::cg_solve_enqueue() {
   if (prm_.vcycle_kernel && (program_npost_ != prm_.n_post || program_order_ != prm_.sublevel_order ||
                              program_bot_ != bot_level_))
     return -1;
+  ensure_derived();
+  if (!err_.empty()) return -1;
   return enqueue_solve();
 }
 
@@ -2310,16 +2324,10 @@ int MacGpu::prepare_device() {
   }
   bind_uniform();
   choose_active();
-  // the FP64 smoother factors serve the FP64 V-cycle and the learned
-  // correction only: an FP32 solve does not build them
-  if (prm_.precision == 0 || learned_active()) ensure_smooth_factors();
+  ensure_derived();
   tune_smoother(prm_.precision);
   if (prm_.precision == 1) ensure_flow();
-  if (prm_.vcycle_out == 1) ensure_df_factors();
-  if (learned_active()) {
-    ensure_fp32_faces();
-    learned_prepare();
-  }
+  if (learned_active()) learned_prepare();
   if (!err_.empty()) return -1;
   if (prm_.vcycle_kernel && (program_npost_ != prm_.n_post || program_order_ != prm_.sublevel_order ||
                              program_bot_ != bot_level_))

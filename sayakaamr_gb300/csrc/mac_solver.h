@@ -406,6 +406,7 @@ class MacGpu {
   float *d_uni32_ = nullptr;
   void build_cf();
   void ensure_df_factors();
+  void ensure_derived();
   void ensure_fp32_faces();
   long df_version_ = -1, faces32_version_ = -1;  // coefficient versions of those copies
   double *d_cf64_ = nullptr;  // coarse/fine face coefficients (Coef::cf)
