@@ -235,7 +235,7 @@ void MacGpu::zero_solid() {
 // list r = entries [a, b) of d, reduced to the active blocks while a solve
 // that walks the reduced lists is recorded
 BlockList MacGpu::active(BlockList r, const DevList &d, int a, int b) const {
-  if (!(solve_lists_ && act_on_) || d.n == 0) return r;
+  if (!(solve_lists_ && reduced()) || d.n == 0) return r;
   r.blocks = d.act.blocks;
   r.ftypes = d.act.ftypes;
   r.hx = d.act.hx;

@@ -1849,7 +1849,7 @@ void MacGpu::vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *o
         // capacity without another capture)
         const int grid = std::min(towers_[l].par.n, flow_capacity_);
         CK(launch_flow(topo_, c, parity_list(l, 0, false), parity_list(l, 1, false), l, prm_.n_post, grid, corr, resid,
-                       guard, d_flow_words_, d_flow_epoch_, act_on_ ? d_active_ : nullptr, stream_));
+                       guard, d_flow_words_, d_flow_epoch_, reduced() ? d_active_ : nullptr, stream_));
         continue;
       }
     }
@@ -1888,7 +1888,7 @@ void MacGpu::vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *o
 
 // tower l can be smoothed by launch_flow
 int MacGpu::flow_entries(int l) const {
-  return act_on_ && l < (int)n_act_par_.size() ? n_act_par_[l] : towers_[l].par.n;
+  return reduced() && l < (int)n_act_par_.size() ? n_act_par_[l] : towers_[l].par.n;
 }
 bool MacGpu::flow_fits(int l) const {
   return d_flow_words_ && prm_.sublevel_order == 1 && prm_.prolong_form == 1 &&
@@ -1980,7 +1980,7 @@ bool MacGpu::vcycle_in_place() const {
   if (learned_active() || prm_.precision != 1) return false;
   if (prm_.vcycle_out != 0) return prm_.vcycle_out != 2;
   const DevList &top = towers_[finest_].all;
-  return tt_.ndim == 2 || (long)top.n * ncell_ <= kDirectF32Cells || (!multi() && 2l * n_iso_ >= n_act_);
+  return tt_.ndim == 2 || (long)top.n * ncell_ <= kDirectF32Cells || (!multi() && act_version_ == coef_version_ && 2l * n_iso_ >= n_act_);
 }
 template <typename T>
 void MacGpu::iteration_device(T *resid, T *corr, const Coef<T> &c) {
@@ -2170,7 +2170,7 @@ void MacGpu::capture_loop(int precision) {
   graph_pform_ = prm_.prolong_form;
   graph_vout_ = prm_.vcycle_out;
   graph_omega_ = prm_.relax_omega;
-  graph_act_ = (int)act_on_;
+  graph_act_ = (int)reduced();
   graph_direct_ = (int)vcycle_in_place();
   graph_flow_ = flow_mask();
 }
@@ -2183,7 +2183,7 @@ bool MacGpu::graph_stale() const {
          graph_order_ != prm_.sublevel_order || graph_smoother_ != prm_.smoother ||
          graph_inner_ != prm_.inner_sweeps || graph_multi_ != (int)multi() || graph_uniform_ != prm_.uniform ||
          graph_pform_ != prm_.prolong_form || graph_vout_ != prm_.vcycle_out ||
-         graph_omega_ != prm_.relax_omega || graph_act_ != (int)act_on_ ||
+         graph_omega_ != prm_.relax_omega || graph_act_ != (int)reduced() ||
          graph_direct_ != (int)vcycle_in_place() || graph_flow_ != flow_mask();
 }
 
@@ -2235,7 +2235,7 @@ int MacGpu::enqueue_solve() {
     for (int c = 0; c < ncomp_; c++) h_stc_[c] = init;
     CKR_(cudaMemcpyAsync(d_stc_, h_stc_, ncomp_ * sizeof(FState), cudaMemcpyHostToDevice, stream_), -1);
   }
-  if (act_on_) zero_solid();
+  if (reduced()) zero_solid();
   // prologue: x0 = sol, x = 0, r = rhs - A x0, rhat = r, |r0|, rho
   k_pro_copy<<<ew_grid(w), kTPB, 0, stream_>>>(TL, ncell_, vec_[kSOL], vec_[kX0], vec_[kX]);
   double *PART = mp ? d_cpart_ : d_part_;

@@ -639,7 +639,7 @@ BlockList MacGpu::sublevel_list(int L, int l) const {
   r.hx = t.all.hx + (long)b * kHX;
   if (L < (int)d_sfac_.size() && d_sfac_[L]) {
     const long w = (long)t.all.n * ncell_;
-    const long o = solve_lists_ && act_on_ ? 0 : (long)b * ncell_;  // reduced: by the entry's full place
+    const long o = solve_lists_ && reduced() ? 0 : (long)b * ncell_;  // reduced: by the entry's full place
     r.sa = d_sfac_[L] + o;
     r.ia = d_sfac_[L] + w + o;
   }
@@ -661,7 +661,7 @@ BlockList MacGpu::parity_list(int L, int g, bool skip_top) const {
   r.hx = t.par.hx + (long)b * kHX;
   if (L < (int)d_pfac_.size() && d_pfac_[L]) {
     const long w = (long)t.par.n * ncell_;
-    const long o = solve_lists_ && act_on_ ? 0 : (long)b * ncell_;
+    const long o = solve_lists_ && reduced() ? 0 : (long)b * ncell_;
     r.sa = d_pfac_[L] + o;
     r.ia = d_pfac_[L] + w + o;
   }

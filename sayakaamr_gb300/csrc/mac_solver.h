@@ -393,7 +393,11 @@ class MacGpu {
   // the BiCGSTAB kernels read the FP32 V-cycle's output in place
   bool vcycle_in_place() const;
   long act_version_ = -1;              // coefficient version of the reduced lists
-  bool act_on_ = false;                // the solve walks the reduced lists
+  bool act_on_ = false;                // enough solid blocks for the reduced lists (choose_active)
+  // the solve walks the reduced lists.  One state per problem and the learned
+  // correction walk the full ones, also when they are switched on after the
+  // preparation
+  bool reduced() const { return act_on_ && !multi() && !learned_active(); }
   Coef<float> c32_{};
   FState *d_st_ = nullptr, *h_st_ = nullptr;
   double *d_part_ = nullptr;
