@@ -416,7 +416,11 @@ int sayaka_mac_residual_norm_noalloc(sayaka_mac *h, int32_t L, const double *x, 
  * `variant` (1..1024) red-black sweeps per block (in = phi, frozen outside
  * each block; in2 = rhs); which 3 = out = A x on the finest tower for x = in
  * rounded to FP32, with the double-float operator the BiCGSTAB iteration
- * applies to the FP32 V-cycle's output (in2 unused) */
+ * applies to the FP32 V-cycle's output (in2 unused).  Failure tests, which
+ * leave out alone: which 4 = the one-launch smoothing of tower L with the
+ * blocks of its second parity group left out and `variant` tries per wait, so
+ * that waits run out (the call reports it); which 5 = the solver's error word
+ * set as by a wait that ran out, for the next solve to find */
 int sayaka_mac_device_kernel_compact(sayaka_mac *h, int32_t which, int32_t L, int32_t variant, const double *in,
                                      const double *in2, double *out);
 /* one mg_smooth_level(L) (src/SayakaMacOperator.cpp:140-159, 1028-1112) */

@@ -647,6 +647,21 @@ class MacSolver:
                                                          out.ctypes.data_as(_f64p)), "device_hybrid_pass", self.h)
         return out
 
+    def fail_wait(self, L, tries):
+        """failure test: the one-launch smoothing of tower L with half of its
+        blocks left out and `tries` tries per wait; raises, as waits run out"""
+        y = self._cells()
+        a, pa = _f64(y)
+        _check(self.lib.sayaka_mac_device_kernel_compact(self.h, 4, int(L), int(tries), pa, None,
+                                                         y.ctypes.data_as(_f64p)), "fail_wait", self.h)
+
+    def set_wait_error(self):
+        """failure test: the solver's error word set as by a wait that ran out"""
+        y = self._cells()
+        a, pa = _f64(y)
+        _check(self.lib.sayaka_mac_device_kernel_compact(self.h, 5, 0, -1, pa, None, y.ctypes.data_as(_f64p)),
+               "set_wait_error", self.h)
+
     def restrict_sweep(self, x):
         out = self._cells()
         a, pa = _f64(x)

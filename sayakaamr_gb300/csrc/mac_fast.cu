@@ -348,9 +348,10 @@ struct EpiEnd {  // |r|, rhat.r of the next iteration
 };
 
 // ---- kernels -------------------------------------------------------------
-__global__ void k_set_cond(cudaGraphConditionalHandle h, const FState *st) {
+// the loop also ends where a bounded wait has run out (err)
+__global__ void k_set_cond(cudaGraphConditionalHandle h, const FState *st, const int *err) {
   pdl_enter();
-  cudaGraphSetConditional(h, st->done ? 0u : 1u);
+  cudaGraphSetConditional(h, st->done || *err ? 0u : 1u);
 }
 
 // x0 = sol, x = 0 on the tower
@@ -469,15 +470,17 @@ __global__ void k_vc_out(BlockList L, int ncell, const FState *st, const T *corr
 }
 
 // every problem's state read: the loop goes on while one is not done; the
-// shared state's done flag (the guard of the V-cycle kernels) is set once all are
-__global__ void k_set_cond_multi(cudaGraphConditionalHandle h, const FState *stc, int ncomp, FState *st) {
+// shared state's done flag (the guard of the V-cycle kernels) is set once all
+// are, or a bounded wait has run out (err)
+__global__ void k_set_cond_multi(cudaGraphConditionalHandle h, const FState *stc, int ncomp, FState *st,
+                                 const int *err) {
   pdl_enter();
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
   int a = 0;
   for (int c = threadIdx.x; c < ncomp; c += blockDim.x) a |= !stc[c].done;
-  if (a) atomicOr(&any, 1);
+  if (a && !*err) atomicOr(&any, 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     st->done = any ? 0 : 1;
@@ -1184,6 +1187,7 @@ void MacGpu::ensure_fast_buffers() {
   }
   if (dev_malloc(&d_st_, sizeof(FState)) != cudaSuccess) fail("alloc state");
   if (cudaMallocHost(&h_st_, sizeof(FState)) != cudaSuccess) fail("alloc pinned state");
+  if (cudaMallocHost(&h_err_, sizeof(int)) != cudaSuccess) fail("alloc pinned error word");
   if (dev_malloc(&d_part_, sizeof(double) * kMaxRedBlocks * 4) != cudaSuccess) fail("alloc partials");
   if (dev_malloc(&d_cnt_, sizeof(unsigned) * 4) != cudaSuccess) fail("alloc counter");
   cudaMemsetAsync(d_cnt_, 0, sizeof(unsigned) * 4, stream_);
@@ -2139,9 +2143,10 @@ void MacGpu::capture_loop(int precision) {
     iteration_device<double>(vec_[kRESID], vec_[kCORR], cd64_);
   solve_lists_ = false;
   if (multi())
-    launch_k(prm_.pdl != 0, k_set_cond_multi, 1, 256, 0, stream_, h, (const FState *)d_stc_, ncomp_, d_st_);
+    launch_k(prm_.pdl != 0, k_set_cond_multi, 1, 256, 0, stream_, h, (const FState *)d_stc_, ncomp_, d_st_,
+             (const int *)topo_.err);
   else
-    launch_k(prm_.pdl != 0, k_set_cond, 1, 1, 0, stream_, h, (const FState *)d_st_);
+    launch_k(prm_.pdl != 0, k_set_cond, 1, 1, 0, stream_, h, (const FState *)d_st_, (const int *)topo_.err);
   cudaGraph_t out = nullptr;
   CK_(cudaStreamEndCapture(stream_, &out));
   // count the kernel nodes of one iteration (reported as launches per step)
@@ -2251,7 +2256,7 @@ int MacGpu::enqueue_solve() {
     mp ? resid(k_op_red<2, 2, double, true>) : resid(k_op_red<2, 2, double, false>);
   else
     mp ? resid(k_op_red<3, 2, double, true>) : resid(k_op_red<3, 2, double, false>);
-  if (mp) k_set_cond_multi<<<1, 256, 0, stream_>>>(0, d_stc_, ncomp_, d_st_);
+  if (mp) k_set_cond_multi<<<1, 256, 0, stream_>>>(0, d_stc_, ncomp_, d_st_, topo_.err);
   if (prm_.max_iter > 0) {
     if (prm_.graph) {
       CKR_(cudaGraphLaunch(graph_exec_, stream_), -1);
@@ -2265,7 +2270,7 @@ int MacGpu::enqueue_solve() {
         else
           iteration_device<double>(vec_[kRESID], vec_[kCORR], cd64_);
         solve_lists_ = false;
-        if (mp) k_set_cond_multi<<<1, 256, 0, stream_>>>(0, d_stc_, ncomp_, d_st_);
+        if (mp) k_set_cond_multi<<<1, 256, 0, stream_>>>(0, d_stc_, ncomp_, d_st_, topo_.err);
         if (record_) {  // a collection solve keeps every iterate
           double *cp = nullptr;
           const size_t n = (size_t)tt_.num_blocks * ncell_;
@@ -2277,8 +2282,9 @@ int MacGpu::enqueue_solve() {
           record_->push_back(cp);
         }
         CKR_(cudaMemcpyAsync(h_st_, d_st_, sizeof(FState), cudaMemcpyDeviceToHost, stream_), -1);
+        CKR_(cudaMemcpyAsync(h_err_, topo_.err, sizeof(int), cudaMemcpyDeviceToHost, stream_), -1);
         CKR_(cudaStreamSynchronize(stream_), -1);
-        if (h_st_->done) break;
+        if (h_st_->done || *h_err_) break;
       }
     }
   }
@@ -2464,12 +2470,29 @@ int MacGpu::enqueue_kernel(int which, int L) {
 // solve's FP64 sweep, launch variant `variant` (-1: the tuned one); in = phi,
 // in2 = rhs.  Uses (and clobbers) the handle's work vectors.
 int MacGpu::device_kernel_compact(int which, int L, int variant, const double *in, const double *in2, double *out) {
-  if (which < 0 || which > 3 || !in || !out || ((which == 1 || which == 2) && !in2)) return 1;
+  if (which < 0 || which > 5 || !in || !out || ((which == 1 || which == 2) && !in2)) return 1;
   if ((which == 1 || which == 2) && (L < 1 || L > finest_ || towers_[L].all.n == 0)) return 1;
   if (which == 1 && variant >= kRbgsVariants) return 1;
   if (which == 2 && (variant < 1 || variant > 1024)) return 1;
+  if (which == 4 && (variant < 1 || variant > kFlowPolls || L < 2 || L > finest_)) return 1;
   if (prepare_device() != 0) return 2;
   ensure_smooth_factors();
+  if (which == 4) {
+    // the one-launch smoothing of tower L without the blocks of its second
+    // parity group: no one writes the words that the first group waits for
+    // across coarse/fine faces
+    const int m = L < (int)towers_.size() && flow_fits(L) ? parity_list(L, 0, false).n : 0;
+    if (m == 0 || m > flow_capacity_) return 1;
+    CKR_(cudaMemsetAsync(d_st_, 0, sizeof(FState), stream_), 2);
+    CKR_(launch_flow(topo_, c32_, parity_list(L, 0, false), BlockList{nullptr, nullptr, 0}, L, prm_.n_post, m,
+                     d_corr32_, d_resid32_, &d_st_->done, d_flow_words_, d_flow_epoch_, nullptr, stream_, variant),
+         2);
+  } else if (which == 5) {  // as a wait that ran out leaves the solver's error word
+    const int one = 1;
+    CKR_(cudaMemcpyAsync(topo_.err, &one, sizeof(int), cudaMemcpyHostToDevice, stream_), 2);
+    CKR_(cudaStreamSynchronize(stream_), 2);
+    return 0;
+  }
   const size_t n = (size_t)tt_.num_blocks * ncell_;
   if (which == 0) {
     const BlockList TL = tower_list(finest_);
@@ -2509,6 +2532,8 @@ int MacGpu::device_kernel_compact(int which, int L, int variant, const double *i
           nullptr, d_opP2_, d_opS2_, d_uni2_);
     CKR_(cudaGetLastError(), 2);
     CKR_(cudaMemcpyAsync(out, vec_[kV], n * sizeof(double), cudaMemcpyDeviceToHost, stream_), 2);
+  } else if (which == 4) {
+    // (above)
   } else if (which == 2) {
     // one block-hybrid pass over every sublevel of tower L, `variant`
     // red-black sweeps per block: in (frozen) -> out
@@ -2534,7 +2559,7 @@ int MacGpu::device_kernel_compact(int which, int L, int variant, const double *i
   }
   CKR_(cudaStreamSynchronize(stream_), 2);
   if (rbgs_bulk_error(topo_.err, stream_, true) > 0) {
-    fail("bulk-copy smoother: an mbarrier wait timed out");
+    fail("device smoother: a bounded wait timed out");
     return 2;
   }
   return err_.empty() ? 0 : 2;

@@ -26,8 +26,10 @@
 //
 // Every warp must be resident at once: the launch is cooperative and the host
 // only uses it when the tower fits (flow_fits).  A poll gives up after
-// kPollLimit tries, sets the solver's error word (the solve then reports a
-// CUDA error) and lets the warp run on without waiting.
+// `limit` tries, sets the solver's error word and lets its thread run on
+// without waiting.  A launch that finds the word set leaves the blocks alone,
+// and the solve's loop ends at its next test (k_set_cond) and reports a CUDA
+// error, so that one lost word costs one limit and not one per launch to come.
 #include <algorithm>
 
 #include "mac_device.h"
@@ -41,8 +43,6 @@ namespace {
 using namespace stencil;
 using Word = unsigned long long;
 
-constexpr int kPollLimit = 1 << 20;  // about half a second
-
 __device__ __forceinline__ void publish(Word *p, float v, unsigned tag) {
   const Word w = ((Word)tag << 32) | __float_as_uint(v);
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
@@ -54,14 +54,22 @@ __device__ __forceinline__ Word look(const Word *p) {
 }
 __device__ __forceinline__ bool tagged(Word w, unsigned tag) { return (unsigned)(w >> 32) == tag; }
 __device__ __forceinline__ float value(Word w) { return __uint_as_float((unsigned)w); }
-__device__ __forceinline__ float poll1(const Word *p, unsigned tag, int *err, bool &dead) {
+// the error word of the bounded waits
+struct Wait {
+  int *err, limit;
+};
+__device__ __forceinline__ bool given_up(const Topo &t) { return *(volatile const int *)t.err != 0; }
+// (unrolled by hand as the compiler does with a constant limit: rolled, a solve of
+// 16 thousand cells took 1,154 us instead of 1,002)
+__device__ __forceinline__ float poll1(const Word *p, unsigned tag, Wait wt, bool &dead) {
   Word w = 0;
-  for (int n = 0; n < kPollLimit; n++) {
+#pragma unroll 4
+  for (int n = 0; n < wt.limit; n++) {
     w = look(p);
     if (tagged(w, tag) || dead) return value(w);
   }
   dead = true;
-  atomicExch(err, 1);
+  atomicExch(wt.err, 1);
   return value(w);
 }
 // N words, on[i]: wanted (else left alone); all of a round's loads are in
@@ -70,9 +78,9 @@ __device__ __forceinline__ float poll1(const Word *p, unsigned tag, int *err, bo
 // instruction cache.)
 template <int N>
 __device__ __forceinline__ void poll(const Word *const (&p)[N], const unsigned (&tag)[N], const bool (&on)[N],
-                                     float (&x)[N], int *err, bool &dead) {
+                                     float (&x)[N], Wait wt, bool &dead) {
   Word w[N] = {};
-  for (int n = dead ? 1 : kPollLimit;;) {
+  for (int n = dead ? 1 : wt.limit;;) {
     bool all = true;
 #pragma unroll
     for (int i = 0; i < N; i++)
@@ -81,7 +89,7 @@ __device__ __forceinline__ void poll(const Word *const (&p)[N], const unsigned (
     for (int i = 0; i < N; i++) all = all && (!on[i] || tagged(w[i], tag[i]));
     if (all) break;
     if (--n > 0) continue;
-    if (!dead) atomicExch(err, 1);
+    if (!dead) atomicExch(wt.err, 1);
     dead = true;
     break;
   }
@@ -92,7 +100,7 @@ __device__ __forceinline__ void poll(const Word *const (&p)[N], const unsigned (
 // `up` words further, times their coefficients, in order; the first has colour
 // `odd`.  (Inlined: a call saves and restores the block's registers.)
 __device__ __forceinline__ float poll_fine(const Word *p, const float *__restrict__ cf, int up, int odd, unsigned red,
-                                           unsigned black, int *err, bool &dead) {
+                                           unsigned black, Wait wt, bool &dead) {
   const Word *q[4];
   unsigned tag[4];
   float f[4], v[4], x = 0.f;
@@ -103,7 +111,7 @@ __device__ __forceinline__ float poll_fine(const Word *p, const float *__restric
     f[n] = cf[(n & 1) + up * (n >> 1)];
     tag[n] = ((odd + n + (n >> 1)) & 1) ? black : red;
   }
-  poll<4>(q, tag, on, v, err, dead);
+  poll<4>(q, tag, on, v, wt, dead);
 #pragma unroll
   for (int n = 0; n < 4; n++) x += f[n] * v[n];
   return x;
@@ -122,7 +130,7 @@ template <int NB>
 __device__ __forceinline__ void flow_block(const Topo &t, const Coef<float> &c, const int *e, int group, int level,
                                            int nsweep, float *__restrict__ phi, const float *__restrict__ rhs,
                                            Word *__restrict__ words, unsigned tag0, const int *__restrict__ alive,
-                                           int lane, FlowHalo<NB> &sh) {
+                                           int limit, int lane, FlowHalo<NB> &sh) {
   constexpr int NC = NB * NB, Q = NB * NB / 64, LPR = 32 / NB;
   const int j = lane / LPR, c0 = (lane % LPR) * 2 * Q;
   const int2 ib = *reinterpret_cast<const int2 *>(e + kHXInfo);
@@ -266,6 +274,7 @@ __device__ __forceinline__ void flow_block(const Topo &t, const Coef<float> &c, 
       diag[k][q] = vf[k][q] > 0.f ? g : 0.f;  // 0: the cell stays at 0
     }
   bool dead = false;
+  const Wait wt{t.err, limit};
   for (int s = 0; s < nsweep; s++) {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
@@ -276,12 +285,12 @@ __device__ __forceinline__ void flow_block(const Topo &t, const Coef<float> &c, 
         const unsigned cross_red = group ? (h >> 1) + 1 : (h + 1) >> 1, cross_black = group ? (h + 1) >> 1 : h >> 1;
         float x;
         if (sl.ty == 0) {
-          x = poll1(sl.w, tag0 + ((h + 1) >> 1), t.err, dead);
+          x = poll1(sl.w, tag0 + ((h + 1) >> 1), wt, dead);
         } else if (sl.ty == 2) {
-          x = poll1(sl.w, tag0 + (sl.odd ? cross_black : cross_red), t.err, dead);
+          x = poll1(sl.w, tag0 + (sl.odd ? cross_black : cross_red), wt, dead);
         } else {
-          const float x0 = poll1(sl.w, tag0 + (sl.odd ? cross_black : cross_red), t.err, dead);
-          const float x1 = poll1(sl.w + 1, tag0 + (sl.odd ? cross_red : cross_black), t.err, dead);
+          const float x0 = poll1(sl.w, tag0 + (sl.odd ? cross_black : cross_red), wt, dead);
+          const float x1 = poll1(sl.w + 1, tag0 + (sl.odd ? cross_red : cross_black), wt, dead);
           x = 0.f;
           x += sl.f0 * x0;
           x += sl.f1 * x1;
@@ -339,18 +348,19 @@ template <int NB>
 __global__ void __launch_bounds__(32, 16) k_flow(Topo t, Coef<float> c, BlockList A, BlockList B, int level, int nsweep,
                                              float *__restrict__ phi, const float *__restrict__ rhs, const int *guard,
                                              Word *__restrict__ words, unsigned *epoch,
-                                             const int *__restrict__ alive) {
+                                             const int *__restrict__ alive, int limit) {
   __shared__ FlowHalo<NB> sh;
+  const bool gone = given_up(t);  // in flight with the loads that follow
   if (guard && *guard) return;
   const unsigned tag0 = epoch[0] * kFlowTags + 1;
   const ListRange ar = list_range(A), br = list_range(B);
   const int na = ar.b - ar.a, n = na + br.b - br.a, p = blockIdx.x;
-  if (p < n) {
+  if (!__any_sync(0xffffffffu, gone) && p < n) {
     const bool ga = p < na;
     const BlockList &L = ga ? A : B;
     const int *e = L.hx + (long)(ga ? ar.a + p : br.a + p - na) * kHX;
     if (!(L.stc && block_off(L, e[kHXBlock])))  // a problem's blocks are off together
-      flow_block<NB>(t, c, e, ga ? 0 : 1, level, nsweep, phi, rhs, words, tag0, alive, threadIdx.x, sh);
+      flow_block<NB>(t, c, e, ga ? 0 : 1, level, nsweep, phi, rhs, words, tag0, alive, limit, threadIdx.x, sh);
   }
   // the next launch's tags: every CTA has read epoch[0] before it counts
   if (threadIdx.x == 0 && atomicAdd(&epoch[1], 1u) == gridDim.x - 1) {
@@ -416,7 +426,7 @@ __device__ __forceinline__ Flow3Setup flow3_slot(const int *__restrict__ e, cons
 __device__ __forceinline__ void flow3_block(const Topo &t, const Coef<float> &c, const int *e, int group, int level,
                                             int nsweep, float *__restrict__ phi, const float *__restrict__ rhs,
                                             Word *__restrict__ words, unsigned tag0, const int *__restrict__ alive,
-                                            Flow3Halo &sh) {
+                                            int limit, Flow3Halo &sh) {
   constexpr int NB = 8, NC = 512, NF = 64, Q = 4;
   const int tid = threadIdx.x, j = tid & 7, k3 = tid >> 3, pr = (j + k3) & 1;
   const int info = e[kHXInfo], b = e[kHXBlock];
@@ -534,6 +544,7 @@ __device__ __forceinline__ void flow3_block(const Topo &t, const Coef<float> &c,
       dg[k][q] = g;
     }
   bool dead = false;
+  const Wait wt{t.err, limit};
   for (int s = 0; s < nsweep; s++) {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
@@ -551,13 +562,13 @@ __device__ __forceinline__ void flow3_block(const Topo &t, const Coef<float> &c,
         on[d] = sl.ty == 0 || sl.ty == 2;
         tag[d] = sl.ty == 0 ? tag0 + ((h + 1) >> 1) : (sl.odd ? cross_black : cross_red);
       }
-      poll<3>(p, tag, on, got, t.err, dead);
+      poll<3>(p, tag, on, got, wt, dead);
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         const Flow3Slot &sl = slot[k][d];
         if (sl.ty == 1) continue;
         float x = got[d];
-        if (sl.ty == 3) x = poll_fine(sl.w, sl.cf, NB, sl.odd, cross_red, cross_black, t.err, dead);
+        if (sl.ty == 3) x = poll_fine(sl.w, sl.cf, NB, sl.odd, cross_red, cross_black, wt, dead);
         const int a0 = 2 * (tid & 3) + ((k + (side ? NB - 1 : 0) + a1) & 1), m = a0 + NB * a1;
         if (d == 0)
           sh.hx[k][side][m] = x;
@@ -604,18 +615,19 @@ __device__ __forceinline__ void flow3_block(const Topo &t, const Coef<float> &c,
 __global__ void __launch_bounds__(64, 8) k_flow3(Topo t, Coef<float> c, BlockList A, BlockList B, int level, int nsweep,
                                                  float *__restrict__ phi, const float *__restrict__ rhs,
                                                  const int *guard, Word *__restrict__ words, unsigned *epoch,
-                                                 const int *__restrict__ alive) {
+                                                 const int *__restrict__ alive, int limit) {
   __shared__ Flow3Halo sh;
+  const bool gone = given_up(t);  // in flight with the loads that follow
   if (guard && *guard) return;
   const unsigned tag0 = epoch[0] * kFlowTags + 1;
   const ListRange ar = list_range(A), br = list_range(B);
   const int na = ar.b - ar.a, n = na + br.b - br.a, p = blockIdx.x;
-  if (p < n) {
+  if (!__syncthreads_or(gone) && p < n) {
     const bool ga = p < na;
     const BlockList &L = ga ? A : B;
     const int *e = L.hx + (long)(ga ? ar.a + p : br.a + p - na) * kHX;
     if (!(L.stc && block_off(L, e[kHXBlock]))) {
-      flow3_block(t, c, e, ga ? 0 : 1, level, nsweep, phi, rhs, words, tag0, alive, sh);
+      flow3_block(t, c, e, ga ? 0 : 1, level, nsweep, phi, rhs, words, tag0, alive, limit, sh);
     }
   }
   __syncthreads();  // every thread has read epoch[0]
@@ -626,7 +638,7 @@ __global__ void __launch_bounds__(64, 8) k_flow3(Topo t, Coef<float> c, BlockLis
 }
 
 using FlowKernel = void (*)(Topo, Coef<float>, BlockList, BlockList, int, int, float *, const float *, const int *,
-                            Word *, unsigned *, const int *);
+                            Word *, unsigned *, const int *, int);
 struct FlowForm {
   FlowKernel kernel;
   int threads;  // per block
@@ -660,7 +672,7 @@ size_t flow_words(const Topo &t) {
 
 cudaError_t launch_flow(const Topo &t, const Coef<float> &c, const BlockList &A, const BlockList &B, int level,
                         int nsweep, int grid, float *phi, const float *rhs, const int *guard,
-                        unsigned long long *words, unsigned *epoch, const int *alive, cudaStream_t s) {
+                        unsigned long long *words, unsigned *epoch, const int *alive, cudaStream_t s, int limit) {
   const FlowForm f = flow_form(t);
   if (!f.kernel) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
@@ -672,7 +684,8 @@ cudaError_t launch_flow(const Topo &t, const Coef<float> &c, const BlockList &A,
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, f.kernel, t, c, A, B, level, nsweep, phi, rhs, guard, words, epoch, alive);
+  return cudaLaunchKernelEx(&cfg, f.kernel, t, c, A, B, level, nsweep, phi, rhs, guard, words, epoch, alive,
+                            limit);
 }
 
 }  // namespace sayaka_gb300

@@ -7,6 +7,8 @@ namespace sayaka_gb300 {
 
 // tags of one launch: a cell's number of updates, at most kFlowTags - 2
 constexpr unsigned kFlowTags = 32;
+// tries of a wait before it gives up: about half a second
+constexpr int kFlowPolls = 1 << 20;
 
 // blocks that one launch can hold (0: blocks of another kind)
 int flow_capacity(const Topo &t);
@@ -17,8 +19,10 @@ size_t flow_words(const Topo &t);
 // launch_rbgs's values in their order.  grid: at least the groups' entries (of
 // reduced lists: their active ones) and at most flow_capacity(t); nsweep <
 // kFlowTags - 1.  alive: with reduced lists, the blocks they hold (else null).
+// limit: tries of a wait.
 cudaError_t launch_flow(const Topo &t, const Coef<float> &c, const BlockList &A, const BlockList &B, int level,
                         int nsweep, int grid, float *phi, const float *rhs, const int *guard,
-                        unsigned long long *words, unsigned *epoch, const int *alive, cudaStream_t s);
+                        unsigned long long *words, unsigned *epoch, const int *alive, cudaStream_t s,
+                        int limit = kFlowPolls);
 
 }  // namespace sayaka_gb300

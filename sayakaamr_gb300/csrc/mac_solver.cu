@@ -610,6 +610,7 @@ MacGpu::~MacGpu() {
   fr(d_phases_);
   fr(d_bar_);
   if (h_st_) cudaFreeHost(h_st_);
+  if (h_err_) cudaFreeHost(h_err_);
   if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
   if (graph_) cudaGraphDestroy(graph_);
   if (h_red_) cudaFreeHost(h_red_);

@@ -400,6 +400,7 @@ class MacGpu {
   bool reduced() const { return act_on_ && !multi() && !learned_active(); }
   Coef<float> c32_{};
   FState *d_st_ = nullptr, *h_st_ = nullptr;
+  int *h_err_ = nullptr;  // pinned: the error word as of the last iteration without a graph
   double *d_part_ = nullptr;
   double *d_opP_ = nullptr, *d_opS_ = nullptr;  // factors of the device solve's operator
   // their nearest double-float pairs, and those of the block records
