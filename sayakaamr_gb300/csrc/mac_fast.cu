@@ -1280,6 +1280,12 @@ void MacGpu::tune_smoother(int precision) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
+  // with one state per problem the sweeps leave finished problems alone, and
+  // after a solve all of them are: no problem is finished while they are timed
+  if (multi()) {
+    CK(cudaMemcpyAsync(h_stc_, d_stc_, ncomp_ * sizeof(FState), cudaMemcpyDeviceToHost, stream_));
+    CK(cudaMemsetAsync(d_stc_, 0, ncomp_ * sizeof(FState), stream_));
+  }
   const int reps = 6;
   float best = 1e30f;
   int bi = 2;
@@ -1308,6 +1314,9 @@ void MacGpu::tune_smoother(int precision) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  // (the last solve's states can still be asked for)
+  if (multi())
+    CK(cudaMemcpyAsync(d_stc_, h_stc_, ncomp_ * sizeof(FState), cudaMemcpyHostToDevice, stream_));
   rbgs_variant_[pi] = bi;
   // the sweeps above scribbled on the V-cycle work vectors
   const size_t n = (size_t)tt_.num_blocks * ncell_;
