@@ -1982,8 +1982,9 @@ void MacGpu::precondition(int L, T *resid, T *corr, const Coef<T> &c, double *ou
 // shat.  params.vcycle_out 0 (auto): in place in 2D and on 3D towers of at
 // most 2M cells, where it saves two launches per iteration (batch workload,
 // 2D, 29M cells: 58.8 in place vs 60.4 ms widened), and on larger 3D towers
-// of which at least half the blocks have one face coefficient, whose operator
-// is formed on the FP32 pipe from the FP32 values (k_op_rows).  Other large 3D
+// of which at least half the blocks have one face coefficient and whose blocks'
+// side is a multiple of four, whose operator is formed on the FP32 pipe from the
+// FP32 values (k_op_rows).  Other large 3D
 // towers widen, since the general 3D operator reads seven cells and their
 // integer widenings cost more than the launches (15.9M cells: 31.6 in place
 // vs 27.3 ms).  1 = in place with the operator in double-float, 2 = always
@@ -1993,7 +1994,8 @@ bool MacGpu::vcycle_in_place() const {
   if (learned_active() || prm_.precision != 1) return false;
   if (prm_.vcycle_out != 0) return prm_.vcycle_out != 2;
   const DevList &top = towers_[finest_].all;
-  return tt_.ndim == 2 || (long)top.n * ncell_ <= kDirectF32Cells || (!multi() && act_version_ == coef_version_ && 2l * n_iso_ >= n_act_);
+  return tt_.ndim == 2 || (long)top.n * ncell_ <= kDirectF32Cells ||
+         (tt_.nb % 4 == 0 && !multi() && act_version_ == coef_version_ && 2l * n_iso_ >= n_act_);
 }
 template <typename T>
 void MacGpu::iteration_device(T *resid, T *corr, const Coef<T> &c) {
