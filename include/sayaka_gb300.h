@@ -155,8 +155,8 @@ typedef struct sayaka_params {
                              exactly on the integer pipe where they read it) in 2D, on 3D towers of at most
                              2,097,152 cells and on larger ones at least half of whose blocks have equal
                              spacings and constant coefficients (block sides a multiple of four), widened once
-                             into FP64 vectors on the others (default); 1 = in place, the operator evaluated in double-float on the FP32 pipe; 2 = always
-                             widened; 3 = always in place */
+                             into FP64 vectors on the others (default); 1 = in place, the operator evaluated in
+                             double-float on the FP32 pipe; 2 = always widened; 3 = always in place */
   int32_t prolong_form;   /* device V-cycle, the prolongation fused with the first red sweep of its level:
                              1 = one warp per 16x16 block with the block in registers, one thread per row of
                              an 8^3 block (FP32; elsewhere form 0), and a tower's prolongation and sweeps in

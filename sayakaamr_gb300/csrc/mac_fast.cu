@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kTPB) k_op_prep(Topo t, Coef<double> c, BlockL
         continue;
       }
       const double vfv = c.vf[q];
-      if (!fpint::positive(vfv)) {
+      if (!positive(vfv)) {  // (a NaN is solid too, as everywhere else)
         P[q] = S[q] = 0.0;
         continue;
       }
