@@ -419,7 +419,9 @@ int sayaka_mac_residual_norm_noalloc(sayaka_mac *h, int32_t L, const double *x, 
  * leave out alone: which 4 = the one-launch smoothing of tower L with the
  * blocks of its second parity group left out and `variant` tries per wait, so
  * that waits run out (the call reports it); which 5 = the solver's error word
- * set as by a wait that ran out, for the next solve to find */
+ * set as by a wait that ran out, for the next solve to find; which 6 = device
+ * memory that a solve can do without is refused from now on (variant 0: given
+ * again) */
 int sayaka_mac_device_kernel_compact(sayaka_mac *h, int32_t which, int32_t L, int32_t variant, const double *in,
                                      const double *in2, double *out);
 /* one mg_smooth_level(L) (src/SayakaMacOperator.cpp:140-159, 1028-1112) */

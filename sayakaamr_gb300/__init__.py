@@ -662,6 +662,13 @@ class MacSolver:
         _check(self.lib.sayaka_mac_device_kernel_compact(self.h, 5, 0, -1, pa, None, y.ctypes.data_as(_f64p)),
                "set_wait_error", self.h)
 
+    def deny_optional_memory(self, on=True):
+        """failure test: device memory that a solve can do without is refused"""
+        y = self._cells()
+        a, pa = _f64(y)
+        _check(self.lib.sayaka_mac_device_kernel_compact(self.h, 6, 0, int(on), pa, None, y.ctypes.data_as(_f64p)),
+               "deny_optional_memory", self.h)
+
     def restrict_sweep(self, x):
         out = self._cells()
         a, pa = _f64(x)

@@ -18,7 +18,9 @@
 // The reduced lists are used when at least a quarter of the finest tower's
 // blocks are solid (kActiveShare): a launch pays one dependent load for the
 // bounds, about 0.4 us, which a launch-bound solve without solid blocks would
-// lose.
+// lose.  Their memory, about 170 bytes an entry of every list, is allocated
+// when that share is first reached; where it cannot be had, the solve walks the
+// full lists.
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -91,21 +93,26 @@ __global__ void __launch_bounds__(256) k_active_copy(const ActiveList *__restric
       l.alinks[i] = l.links[(long)l.orig[i / l.nlinks] * l.nlinks + i % l.nlinks];
 }
 
-// head[0], head[1]: the active blocks of the finest tower, and those of them
-// with one face coefficient (see k_iso); head[2 + i]: active entries of list i
-__global__ void __launch_bounds__(kScanThreads) k_active_head(ActiveList top, const double *__restrict__ iso, int *head,
-                                                             const ActiveList *__restrict__ lists, int nlists) {
-  for (int i = threadIdx.x; i < nlists; i += blockDim.x) head[2 + i] = lists[i].pre[lists[i].n];
-  const int n = top.pre[top.n];
-  int k = 0;
-  for (int i0 = 0; i0 < n; i0 += kScanThreads) {
+// count[0], count[1]: the active blocks of the finest tower, and those of them
+// with one face coefficient (see k_iso); zeroed by the caller
+__global__ void __launch_bounds__(kScanThreads) k_active_count(int n, const int *__restrict__ blocks,
+                                                              const int *__restrict__ flag,
+                                                              const double *__restrict__ iso, int *count) {
+  for (int i0 = blockIdx.x * kScanThreads; i0 < n; i0 += gridDim.x * kScanThreads) {
     const int i = i0 + threadIdx.x;
-    k += __syncthreads_count(i < n && iso[top.ablocks[i]] != 0.0);
+    const bool on = i < n && flag[blocks[i]] != 0;
+    const int a = __syncthreads_count(on), k = __syncthreads_count(on && iso[blocks[i]] != 0.0);
+    if (threadIdx.x == 0 && a) {
+      atomicAdd(&count[0], a);
+      atomicAdd(&count[1], k);
+    }
   }
-  if (threadIdx.x == 0) {
-    head[0] = n;
-    head[1] = k;
-  }
+}
+
+// head[i]: active entries of list i
+__global__ void __launch_bounds__(kScanThreads) k_active_head(int *head, const ActiveList *__restrict__ lists,
+                                                             int nlists) {
+  for (int i = threadIdx.x; i < nlists; i += blockDim.x) head[i] = lists[i].pre[lists[i].n];
 }
 
 // zeros on the solid blocks of up to four vectors
@@ -127,15 +134,41 @@ __global__ void __launch_bounds__(256) k_zero_solid(int nblocks, int ncell, cons
 
 }  // namespace
 
-// the reduced lists of the current volume fractions; their arrays lie in one
-// allocation, made once
-void MacGpu::build_active() {
+// device memory that a solve can do without: null where it cannot be had
+bool MacGpu::optional_malloc(char **p, size_t bytes) {
+  if (!deny_optional_ && dev_malloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
+// the blocks that hold fluid, by the current volume fractions
+bool MacGpu::count_active() {
   const int nbk = tt_.num_blocks;
   const DevList &top = towers_[finest_].all;
   n_act_ = top.n;
   n_iso_ = 0;
-  if (top.n == 0) return;
-  if (!d_active_) {
+  if (top.n == 0) return true;
+  char *mem = nullptr;
+  if (!d_active_ && !optional_malloc(&mem, ((size_t)nbk + 2) * sizeof(int))) return false;
+  if (mem) d_active_ = reinterpret_cast<int *>(mem);
+  int *count = d_active_ + nbk, h[2] = {0, 0};
+  CKR_(cudaMemsetAsync(count, 0, sizeof(h), stream_), false);
+  k_block_active<<<std::min((nbk + 7) / 8, 152 * 8), 256, 0, stream_>>>(nbk, ncell_, d_vf_, d_active_);
+  k_active_count<<<std::min((top.n + kScanThreads - 1) / kScanThreads, 152), kScanThreads, 0, stream_>>>(
+      top.n, top.blocks, d_active_, d_iso_, count);
+  CKR_(cudaGetLastError(), false);
+  CKR_(cudaMemcpyAsync(h, count, sizeof(h), cudaMemcpyDeviceToHost, stream_), false);
+  CKR_(cudaStreamSynchronize(stream_), false);
+  n_act_ = h[0];
+  n_iso_ = h[1];
+  return true;
+}
+
+// the reduced lists of these blocks; their arrays lie in one allocation, made
+// once
+bool MacGpu::build_active() {
+  if (!d_act_lists_) {
     std::vector<ActiveList> h;
     size_t used = 0;
     char *base = nullptr;
@@ -143,13 +176,12 @@ void MacGpu::build_active() {
       p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base ? base + used : nullptr);
       used += (n * sizeof(*p) + 15) / 16 * 16;
     };
-    int *flags = nullptr, *head = nullptr;
+    int *head = nullptr;
     ActiveList *lists = nullptr;
     auto lay = [&] {  // sizes first, then places
       used = 0;
       h.clear();
-      take(flags, nbk);
-      take(head, 2 + 2 * towers_.size() + levels_.size() + nonleaf_.size());
+      take(head, 2 * towers_.size() + levels_.size() + nonleaf_.size());
       auto reduce = [&](DevList &d, int nlinks) {
         if (d.n == 0) return;
         take(d.act.blocks, d.n);
@@ -170,38 +202,29 @@ void MacGpu::build_active() {
       take(lists, h.size());
     };
     lay();
-    if (dev_malloc(&base, used) != cudaSuccess) {
-      fail("out of device memory (active blocks)");
-      return;
-    }
+    if (!optional_malloc(&base, used)) return false;
     d_active_mem_ = base;
     lay();
     n_act_lists_ = (int)h.size();
-    CK_(cudaMemcpyAsync(lists, h.data(), h.size() * sizeof(ActiveList), cudaMemcpyHostToDevice, stream_));
-    CK_(cudaStreamSynchronize(stream_));
+    CKR_(cudaMemcpyAsync(lists, h.data(), h.size() * sizeof(ActiveList), cudaMemcpyHostToDevice, stream_), false);
+    CKR_(cudaStreamSynchronize(stream_), false);
     d_act_lists_ = lists;
-    d_active_ = flags;
     d_act_head_ = head;
   }
-  k_block_active<<<std::min((nbk + 7) / 8, 152 * 8), 256, 0, stream_>>>(nbk, ncell_, d_vf_, d_active_);
   k_active_scan<<<n_act_lists_, kScanThreads, 0, stream_>>>(d_act_lists_, d_active_);
   k_active_copy<<<dim3(152, n_act_lists_), 256, 0, stream_>>>(d_act_lists_);
-  CK_(cudaGetLastError());
-  const ActiveList t{top.blocks, nullptr, nullptr, nullptr, 0, top.n, top.act.blocks, nullptr, nullptr, nullptr,
-                     top.act.pre, top.act.orig};
-  k_active_head<<<1, kScanThreads, 0, stream_>>>(t, d_iso_, d_act_head_, d_act_lists_, n_act_lists_);
-  CK_(cudaGetLastError());
-  std::vector<int> head(2 + n_act_lists_, 0);
-  CK_(cudaMemcpyAsync(head.data(), d_act_head_, head.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_));
-  CK_(cudaStreamSynchronize(stream_));
+  k_active_head<<<1, kScanThreads, 0, stream_>>>(d_act_head_, d_act_lists_, n_act_lists_);
+  CKR_(cudaGetLastError(), false);
+  std::vector<int> head(n_act_lists_, 0);
+  CKR_(cudaMemcpyAsync(head.data(), d_act_head_, head.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_), false);
+  CKR_(cudaStreamSynchronize(stream_), false);
   // active entries of every tower's parity-grouped list
   n_act_par_.assign(towers_.size(), 0);
-  for (size_t i = 0, q = 2; i < towers_.size(); i++) {
+  for (size_t i = 0, q = 0; i < towers_.size(); i++) {
     if (towers_[i].all.n) q++;
     if (towers_[i].par.n) n_act_par_[i] = head[q++];
   }
-  n_act_ = head[0];
-  n_iso_ = head[1];
+  return true;
 }
 
 // whether the next solve walks the reduced lists: one shared BiCGSTAB state,
@@ -210,12 +233,16 @@ void MacGpu::choose_active() {
   act_on_ = false;
   if (multi() || learned_active()) return;
   if (act_version_ != coef_version_) {
-    build_active();
-    if (!err_.empty()) return;
+    if (!count_active()) return;
     act_version_ = coef_version_;
   }
   const long n = towers_[finest_].all.n;
-  act_on_ = n_act_ > 0 && (n - n_act_) * kActiveShare >= n;
+  if (n_act_ == 0 || (n - n_act_) * kActiveShare < n) return;
+  if (act_lists_version_ != coef_version_) {
+    if (!build_active()) return;
+    act_lists_version_ = coef_version_;
+  }
+  act_on_ = true;
 }
 
 // the solid blocks of the vectors whose neighbours read them are 0 before a

@@ -1914,21 +1914,20 @@ unsigned MacGpu::flow_mask() const {
   return m;
 }
 
-// the exchange buffers of launch_flow, if any tower fits it
+// the exchange buffers of launch_flow, if any tower fits it (where they cannot be
+// had, towers keep their separate launches)
 void MacGpu::ensure_flow() {
   if (d_flow_words_) return;
   if (flow_capacity_ < 0) flow_capacity_ = flow_capacity(topo_);
   bool any = false;
   for (int l = 2; l <= finest_; l++) any = any || (flow_entries(l) > 0 && flow_entries(l) <= flow_capacity_);
   if (!any) return;
-  const size_t n = flow_words(topo_);
-  if (dev_malloc(&d_flow_words_, n * sizeof(unsigned long long)) != cudaSuccess ||
-      dev_malloc(&d_flow_epoch_, 2 * sizeof(unsigned)) != cudaSuccess) {
-    fail("out of device memory (edge exchange)");
-    return;
-  }
-  CK(cudaMemsetAsync(d_flow_words_, 0, n * sizeof(unsigned long long), stream_));
-  CK(cudaMemsetAsync(d_flow_epoch_, 0, 2 * sizeof(unsigned), stream_));
+  const size_t n = flow_words(topo_) * sizeof(unsigned long long) + 2 * sizeof(unsigned);
+  char *mem = nullptr;
+  if (!optional_malloc(&mem, n)) return;
+  CK(cudaMemsetAsync(mem, 0, n, stream_));
+  d_flow_words_ = reinterpret_cast<unsigned long long *>(mem);
+  d_flow_epoch_ = reinterpret_cast<unsigned *>(d_flow_words_ + flow_words(topo_));
 }
 
 // V-cycle result on the tower, widened to FP64: out = 0 + corr
@@ -2481,11 +2480,15 @@ int MacGpu::enqueue_kernel(int which, int L) {
 // solve's FP64 sweep, launch variant `variant` (-1: the tuned one); in = phi,
 // in2 = rhs.  Uses (and clobbers) the handle's work vectors.
 int MacGpu::device_kernel_compact(int which, int L, int variant, const double *in, const double *in2, double *out) {
-  if (which < 0 || which > 5 || !in || !out || ((which == 1 || which == 2) && !in2)) return 1;
+  if (which < 0 || which > 6 || !in || !out || ((which == 1 || which == 2) && !in2)) return 1;
   if ((which == 1 || which == 2) && (L < 1 || L > finest_ || towers_[L].all.n == 0)) return 1;
   if (which == 1 && variant >= kRbgsVariants) return 1;
   if (which == 2 && (variant < 1 || variant > 1024)) return 1;
   if (which == 4 && (variant < 1 || variant > kFlowPolls || L < 2 || L > finest_)) return 1;
+  if (which == 6) {
+    deny_optional_ = variant != 0;
+    return 0;
+  }
   if (prepare_device() != 0) return 2;
   ensure_smooth_factors();
   if (which == 4) {

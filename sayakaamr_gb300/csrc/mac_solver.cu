@@ -576,8 +576,8 @@ MacGpu::~MacGpu() {
   fr(d_corr32_);
   fr(d_corr32b_);
   fr(d_flow_words_);
-  fr(d_flow_epoch_);
   fr(d_corr64b_);
+  fr(d_active_);
   fr(d_active_mem_);
   fr(tlc_.blocks);
   fr(tlc_.ftypes);

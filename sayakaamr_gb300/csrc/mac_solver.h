@@ -379,12 +379,15 @@ class MacGpu {
   bool multi() const { return ncomp_ > 1 && prm_.per_problem != 0 && d_stc_ != nullptr; }
   BlockList attach(BlockList r) const;
   // blocks that hold fluid, and the lists reduced to them (mac_active.cu)
-  void build_active();
+  bool count_active();
+  bool build_active();
   void choose_active();
+  bool optional_malloc(char **p, size_t bytes);
+  bool deny_optional_ = false;  // a test's: as if no such memory could be had
   void zero_solid();
   BlockList active(BlockList r, const DevList &d, int a, int b) const;
-  char *d_active_mem_ = nullptr;       // the allocation behind these
   int *d_active_ = nullptr;            // per block: holds fluid
+  char *d_active_mem_ = nullptr;       // the allocation behind these
   ActiveList *d_act_lists_ = nullptr;  // every list and its reduced form
   int n_act_lists_ = 0;
   int n_act_ = 0, n_iso_ = 0;  // active blocks of the finest tower, and those with one face coefficient
@@ -392,7 +395,8 @@ class MacGpu {
   std::vector<int> n_act_par_;  // active entries of every tower's parity-grouped list
   // the BiCGSTAB kernels read the FP32 V-cycle's output in place
   bool vcycle_in_place() const;
-  long act_version_ = -1;              // coefficient version of the reduced lists
+  // coefficient versions of the counts and of the reduced lists
+  long act_version_ = -1, act_lists_version_ = -1;
   bool act_on_ = false;                // enough solid blocks for the reduced lists (choose_active)
   // the solve walks the reduced lists.  One state per problem and the learned
   // correction walk the full ones, also when they are switched on after the
