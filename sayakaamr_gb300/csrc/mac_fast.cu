@@ -1064,9 +1064,9 @@ __global__ void __launch_bounds__(kTPB) k_bottom_gemv(BottomDev bd, const T *__r
 
 // Gauss-Jordan inversion step k of nmat matrices of order m at offsets offs
 // (no pivoting: the pinned, row-scaled bottom operator has positive pivots),
-// from a into b, so that one launch per step is enough: the pivot row and
-// column are read where they are while every other entry is written.  One
-// CTA per matrix row; the row of the next pivot also writes its reciprocal,
+// from a into b (there at offsets `to`), so that one launch per step is enough:
+// the pivot row and column are read where they are while every other entry is
+// written.  One CTA per matrix row; the row of the next pivot also writes its reciprocal,
 // ipiv[mat][k + 1], so that no CTA waits for a division.  (With the row and
 // column saved by a launch of their own and the step in place, an inversion
 // of order 512 took 2.6 ms, half of it the saving launches.)
@@ -1076,13 +1076,13 @@ __global__ void k_gj_first(int m, int nmat, const long long *__restrict__ offs, 
   if (mat < nmat) ipiv[(long)mat * m] = 1.0 / a[offs[mat]];
 }
 __global__ void __launch_bounds__(kTPB) k_gj_step(int m, int k, int nmat, const long long *__restrict__ offs,
-                                                const double *__restrict__ a, double *__restrict__ b,
-                                                double *__restrict__ ipiv) {
+                                                const double *__restrict__ a, const long long *__restrict__ to,
+                                                double *__restrict__ b, double *__restrict__ ipiv) {
   const long rows = (long)nmat * m;
   for (long r = blockIdx.x; r < rows; r += gridDim.x) {
     const int mat = (int)(r / m), i = (int)(r - (long)mat * m);
     const double *am = a + offs[mat], *rw = am + (long)k * m, *ar = am + (long)i * m;
-    double *br = b + offs[mat] + (long)i * m;
+    double *br = b + to[mat] + (long)i * m;
     const double ip = ipiv[(long)mat * m + k];
     if (i == k) {
       for (int j = threadIdx.x; j < m; j += blockDim.x) br[j] = j == k ? ip : rw[j] * ip;
@@ -1718,24 +1718,31 @@ void MacGpu::build_bottom() {
     for (int c = 0; c < nc; c++)
       if (comp_n[c] == m) offs.push_back(comp_off[c]);
     const int nmat = (int)offs.size();
+    const long long mm = (long long)m * m;
+    // the matrices after every other step: all at once, or as many as there is
+    // memory for
+    char *mem = nullptr;
+    int per = nmat;
+    while (per > 1 && !optional_malloc(&mem, (size_t)per * mm * sizeof(double))) per = (per + 1) / 2;
+    if (!mem) CK_(dev_malloc(&mem, (size_t)mm * sizeof(double)));
+    double *const other = reinterpret_cast<double *>(mem);
+    for (int q = 0; q < nmat; q++) offs.push_back(q % per * mm);
     long long *d_offs = nullptr;
-    double *other = nullptr;  // the matrices after every other step, at the same offsets
-    CK_(dev_malloc(&d_offs, nmat * sizeof(long long)));
     double *ipiv = nullptr;
-    CK_(dev_malloc(&other, (size_t)tot * sizeof(double)));
-    CK_(dev_malloc(&ipiv, (size_t)nmat * m * sizeof(double)));
-    CK_(cudaMemcpyAsync(d_offs, offs.data(), nmat * sizeof(long long), cudaMemcpyHostToDevice, stream_));
-    const int step_grid = (int)std::min<long>((long)nmat * m, 152 * 16);
-    // (the order is even, as the blocks' sides are: the last step ends in d_binv_)
-    const double *from = d_binv_;
-    double *to = other;
-    k_gj_first<<<(nmat + kTPB - 1) / kTPB, kTPB, 0, stream_>>>(m, nmat, d_offs, from, ipiv);
-    for (int k = 0; k < m; k++) {
-      k_gj_step<<<step_grid, kTPB, 0, stream_>>>(m, k, nmat, d_offs, from, to, ipiv);
-      double *t = const_cast<double *>(from);
-      from = to;
-      to = t;
+    CK_(dev_malloc(&d_offs, offs.size() * sizeof(long long)));
+    CK_(dev_malloc(&ipiv, (size_t)per * m * sizeof(double)));
+    CK_(cudaMemcpyAsync(d_offs, offs.data(), offs.size() * sizeof(long long), cudaMemcpyHostToDevice, stream_));
+    for (int q = 0; q < nmat; q += per) {
+      const int n = std::min(per, nmat - q), grid = (int)std::min<long>((long)n * m, 152 * 16);
+      const long long *at = d_offs + q, *at2 = d_offs + nmat + q;
+      k_gj_first<<<(n + kTPB - 1) / kTPB, kTPB, 0, stream_>>>(m, n, at, d_binv_, ipiv);
+      // (the order is even, as the blocks' sides are: the last step ends in d_binv_)
+      for (int k = 0; k < m; k += 2) {
+        k_gj_step<<<grid, kTPB, 0, stream_>>>(m, k, n, at, d_binv_, at2, other, ipiv);
+        k_gj_step<<<grid, kTPB, 0, stream_>>>(m, k + 1, n, at2, other, at, d_binv_, ipiv);
+      }
     }
+    CK_(cudaGetLastError());
     CK_(cudaStreamSynchronize(stream_));
     dev_free(d_offs);
     dev_free(other);

@@ -66,3 +66,17 @@ def test_no_lists_without_solid_blocks():
         del S
     # the flags of the blocks; the lists would be 170 bytes for each entry of every list
     assert 0 <= used[1] - used[0] < 170 * p.num_blocks, used
+
+
+def test_bottom_inverse_without_a_second_copy_of_all_matrices():
+    p = W.forest([W.batch_problem(np.random.default_rng(k), "p%d" % k) for k in range(5)], "f")
+    out = []
+    for deny in (True, False):
+        S = W.make_solver(p, **dict(PARAMS, tol_rel=1e-8, bottom_level=1))
+        S.deny_optional_memory(deny)
+        S.set_params(prolong_form=0)  # the edge words are not what is compared
+        info = S.cg_solve()
+        assert info["status"] == 0, info
+        out.append((info["iterations"], S.get_sol_compact()))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1])
