@@ -142,7 +142,27 @@ bool MacGpu::optional_malloc(char **p, size_t bytes) {
   return false;
 }
 
-// the blocks that hold fluid, by the current volume fractions
+// the counts (and the entries of the reduced lists) as the launches before left
+// them; one copy and one wait
+bool MacGpu::read_active(bool lists) {
+  std::vector<int> h(2 + (lists ? n_act_lists_ : 0), 0);
+  CKR_(cudaMemcpyAsync(h.data(), d_act_head_, h.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_), false);
+  CKR_(cudaStreamSynchronize(stream_), false);
+  n_act_ = h[0];
+  n_iso_ = h[1];
+  if (!lists) return true;
+  // active entries of every tower's parity-grouped list
+  n_act_par_.assign(towers_.size(), 0);
+  for (size_t i = 0, q = 2; i < towers_.size(); i++) {
+    if (towers_[i].all.n) q++;
+    if (towers_[i].par.n) n_act_par_[i] = h[q++];
+  }
+  act_lists_version_ = coef_version_;
+  return true;
+}
+
+// the blocks that hold fluid, by the current volume fractions, and the lists
+// reduced to them where they exist
 bool MacGpu::count_active() {
   const int nbk = tt_.num_blocks;
   const DevList &top = towers_[finest_].all;
@@ -150,81 +170,69 @@ bool MacGpu::count_active() {
   n_iso_ = 0;
   if (top.n == 0) return true;
   char *mem = nullptr;
-  if (!d_active_ && !optional_malloc(&mem, ((size_t)nbk + 2) * sizeof(int))) return false;
+  const size_t nhead = 2 + 2 * towers_.size() + levels_.size() + nonleaf_.size();
+  if (!d_active_ && !optional_malloc(&mem, (nbk + nhead) * sizeof(int))) return false;
   if (mem) d_active_ = reinterpret_cast<int *>(mem);
-  int *count = d_active_ + nbk, h[2] = {0, 0};
-  CKR_(cudaMemsetAsync(count, 0, sizeof(h), stream_), false);
+  d_act_head_ = d_active_ + nbk;
+  CKR_(cudaMemsetAsync(d_act_head_, 0, 2 * sizeof(int), stream_), false);
   k_block_active<<<std::min((nbk + 7) / 8, 152 * 8), 256, 0, stream_>>>(nbk, ncell_, d_vf_, d_active_);
   k_active_count<<<std::min((top.n + kScanThreads - 1) / kScanThreads, 152), kScanThreads, 0, stream_>>>(
-      top.n, top.blocks, d_active_, d_iso_, count);
+      top.n, top.blocks, d_active_, d_iso_, d_act_head_);
   CKR_(cudaGetLastError(), false);
-  CKR_(cudaMemcpyAsync(h, count, sizeof(h), cudaMemcpyDeviceToHost, stream_), false);
-  CKR_(cudaStreamSynchronize(stream_), false);
-  n_act_ = h[0];
-  n_iso_ = h[1];
-  return true;
+  if (d_act_lists_) reduce_lists();
+  return read_active(d_act_lists_ != nullptr);
 }
 
-// the reduced lists of these blocks; their arrays lie in one allocation, made
-// once
-bool MacGpu::build_active() {
-  if (!d_act_lists_) {
-    std::vector<ActiveList> h;
-    size_t used = 0;
-    char *base = nullptr;
-    auto take = [&](auto *&p, size_t n) {
-      p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base ? base + used : nullptr);
-      used += (n * sizeof(*p) + 15) / 16 * 16;
-    };
-    int *head = nullptr;
-    ActiveList *lists = nullptr;
-    auto lay = [&] {  // sizes first, then places
-      used = 0;
-      h.clear();
-      take(head, 2 * towers_.size() + levels_.size() + nonleaf_.size());
-      auto reduce = [&](DevList &d, int nlinks) {
-        if (d.n == 0) return;
-        take(d.act.blocks, d.n);
-        take(d.act.pre, d.n + 1);
-        take(d.act.orig, d.n);
-        if (d.ftypes) take(d.act.ftypes, d.n);
-        if (d.hx) take(d.act.hx, (size_t)d.n * kHX);
-        if (d.links) take(d.act.links, (size_t)d.n * nlinks);
-        h.push_back(ActiveList{d.blocks, d.ftypes, d.hx, d.links, nlinks, d.n, d.act.blocks, d.act.ftypes, d.act.hx,
-                               d.act.links, d.act.pre, d.act.orig});
-      };
-      for (DevTower &t : towers_) {
-        reduce(t.all, 0);
-        reduce(t.par, 0);
-      }
-      for (DevList &l : levels_) reduce(l, 1);
-      for (DevList &l : nonleaf_) reduce(l, 8);
-      take(lists, h.size());
-    };
-    lay();
-    if (!optional_malloc(&base, used)) return false;
-    d_active_mem_ = base;
-    lay();
-    n_act_lists_ = (int)h.size();
-    CKR_(cudaMemcpyAsync(lists, h.data(), h.size() * sizeof(ActiveList), cudaMemcpyHostToDevice, stream_), false);
-    CKR_(cudaStreamSynchronize(stream_), false);
-    d_act_lists_ = lists;
-    d_act_head_ = head;
-  }
+// the reduced lists of these blocks
+void MacGpu::reduce_lists() {
   k_active_scan<<<n_act_lists_, kScanThreads, 0, stream_>>>(d_act_lists_, d_active_);
   k_active_copy<<<dim3(152, n_act_lists_), 256, 0, stream_>>>(d_act_lists_);
-  k_active_head<<<1, kScanThreads, 0, stream_>>>(d_act_head_, d_act_lists_, n_act_lists_);
-  CKR_(cudaGetLastError(), false);
-  std::vector<int> head(n_act_lists_, 0);
-  CKR_(cudaMemcpyAsync(head.data(), d_act_head_, head.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_), false);
+  k_active_head<<<1, kScanThreads, 0, stream_>>>(d_act_head_ + 2, d_act_lists_, n_act_lists_);
+  CK(cudaGetLastError());
+}
+
+// the same for the first time; their arrays lie in one allocation
+bool MacGpu::build_active() {
+  std::vector<ActiveList> h;
+  size_t used = 0;
+  char *base = nullptr;
+  auto take = [&](auto *&p, size_t n) {
+    p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base ? base + used : nullptr);
+    used += (n * sizeof(*p) + 15) / 16 * 16;
+  };
+  ActiveList *lists = nullptr;
+  auto lay = [&] {  // sizes first, then places
+    used = 0;
+    h.clear();
+    auto reduce = [&](DevList &d, int nlinks) {
+      if (d.n == 0) return;
+      take(d.act.blocks, d.n);
+      take(d.act.pre, d.n + 1);
+      take(d.act.orig, d.n);
+      if (d.ftypes) take(d.act.ftypes, d.n);
+      if (d.hx) take(d.act.hx, (size_t)d.n * kHX);
+      if (d.links) take(d.act.links, (size_t)d.n * nlinks);
+      h.push_back(ActiveList{d.blocks, d.ftypes, d.hx, d.links, nlinks, d.n, d.act.blocks, d.act.ftypes, d.act.hx,
+                             d.act.links, d.act.pre, d.act.orig});
+    };
+    for (DevTower &t : towers_) {
+      reduce(t.all, 0);
+      reduce(t.par, 0);
+    }
+    for (DevList &l : levels_) reduce(l, 1);
+    for (DevList &l : nonleaf_) reduce(l, 8);
+    take(lists, h.size());
+  };
+  lay();
+  if (!optional_malloc(&base, used)) return false;
+  d_active_mem_ = base;
+  lay();
+  n_act_lists_ = (int)h.size();
+  CKR_(cudaMemcpyAsync(lists, h.data(), h.size() * sizeof(ActiveList), cudaMemcpyHostToDevice, stream_), false);
   CKR_(cudaStreamSynchronize(stream_), false);
-  // active entries of every tower's parity-grouped list
-  n_act_par_.assign(towers_.size(), 0);
-  for (size_t i = 0, q = 0; i < towers_.size(); i++) {
-    if (towers_[i].all.n) q++;
-    if (towers_[i].par.n) n_act_par_[i] = head[q++];
-  }
-  return true;
+  d_act_lists_ = lists;
+  reduce_lists();
+  return read_active(true);
 }
 
 // whether the next solve walks the reduced lists: one shared BiCGSTAB state,
@@ -238,10 +246,7 @@ void MacGpu::choose_active() {
   }
   const long n = towers_[finest_].all.n;
   if (n_act_ == 0 || (n - n_act_) * kActiveShare < n) return;
-  if (act_lists_version_ != coef_version_) {
-    if (!build_active()) return;
-    act_lists_version_ = coef_version_;
-  }
+  if (act_lists_version_ != coef_version_ && !build_active()) return;
   act_on_ = true;
 }
 

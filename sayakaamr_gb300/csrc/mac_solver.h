@@ -381,6 +381,8 @@ class MacGpu {
   // blocks that hold fluid, and the lists reduced to them (mac_active.cu)
   bool count_active();
   bool build_active();
+  void reduce_lists();
+  bool read_active(bool lists);
   void choose_active();
   bool optional_malloc(char **p, size_t bytes);
   bool deny_optional_ = false;  // a test's: as if no such memory could be had
