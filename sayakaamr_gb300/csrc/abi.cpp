@@ -773,7 +773,7 @@ int sayaka_mac_enqueue_kernel(sayaka_mac *h, int32_t which, int32_t L) {
 }
 int sayaka_mac_launch_counts(sayaka_mac *h, int32_t *pro, int32_t *per, int32_t *epi) {
   return guarded(h, [&] {
-    if (pro) *pro = MacGpu::kPrologueKernels;
+    if (pro) *pro = h->gpu->prologue_kernels();
     if (per) *per = h->gpu->kernels_per_iteration();
     if (epi) *epi = MacGpu::kEpilogueKernels;
     return (int)SAYAKA_OK;

@@ -478,9 +478,12 @@ class MacGpu {
 
  public:
   // kernel launches of one captured BiCGSTAB iteration; a device solve
-  // launches kPrologueKernels + iterations * this + kEpilogueKernels
+  // launches prologue_kernels() + iterations * this + kEpilogueKernels
   int kernels_per_iteration() const { return kernels_per_iter_; }
-  static constexpr int kPrologueKernels = 2, kEpilogueKernels = 1;
+  // x0 and the first residual; the shared done flag of one state per problem;
+  // the solid blocks' zeros (FP32 and FP64 vectors are two launches)
+  int prologue_kernels() const { return 2 + (multi() ? 1 : 0) + (reduced() ? (prm_.precision == 1 ? 2 : 1) : 0); }
+  static constexpr int kEpilogueKernels = 1;
 };
 
 // integer-pipe precision conversions of the vector kernels against the
