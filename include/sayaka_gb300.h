@@ -415,7 +415,10 @@ int sayaka_mac_residual_norm_noalloc(sayaka_mac *h, int32_t L, const double *x, 
  * `variant` (1..1024) red-black sweeps per block (in = phi, frozen outside
  * each block; in2 = rhs); which 3 = out = A x on the finest tower for x = in
  * rounded to FP32, with the double-float operator the BiCGSTAB iteration
- * applies to the FP32 V-cycle's output (in2 unused).  Failure tests, which
+ * applies to the FP32 V-cycle's output (in2 unused); which 7 = which 2 in FP32
+ * (in, in2 rounded), variant + 1024: by the general kernel instead of the one
+ * that the V-cycle takes, + 2048: after the prolongation of level L, which the
+ * V-cycle's kernel does itself.  Failure tests, which
  * leave out alone: which 4 = the one-launch smoothing of tower L with the
  * blocks of its second parity group left out and `variant` tries per wait, so
  * that waits run out (the call reports it); which 5 = the solver's error word

@@ -669,6 +669,17 @@ class MacSolver:
         _check(self.lib.sayaka_mac_device_kernel_compact(self.h, 6, 0, int(on), pa, None, y.ctypes.data_as(_f64p)),
                "deny_optional_memory", self.h)
 
+    def device_hybrid_pass_f32(self, L, phi, rhs, sweeps, general=False, prolong=False):
+        """the pass in FP32, by the V-cycle's kernel or by the general one, on
+        phi or with level L prolonged from its parents first"""
+        out = self._cells()
+        a, pa = _f64(phi)
+        b, pb = _f64(rhs)
+        _check(self.lib.sayaka_mac_device_kernel_compact(self.h, 7, int(L), int(sweeps) + 1024 * general + 2048 * prolong,
+                                                         pa, pb, out.ctypes.data_as(_f64p)),
+               "device_hybrid_pass_f32", self.h)
+        return out
+
     def restrict_sweep(self, x):
         out = self._cells()
         a, pa = _f64(x)

@@ -2487,10 +2487,11 @@ int MacGpu::enqueue_kernel(int which, int L) {
 // solve's FP64 sweep, launch variant `variant` (-1: the tuned one); in = phi,
 // in2 = rhs.  Uses (and clobbers) the handle's work vectors.
 int MacGpu::device_kernel_compact(int which, int L, int variant, const double *in, const double *in2, double *out) {
-  if (which < 0 || which > 6 || !in || !out || ((which == 1 || which == 2) && !in2)) return 1;
-  if ((which == 1 || which == 2) && (L < 1 || L > finest_ || towers_[L].all.n == 0)) return 1;
+  if (which < 0 || which > 7 || !in || !out || ((which == 1 || which == 2 || which == 7) && !in2)) return 1;
+  if ((which == 1 || which == 2 || which == 7) && (L < 1 || L > finest_ || towers_[L].all.n == 0)) return 1;
   if (which == 1 && variant >= kRbgsVariants) return 1;
   if (which == 2 && (variant < 1 || variant > 1024)) return 1;
+  if (which == 7 && (variant < 1 || variant > 4 * 1024)) return 1;
   if (which == 4 && (variant < 1 || variant > kFlowPolls || L < 2 || L > finest_)) return 1;
   if (which == 6) {
     deny_optional_ = variant != 0;
@@ -2555,6 +2556,29 @@ int MacGpu::device_kernel_compact(int which, int L, int variant, const double *i
     CKR_(cudaMemcpyAsync(out, vec_[kV], n * sizeof(double), cudaMemcpyDeviceToHost, stream_), 2);
   } else if (which == 4) {
     // (above)
+  } else if (which == 7) {
+    // the FP32 pass, as the V-cycle runs it or by the general kernel (a list
+    // without halo descriptors), from in or with level L prolonged first
+    const int sweeps = (variant - 1) % 1024 + 1, form = (variant - 1) / 1024;
+    const bool general = form & 1, top = form & 2;
+    float *a = d_corr32_, *b = corr_alt<float>();
+    std::vector<float> h(n);
+    if (!err_.empty()) return 2;
+    for (const auto &[src, dst] : {std::pair(in, a), std::pair(in2, d_resid32_)}) {
+      for (size_t i = 0; i < n; i++) h[i] = (float)src[i];
+      CKR_(cudaMemcpyAsync(dst, h.data(), n * sizeof(float), cudaMemcpyHostToDevice, stream_), 2);
+      CKR_(cudaStreamSynchronize(stream_), 2);
+    }
+    BlockList TL = smooth_list(L);
+    if (general) TL.hx = nullptr;
+    const bool fused = top && !general && bhgs_prolongs<float>(topo_, c32_, TL);
+    if (top && !fused) launch_prolong<float>(topo_, c32_, level_list(L), a, nullptr, stream_);
+    CKR_(cudaMemcpyAsync(b, a, n * sizeof(float), cudaMemcpyDeviceToDevice, stream_), 2);
+    launch_bhgs<float>(topo_, c32_, TL, sweeps, a, b, d_resid32_, nullptr, stream_, false, fused ? L : 0);
+    CKR_(cudaGetLastError(), 2);
+    CKR_(cudaMemcpyAsync(h.data(), b, n * sizeof(float), cudaMemcpyDeviceToHost, stream_), 2);
+    CKR_(cudaStreamSynchronize(stream_), 2);
+    for (size_t i = 0; i < n; i++) out[i] = (double)h[i];
   } else if (which == 2) {
     // one block-hybrid pass over every sublevel of tower L, `variant`
     // red-black sweeps per block: in (frozen) -> out
