@@ -604,7 +604,10 @@ __global__ void __launch_bounds__(kTPB) k_smooth_factors(Topo t, Coef<double> c,
 // the FP64 pipe).  Its interior cells'
 // factors are those k_op_prep and k_smooth_factors compute, in the same
 // order: diag = alpha*dv + T_0 + T_0 + T_1 + T_1 (+ T_2 + T_2).  The FP32
-// record holds the FP32 coefficients, equal throughout the block too.
+// record holds the FP32 coefficients, equal throughout the block too.  The FP32
+// coefficients of a coarse/fine face (c32.cf) have to be one value as well, as
+// the hybrid pass takes them per row: where B and the area fraction vary and
+// their product doesn't, these may round apart.
 template <int ND>
 __global__ void __launch_bounds__(kTPB) k_uniform(Topo t, Coef<double> c, Coef<float> c32, double *u64,
                                                 float *u32) {
@@ -621,6 +624,14 @@ __global__ void __launch_bounds__(kTPB) k_uniform(Topo t, Coef<double> c, Coef<f
     }
     for (int i = threadIdx.x; i < t.ncell; i += blockDim.x)
       good = good && __double_as_longlong(c.vf[cb + i]) == __double_as_longlong(1.0);
+    const int nface = ND == 3 ? t.nb * t.nb : t.nb;
+    for (int f = 0; f < 2 * ND; f++) {
+      const int n = t.neighbor[b * 6 + f];
+      if (n != -1 && (n < 0 || t.child[n * 8] < 0)) continue;  // coarser, refined
+      const float *cf = c32.cf + ((long)b * (2 * ND) + f) * nface;
+      for (int i = threadIdx.x; i < nface; i += blockDim.x)
+        good = good && __float_as_uint(cf[i]) == __float_as_uint(cf[0]);
+    }
     if (!good) ok = 0;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1395,10 +1406,12 @@ void MacGpu::build_uniform() {
   const int nbk = tt_.num_blocks;
   if (nbk == 0) return;
   const int grid = std::min(nbk, 152 * 8);
+  Coef<float> c32 = c32_;
+  c32.cf = d_cf32_;
   if (tt_.ndim == 2)
-    k_uniform<2><<<grid, kTPB, 0, stream_>>>(topo_, c64_, c32_, d_uni64_, d_uni32_);
+    k_uniform<2><<<grid, kTPB, 0, stream_>>>(topo_, c64_, c32, d_uni64_, d_uni32_);
   else
-    k_uniform<3><<<grid, kTPB, 0, stream_>>>(topo_, c64_, c32_, d_uni64_, d_uni32_);
+    k_uniform<3><<<grid, kTPB, 0, stream_>>>(topo_, c64_, c32, d_uni64_, d_uni32_);
   k_iso<<<std::min((nbk + kTPB - 1) / kTPB, 152 * 8), kTPB, 0, stream_>>>(nbk, tt_.ndim, alpha_, d_uni64_, d_iso_);
   CK(cudaGetLastError());
 }

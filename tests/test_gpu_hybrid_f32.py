@@ -53,3 +53,47 @@ def test_same_bits_as_the_general_kernel(nd, nb, radius, kw):
     assert len(set(p.tables["level"][p.leaf])) > 1
     assert S.uniform_blocks() > 0
     _same(S, p.tables, nb)
+
+
+def _pairs(q, nd, g):
+    """(B, a) with a = 1 and a = 3/4 whose face coefficients (q B) a agree to the
+    last bit, while the FP32 diagonals of a cell with its third face at a coarser
+    neighbour do not"""
+    f = np.float32
+
+    def diagonal(b, a):
+        t = f((q * b) * a)
+        s = f(f(t + t) + f(f(f(f(q) / f(1.5)) * f(b)) * f(a)))
+        for _ in range(2 * nd - 3):
+            s = f(s + t)
+        return s
+    while True:
+        b1 = 1.0 + g.random()
+        for k in range(-3, 4):
+            b2 = b1 / 0.75 + k * np.spacing(b1 / 0.75)
+            if (q * b2) * 0.75 == q * b1 and diagonal(b1, 1.0) != diagonal(b2, 0.75):
+                return (b1, 1.0), (b2, 0.75)
+
+
+@pytest.mark.parametrize("nd, nb", [(2, 16), (3, 8), (3, 16)])
+def test_coefficient_of_varying_factors(nd, nb):
+    """B and the area fraction vary against each other and their product does
+    not: one coefficient on every face of a block, but two on those at a coarser
+    neighbour"""
+    p = _problem(nd, nb, 0.0)
+    tb = p.tables
+    g = np.random.default_rng(5)
+    fine = int(tb["level"].max())
+    for d in range(nd):
+        x = W.face_centres(tb, d)
+        dx = tb["block_len"].reshape(-1, 3)[:, 0] / nb
+        # beta ds / dx, a power of two as the spacings are (the factor's own bits do not matter)
+        h = dx[tb["level"] == fine][0]
+        (b1, a1), (b2, a2) = _pairs(h ** (nd - 1) / h, nd, g)
+        assert len(np.unique(dx)) == fine
+        step = np.round(2 * x / dx.reshape((-1,) + (1,) * (x.ndim - 1))).astype(np.int64)[..., :nd].sum(axis=-1) // 2
+        p.bface[d][...] = np.where(step % 2 == 0, b1, b2).reshape(p.bface[d].shape)
+        p.area[d][...] = np.where(step % 2 == 0, a1, a2).reshape(p.area[d].shape)
+    S = W.make_solver(p, use_mg_precond=1, bottom=1, precision=1)
+    assert S.uniform_blocks() > 0
+    _same(S, tb, 3)
