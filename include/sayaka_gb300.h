@@ -418,7 +418,9 @@ int sayaka_mac_residual_norm_noalloc(sayaka_mac *h, int32_t L, const double *x, 
  * applies to the FP32 V-cycle's output (in2 unused); which 7 = which 2 in FP32
  * (in, in2 rounded), variant + 1024: by the general kernel instead of the one
  * that the V-cycle takes, + 2048: after the prolongation of level L, which the
- * V-cycle's kernel does itself.  Failure tests, which
+ * V-cycle's kernel does itself; which 8 = which 3 by the operator by rows, which
+ * the iteration applies by default, on the blocks that a solve walks (0
+ * elsewhere).  Failure tests, which
  * leave out alone: which 4 = the one-launch smoothing of tower L with the
  * blocks of its second parity group left out and `variant` tries per wait, so
  * that waits run out (the call reports it); which 5 = the solver's error word

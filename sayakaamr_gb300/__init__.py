@@ -628,6 +628,15 @@ class MacSolver:
                "device_apply_f32", self.h)
         return y
 
+    def device_apply_rows(self, x):
+        """the iteration's operator by rows on x rounded to FP32, on the blocks
+        that a solve walks"""
+        y = self._cells()
+        a, pa = _f64(x)
+        _check(self.lib.sayaka_mac_device_kernel_compact(self.h, 8, 0, -1, pa, None, y.ctypes.data_as(_f64p)),
+               "device_apply_rows", self.h)
+        return y
+
     def device_smooth(self, L, phi, rhs, variant=-1):
         """one smoothing pass of tower L by the device solve's FP64 sweep"""
         out = self._cells()

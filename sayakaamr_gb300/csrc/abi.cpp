@@ -1024,7 +1024,7 @@ int sayaka_mac_device_kernel_compact(sayaka_mac *h, int32_t which, int32_t L, in
   return guarded(h, [&] {
     const int r = h->gpu->device_kernel_compact(which, L, variant, in, in2, out);
     if (r == 1) {
-      h->err = "device_kernel_compact: which must be 0..7, L a tower of the tree (which 1, 2, 7) or one that a launch "
+      h->err = "device_kernel_compact: which must be 0..8 (8: block sides a multiple of 4), L a tower of the tree (which 1, 2, 7) or one that a launch "
                "holds (which 4), a smoother variant (which 1), 1..1024 (which 2; times 4: which 7) or a number of tries (which 4), "
                "pointers non-null";
       return (int)SAYAKA_BAD_INPUT;

@@ -2029,6 +2029,27 @@ void MacGpu::iteration_device(T *resid, T *corr, const Coef<T> &c) {
   }
 }
 
+// the operator by rows on the blocks of the finest tower that the solve walks
+template <int M>
+void MacGpu::launch_op_rows(const float *x, double *y, const double *w) {
+  const bool mp = multi();
+  const BlockList TL =
+      mp ? BlockList{tlc_.blocks, tlc_.ftypes, tlc_.n, nullptr, nullptr, tlc_.hx} : tower_list(finest_);
+  // threads at work per CTA: 32 .. 256, enough for about two CTAs per SM
+  const long cells = (long)TL.n * ncell_, groups = std::max<long>(1, cells / 4), cap = red_grid(cells);
+  const int per = (int)std::min<long>(kTPB, std::max<long>(32, (groups / (152 * 2) + 31) / 32 * 32));
+  const int g = mp ? nchunks_ : (int)std::min<long>(std::max<long>(cap, 152 * 2), (groups + per - 1) / per);
+  auto rows = [&](auto kern) {
+    launch_k(prm_.pdl != 0, kern, g, kTPB, 0, stream_, topo_, cd64_, TL, chunks(), x, y, w, (const double *)d_opP_,
+             (const double *)d_opS_, mp ? d_stc_ : d_st_, mp ? d_cpart_ : d_part_, mp ? d_ccnt_ : d_cnt_,
+             (const double *)d_iso_, per);
+  };
+  if (tt_.ndim == 2)
+    mp ? rows(k_op_rows<2, M, true>) : rows(k_op_rows<2, M, false>);
+  else
+    mp ? rows(k_op_rows<3, M, true>) : rows(k_op_rows<3, M, false>);
+}
+
 // One BiCGSTAB iteration.  The V-cycle's output PH (the first
 // preconditioner application) is consumed by the operator and the x update
 // before the second application overwrites it (SH); out_p / out_s, when
@@ -2052,7 +2073,6 @@ void MacGpu::iteration_body(T *resid, T *corr, const Coef<T> &c, const TO *PH, c
   const bool pdl = prm_.pdl != 0;
   const double *OP = d_opP_, *OS = d_opS_;
   const float2 *OP2 = d_opP2_, *OS2 = d_opS2_, *U2 = d_uni2_;
-  const double *ISO = d_iso_;
   // params.vcycle_out 1: the operator of the FP32 V-cycle's output in double-float
   const bool dfop = prm_.vcycle_out == 1;
   auto op = [&](auto mode, const auto *x, double *y, const double *wv, double *y2) {
@@ -2078,17 +2098,7 @@ void MacGpu::iteration_body(T *resid, T *corr, const Coef<T> &c, const TO *PH, c
     };
     if constexpr (sizeof(TX) == 4 && M < 2) {
       if (!dfop && tt_.nb % 4 == 0) {
-        // threads at work per CTA: 32 .. 256, enough for about two CTAs per SM
-        const long groups = std::max<long>(1, w / 4), cap = red_grid(w);
-        const int per = (int)std::min<long>(kTPB, std::max<long>(32, (groups / (152 * 2) + 31) / 32 * 32));
-        const int g = mp ? nchunks_ : (int)std::min<long>(std::max<long>(cap, 152 * 2), (groups + per - 1) / per);
-        auto rows = [&](auto kern) {
-          launch_k(pdl, kern, g, kTPB, 0, stream_, topo_, cd64_, TL, ch, x, y, wv, OP, OS, ST, PART, CNT, ISO, per);
-        };
-        if (tt_.ndim == 2)
-          mp ? rows(k_op_rows<2, M, true>) : rows(k_op_rows<2, M, false>);
-        else
-          mp ? rows(k_op_rows<3, M, true>) : rows(k_op_rows<3, M, false>);
+        launch_op_rows<M>(x, y, wv);
         return;
       }
       if (dfop) {
@@ -2500,7 +2510,7 @@ int MacGpu::enqueue_kernel(int which, int L) {
 // solve's FP64 sweep, launch variant `variant` (-1: the tuned one); in = phi,
 // in2 = rhs.  Uses (and clobbers) the handle's work vectors.
 int MacGpu::device_kernel_compact(int which, int L, int variant, const double *in, const double *in2, double *out) {
-  if (which < 0 || which > 7 || !in || !out || ((which == 1 || which == 2 || which == 7) && !in2)) return 1;
+  if (which < 0 || which > 8 || !in || !out || ((which == 1 || which == 2 || which == 7) && !in2)) return 1;
   if ((which == 1 || which == 2 || which == 7) && (L < 1 || L > finest_ || towers_[L].all.n == 0)) return 1;
   if (which == 1 && variant >= kRbgsVariants) return 1;
   if (which == 2 && (variant < 1 || variant > 1024)) return 1;
@@ -2569,6 +2579,20 @@ int MacGpu::device_kernel_compact(int which, int L, int variant, const double *i
     CKR_(cudaMemcpyAsync(out, vec_[kV], n * sizeof(double), cudaMemcpyDeviceToHost, stream_), 2);
   } else if (which == 4) {
     // (above)
+  } else if (which == 8) {
+    // the operator by rows on the lists that a solve walks, in rounded to FP32
+    if (tt_.nb % 4 != 0) return 1;
+    CKR_(cudaMemcpyAsync(vec_[kTMP], in, n * sizeof(double), cudaMemcpyHostToDevice, stream_), 2);
+    k_narrow<<<ew_grid((long)n), kTPB, 0, stream_>>>((long long)n, vec_[kTMP], d_corr32_);
+    CKR_(cudaMemsetAsync(vec_[kV], 0, n * sizeof(double), stream_), 2);
+    CKR_(cudaMemsetAsync(vec_[kRHAT], 0, n * sizeof(double), stream_), 2);
+    CKR_(cudaMemsetAsync(d_st_, 0, sizeof(FState), stream_), 2);
+    if (multi()) CKR_(cudaMemsetAsync(d_stc_, 0, ncomp_ * sizeof(FState), stream_), 2);
+    solve_lists_ = true;
+    launch_op_rows<0>(d_corr32_, vec_[kV], vec_[kRHAT]);
+    solve_lists_ = false;
+    CKR_(cudaGetLastError(), 2);
+    CKR_(cudaMemcpyAsync(out, vec_[kV], n * sizeof(double), cudaMemcpyDeviceToHost, stream_), 2);
   } else if (which == 7) {
     // the FP32 pass, as the V-cycle runs it or by the general kernel (a list
     // without halo descriptors), from in or with level L prolonged first

@@ -288,6 +288,8 @@ class MacGpu {
   void vcycle_device(int L, T *resid, T *corr, const Coef<T> &c, double *out);
   template <typename T>
   void iteration_device(T *resid, T *corr, const Coef<T> &c);
+  template <int M>
+  void launch_op_rows(const float *x, double *y, const double *w);
   template <typename T, typename TO>
   void iteration_body(T *resid, T *corr, const Coef<T> &c, const TO *PH, const TO *SH, double *out_p, double *out_s);
   void capture_loop(int precision);
