@@ -781,9 +781,9 @@ __global__ void __launch_bounds__(kThreads) k_restrict(Topo t, Coef<T> c, BlockL
 // A factor vf = 1 is not multiplied or divided by (the same bits; in FP64 the
 // division alone is half of the kernel's FP64 work), and where a block's record
 // says that all its cells have vf = 1 it isn't read.  Bound by bytes on large
-// levels, by the chain block id -> child -> cells on small ones: 256 problems,
-// FP32, 15.6 us a launch with one cell per thread, 10.9 with two; 32 problems,
-// FP64, 12.7 and 11.6.
+// levels, where it is used (launch_restrict): 128 problems, FP32, 1.2 million
+// cells, 25.7 us a launch with one cell per thread, 18.3 with two; 32 problems,
+// FP64, 552 thousand cells, 27.7 and 23.4.
 template <typename T>
 struct alignas(16) Quad {
   T v[4];
@@ -2385,12 +2385,20 @@ void launch_smooth(const Topo &t, const Coef<T> &c, const BlockList &L, int colo
     launch_k(pdl, k_smooth<T, 3>, grid_for(work), kThreads, 0, s, t, c, L, color, phi, rhs, guard);
 }
 
+constexpr long kRestrictPairs = 1l << 17;
 template <typename T>
 void launch_restrict(const Topo &t, const Coef<T> &c, const BlockList &L, T *phi, const int *guard,
                      cudaStream_t s, bool pdl) {
   const long work = (long)L.n * t.ncell;
   if (work == 0) return;
-  if (t.nb % 4 == 0) {  // a child covers an even number of coarse cells: rows of four fine cells are aligned
+  // Two cells per thread from 131,072 cells of a level on (a side that is a
+  // multiple of four: rows of four fine cells are aligned).  The form reads a
+  // record before it knows whether it needs vf, one more load in the chain, and
+  // has half the threads to hide it: us a launch with one and with two cells, 2D
+  // FP32 30 thousand cells 3.4 and 3.7, 138 thousand 5.5 and 5.7, 364 thousand
+  // 7.9 and 6.4; FP64 30 thousand 5.1 and 7.3, 131 thousand 11.0 and 9.9; 3D FP64
+  // 33 thousand 6.2 and 8.4, 246 thousand 17.7 and 14.8.
+  if (t.nb % 4 == 0 && work >= kRestrictPairs) {
     const auto k = t.ndim == 2 ? k_restrict_pairs<T, 2> : k_restrict_pairs<T, 3>;
     launch_k(pdl, k, grid_for(work / 2), kThreads, 0, s, t, c, L, phi, guard);
     return;
