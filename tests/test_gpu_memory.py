@@ -68,11 +68,14 @@ def test_no_lists_without_solid_blocks():
     assert 0 <= used[1] - used[0] < 170 * p.num_blocks, used
 
 
-def test_bottom_inverse_without_a_second_copy_of_all_matrices():
-    p = W.forest([W.batch_problem(np.random.default_rng(k), "p%d" % k) for k in range(5)], "f")
+@pytest.mark.parametrize("n, level", [(5, 1), (8, 2), (9, 2)])
+def test_bottom_inverse_without_a_second_copy_of_all_matrices(n, level):
+    # (8 and 9 matrices of order 1024: two copies of all do not fit the L2, and
+    # two halves are inverted one after the other)
+    p = W.forest([W.batch_problem(np.random.default_rng(k), "p%d" % k) for k in range(n)], "f")
     out = []
     for deny in (True, False):
-        S = W.make_solver(p, **dict(PARAMS, tol_rel=1e-8, bottom_level=1))
+        S = W.make_solver(p, **dict(PARAMS, tol_rel=1e-8, bottom_level=level))
         S.deny_optional_memory(deny)
         S.set_params(prolong_form=0)  # the edge words are not what is compared
         info = S.cg_solve()
