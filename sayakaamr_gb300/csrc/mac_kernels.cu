@@ -1092,6 +1092,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_tile(Topo t, Coef<T> c,
     const int *hxe = L.hx ? L.hx + (long)p * kHX : nullptr;
     const int b = hxe ? hxe[kHXBlock] : L.blocks[p];
     if (block_off(L, b)) continue;  // uniform over the CTA
+    const long f0 = factor_entry(L, p) * ncell;
     const uint16_t ft = hxe ? (uint16_t)(hxe[kHXInfo] & 0xffff) : L.ftypes[p];
     const long cb = (long)b * ncell;
     const long fb = (long)b * t.nfb;
@@ -1178,7 +1179,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_rbgs_tile(Topo t, Coef<T> c,
           o.sa = u[6];
           o.ia = u[7];
         } else {
-          const long fo = factor_entry(L, p) * ncell + o.ci;
+          const long fo = f0 + o.ci;
           o.sa = L.sa[fo];
           o.ia = L.ia[fo];
         }
@@ -1263,6 +1264,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bhgs(Topo t, Coef<T> c, Bloc
     const int *hxe = L.hx ? L.hx + (long)p * kHX : nullptr;
     const int b = hxe ? hxe[kHXBlock] : L.blocks[p];
     if (block_off(L, b)) continue;  // uniform over the CTA
+    const long f0 = factor_entry(L, p) * ncell;
     const uint16_t ft = hxe ? (uint16_t)(hxe[kHXInfo] & 0xffff) : L.ftypes[p];
     const long cb = (long)b * ncell;
     const long fb = (long)b * t.nfb;
@@ -1345,7 +1347,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bhgs(Topo t, Coef<T> c, Bloc
             bool inner = true;
 #pragma unroll
             for (int q = 0; q < ND; q++) inner = inner && ijk[q] > 0 && ijk[q] < nb - 1;
-            const long fo = factor_entry(L, p) * ncell + ci;
+            const long fo = f0 + ci;
             const bool ui = u && inner;
             const T iav = ui ? u[7] : (T)L.ia[fo];  // 0 in a solid cell
             unew = fma_t(rhs[cb + ci], ui ? u[6] : (T)L.sa[fo], off * iav);
@@ -2073,6 +2075,7 @@ __global__ void __launch_bounds__(kThreads, FAC ? 6 : 4) k_prolong_red(Topo t, C
     const int *hxe = L.hx ? L.hx + (long)pl * kHX : nullptr;
     const int b = hxe ? hxe[kHXBlock] : L.blocks[pl];
     if (block_off(L, b)) continue;  // uniform over the CTA
+    const long f0 = factor_entry(L, pl) * ncell;
     const uint16_t ft = hxe ? (uint16_t)(hxe[kHXInfo] & 0xffff) : L.ftypes[pl];
     const long cb = (long)b * ncell;
     const long fb = (long)b * t.nfb;
@@ -2157,7 +2160,7 @@ __global__ void __launch_bounds__(kThreads, FAC ? 6 : 4) k_prolong_red(Topo t, C
         bool inner = true;
 #pragma unroll
         for (int q = 0; q < ND; q++) inner = inner && ijk[q] > 0 && ijk[q] < nb - 1;
-        const long fo = factor_entry(L, pl) * ncell + ci;
+        const long fo = f0 + ci;
         const bool ui = u && inner;
         const T iav = ui ? u[7] : (T)L.ia[fo];  // 0 in a solid cell
         unew = fma_t(rhs[cb + ci], ui ? u[6] : (T)L.sa[fo], off * iav);
