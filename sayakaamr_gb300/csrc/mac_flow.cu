@@ -59,11 +59,13 @@ struct Wait {
   int *err, limit;
 };
 __device__ __forceinline__ bool given_up(const Topo &t) { return *(volatile const int *)t.err != 0; }
-// (unrolled by hand as the compiler does with a constant limit: rolled, a solve of
-// 16 thousand cells took 1,154 us instead of 1,002)
+// (unrolled, as the compiler does with a constant limit.  us of a solve of 16
+// thousand cells and of one of 1.9 million, with a constant limit and here on the
+// same inputs: rolled 1,002 and 1,154, 5,704 and 5,877; by four 1,109 and 1,083,
+// 5,832 and 5,879; by eight 1,108 and 1,062, 5,964 and 5,983)
 __device__ __forceinline__ float poll1(const Word *p, unsigned tag, Wait wt, bool &dead) {
   Word w = 0;
-#pragma unroll 4
+#pragma unroll 8
   for (int n = 0; n < wt.limit; n++) {
     w = look(p);
     if (tagged(w, tag) || dead) return value(w);
