@@ -1738,7 +1738,7 @@ void MacGpu::build_bottom() {
     int per = nmat;
     // (halves where both copies of a half fit the L2, 129 MB, and both of the
     // group do not: 8 matrices of order 1024 take 38 ms together and 34 as halves)
-    const long long copy = nmat * mm * 8, l2 = 104ll << 20;
+    const long long copy = nmat * mm * 8, l2 = 100ll << 20;
     if (nmat > 1 && copy <= l2 && 2 * copy > l2) per = (nmat + 1) / 2;
     while (per > 1 && !optional_malloc(&mem, (size_t)per * mm * sizeof(double))) per = (per + 1) / 2;
     if (!mem) CK_(dev_malloc(&mem, (size_t)mm * sizeof(double)));
