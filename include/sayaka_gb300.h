@@ -118,7 +118,8 @@ typedef struct sayaka_params {
   int32_t smooth_variant; /* device smoother launch bounds (register cap): -1 = autotuned at prepare by
                              timing every variant on the finest level (default), 0..13 = fixed: 10 two
                              cells per thread; 11..13, FP32, one warp per 16x16 block (register caps 64, 48,
-                             80) or one thread per row of an 8^3 block, elsewhere as 3.  The same values */
+                             80) or one thread per row of an 8^3 block, elsewhere as 3.  The same values.
+                             A tower that is smoothed in one launch (prolong_form 1) takes no variant */
   int32_t learned;        /* device path with the FP32 V-cycle: 1 = add the trained learned block
                              correction after every V-cycle (default 0); see sayaka_mac_learned_* */
   int32_t bottom_level;   /* device path: level of the dense bottom solve; 0 = auto (the finest level below the
@@ -143,7 +144,9 @@ typedef struct sayaka_params {
   int32_t uniform;        /* device path: 1 = blocks whose face coefficients are constant per direction and
                              whose cells are all fluid (vf = 1) read the coefficients from a per-block record
                              instead of the face arrays and vf (same arithmetic, same results; default);
-                             0 = every block reads the arrays */
+                             0 = the smoothers, the transfers and the general operator read the arrays in
+                             every block (the operator by rows, which an FP32 solve applies by default, and the
+                             operator's factors take a block's single coefficient from its record either way) */
   int32_t bottom_refresh; /* device path: 1 = the dense bottom inverse is rebuilt after every coefficient change
                              (default); 0 = the inverse of the last build is kept while only coefficients change
                              (a fixed coarsest-level solve of the preconditioner, slightly stale; the outer

@@ -152,10 +152,11 @@ __device__ __forceinline__ long factor_entry(const BlockList &L, int p) { return
 // chunks of a block list listed problem by problem (one BiCGSTAB state per
 // problem): the BiCGSTAB kernels run one CTA per chunk of at most
 // chunk_cells(total) cells of one problem.  4096 cells, 16 per thread, spread
-// the FP64 epilogue of a chunk's reduction thin (29M cells: 58.8 ms a solve,
-// 59.5 with 2048 or 8192); a smaller forest takes smaller chunks, so that its
-// launches still fill the 608 resident CTAs about twice over and a thread
-// waits for one round of loads instead of four.
+// the FP64 epilogue of a chunk's reduction thin (29 M cells: 35.8 ms a solve, 36.7
+// with 2048, 36.1 with 8192); a smaller forest takes smaller chunks, so that its
+// launches still fill the 608 resident CTAs about twice over and a thread waits
+// for one round of loads instead of four (7.7 M cells: 12.7 ms with 2048, 12.9 with
+// 4096, 13.1 with 1024; 1.9 M: 4.84 with 1024, 4.99 with 2048, 5.45 with 4096).
 inline long chunk_cells(long total) { return total >= (1l << 24) ? 4096 : total >= (1l << 22) ? 2048 : 1024; }
 struct Chunks {
   const int *comp;       // per chunk: its problem

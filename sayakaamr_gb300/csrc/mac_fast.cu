@@ -2003,14 +2003,16 @@ void MacGpu::precondition(int L, T *resid, T *corr, const Coef<T> &c, double *ou
 // FP32 V-cycle output read in place by the BiCGSTAB kernels, widened exactly
 // on the integer pipe where they read it, or widened once into FP64 phat /
 // shat.  params.vcycle_out 0 (auto): in place in 2D and on 3D towers of at
-// most 2M cells, where it saves two launches per iteration (batch workload,
-// 2D, 29M cells: 58.8 in place vs 60.4 ms widened), and on larger 3D towers
+// most 2M cells, where it saves two launches per iteration and the operator forms
+// its differences on the FP32 pipe (256 problems, 2D, 29 M cells: 35.8 ms in place,
+// 41.9 widened, 44.5 with the double-float operator), and on larger 3D towers
 // of which at least half the blocks have one face coefficient and whose blocks'
 // side is a multiple of four, whose operator is formed on the FP32 pipe from the
-// FP32 values (k_op_rows).  Other large 3D
-// towers widen, since the general 3D operator reads seven cells and their
-// integer widenings cost more than the launches (15.9M cells: 31.6 in place
-// vs 27.3 ms).  1 = in place with the operator in double-float, 2 = always
+// FP32 values (k_op_rows; 15.9 M cells of 16^3 blocks: 16.2 in place, 20.0
+// widened).  Other large 3D towers widen, since the general 3D operator reads seven
+// cells and widens each on the integer pipe: no difference on 3.9 M cells of 10^3
+// blocks (10.9 ms).  (16^3 blocks of variable B, which this rule widens too, take
+// 22.7 ms widened and 20.0 in place: the rows form gains there as well.)  1 = in place with the operator in double-float, 2 = always
 // widened, 3 = always in place.
 constexpr long kDirectF32Cells = 1l << 21;
 bool MacGpu::vcycle_in_place() const {

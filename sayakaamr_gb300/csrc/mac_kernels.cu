@@ -881,8 +881,8 @@ __global__ void __launch_bounds__(kThreads) k_face_coef(Topo t, const double *ge
                             const T *a1, const T *a2, double beta, T *t0, T *t1, T *t2) {
   // One warp per block and direction divides once for all its faces (a
   // division is about 20 operations of the FP64 pipe, whatever the number of
-  // lanes that need it), and a product with 1 or 0 is not formed: B and the
-  // area fraction are 1 or 0 on most faces.  13.75 M cells: 1050 us with a
+  // lanes that need it), and a product with 1 is not formed: B and the area
+  // fraction are 1 on most faces.  13.75 M cells: 1050 us with a
   // division per face, 587 with one per thread of a CTA, 262 now.
   const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
   for (long it = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; it < (long)t.nblocks * t.ndim; it += warps) {
@@ -1427,9 +1427,9 @@ __device__ __forceinline__ void h3_stage(const float *__restrict__ src, float4 (
 // block, coefficients T[]; else from the face arrays).  The diagonal is not
 // kept per cell: in a constant-coefficient block every cell of a row but its
 // two ends has the same (a boundary face's part is one value per face there,
-// coarse/fine faces included), elsewhere it is summed along with the
-// off-diagonal from the same loads.  With 16 registers less, three CTAs of a
-// 16^3 block fit an SM instead of two.
+// coarse/fine faces included: k_uniform), elsewhere it is summed along with the
+// off-diagonal from the same loads.  Two CTAs of a 16^3 block fit an SM: 28.9 KB
+// of H3 and 68.6 KB of H3Var each, reserved for blocks with a record too.
 template <int NB, bool U>
 __device__ __forceinline__ void h3_sweeps(const Topo &t, const Coef<float> &c, int b, const float *u, float dv,
                                           int nsweep, const float4 (&r4)[NB / 4], H3<NB> &sh,

@@ -63,7 +63,8 @@ struct SolverParams {
                               // change; 0 = kept from the last build until the tree or the bottom level changes
                               // (a fixed, slightly stale coarsest-level solve inside the preconditioner)
   int uniform = 1;            // device path: constant-coefficient blocks read their face coefficients from a
-                              // per-block record (same results; 0 = every block reads the face arrays)
+                              // per-block record (same results; 0 = the face arrays, but in the operator by rows
+                              // and the operator's factors)
   int per_problem = 1;        // device path, a tree of several independent problems (connected components):
                               // 1 = one BiCGSTAB state per problem, each stopping at its own tolerance;
                               // 0 = one state shared by all
