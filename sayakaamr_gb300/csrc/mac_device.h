@@ -218,9 +218,8 @@ void launch_smooth(const Topo &t, const Coef<T> &c, const BlockList &L, int colo
 // the device solve's smoother (smooth_cell_fast); `variant` picks the
 // launch bounds (0..kRbgsVariants-1), chosen per workload by the autotuner
 constexpr int kRbgsVariants = 14;
-// error word of the bulk-copy smoother variant (an mbarrier wait timed out);
-// read (and cleared) by the host after a solve
-// the solver's error word (Topo::err) after its stream is idle; clear: reset it
+// the solver's error word (Topo::err: a bounded wait of the bulk-copy sweeps or of
+// the one-launch towers ran out) after its stream is idle; clear: reset it
 int rbgs_bulk_error(int *err, cudaStream_t s, bool clear);
 template <typename T>
 void launch_rbgs(const Topo &t, const Coef<T> &c, const BlockList &L, int color, T *phi,
